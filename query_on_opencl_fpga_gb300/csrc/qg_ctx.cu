@@ -36,6 +36,13 @@ QG_API qg_status qg_ctx_create(qg_ctx **out, void *stream) {
         e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, ctx->device);
     if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->ctl, sizeof(qg_control));
     if (e == cudaSuccess) e = cudaMemset(ctx->ctl, 0, sizeof(qg_control));
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&ctx->hres, sizeof(qg_hostres));
+    if (e == cudaSuccess) {
+        memset((void *)ctx->hres, 0, sizeof(qg_hostres));
+        // pinned memory has one address for host and device
+        const unsigned long long at = (unsigned long long)(uintptr_t)&ctx->hres->err;
+        e = cudaMemcpy(&ctx->ctl->herr, &at, sizeof(at), cudaMemcpyHostToDevice);
+    }
     if (e == cudaSuccess) e = cudaMallocHost((void **)&ctx->pinned, 8 * sizeof(long long));
     if (e == cudaSuccess) e = cudaMallocHost((void **)&ctx->pin_ctl, sizeof(qg_control));
     if (e == cudaSuccess) e = cudaMallocHost((void **)&ctx->pin_bases, 8 * 1024 * sizeof(uint32_t));
@@ -43,6 +50,7 @@ QG_API qg_status qg_ctx_create(qg_ctx **out, void *stream) {
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         if (ctx->ctl) cudaFree(ctx->ctl);
+        if (ctx->hres) cudaFreeHost((void *)ctx->hres);
         if (ctx->pinned) cudaFreeHost(ctx->pinned);
         if (ctx->pin_ctl) cudaFreeHost(ctx->pin_ctl);
         if (ctx->pin_bases) cudaFreeHost(ctx->pin_bases);
@@ -69,6 +77,7 @@ QG_API qg_status qg_ctx_destroy(qg_ctx *ctx) {
     if (ctx->table) cudaFree(ctx->table);
     if (ctx->aux) cudaFree(ctx->aux);
     if (ctx->ctl) cudaFree(ctx->ctl);
+    if (ctx->hres) cudaFreeHost((void *)ctx->hres);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->pin_ctl) cudaFreeHost(ctx->pin_ctl);
     if (ctx->pin_bases) cudaFreeHost(ctx->pin_bases);
@@ -334,6 +343,7 @@ static qg_status map_error(qg_ctx *ctx, const int32_t *h) {
     if (h[0] == 0) return QG_OK;
     // A kernel that gave up may have left the single-pass counters or the
     // group-by table mid-way: reset them (in stream order).
+    ctx->hres->err = 0;
     cudaMemsetAsync(&ctx->ctl->err, 0, 2 * sizeof(int32_t), ctx->stream);
     cudaMemsetAsync(&ctx->ctl->tile_ctr, 0, 2 * sizeof(uint32_t), ctx->stream);
     cudaMemsetAsync(ctx->ctl->gbd, 0, sizeof(ctx->ctl->gbd), ctx->stream);  // dense group-by state words
@@ -345,6 +355,8 @@ static qg_status map_error(qg_ctx *ctx, const int32_t *h) {
 }
 
 qg_status qg_collect_error(qg_ctx *ctx) {
+    QG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
+    if (ctx->hres->err == 0) return QG_OK;
     int32_t *h = reinterpret_cast<int32_t *>(ctx->pinned + 7);
     QG_TRY_CUDA(ctx, cudaMemcpyAsync(h, &ctx->ctl->err, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream),
                 "read error word");
@@ -352,26 +364,16 @@ qg_status qg_collect_error(qg_ctx *ctx) {
     return map_error(ctx, h);
 }
 
+qg_status qg_host_count(qg_ctx *ctx, long long *h) {
+    QG_TRY(qg_collect_error(ctx));
+    *h = ctx->hres->count;
+    return QG_OK;
+}
+
 qg_status qg_read_count(qg_ctx *ctx, const long long *d, long long *h) {
-    const uintptr_t base = (uintptr_t)ctx->ctl, at = (uintptr_t)d;
-    const size_t off = (size_t)(at - base);
-    if (at >= base && off + sizeof(long long) <= offsetof(qg_control, gbd)) {
-        // A count kept in the control block comes back with the error word
-        // in one copy.
-        QG_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->pin_ctl, ctx->ctl, off + sizeof(long long), cudaMemcpyDeviceToHost,
-                                         ctx->stream),
-                    "cudaMemcpyAsync count");
-        QG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
-        memcpy(h, (const char *)ctx->pin_ctl + off, sizeof(long long));
-        const int32_t e[2] = {ctx->pin_ctl->err, ctx->pin_ctl->err_site};
-        return map_error(ctx, e);
-    }
-    int32_t *e = reinterpret_cast<int32_t *>(ctx->pinned + 7);
     QG_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, d, sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream),
                 "cudaMemcpyAsync count");
-    QG_TRY_CUDA(ctx, cudaMemcpyAsync(e, &ctx->ctl->err, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream),
-                "read error word");
-    QG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
+    QG_TRY(qg_collect_error(ctx));
     *h = ctx->pinned[0];
-    return map_error(ctx, e);
+    return QG_OK;
 }

@@ -316,9 +316,9 @@ k_filter_cols_tma(const int32_t *__restrict__ key, const int32_t *__restrict__ p
 
 }  // namespace
 
-static qg_status finish_count(qg_ctx *ctx, long long *d_count, int64_t cap, int64_t *out_n) {
+static qg_status finish_count(qg_ctx *ctx, int64_t cap, int64_t *out_n) {
     long long h = 0;
-    QG_TRY(qg_read_count(ctx, d_count, &h));
+    QG_TRY(qg_host_count(ctx, &h));
     *out_n = h;
     if (h > cap) return QG_ERR_CAPACITY;
     return QG_OK;
@@ -483,12 +483,18 @@ k_filter_write(const uint16_t *__restrict__ mask, const int32_t *__restrict__ pa
     }
 }
 
+// The count of an empty input: the host word directly, a device word in stream order.
+static qg_status qg_zero_count(qg_ctx *ctx, long long *d_count) {
+    if (d_count == (long long *)&ctx->hres->count) ctx->hres->count = 0;
+    else QG_TRY_CUDA(ctx, cudaMemsetAsync(d_count, 0, sizeof(long long), ctx->stream), "memset");
+    return QG_OK;
+}
+
 qg_status qg_filter_rec_launch(qg_ctx *ctx, const void *in, int64_t n, int32_t lo, int32_t hi,
                                void *out, int64_t cap, long long *d_count) {
     constexpr int TILE = FT_THREADS * REC_ROUNDS * 2;
     if (n == 0) {
-        QG_TRY_CUDA(ctx, cudaMemsetAsync(d_count, 0, sizeof(long long), ctx->stream), "memset");
-        return QG_OK;
+        return qg_zero_count(ctx, d_count);
     }
     if (((uintptr_t)in & 15) != 0 || ((uintptr_t)out & 7) != 0) return QG_ERR_INVALID;
     int64_t tiles = qg_ceil_div(n, TILE);
@@ -508,8 +514,7 @@ qg_status qg_filter_cols_launch(qg_ctx *ctx, const int32_t *key, const int32_t *
                                 long long *d_count) {
     constexpr int TILE = FT_THREADS * COL_ROUNDS * 4;
     if (n == 0) {
-        QG_TRY_CUDA(ctx, cudaMemsetAsync(d_count, 0, sizeof(long long), ctx->stream), "memset");
-        return QG_OK;
+        return qg_zero_count(ctx, d_count);
     }
     if (((uintptr_t)key & 15) || ((uintptr_t)pay & 15) || ((uintptr_t)out & 7))
         return QG_ERR_INVALID;
@@ -580,9 +585,9 @@ QG_API qg_status qg_filter_range_rec_async(qg_ctx *ctx, const void *in, int64_t 
 QG_API qg_status qg_filter_range_rec(qg_ctx *ctx, const void *in, int64_t n, int32_t lo,
                                      int32_t hi, void *out, int64_t cap, int64_t *out_n) {
     if (!ctx || !out_n) return QG_ERR_INVALID;
-    long long *d_count = (long long *)&ctx->ctl->counter[0];
+    long long *d_count = (long long *)&ctx->hres->count;  // the kernel stores the count in host memory
     QG_TRY(qg_filter_range_rec_async(ctx, in, n, lo, hi, out, cap, (int64_t *)d_count));
-    return finish_count(ctx, d_count, cap, out_n);
+    return finish_count(ctx, cap, out_n);
 }
 
 QG_API qg_status qg_filter_cols_async(qg_ctx *ctx, const int32_t *key, const int32_t *pay,
@@ -601,9 +606,9 @@ QG_API qg_status qg_filter_cols(qg_ctx *ctx, const int32_t *key, const int32_t *
     // selectivity estimate is the predicate's share of the int32 range.
     qg_steer_call sc;
     qg_steer_begin(ctx, QG_STEER_FILTER, n, 0, ((double)hi - (double)lo + 1.0) / 4294967296.0, &sc);
-    long long *d_count = (long long *)&ctx->ctl->counter[0];
+    long long *d_count = (long long *)&ctx->hres->count;  // the kernel stores the count in host memory
     qg_status st = qg_filter_cols_async(ctx, key, pay, n, lo, hi, out, cap, (int64_t *)d_count);
-    if (st == QG_OK) st = finish_count(ctx, d_count, cap, out_n);
+    if (st == QG_OK) st = finish_count(ctx, cap, out_n);
     qg_steer_end(ctx, &sc, st);
     return st;
 }

@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(GBD_THREADS)
 k_gbd_emit(unsigned long long *__restrict__ dense, long long *__restrict__ extra,
            unsigned long long *__restrict__ img, uint32_t *__restrict__ sketch, const uint32_t *__restrict__ st,
            uint32_t shift, int32_t *__restrict__ gkey, long long *__restrict__ gsum, long long *__restrict__ gcnt,
-           long long cap, long long *__restrict__ d_num, qg_lookback lb) {
+           long long cap, long long *__restrict__ d_num, volatile uint32_t *outside, qg_lookback lb) {
     __shared__ uint32_t s_tile, s_epoch, s_tot, s_wsum[GBD_ENW], s_off[GBD_EPER * GBD_ENW], s_tmp[2 * 8];
     gbd_clear_sample(img, sketch, blockIdx.x, gridDim.x);
     qg_lb_begin_dyn(lb, &s_tile, &s_epoch);  // chunk ids in CTA start order: predecessors are running
@@ -504,7 +504,10 @@ k_gbd_emit(unsigned long long *__restrict__ dense, long long *__restrict__ extra
         const uint32_t excl = qg_lb_wide_exclusive<8>(lb, chunk, epoch, total, s_tmp);
         if (threadIdx.x == 0) {
             s_wsum[0] = excl;
-            if (chunk == C - 1) *d_num = (long long)excl + total;
+            if (chunk == C - 1) {
+                *d_num = (long long)excl + total;
+                if (outside) *outside = st[G_OUTSIDE];
+            }
         }
     }
     __syncthreads();
@@ -568,8 +571,8 @@ k_gbd_single(const int32_t *__restrict__ key, const int32_t *__restrict__ val, c
              int32_t lo2, int32_t hi2, long long n, int runs, bool every_row, uint32_t *sketch,
              unsigned long long *img, uint32_t *st, unsigned long long *dense, long long *extra, uint32_t shift,
              uint32_t fast_max, int32_t *__restrict__ gkey, long long *__restrict__ gsum,
-             long long *__restrict__ gcnt, long long cap, long long *d_num, uint32_t *counts, qg_control *ctl,
-             uint32_t spin_limit) {
+             long long *__restrict__ gcnt, long long cap, long long *d_num, volatile uint32_t *outside,
+             uint32_t *counts, qg_control *ctl, uint32_t spin_limit) {
     extern __shared__ __align__(16) unsigned char gbd_main_raw[];
     __shared__ uint32_t s_red[4], s_wsum[GBD_ENW], s_off[GBD_EPER * GBD_ENW];
     __shared__ volatile uint32_t s_ok;
@@ -696,7 +699,10 @@ k_gbd_single(const int32_t *__restrict__ key, const int32_t *__restrict__ val, c
         }
         if (lane == 0) {
             s_base = before;
-            if (b == 0) *d_num = (long long)all;
+            if (b == 0) {
+                *d_num = (long long)all;
+                if (outside) *outside = __ldcg(&st[G_OUTSIDE]);
+            }
         }
     }
     __syncthreads();
@@ -715,7 +721,7 @@ extern "C" QG_API qg_status qg_groupby_set_single_launch(int enable) {
 
 qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, const int32_t *val2, int32_t lo2,
                         int32_t hi2, int64_t n, int32_t *gkey, int64_t *gsum, int64_t *gcnt, int64_t cap,
-                        long long *d_num) {
+                        long long *d_num, volatile uint32_t *outside) {
     // table arena (kept all-zero between calls):
     //   dense [W] u64 | extra [W] i64 | sample sketch [2][2^19] u32 | slot image [GBD_S] u64
     const size_t dense_b = (size_t)GBD_W * 8, sk_b = ((size_t)2 << GBD_TLOG2) * 4, img_b = (size_t)GBD_S * 8;
@@ -786,7 +792,7 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
             qg_control *ctl = ctx->ctl;
             long long *gs = (long long *)gsum, *gc = (long long *)gcnt;
             void *args[] = {&k0, &v0, &w0, &l2, &h2, &nn, &rn, &er, &sketch, &img, &st, &dense, &extra, &sh,
-                            &fm32, &gkey, &gs, &gc, &cp, &d_num, &counts, &ctl, &spin};
+                            &fm32, &gkey, &gs, &gc, &cp, &d_num, &outside, &counts, &ctl, &spin};
             qg_pre_launch(ctx);
             const cudaError_t e = cudaLaunchCooperativeKernel((const void *)singlef, dim3(C), dim3(GBD_THREADS), args,
                                                               smem_main, ctx->stream);
@@ -818,7 +824,7 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
     if (s == QG_OK) {
         qg_pre_launch(ctx);
         k_gbd_emit<<<C, GBD_THREADS, 0, ctx->stream>>>(dense, extra, img, sketch, st, shift, gkey, (long long *)gsum,
-                                                       (long long *)gcnt, cap, d_num, lb);
+                                                       (long long *)gcnt, cap, d_num, outside, lb);
         s = qg_check_launch(ctx, "k_gbd_emit");
     }
     if (s != QG_OK) ctx->table_dirty = true;  // the dense table may hold partial sums

@@ -1045,13 +1045,13 @@ extern "C" QG_API qg_status qg_groupby_rec(qg_ctx *ctx, const void *in, int64_t 
         qg_lookback lb;
         s = qg_lb_make(ctx, tiles, QG_SITE_GROUPBY, &lb);
         if (s == QG_OK) {
-            long long *d_count = (long long *)&ctx->ctl->counter[0];
+            long long *d_count = (long long *)&ctx->hres->count;
             qg_pre_launch(ctx);
             k_group_bounds<<<(unsigned)tiles, GBD_THREADS, 0, ctx->stream>>>(
                 (const uint4 *)sorted_out, n, startPos, cap_groups, d_count, lb);
             s = qg_check_launch(ctx, "k_group_bounds");
             long long h = 0;
-            if (s == QG_OK) s = qg_read_count(ctx, d_count, &h);
+            if (s == QG_OK) s = qg_host_count(ctx, &h);
             if (s == QG_OK) {
                 *num_groups = h;
                 if (h > cap_groups) s = QG_ERR_CAPACITY;
@@ -1405,7 +1405,7 @@ qg_status qg_groupby_dense_async(qg_ctx *ctx, const int32_t *key, const int32_t 
     if ((((uintptr_t)key) | ((uintptr_t)val) | ((uintptr_t)val2)) & 15) return QG_ERR_INVALID;
     if (n == 0 || n >= (1LL << 32))
         return qg_groupby_cols_async(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, QG_ORDER_NONE, d_num);
-    QG_TRY(qg_gbd_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, (long long *)d_num));
+    QG_TRY(qg_gbd_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, (long long *)d_num, nullptr));
     qg_pre_launch(ctx);
     k_gbd_outside_error<<<1, 1, 0, ctx->stream>>>(ctx->ctl);
     return qg_check_launch(ctx, "k_gbd_outside_error");
@@ -1419,7 +1419,7 @@ qg_status qg_groupby_dense_probe(qg_ctx *ctx, const int32_t *key, const int32_t 
     *ok = false;
     if (!ctx || n <= 0 || n >= (1LL << 32) || !key || !val || !d_num) return QG_OK;
     if ((((uintptr_t)key) | ((uintptr_t)val) | ((uintptr_t)val2)) & 15) return QG_OK;
-    QG_TRY(qg_gbd_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, (long long *)d_num));
+    QG_TRY(qg_gbd_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, (long long *)d_num, nullptr));
     QG_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->pin_ctl, ctx->ctl, offsetof(qg_control, ghist), cudaMemcpyDeviceToHost,
                                      ctx->stream),
                 "ctl d2h");
@@ -1474,17 +1474,12 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
     // read the count.
     if (gm == 0 && !global && n > 0) {
         // Dense-window path: output in key order whatever `order` asks for;
-        // one read of the control block brings the error word, the group
-        // count and whether every row fell inside the window.
-        QG_TRY(qg_gbd_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, d_num));
-        QG_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->pin_ctl, ctx->ctl, offsetof(qg_control, ghist),
-                                         cudaMemcpyDeviceToHost, ctx->stream),
-                    "ctl d2h");
-        QG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-        if (ctx->pin_ctl->err != 0) return qg_collect_error(ctx);
-        const uint32_t outside = ctx->pin_ctl->gbd[QG_GBD_OUTSIDE];
-        if (outside == 0) {
-            g = (long long)ctx->pin_ctl->counter[1];
+        // its last kernel stores the group count and the rows outside the
+        // window in host memory.
+        QG_TRY(qg_gbd_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap,
+                             (long long *)&ctx->hres->count, &ctx->hres->aux));
+        QG_TRY(qg_host_count(ctx, &g));
+        if (ctx->hres->aux == 0) {
             ctx->gb_stats[0] = 2u;
             ctx->gb_stats[1] = ctx->gb_stats[2] = ctx->gb_stats[3] = 0;
             *num_groups = g;

@@ -23,6 +23,20 @@ struct qg_control {
     // (inputs below 2^31 rows make at most 2048 groups).  The last tile of a
     // group wraps its counter back to zero, so no launch has to clear them.
     uint32_t fgroup[2048];
+    // Address of the context's host error word (0: none), written with the
+    // first error only: a call that met no error reads it after its
+    // synchronisation instead of copying this block back.
+    unsigned long long herr;
+};
+
+// Host pinned words that kernels write directly (one set per context).  A
+// result the last kernel stores here is in host memory once the stream is
+// synchronised: a 4K-row filter call spent 9 of its 37 us on the copy-engine
+// read of its count that this replaces.
+struct qg_hostres {
+    volatile uint32_t err;         // first error code (qg_record_error), 0 = none
+    volatile uint32_t aux;         // an operator's second result word
+    volatile long long count;      // an operator's row or group count
 };
 
 #define QG_MAX_TIMED 4096
@@ -39,6 +53,7 @@ struct qg_ctx {
     unsigned long long *lbstat;  // look-back status words, used by nothing else
     size_t lbstat_words;
     qg_control *ctl;        // device
+    qg_hostres *hres;       // host pinned result words, written by kernels
     long long *pinned;      // host pinned readback slots (8)
     qg_control *pin_ctl;    // host pinned copy of the control block (one read brings error, counters, ghist)
     uint32_t *pin_bases;    // ring of 8 host pinned 4 KB slots for radix digit bases
@@ -83,10 +98,11 @@ qg_status qg_cuda_fail(qg_ctx *ctx, cudaError_t e, const char *what);
 // Dense-window column group-by (qg_gbdense.cu): launches the whole path on the
 // context's stream, output in ascending unsigned key order; the caller reads
 // ctl->gbd[QG_GBD_OUTSIDE] (non-zero: the path did not apply, nothing valid
-// was written) and the group count (*d_num) after its one synchronisation.
+// was written; also stored to *outside when set) and the group count
+// (*d_num) after its one synchronisation.
 qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, const int32_t *val2,
                         int32_t lo2, int32_t hi2, int64_t n, int32_t *gkey, int64_t *gsum, int64_t *gcnt,
-                        int64_t cap, long long *d_num);
+                        int64_t cap, long long *d_num, volatile uint32_t *outside);
 enum { QG_GBD_OUTSIDE = 6 };
 qg_status qg_groupby_dense_async(qg_ctx *ctx, const int32_t *key, const int32_t *val, const int32_t *val2,
                                  int32_t lo2, int32_t hi2, int64_t n, int32_t *gkey, int64_t *gsum, int64_t *gcnt,
@@ -137,6 +153,9 @@ qg_status qg_read_i64(qg_ctx *ctx, const long long *d, long long *h);
 qg_status qg_check_launch(qg_ctx *ctx, const char *what);
 // Read the device error word (after the stream's work), clear it and map it.
 qg_status qg_collect_error(qg_ctx *ctx);
+// Synchronise; the count a kernel stored in ctx->hres->count goes to *h, a
+// device error (if any) is the status.
+qg_status qg_host_count(qg_ctx *ctx, long long *h);
 // qg_read_i64 and qg_collect_error with one synchronisation: the count in *h,
 // the device error (if any) as the status.
 qg_status qg_read_count(qg_ctx *ctx, const long long *d, long long *h);
@@ -161,7 +180,10 @@ static inline int64_t qg_ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b
 #define QG_FULL_MASK 0xffffffffu
 
 __device__ __forceinline__ void qg_record_error(qg_control *ctl, int code, int site) {
-    if (atomicCAS(&ctl->err, 0, code) == 0) ctl->err_site = site;
+    if (atomicCAS(&ctl->err, 0, code) == 0) {
+        ctl->err_site = site;
+        if (ctl->herr) *reinterpret_cast<volatile uint32_t *>(ctl->herr) = (uint32_t)code;
+    }
 }
 
 __device__ __forceinline__ unsigned long long qg_ld_relaxed_u64(const unsigned long long *p) {

@@ -45,6 +45,7 @@
 //      bucket sends the call to the general path (R's records made then, the
 //      S' partitioning reused).
 #include <algorithm>
+#include <stddef.h>
 #include <string.h>
 #include <vector>
 #include "qg_internal.cuh"
@@ -99,7 +100,10 @@ struct PjPackOut {
 // payload exists, [7] the sentinel.
 enum { PJ_F_DENSE = 1, PJ_F_DISTINCT = 2, PJ_F_PMIN = 4, PJ_F_PMAX = 5, PJ_F_SENT_OK = 6, PJ_F_SENT = 7, PJ_F_WORDS = 8 };
 
-__global__ void k_pj_range_init(PjRange *r, uint32_t *flags) {
+// One CTA: the head block (range, digit histograms, flags) of a new call.
+__global__ void k_pj_range_init(PjRange *r, uint32_t *dh, uint32_t *flags) {
+    for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) dh[i] = 0;
+    if (threadIdx.x != 0) return;
     r->kmin = 0xffffffffu;
     r->kmax = 0;
     r->count = 0;
@@ -180,13 +184,21 @@ __device__ __forceinline__ bool pj_sentinel(int32_t pmin, int32_t pmax, uint32_t
 }
 
 // Dense span with a sentinel payload: T[0 .. w) = the sentinel (no row yet),
-// flags[PJ_F_SENT_OK] = 1, flags[PJ_F_SENT] = the sentinel.
+// flags[PJ_F_SENT_OK] = 1, flags[PJ_F_SENT] = the sentinel.  Without one the
+// presence bitmap is cleared instead.
 __global__ void __launch_bounds__(256)
-k_pj_tfill(uint32_t *__restrict__ T, const PjRange *__restrict__ range, int lb2, long long nR, uint32_t *flags) {
+k_pj_tfill(uint32_t *__restrict__ T, uint32_t *__restrict__ bitmap, const PjRange *__restrict__ range, int lb2,
+           long long nR, uint32_t *flags) {
     const uint32_t kmin = range->kmin, kmax = range->kmax;
     if (!pj_dense_span(kmin, kmax, lb2, nR)) return;
     uint32_t sent;
-    if (!pj_sentinel((int32_t)flags[PJ_F_PMIN], (int32_t)flags[PJ_F_PMAX], &sent)) return;
+    if (!pj_sentinel((int32_t)flags[PJ_F_PMIN], (int32_t)flags[PJ_F_PMAX], &sent)) {
+        const unsigned long long words = ((unsigned long long)(kmax - kmin) + 32ull) >> 5;
+        for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < words;
+             i += (unsigned long long)gridDim.x * blockDim.x)
+            bitmap[i] = 0u;
+        return;
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         flags[PJ_F_SENT_OK] = 1u;
         flags[PJ_F_SENT] = sent;
@@ -1572,11 +1584,12 @@ struct PjLevel {
     uint32_t *gr, *gs;     // [nb + 1] first row of each join group
     uint32_t *big, *mm;    // [nb] group handled outside the bucket kernel; [2 nb] key ranges
     uint32_t *scnt;        // [2 nb] sample counts under radix, learned
-    unsigned long long *bigcnt, *off, *total;
+    unsigned long long *bigcnt, *off;
+    unsigned long long *total;  // the output count (host pinned, written by the bucket kernel)
     PjCross *cross;
     PjMj *mj;
     unsigned long long *mjtot;  // matches of the sort-merge buckets
-    PjPackOut *pk;              // the packing's counts
+    PjPackOut *pk;              // the packing's counts (host pinned, written by k_pj_place)
     uint32_t *dflags;           // [PJ_F_WORDS] flags of the dense build side (set by k_pj_range_init)
     PjPackCta *pkc;             // [nb / (PK_THREADS * 8) + 1] the pack CTAs' totals
     uint32_t *tg;               // [3][nb + PK_THREADS * PK_SEG] the packing's staging (group ends, flags)
@@ -1591,18 +1604,16 @@ size_t pj_level_bytes(uint32_t nb, bool learned) {
     auto add = [&](size_t x) { b += qg_align_up(x, 256); };
     add(sizeof(PjRange));
     add(4 * 256 * 4);
+    add(PJ_F_WORDS * 4);
     for (int i = 0; i < 4; i++) add((size_t)(nb + 16) * 4);  // the packing reads bounds 8 ahead
     add((size_t)nb * 4);
     add((size_t)2 * nb * 4);
     add((size_t)2 * nb * 4);
     add((size_t)nb * 8);
     add((size_t)nb * 8);
-    add(8);
     add((size_t)nb * sizeof(PjCross));
     add((size_t)nb * sizeof(PjMj));
     add(8);
-    add(sizeof(PjPackOut));
-    add(PJ_F_WORDS * 4);
     add(((size_t)nb / (PK_THREADS * 8) + 1) * sizeof(PjPackCta));
     add((size_t)3 * (nb + PK_THREADS * PK_SEG) * 4);
     add((size_t)(nb + PK_THREADS * PK_SEG) * sizeof(PjCross));
@@ -1619,6 +1630,7 @@ void pj_level_carve(char *p, uint32_t nb, bool learned, PjLevel *L) {
     auto take = [&](size_t x) { char *q = p; p += qg_align_up(x, 256); return q; };
     L->range = (PjRange *)take(sizeof(PjRange));
     L->dh = (uint32_t *)take(4 * 256 * 4);
+    L->dflags = (uint32_t *)take(PJ_F_WORDS * 4);  // range, dh and dflags are read back together (PjHead)
     L->rbk = (uint32_t *)take((size_t)(nb + 16) * 4);
     L->sbk = (uint32_t *)take((size_t)(nb + 16) * 4);
     L->gr = (uint32_t *)take((size_t)(nb + 16) * 4);
@@ -1628,12 +1640,9 @@ void pj_level_carve(char *p, uint32_t nb, bool learned, PjLevel *L) {
     L->scnt = (uint32_t *)take((size_t)2 * nb * 4);
     L->bigcnt = (unsigned long long *)take((size_t)nb * 8);
     L->off = (unsigned long long *)take((size_t)nb * 8);
-    L->total = (unsigned long long *)take(8);
     L->cross = (PjCross *)take((size_t)nb * sizeof(PjCross));
     L->mj = (PjMj *)take((size_t)nb * sizeof(PjMj));
     L->mjtot = (unsigned long long *)take(8);
-    L->pk = (PjPackOut *)take(sizeof(PjPackOut));
-    L->dflags = (uint32_t *)take(PJ_F_WORDS * 4);
     L->pkc = (PjPackCta *)take(((size_t)nb / (PK_THREADS * 8) + 1) * sizeof(PjPackCta));
     L->tg = (uint32_t *)take((size_t)3 * (nb + PK_THREADS * PK_SEG) * 4);
     L->tover = (PjCross *)take((size_t)(nb + PK_THREADS * PK_SEG) * sizeof(PjCross));
@@ -1771,8 +1780,12 @@ qg_status pj_compare(qg_ctx *ctx, const PjLevel &L, long long m, long long ntot,
 // oversize buckets and their key ranges.  Every call ends with a stream sync,
 // so the next call may overwrite it.
 struct PjPin {
+    // the level's head block (pj_level_carve's first three arrays), one copy
+    PjRange range;
+    unsigned char pad0[256 - sizeof(PjRange)];
     uint32_t h[1024];                 // [side R, S'][digit 0, 1][256]
     uint32_t dflags[PJ_F_WORDS];
+    unsigned char pad1[256 - PJ_F_WORDS * 4];
     PjPackOut pk;
     PjCross over[PJ_MAX_BUCKETS];
     uint32_t mm[2 * PJ_MAX_BUCKETS];  // [mins][maxes] of the listed buckets
@@ -1927,7 +1940,6 @@ qg_status pj_core(qg_ctx *ctx, const PjLevel &L, PjPin *pin, uint32_t nb, int lb
     // fine bucket bounds, then the join groups packed on the device (one read of the counts)
     auto pack = [&](uint32_t rmax, PjPackOut *pk) -> qg_status {
         QG_TRY(pack_launch(rmax));
-        QG_TRY_CUDA(ctx, cudaMemcpyAsync(&pin->pk, L.pk, sizeof(PjPackOut), cudaMemcpyDeviceToHost, ctx->stream), "pack d2h");
         QG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "sync");
         *pk = pin->pk;
         return pack_check(*pk);
@@ -1960,9 +1972,7 @@ qg_status pj_core(qg_ctx *ctx, const PjLevel &L, PjPin *pin, uint32_t nb, int lb
             auto kern = full ? k_pj_join_dense<PB_THREADS, PB_SMAX, true> : k_pj_join_dense<PB_THREADS, PB_SMAX, false>;
             kern<<<pk.groups, PB_THREADS, sizeof(PdSmem<PB_SMAX, PB_WARPS>), ctx->stream>>>(da, lb);
             QG_TRY(qg_check_launch(ctx, "k_pj_join_dense"));
-            QG_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, L.total, 8, cudaMemcpyDeviceToHost, ctx->stream), "total d2h");
-            QG_TRY(qg_collect_error(ctx));
-            *M_out = ctx->pinned[0];
+            QG_TRY(qg_host_count(ctx, M_out));
             ctx->pj_stats[0] = 4;
             ctx->pj_stats[1] = nbu;
             for (int i = 2; i < 8; i++) ctx->pj_stats[i] = 0;
@@ -2071,12 +2081,11 @@ qg_status pj_core(qg_ctx *ctx, const PjLevel &L, PjPin *pin, uint32_t nb, int lb
         QG_TRY(qg_check_launch(ctx, "k_pj_mj_write"));
     }
     QG_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->pinned + 1, L.mjtot, 8, cudaMemcpyDeviceToHost, ctx->stream), "mjtot d2h");
-    QG_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, L.total, 8, cudaMemcpyDeviceToHost, ctx->stream), "total d2h");
     if (use_learned)  // the model's knot and heavy-key counts, for qg_join_stats
         QG_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->pinned + 2, L.model, 16, cudaMemcpyDeviceToHost, ctx->stream),
                     "model header d2h");
     QG_TRY(qg_collect_error(ctx));  // synchronises: the counts (and header) are in
-    const unsigned long long total = (unsigned long long)ctx->pinned[0];
+    const unsigned long long total = (unsigned long long)ctx->hres->count;
     // The look-back sums are 32-bit: report the outside groups' 64-bit sum
     // when they alone could wrap it (a capacity error follows).
     *M_out = (long long)total;
@@ -2182,17 +2191,17 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     while ((1u << lb2) < nb) lb2++;
     PjLevel L;
     pj_level_carve(aux + 2 * rb + 2 * sb + bmb, nb, variant != 1, &L);
-    QG_TRY_CUDA(ctx, cudaMemsetAsync(L.dh, 0, 4 * 256 * 4, ctx->stream), "memset dhist");
-    QG_TRY_CUDA(ctx, cudaMemsetAsync(bitmap, 0, bmb, ctx->stream), "memset bitmap");
+    L.pk = &pin->pk;
+    L.total = (unsigned long long *)&ctx->hres->count;
     qg_pre_launch(ctx);
-    k_pj_range_init<<<1, 1, 0, ctx->stream>>>(L.range, L.dflags);
+    k_pj_range_init<<<1, 1024, 0, ctx->stream>>>(L.range, L.dh, L.dflags);
     QG_TRY(qg_check_launch(ctx, "k_pj_range_init"));
     qg_pre_launch(ctx);
     k_pj_rrange<<<pj_grid(ctx, nR, 256, 8), 256, 0, ctx->stream>>>(rkey, rpay, nR, L.range, L.dflags);
     QG_TRY(qg_check_launch(ctx, "k_pj_rrange"));
     // R: payload table (+ presence bitmap without a sentinel) on a dense span, else records + digit histograms
     qg_pre_launch(ctx);
-    k_pj_tfill<<<pj_grid(ctx, nR / 2, 256, 8), 256, 0, ctx->stream>>>(T, L.range, lb2, nR, L.dflags);
+    k_pj_tfill<<<pj_grid(ctx, nR / 2, 256, 8), 256, 0, ctx->stream>>>(T, bitmap, L.range, lb2, nR, L.dflags);
     QG_TRY(qg_check_launch(ctx, "k_pj_tfill"));
     qg_pre_launch(ctx);
     k_pj_rtab<<<pj_grid(ctx, nR, 256, 8), 256, 0, ctx->stream>>>(rkey, rpay, nR, L.range, lb2, bitmap, T,
@@ -2209,14 +2218,12 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     k_pj_sfilter<<<(unsigned)std::min<long long>(tiles, (long long)ctx->sm_count * 4), SF_THREADS, 0, ctx->stream>>>(
         skey, spay, nS, slo, shi, L.range, S, &L.range->count, ctx->ctl, lb2, L.dh + 512);
     QG_TRY(qg_check_launch(ctx, "k_pj_sfilter"));
-    // one read brings R's key range, the S' count, the histograms, the dense flags and the error word
-    static_assert(sizeof(PjRange) <= 2 * sizeof(long long), "two pinned slots");
-    PjRange *hp = reinterpret_cast<PjRange *>(ctx->pinned + 4);
-    QG_TRY_CUDA(ctx, cudaMemcpyAsync(hp, L.range, sizeof(PjRange), cudaMemcpyDeviceToHost, ctx->stream), "range d2h");
-    QG_TRY_CUDA(ctx, cudaMemcpyAsync(pin->h, L.dh, 4 * 256 * 4, cudaMemcpyDeviceToHost, ctx->stream), "dhist d2h");
-    QG_TRY_CUDA(ctx, cudaMemcpyAsync(pin->dflags, L.dflags, PJ_F_WORDS * 4, cudaMemcpyDeviceToHost, ctx->stream), "flags d2h");
+    // one copy brings R's key range, the S' count, the histograms and the dense flags
+    constexpr size_t head = offsetof(PjPin, dflags) + PJ_F_WORDS * 4;
+    static_assert(offsetof(PjPin, h) == 256 && offsetof(PjPin, dflags) == 256 + 4096, "as carved");
+    QG_TRY_CUDA(ctx, cudaMemcpyAsync(pin, L.range, head, cudaMemcpyDeviceToHost, ctx->stream), "head d2h");
     QG_TRY(qg_collect_error(ctx));
-    const PjRange hr = *hp;
+    const PjRange hr = pin->range;
     const long long ns1 = (long long)hr.count;
     unsigned long long distinct;
     memcpy(&distinct, pin->dflags + PJ_F_DISTINCT, 8);
