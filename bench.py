@@ -449,9 +449,9 @@ def operator_lines(ctx, args, peak, stream):
 
     ms, kern, _ = timed(ctx, fstep, steps, 3, 1, stream)
     sel = res["o"].shape[0]
-    # The default column filter is two kernels (count, then write): its
-    # roofline is the operator's algorithmic bytes over their summed launch times.
-    fk = [k for k in ("k_filter_count", "k_filter_write", "k_filter_cols") if kern.get(k, (0, 0.0))[0]]
+    # The column filter is one kernel: its roofline is the operator's
+    # algorithmic bytes over its launch time.
+    fk = [k for k in ("k_filter_two", "k_filter_cols") if kern.get(k, (0, 0.0))[0]]
     f_ms = sum(kern[k][1] / kern[k][0] for k in fk)
     f_alg = n * 8 + sel * 8
     out["filter_config0"] = {"rows_per_s": n / (ms * 1e-3), "ms_per_op": ms, "rows": n, "selected": sel,

@@ -130,9 +130,9 @@ QG_API qg_status qg_noalloc_forget(void);
 
 /* Column filter kernel choice (process-wide): 0 = one 4096-row tile per CTA
  * held in registers with a decoupled look-back, 1 = persistent CTAs
- * streaming tiles through a 3-stage bulk-copy (TMA) ring, 2 = two passes
- * (per-tile counts from the keys, then the writes) with no look-back, the
- * default.  Results are identical. */
+ * streaming tiles through a 3-stage bulk-copy (TMA) ring, 2 = two phases of
+ * one launch (per-CTA counts from the keys, then the writes) around a single
+ * exchange of counts, the default.  Results are identical. */
 QG_API qg_status qg_filter_set_variant(int variant);
 
 /* ---- scan (ScanLargeArrays/prefixSum/blockAddition, host/host/testScan.cpp:278-340) */

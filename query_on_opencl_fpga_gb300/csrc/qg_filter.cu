@@ -1,4 +1,4 @@
-// qg_filter.cu -- single-pass stable range filter.
+// qg_filter.cu -- stable range filter.
 //
 // Reference chain replaced (kernel/filter/filter_op.cl, host/host/testFilter.cpp:92-154):
 //   filterImpl_map_kernel (:6-31)       mark[i] = lo <= (int)Rin[i].y <= hi
@@ -6,10 +6,10 @@
 //   filterImpl_outSize_kernel (:211-215) count = mark[n-1] + scan[n-1]
 //   filterImpl_write_kernel (:220-238)   Rout[scan[i]] = Rin[i] if mark[i]
 // The reference moves each row through HBM about six times and launches
-// 2*pass+3 kernels.  Here one kernel reads each row once with 128-bit loads,
-// ranks the selected rows with warp ballots + popc, gets the tile's output
-// offset from a decoupled look-back over earlier tiles, and writes the
-// selected rows in input order (stable, as the reference's scatter is).
+// 2*pass+3 kernels.  Here one kernel counts the selected rows with 128-bit
+// loads, gets each CTA's output offset from one exchange of counts, and writes
+// the selected rows in input order (stable, as the reference's scatter is).
+#include <algorithm>
 #include "qg_internal.cuh"
 
 namespace {
@@ -18,68 +18,148 @@ constexpr int FT_THREADS = 256;
 constexpr int FT_WARPS = FT_THREADS / 32;
 constexpr int FT_LB_WARPS = 4;  // warps doing the look-back: 128 predecessors per round
 
-// Records (uint2 {x, y}), two per 128-bit load.  ROUNDS loads per thread.
-template <int ROUNDS>
-__global__ void __launch_bounds__(FT_THREADS, 5)
-k_filter_rec(const uint4 *__restrict__ in, long long n, int32_t lo, int32_t hi,
-             uint2 *__restrict__ out, long long cap, long long *__restrict__ d_count,
-             qg_lookback lb) {
-    constexpr int TILE = FT_THREADS * ROUNDS * 2;
-    __shared__ uint32_t s_tile, s_epoch, s_excl;
-    __shared__ uint32_t s_woff[ROUNDS * FT_WARPS];
-    const uint32_t tile = blockIdx.x;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const long long base = (long long)tile * TILE;
-    const uint32_t lt = qg_lanemask_lt();
+// Two phases in one launch (records, and the default column form).  The rows
+// are cut into units of four 128-bit loads per lane of a warp, and every warp
+// owns a contiguous range of units:
+//   phase 1: the warp reads its keys (or records), keeps each row's predicate
+//            bit and counts them, with no exchange between warps;
+//   exchange: one count per CTA, a wide look-back over the CTAs before it
+//            (CTAs are numbered as they start, so they are running);
+//   phase 2: the warp walks its units backwards from its end position and
+//            writes the selected rows in input order.  Columns read payloads
+//            of lanes with a selected row only; records are read again, the
+//            last unit from registers and the most recent ones from L2.
+// What bounds it is the memory's pace in both phases plus one exchange per
+// launch: neither a chain of look-backs, tile by tile (what records had:
+// 5M of them, 40 % kept, 30.8 us, now 23), nor a second launch (what columns
+// had: 16M rows, 10 % kept, 45.6 us in two launches, now 36.9; 4096-row tiles
+// with a look-back each 67).  One CTA per SM: with four to eight smaller ones
+// the exchange took longer (49 us with six).  Loading a unit ahead did not help.
+// The selected rows pass through shared memory so that a warp's stores are
+// consecutive (16M rows, 90 % kept: 87 -> 53 us).
+constexpr int F2_MAX_WARPS = 32;  // one CTA of up to 1024 threads per SM
+constexpr int F2_MIN_WARPS = 8;   // the look-back's warps
+constexpr int F2_LOADS = 4;       // 128-bit loads per lane and unit
+constexpr int F2_SUNITS = 16;     // units of a warp whose predicate bits stay in shared memory
 
-    uint4 v[ROUNDS];
-    uint32_t fl = 0;            // bit 2r: first record of round r, bit 2r+1: second
-    uint32_t lpre[ROUNDS];      // selected records of lower lanes in this round
-    // Every load of the tile is issued before the first ballot, so the
-    // rounds' DRAM latencies overlap instead of adding up.
+template <bool REC>
+struct F2 {
+    static constexpr int PER = REC ? 2 : 4;                      // rows per 128-bit load
+    static constexpr int UNIT = 32 * F2_LOADS * PER;             // rows per unit
+    static constexpr uint32_t FM = (1u << PER) - 1u;             // predicate bits of one load
+};
+
+// Lane's load r of unit u: rows [idx, idx + PER), zero past the end.
+template <bool REC>
+__device__ __forceinline__ int4 f2_load(const int32_t *__restrict__ src, long long idx, long long n) {
+    constexpr int PER = F2<REC>::PER, WORDS = 4 / PER;  // words per row
+    if (idx + PER <= n) return qg_ldg_stream(reinterpret_cast<const int4 *>(src + idx * WORDS));
+    int t[4] = {0, 0, 0, 0};
+    for (int j = 0; j < 4; j++)
+        if (idx + j / WORDS < n) t[j] = src[idx * WORDS + j];
+    return make_int4(t[0], t[1], t[2], t[3]);
+}
+
+template <bool REC>
+__device__ __forceinline__ uint32_t f2_flags(const int4 &k, long long idx, long long n, int32_t lo, int32_t hi) {
+    if (REC)
+        return (uint32_t)((k.y >= lo) & (k.y <= hi) & (idx + 0 < n)) |
+               ((uint32_t)((k.w >= lo) & (k.w <= hi) & (idx + 1 < n)) << 1);
+    return (uint32_t)((k.x >= lo) & (k.x <= hi) & (idx + 0 < n)) |
+           ((uint32_t)((k.y >= lo) & (k.y <= hi) & (idx + 1 < n)) << 1) |
+           ((uint32_t)((k.z >= lo) & (k.z <= hi) & (idx + 2 < n)) << 2) |
+           ((uint32_t)((k.w >= lo) & (k.w <= hi) & (idx + 3 < n)) << 3);
+}
+
+template <bool REC>
+__global__ void __launch_bounds__(32 * F2_MAX_WARPS, 1)
+k_filter_two(const int32_t *__restrict__ src, const int32_t *__restrict__ pay, long long n, long long units,
+             int32_t lo, int32_t hi, int2 *__restrict__ out, long long cap, long long *__restrict__ d_count,
+             uint16_t *__restrict__ spill, qg_lookback lb) {
+    constexpr int PER = F2<REC>::PER, UNIT = F2<REC>::UNIT;
+    // per warp: the unit's selected rows on their way out; per thread: predicate bits
+    extern __shared__ __align__(16) unsigned char f2_raw[];
+    __shared__ uint32_t s_tile, s_epoch, s_excl, s_cnt[F2_MAX_WARPS], s_tmp[2 * F2_MIN_WARPS];
+    const uint32_t nw = blockDim.x >> 5;
+    int2 *stage = reinterpret_cast<int2 *>(f2_raw) + (size_t)(threadIdx.x >> 5) * UNIT;
+    uint16_t *s_mask = reinterpret_cast<uint16_t *>(reinterpret_cast<int2 *>(f2_raw) + (size_t)nw * UNIT);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t lt = qg_lanemask_lt();
+    qg_lb_begin_dyn(lb, &s_tile, &s_epoch);
+    const uint32_t tile = s_tile;
+    const long long W = (long long)gridDim.x * nw, gw = (long long)tile * nw + warp;
+    const long long ub = units * gw / W, ue = units * (gw + 1) / W;
+    int4 v[F2_LOADS];
+    uint32_t cnt = 0, fl = 0;
+    for (long long u = ub; u < ue; u++) {
+        const long long r0 = u * UNIT + lane * PER;
 #pragma unroll
-    for (int r = 0; r < ROUNDS; r++) {
-        long long idx = base + (long long)(r * FT_THREADS + tid) * 2;
-        if (idx + 1 < n) {
-            int4 t = qg_ldg_stream(reinterpret_cast<const int4 *>(in) + (idx >> 1));
-            v[r] = make_uint4(t.x, t.y, t.z, t.w);
-        } else if (idx < n) {
-            uint2 a = reinterpret_cast<const uint2 *>(in)[idx];
-            v[r] = make_uint4(a.x, a.y, 0, 0);
-        } else {
-            v[r] = make_uint4(0, 0, 0, 0);
+        for (int r = 0; r < F2_LOADS; r++) v[r] = f2_load<REC>(src, r0 + r * 32 * PER, n);
+        fl = 0;
+#pragma unroll
+        for (int r = 0; r < F2_LOADS; r++) fl |= f2_flags<REC>(v[r], r0 + r * 32 * PER, n, lo, hi) << (PER * r);
+        cnt += __popc(fl);
+        // only this thread reads its bits back
+        if (u - ub < F2_SUNITS) s_mask[(u - ub) * blockDim.x + tid] = (uint16_t)fl;
+        else spill[u * 32 + lane] = (uint16_t)fl;
+    }
+    cnt = __reduce_add_sync(QG_FULL_MASK, cnt);
+    if (lane == 0) s_cnt[warp] = cnt;
+    __syncthreads();
+    const uint32_t wc = lane < (int)nw ? s_cnt[lane] : 0u;
+    const uint32_t before = __reduce_add_sync(QG_FULL_MASK, lane < warp ? wc : 0u);
+    if (warp < F2_MIN_WARPS) {
+        const uint32_t total = __reduce_add_sync(QG_FULL_MASK, wc);
+        const uint32_t e = qg_lb_wide_exclusive<F2_MIN_WARPS>(lb, tile, s_epoch, total, s_tmp);
+        if (tid == 0) {
+            s_excl = e;
+            if (tile == gridDim.x - 1) *d_count = (long long)e + total;
         }
     }
-    qg_lb_begin(lb, &s_tile, &s_epoch);  // epoch read while the loads are in flight
-#pragma unroll
-    for (int r = 0; r < ROUNDS; r++) {
-        long long idx = base + (long long)(r * FT_THREADS + tid) * 2;
-        bool f0 = (idx < n) & ((int32_t)v[r].y >= lo) & ((int32_t)v[r].y <= hi);
-        bool f1 = (idx + 1 < n) & ((int32_t)v[r].w >= lo) & ((int32_t)v[r].w <= hi);
-        uint32_t b0 = __ballot_sync(QG_FULL_MASK, f0), b1 = __ballot_sync(QG_FULL_MASK, f1);
-        lpre[r] = __popc(b0 & lt) + __popc(b1 & lt);
-        if (lane == 0) s_woff[r * FT_WARPS + warp] = __popc(b0) + __popc(b1);
-        fl |= (uint32_t)f0 << (2 * r);
-        fl |= (uint32_t)f1 << (2 * r + 1);
-    }
-    // Exclusive offsets of the ROUNDS*WARPS per-warp counts, round-major (the
-    // order of the rows they cover), and the tile's offset from the look-back.
-    __shared__ uint32_t s_tmp[2 * FT_LB_WARPS + 1];
-    qg_tile_offsets_wide<ROUNDS * FT_WARPS, FT_LB_WARPS>(s_woff, lb, tile, s_epoch, &s_excl, s_tmp,
-                                                         d_count, gridDim.x - 1);
-    const long long excl = s_excl;
-#pragma unroll
-    for (int r = 0; r < ROUNDS; r++) {
-        long long pos = excl + s_woff[r * FT_WARPS + warp] + lpre[r];
-        if ((fl >> (2 * r)) & 1u) {
-            if (pos < cap) out[pos] = make_uint2(v[r].x, v[r].y);
-            pos++;
+    __syncthreads();
+    long long end = (long long)s_excl + before + cnt;  // one past the warp's last output row
+    for (long long u = ue - 1; u >= ub; u--) {
+        const long long r0 = u * UNIT + lane * PER;
+        if (u < ue - 1) {
+            fl = u - ub < F2_SUNITS ? (uint32_t)s_mask[(u - ub) * blockDim.x + tid] : (uint32_t)spill[u * 32 + lane];
+            if (!__any_sync(QG_FULL_MASK, fl != 0u)) continue;
         }
-        if ((fl >> (2 * r + 1)) & 1u) {
-            if (pos < cap) out[pos] = make_uint2(v[r].z, v[r].w);
+        if (!REC || u < ue - 1) {
+#pragma unroll
+            for (int r = 0; r < F2_LOADS; r++) {
+                v[r] = make_int4(0, 0, 0, 0);
+                if ((fl >> (PER * r)) & F2<REC>::FM) v[r] = f2_load<REC>(REC ? src : pay, r0 + r * 32 * PER, n);
+            }
         }
+        uint32_t pre[F2_LOADS], tot = 0;  // selected rows of the unit before this lane's load r
+#pragma unroll
+        for (int r = 0; r < F2_LOADS; r++) {
+            pre[r] = tot;
+#pragma unroll
+            for (int j = 0; j < PER; j++) {
+                const uint32_t b = __ballot_sync(QG_FULL_MASK, (fl >> (PER * r + j)) & 1u);
+                pre[r] += __popc(b & lt);
+                tot += __popc(b);
+            }
+        }
+        // through shared memory, so that the warp's stores are consecutive
+#pragma unroll
+        for (int r = 0; r < F2_LOADS; r++) {
+            uint32_t pos = pre[r];
+            const int x[4] = {v[r].x, v[r].y, v[r].z, v[r].w};
+#pragma unroll
+            for (int j = 0; j < PER; j++)
+                if ((fl >> (PER * r + j)) & 1u)
+                    stage[pos++] = REC ? make_int2(x[2 * j & 3], x[(2 * j + 1) & 3])
+                                       : make_int2((int)(r0 + r * 32 * PER + j), x[j]);
+        }
+        __syncwarp();
+        end -= tot;
+        const uint32_t lim = end >= cap ? 0u : (uint32_t)min((long long)tot, cap - end);
+        for (uint32_t i = lane; i < lim; i += 32) out[end + i] = stage[i];
+        __syncwarp();
     }
-    qg_lb_finish(lb, tile, gridDim.x - 1, s_epoch);
+    qg_lb_finish_dyn(lb, tile, gridDim.x - 1, s_epoch);
 }
 
 // Columns: int32 key and payload, four rows per 128-bit load.  Output is the
@@ -157,7 +237,6 @@ k_filter_cols(const int32_t *__restrict__ key, const int32_t *__restrict__ pay, 
     qg_lb_finish_dyn(lb, tile, gridDim.x - 1, s_epoch);
 }
 
-constexpr int REC_ROUNDS = 8;   // 4096 records per tile
 constexpr int COL_ROUNDS = 4;   // 4096 rows per tile
 
 // Persistent column filter: each CTA streams tiles of 4096 rows (keys and
@@ -324,163 +403,35 @@ static qg_status finish_count(qg_ctx *ctx, int64_t cap, int64_t *out_n) {
     return QG_OK;
 }
 
-// ---------------------------------------------------------------------------
-// Column filter, two passes with no waiting between tiles (variant 2).
-//   pass A (k_filter_count): keys only; the selected-row count of every tile,
-//          per group of 256 tiles the sum of their counts, and every row's
-//          predicate bit (16 bits per thread);
-//   pass B (k_filter_write): the predicate bits and the payloads of the
-//          selected rows only (the output is row id + payload); each tile's
-//          output offset is the sum of the group sums before it plus its
-//          group's earlier tile counts (at most 255), read while its own
-//          loads are in flight.
-// No tile waits for another: both passes stream at the memory's pace, where
-// the single-pass chain of look-backs does not.
-// ---------------------------------------------------------------------------
-constexpr int TP_THREADS = 256;
-constexpr int TP_WARPS = TP_THREADS / 32;
-constexpr int TP_ROUNDS = 4;
-constexpr int TP_TILE = TP_THREADS * TP_ROUNDS * 4;  // 4096 rows
-constexpr int TP_GROUP = 256;                         // tiles per group sum
-
-__device__ __forceinline__ void tp_load_keys(const int32_t *__restrict__ key, long long idx, long long n, int4 &k) {
-    if (idx + 3 < n) {
-        k = qg_ldg_stream(reinterpret_cast<const int4 *>(key + idx));
-    } else {
-        int t[4] = {0, 0, 0, 0};
-        for (int j = 0; j < 4; j++)
-            if (idx + j < n) t[j] = key[idx + j];
-        k = make_int4(t[0], t[1], t[2], t[3]);
+// Launch of k_filter_two: a warp per unit until every SM is full, then
+// contiguous ranges.  `spill` holds the predicate bits of a warp's units past
+// the 16 it keeps in shared memory (inputs above about 60M column rows).
+template <bool REC>
+static qg_status f2_launch(qg_ctx *ctx, const int32_t *src, const int32_t *pay, int64_t n, int32_t lo, int32_t hi,
+                           void *out, int64_t cap, long long *d_count) {
+    const long long units = qg_ceil_div(n, F2<REC>::UNIT);
+    const long long warps = std::max<long long>(F2_MIN_WARPS, std::min<long long>(F2_MAX_WARPS, qg_ceil_div(units, ctx->sm_count)));
+    const long long grid = std::min<long long>(qg_ceil_div(units, warps), ctx->sm_count);
+    qg_lookback lb;
+    QG_TRY(qg_lb_make(ctx, grid, QG_SITE_FILTER, &lb));
+    const long long per_warp = qg_ceil_div(units, grid * warps);  // a warp's units, at most
+    uint16_t *spill = nullptr;
+    if (per_warp > F2_SUNITS) {
+        char *scr;
+        QG_TRY(qg_scratch(ctx, (size_t)units * 64, &scr));
+        spill = (uint16_t *)scr;
     }
-}
-
-__device__ __forceinline__ uint32_t tp_flags(const int4 &k, long long idx, long long n, int32_t lo, int32_t hi) {
-    return (uint32_t)((k.x >= lo) & (k.x <= hi) & (idx + 0 < n)) | ((uint32_t)((k.y >= lo) & (k.y <= hi) & (idx + 1 < n)) << 1) |
-           ((uint32_t)((k.z >= lo) & (k.z <= hi) & (idx + 2 < n)) << 2) |
-           ((uint32_t)((k.w >= lo) & (k.w <= hi) & (idx + 3 < n)) << 3);
-}
-
-// With mask set, each thread also stores its 16 rows' predicate bits (bit
-// 4 * round + j), so that pass B need not read the keys again.
-__global__ void __launch_bounds__(TP_THREADS)
-k_filter_count(const int32_t *__restrict__ key, long long n, int32_t lo, int32_t hi, uint32_t *__restrict__ counts,
-               uint32_t *__restrict__ gsum, uint16_t *__restrict__ mask, uint32_t *__restrict__ arrivals) {
-    __shared__ uint32_t ws[TP_WARPS];
-    __shared__ uint32_t s_last;
-    const int tid = threadIdx.x;
-    const long long base = (long long)blockIdx.x * TP_TILE;
-    int4 kv[TP_ROUNDS];
-#pragma unroll
-    for (int r = 0; r < TP_ROUNDS; r++) tp_load_keys(key, base + (long long)(r * TP_THREADS + tid) * 4, n, kv[r]);
-    uint32_t fl = 0;
-#pragma unroll
-    for (int r = 0; r < TP_ROUNDS; r++)
-        fl |= tp_flags(kv[r], base + (long long)(r * TP_THREADS + tid) * 4, n, lo, hi) << (4 * r);
-    if (mask) mask[(size_t)blockIdx.x * TP_THREADS + tid] = (uint16_t)fl;
-    uint32_t c = __popc(fl);
-    c = __reduce_add_sync(QG_FULL_MASK, c);
-    if ((tid & 31) == 0) ws[tid >> 5] = c;
-    __syncthreads();
-    const uint32_t g = blockIdx.x / TP_GROUP;
-    const uint32_t gsize = min((uint32_t)TP_GROUP, gridDim.x - g * TP_GROUP);
-    if (tid == 0) {
-        uint32_t t = 0;
-        for (int w = 0; w < TP_WARPS; w++) t += ws[w];
-        counts[blockIdx.x] = t;
-        __threadfence();
-        // atomicInc wraps to zero on the group's last arrival, which then
-        // sums the group's counts (all stored and fenced before their arrivals)
-        s_last = atomicInc(&arrivals[g], gsize - 1) == gsize - 1;
+    const size_t smem = (size_t)warps * (F2<REC>::UNIT * 8 + std::min<long long>(per_warp, F2_SUNITS) * 64);
+    static bool attr = false;
+    if (!attr) {
+        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_filter_two<REC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              F2_MAX_WARPS * (F2<REC>::UNIT * 8 + F2_SUNITS * 64)), "attr");
+        attr = true;
     }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    uint32_t gc = tid < (int)gsize ? __ldcg(counts + (size_t)g * TP_GROUP + tid) : 0u;
-    static_assert(TP_GROUP == TP_THREADS, "one count per thread");
-    gc = __reduce_add_sync(QG_FULL_MASK, gc);
-    if ((tid & 31) == 0) ws[tid >> 5] = gc;
-    __syncthreads();
-    if (tid == 0) {
-        uint32_t t = 0;
-        for (int w = 0; w < TP_WARPS; w++) t += ws[w];
-        gsum[g] = t;
-    }
-}
-
-// Pass B from pass A's predicate bits: the keys are not read again, and a
-// thread loads its four payloads only when one of them is selected (the
-// output holds row ids and payloads, never keys).
-__global__ void __launch_bounds__(TP_THREADS)
-k_filter_write(const uint16_t *__restrict__ mask, const int32_t *__restrict__ pay, long long n,
-                 const uint32_t *__restrict__ counts, const uint32_t *__restrict__ gsum, int2 *__restrict__ out,
-                 long long cap, long long *__restrict__ d_count) {
-    __shared__ uint32_t s_woff[TP_ROUNDS * TP_WARPS];
-    __shared__ unsigned long long s_pre[TP_WARPS];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t tile = blockIdx.x;
-    const long long base = (long long)tile * TP_TILE;
-    const uint32_t lt = qg_lanemask_lt();
-    const uint32_t fl = __ldg(mask + (size_t)tile * TP_THREADS + tid);
-    int4 pv[TP_ROUNDS];
-#pragma unroll
-    for (int r = 0; r < TP_ROUNDS; r++) {
-        pv[r] = make_int4(0, 0, 0, 0);
-        if ((fl >> (4 * r)) & 0xfu) tp_load_keys(pay, base + (long long)(r * TP_THREADS + tid) * 4, n, pv[r]);
-    }
-    // offset of this tile: earlier groups' sums, then this group's earlier tiles
-    unsigned long long pre = 0;
-    const uint32_t g = tile / TP_GROUP;
-    for (uint32_t i = tid; i < g; i += TP_THREADS) pre += __ldg(gsum + i);
-    for (uint32_t i = g * TP_GROUP + tid; i < tile; i += TP_THREADS) pre += __ldg(counts + i);
-    uint32_t lpre[TP_ROUNDS];
-#pragma unroll
-    for (int r = 0; r < TP_ROUNDS; r++) {
-        const uint32_t f = (fl >> (4 * r)) & 0xfu;
-        uint32_t c = 0, tot = 0;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint32_t b = __ballot_sync(QG_FULL_MASK, (f >> j) & 1u);
-            c += __popc(b & lt);
-            tot += __popc(b);
-        }
-        lpre[r] = c;
-        if (lane == 0) s_woff[r * TP_WARPS + warp] = tot;
-    }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) pre += __shfl_down_sync(QG_FULL_MASK, pre, d);
-    if (lane == 0) s_pre[warp] = pre;
-    __syncthreads();
-    if (warp == 0) {  // exclusive scan of the 32 (round, warp) counts in row order
-        const uint32_t x = s_woff[lane];
-        uint32_t inc = x;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(QG_FULL_MASK, inc, d);
-            if (lane >= d) inc += y;
-        }
-        s_woff[lane] = inc - x;
-        if (lane == 31) {
-            unsigned long long e = 0;
-            for (int w = 0; w < TP_WARPS; w++) e += s_pre[w];
-            s_pre[0] = e;
-            if (tile == gridDim.x - 1) *d_count = (long long)(e + inc);
-        }
-    }
-    __syncthreads();
-    const long long excl = (long long)s_pre[0];
-#pragma unroll
-    for (int r = 0; r < TP_ROUNDS; r++) {
-        long long pos = excl + s_woff[r * TP_WARPS + warp] + lpre[r];
-        const long long idx = base + (long long)(r * TP_THREADS + tid) * 4;
-        const int pp[4] = {pv[r].x, pv[r].y, pv[r].z, pv[r].w};
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            if ((fl >> (4 * r + j)) & 1u) {
-                if (pos < cap) out[pos] = make_int2((int)(idx + j), pp[j]);
-                pos++;
-            }
-        }
-    }
+    qg_pre_launch(ctx);
+    k_filter_two<REC><<<(unsigned)grid, (unsigned)(32 * warps), smem, ctx->stream>>>(src, pay, n, units, lo, hi,
+                                                                                    (int2 *)out, cap, d_count, spill, lb);
+    return qg_check_launch(ctx, REC ? "k_filter_rec" : "k_filter_two");
 }
 
 // The count of an empty input: the host word directly, a device word in stream order.
@@ -492,22 +443,23 @@ static qg_status qg_zero_count(qg_ctx *ctx, long long *d_count) {
 
 qg_status qg_filter_rec_launch(qg_ctx *ctx, const void *in, int64_t n, int32_t lo, int32_t hi,
                                void *out, int64_t cap, long long *d_count) {
-    constexpr int TILE = FT_THREADS * REC_ROUNDS * 2;
     if (n == 0) {
         return qg_zero_count(ctx, d_count);
     }
     if (((uintptr_t)in & 15) != 0 || ((uintptr_t)out & 7) != 0) return QG_ERR_INVALID;
-    int64_t tiles = qg_ceil_div(n, TILE);
-    if (tiles > 0x7fffffff) return QG_ERR_UNSUPPORTED;
-    qg_lookback lb;
-    QG_TRY(qg_lb_make(ctx, tiles, QG_SITE_FILTER, &lb));
-    qg_pre_launch(ctx);
-    k_filter_rec<REC_ROUNDS><<<(unsigned)tiles, FT_THREADS, 0, ctx->stream>>>(
-        (const uint4 *)in, n, lo, hi, (uint2 *)out, cap, d_count, lb);
-    return qg_check_launch(ctx, "k_filter_rec");
+    // Phase 2 reads rows that other warps' writes may have reached by then
+    // when the output overlaps the input: such a call filters a copy.
+    const uintptr_t ib = (uintptr_t)in, ob = (uintptr_t)out;
+    if (ib < ob + (size_t)std::min(cap, n) * 8 && ob < ib + (size_t)n * 8) {
+        char *tmp;
+        QG_TRY(qg_aux(ctx, (size_t)n * 8, &tmp));
+        QG_TRY_CUDA(ctx, cudaMemcpyAsync(tmp, in, (size_t)n * 8, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
+        in = tmp;
+    }
+    return f2_launch<true>(ctx, (const int32_t *)in, nullptr, n, lo, hi, out, cap, d_count);
 }
 
-static int g_filter_variant = 2;  // two passes: fastest measured (42 us vs 68 us at 16M rows)
+static int g_filter_variant = 2;  // two phases: fastest measured at every size
 
 qg_status qg_filter_cols_launch(qg_ctx *ctx, const int32_t *key, const int32_t *pay, int64_t n,
                                 int32_t lo, int32_t hi, int32_t *out, int64_t cap,
@@ -520,28 +472,10 @@ qg_status qg_filter_cols_launch(qg_ctx *ctx, const int32_t *key, const int32_t *
         return QG_ERR_INVALID;
     int64_t tiles = qg_ceil_div(n, TILE);
     if (tiles > 0x7fffffff || n > 0x7fffffffLL) return QG_ERR_UNSUPPORTED;
+    const int variant = qg_effective_variant(ctx, QG_STEER_FILTER, g_filter_variant);
+    if (variant == 2) return f2_launch<false>(ctx, key, pay, n, lo, hi, out, cap, d_count);
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, tiles, QG_SITE_FILTER, &lb));
-    const int variant = qg_effective_variant(ctx, QG_STEER_FILTER, g_filter_variant);
-    if (variant == 2) {
-        const long long tp_tiles = qg_ceil_div(n, TP_TILE);
-        const long long groups = qg_ceil_div(tp_tiles, TP_GROUP);
-        char *scr;
-        const size_t cg_bytes = qg_align_up((size_t)(tp_tiles + groups) * 4, 256);
-        QG_TRY(qg_scratch(ctx, cg_bytes + (size_t)tp_tiles * TP_THREADS * 2, &scr));
-        uint32_t *counts = (uint32_t *)scr, *gsum = counts + tp_tiles;
-        uint16_t *mask = (uint16_t *)(scr + cg_bytes);
-        static_assert(sizeof(((qg_control *)0)->fgroup) / 4 * (long long)TP_GROUP * TP_TILE >= 0x7fffffffLL,
-                      "one arrival counter per group of the largest accepted input");
-        qg_pre_launch(ctx);
-        k_filter_count<<<(unsigned)tp_tiles, TP_THREADS, 0, ctx->stream>>>(key, n, lo, hi, counts, gsum, mask,
-                                                                         ctx->ctl->fgroup);
-        QG_TRY(qg_check_launch(ctx, "k_filter_count"));
-        qg_pre_launch(ctx);
-        k_filter_write<<<(unsigned)tp_tiles, TP_THREADS, 0, ctx->stream>>>(mask, pay, n, counts, gsum, (int2 *)out,
-                                                                         cap, d_count);
-        return qg_check_launch(ctx, "k_filter_write");
-    }
     if (variant == 1) {
         static bool attr = false;
         if (!attr) {
@@ -563,8 +497,8 @@ qg_status qg_filter_cols_launch(qg_ctx *ctx, const int32_t *key, const int32_t *
 }
 
 // 0: one tile per CTA, rows staged in registers, decoupled look-back;
-// 1: persistent CTAs with a bulk-copy ring; 2: two passes (count, write)
-// with no look-back (all bit-identical; chosen by measurement).
+// 1: persistent CTAs with a bulk-copy ring; 2: two phases (count, write)
+// around one exchange (all bit-identical; chosen by measurement).
 int qg_filter_default_variant() { return g_filter_variant; }
 
 extern "C" QG_API qg_status qg_filter_set_variant(int variant) {

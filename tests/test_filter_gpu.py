@@ -136,3 +136,36 @@ def test_filter_cols_variants(ctx, orc, variant, n):
         assert np.array_equal(got, orc.filter_cols(key, pay, d["lo"], d["hi"]))
     finally:
         ctx.lib.qg_filter_set_variant(2)  # the default
+
+
+# Edges of the two-phase kernel: a warp's unit (512 column rows, 256 records),
+# a CTA of 8 warps, one unit per warp on every SM, and more units per warp than
+# its shared memory keeps predicate bits for.
+@pytest.mark.parametrize("rec", [False, True])
+@pytest.mark.parametrize("units,extra", [(1, -1), (1, 0), (1, 1), (8, 0), (8, 1), (152 * 8, 3), (152 * 32, 0),
+                                         (152 * 32, 1), (152 * 32 * 16, 1)])
+def test_filter_two_phase_edges(ctx, orc, rec, units, extra):
+    n = units * (256 if rec else 512) + extra
+    d = datagen.config0_filter(n, seed=units, device="cuda")
+    key, pay = d["key"], d["payload"]
+    for lo, hi in [(d["lo"], d["hi"]), (1 << 29, 2 ** 31 - 1)]:
+        if rec:
+            r = datagen.records(key, pay)
+            got = ctx.filter_range_rec(r, lo, hi).cpu().numpy()
+            exp = orc.filter_rec(r.cpu().numpy(), lo, hi)
+        else:
+            got = ctx.filter_cols(key, pay, lo, hi).cpu().numpy()
+            exp = orc.filter_cols(key.cpu().numpy(), pay.cpu().numpy(), lo, hi, mt=True)
+        assert np.array_equal(got, exp)
+
+
+def test_filter_rec_into_its_input(ctx, orc):
+    import ctypes
+
+    n = 300_007
+    r = orc.generate_rand(1000, n, 9)
+    buf = dev(r)
+    cnt = ctypes.c_int64()
+    st = ctx.lib.qg_filter_range_rec(ctx.handle, buf.data_ptr(), n, 0, 400, buf.data_ptr(), n, ctypes.byref(cnt))
+    exp = orc.filter_rec(r, 0, 400)
+    assert st == 0 and np.array_equal(buf[: cnt.value].cpu().numpy(), exp)
