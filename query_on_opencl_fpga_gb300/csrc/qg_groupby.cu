@@ -27,6 +27,7 @@
 //    updated with atomicCAS / 64-bit atomicAdd) is the fallback for inputs
 //    that overflow the spill buckets.  QG_ORDER_KEY then ranks or sorts the
 //    groups by key (unsigned, the order groupByImpl's sorted array gives).
+#include <algorithm>
 #include "qg_internal.cuh"
 #include "qg_sort.cuh"
 
@@ -35,77 +36,111 @@ namespace {
 // ---------------------------------------------------------------------------
 // 1a. group boundaries of sorted records -> startPos (stable compaction)
 // ---------------------------------------------------------------------------
-constexpr int GBD_THREADS = 256;
-constexpr int GBD_WARPS = GBD_THREADS / 32;
-constexpr int GBD_ROUNDS = 8;  // 2 records per round: 4096 records per tile
+// Two phases in one launch, as the filters (qg_filter.cu): every warp owns a
+// contiguous range of units of 256 records, finds and counts the group heads
+// (a key unlike the one before it), the CTAs exchange their counts once, and
+// the warp writes the heads' row indices from its bits -- the records are read
+// once.  16M records: 64 us with a look-back per 4096-record tile, 37 us now
+// (floor 20).
+constexpr int GH_MAX_WARPS = 32, GH_MIN_WARPS = 8;  // one CTA per SM; the look-back's warps
+constexpr int GH_UNIT = 256;                        // records: 4 loads of 2 per lane
+constexpr int GH_SUNITS = 32;                       // units of a warp whose head bits stay in shared memory
 
-__global__ void __launch_bounds__(GBD_THREADS)
-k_group_bounds(const uint4 *__restrict__ in, long long n, int32_t *__restrict__ startPos,
-               long long cap, long long *__restrict__ d_count, qg_lookback lb) {
-    constexpr int TILE = GBD_THREADS * GBD_ROUNDS * 2;
-    __shared__ uint32_t s_tile, s_epoch, s_excl;
-    __shared__ uint32_t s_woff[GBD_ROUNDS * GBD_WARPS];
-    qg_lb_begin(lb, &s_tile, &s_epoch);
-    const uint32_t tile = s_tile;
+__global__ void __launch_bounds__(32 * GH_MAX_WARPS, 1)
+k_group_bounds(const uint2 *__restrict__ in, long long n, long long units, int32_t *__restrict__ startPos,
+               long long cap, long long *__restrict__ d_count, uint8_t *__restrict__ spill, qg_lookback lb) {
+    extern __shared__ __align__(16) unsigned char gh_raw[];
+    __shared__ uint32_t s_tile, s_epoch, s_excl, s_cnt[GH_MAX_WARPS], s_tmp[2 * GH_MIN_WARPS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const long long base = (long long)tile * TILE;
-    const uint32_t lt = qg_lanemask_lt();
-    const uint2 *in2 = reinterpret_cast<const uint2 *>(in);
-    uint32_t fl = 0, lpre[GBD_ROUNDS];
-    // Loads of all rounds first (keys of the thread's pair and of the record
-    // before it), then the ballots, so the DRAM latencies overlap.
-    uint32_t k0[GBD_ROUNDS], k1[GBD_ROUNDS], kp[GBD_ROUNDS];
+    const uint32_t nw = blockDim.x >> 5, lt = qg_lanemask_lt();
+    int32_t *stage = reinterpret_cast<int32_t *>(gh_raw) + (size_t)warp * GH_UNIT;
+    uint8_t *s_mask = gh_raw + (size_t)nw * GH_UNIT * 4;
+    qg_lb_begin_dyn(lb, &s_tile, &s_epoch);
+    const uint32_t tile = s_tile;
+    const long long W = (long long)gridDim.x * nw, gw = (long long)tile * nw + warp;
+    const long long ub = units * gw / W, ue = units * (gw + 1) / W;
+    uint32_t cnt = 0, prev = ub < ue && ub > 0 ? in[ub * GH_UNIT - 1].y : 0u;  // the key before the unit
+    for (long long u = ub; u < ue; u++) {
+        const long long r0 = u * GH_UNIT + lane * 2;
+        uint32_t k0[4], k1[4];
 #pragma unroll
-    for (int r = 0; r < GBD_ROUNDS; r++) {
-        long long idx = base + (long long)(r * GBD_THREADS + tid) * 2;
-        k0[r] = k1[r] = kp[r] = 0;
-        if (idx < n) {
-            if (idx + 1 < n) {
-                int4 t = qg_ldg_stream(reinterpret_cast<const int4 *>(in) + (idx >> 1));
+        for (int r = 0; r < 4; r++) {
+            const long long i = r0 + r * 64;
+            k0[r] = k1[r] = 0;
+            if (i + 1 < n) {
+                const int4 t = qg_ldg_stream(reinterpret_cast<const int4 *>(in) + (i >> 1));
                 k0[r] = (uint32_t)t.y;
                 k1[r] = (uint32_t)t.w;
             } else {
-                k0[r] = in2[idx].y;
+                if (i < n) k0[r] = in[i].y;
             }
-            if (idx > 0) kp[r] = __ldg(&in2[idx - 1].y);
+        }
+        uint32_t fl = 0;
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const long long i = r0 + r * 64;
+            uint32_t p = __shfl_up_sync(QG_FULL_MASK, k1[r], 1);
+            if (lane == 0) p = prev;
+            prev = __shfl_sync(QG_FULL_MASK, k1[r], 31);
+            fl |= (uint32_t)((i < n) & ((i == 0) | (k0[r] != p))) << (2 * r);
+            fl |= (uint32_t)((i + 1 < n) & (k1[r] != k0[r])) << (2 * r + 1);
+        }
+        cnt += __popc(fl);
+        if (u - ub < GH_SUNITS) s_mask[(u - ub) * blockDim.x + tid] = (uint8_t)fl;
+        else spill[u * 32 + lane] = (uint8_t)fl;
+    }
+    cnt = __reduce_add_sync(QG_FULL_MASK, cnt);
+    if (lane == 0) s_cnt[warp] = cnt;
+    __syncthreads();
+    const uint32_t wc = lane < (int)nw ? s_cnt[lane] : 0u;
+    const uint32_t before = __reduce_add_sync(QG_FULL_MASK, lane < warp ? wc : 0u);
+    if (warp < GH_MIN_WARPS) {
+        const uint32_t total = __reduce_add_sync(QG_FULL_MASK, wc);
+        const uint32_t e = qg_lb_wide_exclusive<GH_MIN_WARPS>(lb, tile, s_epoch, total, s_tmp);
+        if (tid == 0) {
+            s_excl = e;
+            if (tile == gridDim.x - 1) *d_count = (long long)e + total;
         }
     }
-#pragma unroll
-    for (int r = 0; r < GBD_ROUNDS; r++) {
-        long long idx = base + (long long)(r * GBD_THREADS + tid) * 2;
-        bool f0 = (idx < n) && ((idx == 0) || (kp[r] != k0[r]));
-        bool f1 = (idx + 1 < n) && (k1[r] != k0[r]);
-        uint32_t b0 = __ballot_sync(QG_FULL_MASK, f0), b1 = __ballot_sync(QG_FULL_MASK, f1);
-        lpre[r] = __popc(b0 & lt) + __popc(b1 & lt);
-        if (lane == 0) s_woff[r * GBD_WARPS + warp] = __popc(b0) + __popc(b1);
-        fl |= ((uint32_t)f0 << (2 * r)) | ((uint32_t)f1 << (2 * r + 1));
-    }
     __syncthreads();
-    if (warp == 0)
-        qg_tile_compact_offsets<GBD_ROUNDS * GBD_WARPS>(s_woff, lb, tile, s_epoch, &s_excl, d_count);
-    __syncthreads();
-    const long long excl = s_excl;
+    long long at = (long long)s_excl + before;
+    for (long long u = ub; u < ue; u++) {
+        const uint32_t fl = u - ub < GH_SUNITS ? s_mask[(u - ub) * blockDim.x + tid] : spill[u * 32 + lane];
+        uint32_t tot = 0;
 #pragma unroll
-    for (int r = 0; r < GBD_ROUNDS; r++) {
-        long long idx = base + (long long)(r * GBD_THREADS + tid) * 2;
-        long long pos = excl + s_woff[r * GBD_WARPS + warp] + lpre[r];
-        if ((fl >> (2 * r)) & 1u) {
-            if (pos < cap) startPos[pos] = (int32_t)idx;
-            pos++;
+        for (int r = 0; r < 4; r++) {
+            const uint32_t b0 = __ballot_sync(QG_FULL_MASK, (fl >> (2 * r)) & 1u);
+            const uint32_t b1 = __ballot_sync(QG_FULL_MASK, (fl >> (2 * r + 1)) & 1u);
+            uint32_t pos = tot + __popc(b0 & lt) + __popc(b1 & lt);
+            const int32_t i = (int32_t)(u * GH_UNIT + r * 64 + lane * 2);
+            if ((fl >> (2 * r)) & 1u) stage[pos++] = i;
+            if ((fl >> (2 * r + 1)) & 1u) stage[pos] = i + 1;
+            tot += __popc(b0) + __popc(b1);
         }
-        if ((fl >> (2 * r + 1)) & 1u)
-            if (pos < cap) startPos[pos] = (int32_t)(idx + 1);
+        __syncwarp();
+        const uint32_t lim = at >= cap ? 0u : (uint32_t)min((long long)tot, cap - at);
+        for (uint32_t q = lane; q < lim; q += 32) startPos[at + q] = stage[q];
+        __syncwarp();
+        at += tot;
     }
-    qg_lb_finish(lb, tile, gridDim.x - 1, s_epoch);
+    qg_lb_finish_dyn(lb, tile, gridDim.x - 1, s_epoch);
 }
 
 // ---------------------------------------------------------------------------
 // 1b. per-group aggregation of .x over sorted records
 // ---------------------------------------------------------------------------
-constexpr int AGG_CHUNK = 2048;  // rows per warp work item
+constexpr int AGG_CHUNK = 1024;  // rows per warp work item
+constexpr int AGG_WARPS = 8;
+constexpr int AGG_PAD = AGG_CHUNK + AGG_CHUNK / 32;
 
 __device__ __forceinline__ int32_t agg_identity(int op) {
     return op == QG_REDUCE_MIN ? (1 << 30) : 0;
+}
+
+// OP: QG_REDUCE_SUM (also AVERAGE, which divides at the end), MAX or MIN.
+template <int OP>
+__device__ __forceinline__ int32_t agg_op(int32_t a, int32_t b) {
+    return OP == QG_REDUCE_MAX ? max(a, b) : OP == QG_REDUCE_MIN ? min(a, b) : (int32_t)((uint32_t)a + (uint32_t)b);
 }
 
 __global__ void k_agg_init(int32_t *agg, long long g0, long long g1, int op) {
@@ -115,56 +150,155 @@ __global__ void k_agg_init(int32_t *agg, long long g0, long long g1, int op) {
         agg[i] = id;
 }
 
-// Groups [g0, g1) of G: rows [startPos[g0], startPos[g1] or n) in chunks of
-// AGG_CHUNK rows counted from the range start.
-__global__ void __launch_bounds__(256)
-k_agg_chunks(const uint2 *__restrict__ rec, long long n, const int32_t *__restrict__ startPos,
-             long long G, long long g0, long long g1, int op, int32_t *__restrict__ agg) {
-    const int lane = threadIdx.x & 31;
-    const long long warp_id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+// Groups [g0, g1) of G, rows [startPos[g0], startPos[g1] or n), a warp per
+// chunk of AGG_CHUNK rows.  The chunk's .x values go to shared memory and its
+// group heads to a bit mask; a lane then folds 32 consecutive rows, storing
+// every group that begins and ends among them, and a segmented scan over the
+// lanes joins the groups that cross lanes.  Groups that cross chunks are added
+// with atomics (agg holds the identity).  One group at a time per warp took
+// 195 us for 16M records in 1M groups (16 of 32 lanes idle, a dependent load
+// per group); this takes 39 us (floor 20).
+template <int OP, bool AVG, bool VEC>
+__global__ void __launch_bounds__(32 * AGG_WARPS, 4)
+k_agg_chunks(const uint2 *__restrict__ rec, long long n, const int32_t *__restrict__ startPos, long long G,
+             long long g0, long long g1, int32_t *__restrict__ agg) {
+    __shared__ int32_t s_x[AGG_WARPS][AGG_PAD];
+    __shared__ uint32_t s_head[AGG_WARPS][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long wid = (long long)blockIdx.x * AGG_WARPS + warp, nwarps = (long long)gridDim.x * AGG_WARPS;
+    const int32_t id = agg_identity(OP);
     const long long rs = __ldg(&startPos[g0]);
     const long long re = (g1 == G) ? n : (long long)__ldg(&startPos[g1]);
-    const long long nchunks = (re - rs + AGG_CHUNK - 1) / AGG_CHUNK;
-    for (long long c = warp_id; c < nchunks; c += nwarps) {
-        const long long cs = rs + c * AGG_CHUNK;
-        const long long ce = (cs + AGG_CHUNK < re) ? cs + AGG_CHUNK : re;
-        // last group of the range starting at or before cs
-        long long lo = g0, hi = g1 - 1;
-        while (lo < hi) {
-            long long mid = (lo + hi + 1) >> 1;
-            if ((long long)__ldg(&startPos[mid]) <= cs) lo = mid; else hi = mid - 1;
-        }
-        long long g = lo;
-        long long pos = cs;
-        while (pos < ce && g < g1) {
-            const long long gs = __ldg(&startPos[g]);
-            const long long ge = (g == G - 1) ? n : (long long)__ldg(&startPos[g + 1]);
-            const long long se = ge < ce ? ge : ce;
-            int32_t acc = agg_identity(op);
-            uint32_t sum = 0;
-            for (long long i = pos + lane; i < se; i += 32) {
-                int32_t v = (int32_t)rec[i].x;
-                if (op == QG_REDUCE_MAX) acc = v > acc ? v : acc;
-                else if (op == QG_REDUCE_MIN) acc = v < acc ? v : acc;
-                else sum += (uint32_t)v;
+    if (rs < 0 || re > n || rs >= re) return;
+    auto group_end = [&](long long g) { return g == G - 1 ? n : (long long)__ldg(&startPos[g + 1]); };
+    // the result of the whole group g, and a part of it
+    auto put = [&](long long g, int32_t v) {
+        if (AVG) v = v / (int32_t)(group_end(g) - __ldg(&startPos[g]));
+        agg[g] = v;
+    };
+    auto part = [&](long long g, int32_t v) {
+        if (OP == QG_REDUCE_MAX) atomicMax(&agg[g], v);
+        else if (OP == QG_REDUCE_MIN) atomicMin(&agg[g], v);
+        else atomicAdd((unsigned int *)&agg[g], (unsigned int)v);
+    };
+    for (long long c = rs / AGG_CHUNK + wid; c * AGG_CHUNK < re; c += nwarps) {
+        const long long cs = c * AGG_CHUNK, lo = max(cs, rs), hi = min(cs + AGG_CHUNK, re);
+        int32_t *x = s_x[warp];
+        uint32_t *head = s_head[warp];
+        const int rlo = (int)(lo - cs), rhi = (int)(hi - cs);
+        const uint2 *rc = rec + cs;
+        const bool inner = rlo == 0 && rhi == AGG_CHUNK;
+        int32_t a[AGG_CHUNK / 64], b[AGG_CHUNK / 64];  // rows, the identity outside [lo, hi)
+#pragma unroll
+        for (int i = 0; i < AGG_CHUNK / 64; i++) {
+            const int k = i * 64 + lane * 2;
+            if (VEC && inner) {
+                const int4 t = qg_ldg_stream(reinterpret_cast<const int4 *>(rc + k));
+                a[i] = t.x;
+                b[i] = t.z;
+            } else {
+                a[i] = k >= rlo && k < rhi ? (int32_t)rc[k].x : id;
+                b[i] = k + 1 >= rlo && k + 1 < rhi ? (int32_t)rc[k + 1].x : id;
             }
-            if (op == QG_REDUCE_MAX) acc = __reduce_max_sync(QG_FULL_MASK, acc);
-            else if (op == QG_REDUCE_MIN) acc = __reduce_min_sync(QG_FULL_MASK, acc);
-            else sum = __reduce_add_sync(QG_FULL_MASK, sum);
-            if (lane == 0) {
-                const bool whole = (pos == gs) && (se == ge);
-                if (op == QG_REDUCE_MAX) { if (whole) agg[g] = acc; else atomicMax(&agg[g], acc); }
-                else if (op == QG_REDUCE_MIN) { if (whole) agg[g] = acc; else atomicMin(&agg[g], acc); }
-                else if (whole) {
-                    agg[g] = (op == QG_REDUCE_AVERAGE) ? ((int32_t)sum) / (int32_t)(ge - gs) : (int32_t)sum;
-                } else {
-                    atomicAdd((unsigned int *)&agg[g], sum);
+        }
+        head[lane] = 0;
+        // last group of the range starting at or before lo: a 32-way search
+        long long gl = g0, gh = g1;  // startPos[gl] <= lo; the answer is in [gl, gh)
+        while (gh - gl > 1) {
+            const long long step = (gh - gl + 31) / 32, g = gl + lane * step;
+            const bool le = g < gh && (long long)__ldg(&startPos[g]) <= lo;
+            const uint32_t m = __ballot_sync(QG_FULL_MASK, le);
+            const int last = m ? 31 - __clz(m) : 0;
+            gl += last * step;
+            gh = min(gh, gl + step);
+        }
+        __syncwarp();
+        // heads in [cs, hi), from group gl on
+        bool ordered = true;
+        for (long long g = gl + lane;; g += 32) {
+            const long long p = g < g1 ? (long long)__ldg(&startPos[g]) : re;
+            if (g < g1 && p < hi) {
+                if (p >= cs) {
+                    const uint32_t bit = (uint32_t)(p - cs);
+                    ordered &= !((atomicOr(&head[bit >> 5], 1u << (bit & 31)) >> (bit & 31)) & 1u);
+                }
+                if (g > gl) ordered &= p > (long long)__ldg(&startPos[g - 1]);
+            }
+            if (__any_sync(QG_FULL_MASK, p >= hi)) break;
+        }
+        const bool plain = __all_sync(QG_FULL_MASK, ordered);
+#pragma unroll
+        for (int i = 0; i < AGG_CHUNK / 64; i++) {
+            const int k = i * 64 + lane * 2, at = k + (k >> 5);
+            x[at] = a[i];
+            x[at + 1] = b[i];
+        }
+        __syncwarp();
+        if (plain) {
+            const uint32_t hw = head[lane];
+            uint32_t hb = __popc(hw);  // inclusive count of heads up to this lane's rows
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t t = __shfl_up_sync(QG_FULL_MASK, hb, d);
+                if (lane >= d) hb += t;
+            }
+            const uint32_t heads_before = hb - __popc(hw);
+            // the group of the lane's first row, when that row is no head
+            const long long gfirst = gl - ((long long)__ldg(&startPos[gl]) >= cs ? 1 : 0) + heads_before;
+            long long g = gfirst;
+            int32_t acc = id, front = id;  // front: the rows before the lane's first head
+            bool seen = false;
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+                if ((hw >> j) & 1u) {
+                    if (seen) put(g, acc);
+                    else front = acc;
+                    seen = true;
+                    g++;
+                    acc = id;
+                }
+                acc = agg_op<OP>(acc, x[lane * 33 + j]);
+            }
+            // fold of the rows since the last head, over the lanes
+            int32_t run = acc;
+            bool cut = seen;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int32_t t = __shfl_up_sync(QG_FULL_MASK, run, d);
+                const bool f = __shfl_up_sync(QG_FULL_MASK, (int)cut, d) != 0;
+                if (lane >= d && !cut) {
+                    run = agg_op<OP>(t, run);
+                    cut = f;
                 }
             }
-            pos = se;
-            g++;
+            const int32_t carry = __shfl_up_sync(QG_FULL_MASK, run, 1);
+            if (seen) {  // the group that the lane's first head ends
+                const int32_t v = lane ? agg_op<OP>(carry, front) : front;
+                const long long h0 = cs + lane * 32 + __ffs(hw) - 1;
+                if (heads_before > 0) put(gfirst, v);
+                else if (h0 > lo) part(gfirst, v);
+            }
+            if (lane == 31) {  // the chunk's last group
+                const long long gt = gl - ((long long)__ldg(&startPos[gl]) >= cs ? 1 : 0) + hb;
+                if (hb > 0 && group_end(gt) <= hi) put(gt, run);
+                else part(gt, run);
+            }
+        } else {  // empty groups among these: one group at a time
+            long long pos = lo;
+            for (long long g = gl; pos < hi && g < g1; g++) {
+                const long long gs = __ldg(&startPos[g]), ge = group_end(g), se = min(ge, hi);
+                int32_t acc = id;
+                for (long long i = pos + lane; i < se; i += 32) acc = agg_op<OP>(acc, x[(i - cs) + ((i - cs) >> 5)]);
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) acc = agg_op<OP>(acc, __shfl_xor_sync(QG_FULL_MASK, acc, d));
+                if (lane == 0) {
+                    if (pos == gs && se == ge && ge > gs) put(g, acc);
+                    else if (ge > gs) part(g, acc);
+                }
+                pos = max(pos, se);
+            }
         }
+        __syncwarp();
     }
 }
 
@@ -172,10 +306,9 @@ k_agg_chunks(const uint2 *__restrict__ rec, long long n, const int32_t *__restri
 __global__ void k_agg_avg_finish(const int32_t *__restrict__ startPos, long long n, long long G,
                                  long long g0, long long g1, int32_t *__restrict__ agg) {
     long long stride = (long long)gridDim.x * blockDim.x;
-    const long long rs = startPos[g0];
     for (long long g = g0 + (long long)blockIdx.x * blockDim.x + threadIdx.x; g < g1; g += stride) {
         long long gs = startPos[g], ge = (g == G - 1) ? n : startPos[g + 1];
-        bool spans = ((gs - rs) / AGG_CHUNK) != ((ge - 1 - rs) / AGG_CHUNK);
+        bool spans = ge > gs && gs / AGG_CHUNK != (ge - 1) / AGG_CHUNK;
         if (spans) agg[g] = agg[g] / (int32_t)(ge - gs);
     }
 }
@@ -1035,30 +1168,37 @@ extern "C" QG_API qg_status qg_groupby_rec(qg_ctx *ctx, const void *in, int64_t 
     if (n == 0) return QG_OK;
     char *tmp = nullptr;
     QG_TRY(qg_aux(ctx, (size_t)n * 8, &tmp));
-    qg_status s = QG_OK;
-    if (in != sorted_out)
-        QG_TRY_CUDA(ctx, cudaMemcpyAsync(sorted_out, in, (size_t)n * 8, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
-    s = qg_sort_rec_inplace(ctx, (unsigned long long *)sorted_out, (unsigned long long *)tmp, n);
-    if (s == QG_OK) {
-        constexpr int TILE = GBD_THREADS * GBD_ROUNDS * 2;
-        int64_t tiles = qg_ceil_div(n, TILE);
-        qg_lookback lb;
-        s = qg_lb_make(ctx, tiles, QG_SITE_GROUPBY, &lb);
-        if (s == QG_OK) {
-            long long *d_count = (long long *)&ctx->hres->count;
-            qg_pre_launch(ctx);
-            k_group_bounds<<<(unsigned)tiles, GBD_THREADS, 0, ctx->stream>>>(
-                (const uint4 *)sorted_out, n, startPos, cap_groups, d_count, lb);
-            s = qg_check_launch(ctx, "k_group_bounds");
-            long long h = 0;
-            if (s == QG_OK) s = qg_host_count(ctx, &h);
-            if (s == QG_OK) {
-                *num_groups = h;
-                if (h > cap_groups) s = QG_ERR_CAPACITY;
-            }
-        }
+    QG_TRY(qg_sort_rec(ctx, (const unsigned long long *)in, (unsigned long long *)sorted_out,
+                       (unsigned long long *)tmp, n));
+    const long long units = qg_ceil_div(n, GH_UNIT);
+    const long long warps =
+        std::max<long long>(GH_MIN_WARPS, std::min<long long>(GH_MAX_WARPS, qg_ceil_div(units, ctx->sm_count)));
+    const long long grid = std::min<long long>(qg_ceil_div(units, warps), ctx->sm_count);
+    const long long per_warp = qg_ceil_div(units, grid * warps);  // a warp's units, at most
+    uint8_t *spill = nullptr;
+    if (per_warp > GH_SUNITS) {
+        char *scr;
+        QG_TRY(qg_scratch(ctx, (size_t)units * 32, &scr));
+        spill = (uint8_t *)scr;
     }
-    return s;
+    const size_t smem = (size_t)warps * (GH_UNIT * 4 + std::min<long long>(per_warp, GH_SUNITS) * 32);
+    static bool attr = false;
+    if (!attr) {
+        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_group_bounds, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              GH_MAX_WARPS * (GH_UNIT * 4 + GH_SUNITS * 32)), "attr");
+        attr = true;
+    }
+    qg_lookback lb;
+    QG_TRY(qg_lb_make(ctx, grid, QG_SITE_GROUPBY, &lb));
+    qg_pre_launch(ctx);
+    k_group_bounds<<<(unsigned)grid, (unsigned)(32 * warps), smem, ctx->stream>>>(
+        (const uint2 *)sorted_out, n, units, startPos, cap_groups, (long long *)&ctx->hres->count, spill, lb);
+    QG_TRY(qg_check_launch(ctx, "k_group_bounds"));
+    long long h = 0;
+    QG_TRY(qg_host_count(ctx, &h));
+    if (in == sorted_out) qg_sort_remember(ctx);
+    *num_groups = h;
+    return h > cap_groups ? QG_ERR_CAPACITY : QG_OK;
 }
 
 extern "C" QG_API qg_status qg_aggregate_group_range(qg_ctx *ctx, const void *sorted, int64_t n,
@@ -1075,10 +1215,15 @@ extern "C" QG_API qg_status qg_aggregate_group_range(qg_ctx *ctx, const void *so
     k_agg_init<<<ib, 256, 0, ctx->stream>>>(agg, g0, g1, op);
     QG_TRY(qg_check_launch(ctx, "k_agg_init"));
     // The row range is only known on the device; size the grid for all rows.
-    long long chunks = (n + AGG_CHUNK - 1) / AGG_CHUNK;
-    int blocks = grid_for(ctx, chunks * 32, 256, 8);
+    const long long chunks = (n + AGG_CHUNK - 1) / AGG_CHUNK;
+    const int blocks = grid_for(ctx, chunks, AGG_WARPS, 6);
+    const bool vec = ((uintptr_t)sorted & 15) == 0;
+    auto kern = op == QG_REDUCE_MAX       ? (vec ? k_agg_chunks<QG_REDUCE_MAX, false, true> : k_agg_chunks<QG_REDUCE_MAX, false, false>)
+                : op == QG_REDUCE_MIN     ? (vec ? k_agg_chunks<QG_REDUCE_MIN, false, true> : k_agg_chunks<QG_REDUCE_MIN, false, false>)
+                : op == QG_REDUCE_AVERAGE ? (vec ? k_agg_chunks<QG_REDUCE_SUM, true, true> : k_agg_chunks<QG_REDUCE_SUM, true, false>)
+                                          : (vec ? k_agg_chunks<QG_REDUCE_SUM, false, true> : k_agg_chunks<QG_REDUCE_SUM, false, false>);
     qg_pre_launch(ctx);
-    k_agg_chunks<<<blocks, 256, 0, ctx->stream>>>((const uint2 *)sorted, n, startPos, G, g0, g1, op, agg);
+    kern<<<blocks, 32 * AGG_WARPS, 0, ctx->stream>>>((const uint2 *)sorted, n, startPos, G, g0, g1, agg);
     QG_TRY(qg_check_launch(ctx, "k_agg_chunks"));
     if (op == QG_REDUCE_AVERAGE) {
         qg_pre_launch(ctx);
@@ -1543,7 +1688,7 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
         // Global-table path (or a very large cap): sort (key, index) records,
         // then gather the sums and counts.
         unsigned long long *tmp = (unsigned long long *)(o.c + (cap > 0 ? cap : 1));
-        QG_TRY(qg_sort_rec_inplace(ctx, o.rec, tmp, g));
+        QG_TRY(qg_sort_rec(ctx, o.rec, o.rec, tmp, g));
         int gb = grid_for(ctx, g, 256, 8);
         qg_pre_launch(ctx);
         k_groupby_gather<<<gb, 256, 0, ctx->stream>>>(o.rec, g, o.s, o.c, gkey, (long long *)gsum,

@@ -19,6 +19,7 @@ struct qg_control {
     unsigned long long counter[6];  // scratch counters (output cursors)
     uint32_t gbd[48];               // per-call state of the dense-window group-by (qg_gbdense.cu)
     uint32_t ghist[4 * 256];        // digit counts of emitted group keys (group-by in key order)
+    uint32_t shist[4 * 256];        // a record sort's digit counts, zero between sorts
     // Address of the context's host error word (0: none), written with the
     // first error only: a call that met no error reads it after its
     // synchronisation instead of copying this block back.
@@ -32,6 +33,8 @@ struct qg_control {
 struct qg_hostres {
     volatile uint32_t err;         // first error code (qg_record_error), 0 = none
     volatile uint32_t aux;         // an operator's second result word
+    volatile uint32_t passes;      // passes of the last record sort
+    uint32_t pad;
     volatile long long count;      // an operator's row or group count
 };
 

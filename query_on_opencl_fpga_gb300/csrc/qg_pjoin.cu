@@ -1732,7 +1732,7 @@ qg_status pj_train(qg_ctx *ctx, const PjLevel &L, uint32_t nb, const unsigned lo
     qg_pre_launch(ctx);
     k_cdf_sample<<<pj_grid(ctx, m, 256, 4), 256, 0, ctx->stream>>>(r, nR, s, nS, mR, m, L.smp);
     QG_TRY(qg_check_launch(ctx, "k_cdf_sample"));
-    QG_TRY(qg_sort_rec_inplace(ctx, L.smp, L.smp2, m));
+    QG_TRY(qg_sort_rec(ctx, L.smp, L.smp, L.smp2, m));
     long long hthr = (3 * m + nb - 1) / nb;
     if (hthr < 2) hthr = 2;
     QG_TRY_CUDA(ctx, cudaMemsetAsync(L.heavy, 0, 4, ctx->stream), "memset heavy");
@@ -2052,8 +2052,8 @@ qg_status pj_core(qg_ctx *ctx, const PjLevel &L, PjPin *pin, uint32_t nb, int lb
         qg_pre_launch(ctx);
         k_pj_mj_gather<<<dim3(mgx, mgy), 256, 0, ctx->stream>>>(L.mj, (uint32_t)mj.size(), r, s, Rb, Sb);
         QG_TRY(qg_check_launch(ctx, "k_pj_mj_gather"));
-        QG_TRY(qg_sort_rec_inplace(ctx, Rb, Rt, nrb));
-        QG_TRY(qg_sort_rec_inplace(ctx, Sb, St, nsb));
+        QG_TRY(qg_sort_rec(ctx, Rb, Rb, Rt, nrb));
+        QG_TRY(qg_sort_rec(ctx, Sb, Sb, St, nsb));
         qg_pre_launch(ctx);
         k_pj_mj_count<<<dim3(mgx, mgy), 256, 0, ctx->stream>>>(L.mj, (uint32_t)mj.size(), Rb, Sb, mcnt, mlob,
                                                                L.bigcnt, L.mjtot);
@@ -2263,7 +2263,7 @@ extern "C" QG_API qg_status qg_part_learn(qg_ctx *ctx, const uint32_t *keys, int
     qg_pre_launch(ctx);
     k_keys_to_items<<<pj_grid(ctx, m, 256, 4), 256, 0, ctx->stream>>>(keys, n, m, smp);
     QG_TRY(qg_check_launch(ctx, "k_keys_to_items"));
-    QG_TRY(qg_sort_rec_inplace(ctx, smp, smp2, m));
+    QG_TRY(qg_sort_rec(ctx, smp, smp, smp2, m));
     long long hthr = (3 * m + nbuckets - 1) / nbuckets;
     if (hthr < 2) hthr = 2;
     QG_TRY_CUDA(ctx, cudaMemsetAsync(heavy, 0, 4, ctx->stream), "memset heavy");

@@ -22,10 +22,9 @@ struct qg_sort_bufs {
 // Number of 8-bit digit positions covering `bits` key bits (1..4).
 int qg_sort_positions(int bits);
 // Device histogram of (key - key_off) digits for `npos` positions into
-// d_hist[4][256]; for records, `copy` (if set) also receives a copy of them.
+// d_hist[4][256].
 qg_status qg_radix_histogram(qg_ctx *ctx, const qg_sort_bufs &src, bool kv3, long long n,
-                             uint32_t key_off, int npos, uint32_t *d_hist,
-                             unsigned long long *copy = nullptr);
+                             uint32_t key_off, int npos, uint32_t *d_hist);
 // From a host copy of the histogram: the non-trivial positions (returned
 // count) and every position's exclusive digit bases.
 int qg_sort_plan(const uint32_t *h_hist, int npos, long long n, int *passes, uint32_t *bases);
@@ -51,6 +50,10 @@ qg_status qg_radix_passes_dev(qg_ctx *ctx, bool kv3, qg_sort_bufs a, qg_sort_buf
                               const unsigned long long *d_n, const uint32_t *d_hist, int npos, uint32_t key_off,
                               char *work, bool *result_in_b);
 size_t qg_radix_dev_work_bytes(long long n_bound);
-// Sort REC items in place with `tmp` as the second buffer (synchronises once).
-qg_status qg_sort_rec_inplace(qg_ctx *ctx, unsigned long long *data, unsigned long long *tmp,
-                              long long n);
+// Sort REC items of `in` into `out` (may be `in`) with `tmp` as the second
+// buffer, planned on the device (no synchronisation, nothing read back).
+qg_status qg_sort_rec(qg_ctx *ctx, const unsigned long long *in, unsigned long long *out, unsigned long long *tmp,
+                      long long n);
+// After the stream of an in-place qg_sort_rec has been waited for: remember the
+// parity of its passes for the next one.
+void qg_sort_remember(qg_ctx *ctx);

@@ -471,3 +471,44 @@ def test_groupby_key_order_fresh_context_window(orc):
         _check_key_order_sequence(c, orc, ["dense", "dense", "low", "dense", "edge", "low", "low"], 10)
     finally:
         c.close()
+
+
+# Groups around the aggregation's chunks (1024 rows) and lanes (32 rows): heads
+# on and beside the edges, one-row groups, one group over several chunks, a
+# sub-range of groups, records that are only 8-byte aligned, empty groups.
+@pytest.mark.parametrize("op", [0, 1, 2, 3])
+@pytest.mark.parametrize("sizes", [[1] * 2100, [32] * 70, [33, 31] * 40, [1024, 1, 1023, 1024], [5000, 1, 1, 3000],
+                                   [1023, 2, 1023, 7], [300_000, 1]])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_aggregate_chunk_edges(ctx, orc, op, sizes, shift):
+    n = sum(sizes)
+    rng = np.random.default_rng(n + op)
+    rec = np.stack([rng.integers(-(2 ** 31), 2 ** 31, n), np.repeat(np.arange(len(sizes)), sizes)], 1).astype(np.int32)
+    sp = np.r_[0, np.cumsum(sizes)[:-1]].astype(np.int32)
+    exp = orc.aggregate_groups(rec, sp, op)
+    buf = torch.zeros((n + 1, 2), dtype=torch.int32, device="cuda")
+    buf[shift: n + shift] = dev(rec)
+    got = ctx.aggregate_groups(buf[shift: n + shift], dev(sp), op).cpu().numpy()
+    assert np.array_equal(got, exp)
+    g0, cnt = len(sizes) // 3, len(sizes) // 3 + 1
+    agg = torch.full((len(sizes),), -7, dtype=torch.int32, device="cuda")
+    st = ctx.lib.qg_aggregate_group_range(ctx.handle, buf[shift:].data_ptr(), n, dev(sp).data_ptr(), len(sizes), g0, cnt,
+                                          op, agg.data_ptr())
+    assert st == 0
+    out = agg.cpu().numpy()
+    assert np.array_equal(out[g0: g0 + cnt], exp[g0: g0 + cnt])
+    assert (out[:g0] == -7).all() and (out[g0 + cnt:] == -7).all()
+
+
+@pytest.mark.parametrize("op", [0, 1, 2])
+def test_aggregate_empty_groups(ctx, op):
+    n = 5000
+    x = np.arange(n, dtype=np.int32) - 2500
+    rec = np.stack([x, np.zeros(n, np.int32)], 1)
+    sp = np.array([0, 10, 10, 10, 1024, 1024, 3000], np.int32)
+    got = ctx.aggregate_groups(dev(rec), dev(sp), op).cpu().numpy()
+    ends = np.r_[sp[1:], n]
+    for g, (a, b) in enumerate(zip(sp, ends)):
+        v = x[a:b].astype(np.int64)
+        exp = v.sum() if op == 0 else max(0, v.max(initial=0)) if op == 1 else min(1 << 30, v.min(initial=1 << 30))
+        assert got[g] == exp, (g, got[g], exp)

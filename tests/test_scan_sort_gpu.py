@@ -108,3 +108,22 @@ def test_sort_ranking_modes_stable(ctx, mode):
         assert np.array_equal(got, rin[order])
     finally:
         assert ctx.lib.qg_sort_set_rank(-1) == 0
+
+
+# Tile edges (5120 records), and key masks whose digit positions give 0 to 4
+# passes: in place (twice, so that both parities are remembered) and into
+# another buffer.  Stable: equal keys keep their input order.
+@pytest.mark.parametrize("n", [2, 5119, 5120, 5121, 3 * 5120 + 1, 100_003])
+@pytest.mark.parametrize("mask", [0, 0xFF, 0xFF00FF, 0xFFFFFF, 0xFFFFFFFF])
+def test_sort_rec_tiles_and_passes(ctx, n, mask):
+    rng = np.random.default_rng(n ^ mask)
+    for _ in range(2):
+        y = (rng.integers(0, 2 ** 32, n, dtype=np.uint64) & np.uint64(mask)).astype(np.uint32)
+        rec = np.stack([np.arange(n, dtype=np.uint32), y], 1).view(np.int32)
+        exp = rec[np.argsort(y, kind="stable")]
+        d = dev(rec)
+        srt, start = ctx.groupby_rec(d)
+        assert np.array_equal(srt.cpu().numpy(), exp) and np.array_equal(d.cpu().numpy(), rec)
+        heads = np.flatnonzero(np.r_[True, exp[1:, 1] != exp[:-1, 1]])
+        assert np.array_equal(start.cpu().numpy(), heads)
+        assert np.array_equal(ctx.sort_rec(d).cpu().numpy(), exp)
