@@ -185,7 +185,9 @@ QG_API qg_status qg_scatter_rec(qg_ctx *ctx, const void *R, int64_t rLen, const 
  * filter_aggregation pipeline, kernel/filter_aggregation/
  * filter_aggregation_cu_op_dp.cl).  Outputs hold `cap` groups; order is
  * QG_ORDER_KEY (ascending unsigned key, the reference's sorted order) or
- * QG_ORDER_NONE.  By default the keys are first aggregated in a direct-indexed
+ * QG_ORDER_NONE.  By default up to 16384 rows are aggregated by one CTA in
+ * shared memory (key order either way).  Larger inputs, and small ones with
+ * too many distinct keys for that, are first aggregated in a direct-indexed
  * window of 2^22 keys placed on a sample's key range (output in key order
  * either way); when the sample spans more than 2^21 keys or any row's key
  * falls outside the window, the call runs the two-pass hash path instead.
@@ -226,7 +228,7 @@ QG_API qg_status qg_groupby_set_knobs(int mode, int hot_slots_log2, int partitio
  * captured into a graph).  Process-wide; results are identical. */
 QG_API qg_status qg_groupby_set_single_launch(int enable);
 /* Diagnostics of the context's last qg_groupby_cols call: out[0] = path
- * (0 two-pass, 1 global table, 2 dense window), out[1] = overflow flags
+ * (0 two-pass, 1 global table, 2 dense window or a small input's one launch), out[1] = overflow flags
  * (bit 0 spill bucket, bit 1 pass-2 table), out[2] = fullest spill bucket,
  * out[3] = bucket capacity (the last three 0 on the dense-window path). */
 QG_API qg_status qg_groupby_stats(qg_ctx *ctx, uint32_t *out4);

@@ -1617,6 +1617,18 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
     // found its keys too widely spread, then the device-planned sort (up to
     // 2^30 records).  Whatever neither placed is sorted after the host has
     // read the count.
+    if (gm == 0 && n > 0 && n <= QG_GBS_MAX_ROWS) {
+        QG_TRY(qg_gbs_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, &ctx->hres->count,
+                             &ctx->hres->aux));
+        QG_TRY(qg_host_count(ctx, &g));
+        if (ctx->hres->aux == 0) {
+            ctx->gb_stats[0] = 2u;
+            ctx->gb_stats[1] = ctx->gb_stats[2] = ctx->gb_stats[3] = 0;
+            *num_groups = g;
+            return g > cap ? QG_ERR_CAPACITY : QG_OK;
+        }
+        // more distinct keys than the small table takes: the general paths
+    }
     if (gm == 0 && !global && n > 0) {
         // Dense-window path: output in key order whatever `order` asks for;
         // its last kernel stores the group count and the rows outside the

@@ -512,3 +512,31 @@ def test_aggregate_empty_groups(ctx, op):
         v = x[a:b].astype(np.int64)
         exp = v.sum() if op == 0 else max(0, v.max(initial=0)) if op == 1 else min(1 << 30, v.min(initial=1 << 30))
         assert got[g] == exp, (g, got[g], exp)
+
+
+# The small form (one CTA): vector tails, the round that starts its checks for
+# too many distinct keys, its largest input and the next row, every row its own
+# key (the table is given up early or late), one key, the key that marks free
+# slots, values whose halves carry signs.
+@pytest.mark.parametrize("n", [1, 3, 1023, 4096, 8191, 8192, 8193, 12_289, 16_384, 16_385])
+@pytest.mark.parametrize("kind", ["own", "few", "one", "wide", "late"])
+@pytest.mark.parametrize("fused", [False, True])
+def test_groupby_small(ctx, orc, n, kind, fused):
+    rng = np.random.default_rng(n)
+    key = {"own": rng.permutation(n).astype(np.int64) * 261_001 - 2 ** 31, "few": rng.integers(-3, 60, n),
+           "one": np.full(n, -1), "wide": rng.choice(rng.integers(-(2 ** 31), 2 ** 31, 2500), n),
+           "late": np.where(np.arange(n) < 9000, np.arange(n) % 50, np.arange(n))}[kind].astype(np.int32)
+    val = rng.choice(np.array([-(2 ** 31), 2 ** 31 - 1, -1, 65535, 65536, 7]), n).astype(np.int32)
+    val2 = rng.integers(0, 1000, n).astype(np.int32) if fused else None
+    got = ctx.groupby_cols(dev(key), dev(val), dev(val2) if fused else None, 0, 499, cap=n)
+    check_groups(got, orc.groupby_cols(key, val, val2, 0, 499))
+
+
+def test_groupby_small_capacity(ctx):
+    from query_on_opencl_fpga_gb300 import QGError
+
+    key = torch.arange(3000, dtype=torch.int32, device="cuda")
+    with pytest.raises(QGError) as e:
+        ctx.groupby_cols(key, key, cap=2999)
+    assert e.value.status == 3
+    assert ctx.groupby_cols(key, key, cap=3000)[0].numel() == 3000
