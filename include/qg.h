@@ -243,10 +243,13 @@ QG_API qg_status qg_join_filter_sort(qg_ctx *ctx, const int32_t *rkey, const int
                                      int64_t nS, int32_t slo, int32_t shi, int32_t *out_key,
                                      int32_t *out_rpay, int32_t *out_spay, int64_t cap,
                                      int64_t *out_n);
-/* Join algorithm knobs (process-wide).  variant: 0 auto -- range
- * partitioning by radix over the key, switching to the learned CDF partition
- * function when radix leaves more than 2% of the rows in buckets too large
- * for shared memory and the model does better on the same counts; 1 radix
+/* Join algorithm knobs (process-wide).  variant: 0 auto -- with the other
+ * knobs at their defaults, a counting join when R's keys are unique over a
+ * dense span (at most 2 nR values) and S has up to 40M rows, the hash join (3)
+ * when R has up to 2^23 keys of no dense span; else range partitioning by
+ * radix over the key, switching to the learned CDF partition function when
+ * radix leaves more than 2% of the rows in buckets too large for shared memory
+ * and the model does better on the same counts; 1 radix
  * only; 2 learned only; 3 the global hash table + radix sort of the output.
  * buckets_log2: 0 = from the input size (about 2560 rows per bucket), else
  * 1..15.  bucket_s_max / bucket_r_max: rows of a bucket that the shared-memory
@@ -263,7 +266,7 @@ QG_API qg_status qg_join_set_knobs(int variant, int buckets_log2, uint32_t bucke
  * general path.  Results are identical. */
 QG_API qg_status qg_join_set_dense(int enable);
 /* Diagnostics of the context's last qg_join_filter_sort: out[0] path
- * (1 radix, 2 learned, 3 hash join + sort, 4 radix with the dense build side,
+ * (1 radix, 2 learned, 3 hash join + sort, 4 dense build side: counting or radix,
  * 0 nothing to join), out[1]
  * buckets, out[2] buckets handled outside the bucket kernel, out[3] their
  * rows, out[4] those of them with several keys (joined together by the

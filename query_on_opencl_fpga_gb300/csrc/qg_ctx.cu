@@ -291,6 +291,24 @@ qg_status qg_aux(qg_ctx *ctx, size_t bytes, char **out) {
     return QG_OK;
 }
 
+qg_status qg_spare(qg_ctx *ctx, size_t bytes, char **out) {
+    bytes = qg_align_up(bytes ? bytes : 256, 256);
+    if (bytes > ctx->pj_tmp_bytes) {
+        QG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "sync");
+        if (ctx->pj_tmp) cudaFree(ctx->pj_tmp);
+        ctx->pj_tmp = nullptr;
+        ctx->pj_tmp_bytes = 0;
+        if (cudaMalloc((void **)&ctx->pj_tmp, bytes + bytes / 4) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->pj_tmp = nullptr;
+            return QG_ERR_OOM;
+        }
+        ctx->pj_tmp_bytes = bytes + bytes / 4;
+    }
+    *out = ctx->pj_tmp;
+    return QG_OK;
+}
+
 qg_status qg_table(qg_ctx *ctx, size_t bytes, char **out) {
     bytes = qg_align_up(bytes ? bytes : 256, 256);
     if (bytes > ctx->table_bytes) {
@@ -348,6 +366,8 @@ static qg_status map_error(qg_ctx *ctx, const int32_t *h) {
     cudaMemsetAsync(&ctx->ctl->tile_ctr, 0, 2 * sizeof(uint32_t), ctx->stream);
     cudaMemsetAsync(ctx->ctl->gbd, 0, sizeof(ctx->ctl->gbd), ctx->stream);  // dense group-by state words
     cudaMemsetAsync(ctx->ctl->shist, 0, sizeof(ctx->ctl->shist), ctx->stream);
+    cudaMemsetAsync(ctx->ctl->jd, 0, sizeof(ctx->ctl->jd), ctx->stream);
+    cudaMemsetAsync(&ctx->ctl->jd_arrived, 0, sizeof(uint32_t), ctx->stream);
     cudaStreamSynchronize(ctx->stream);  // done before any later stream of this context runs
     ctx->table_dirty = true;
     snprintf(ctx->msg, sizeof(ctx->msg), "device error %d (%s) at site %d", h[0],

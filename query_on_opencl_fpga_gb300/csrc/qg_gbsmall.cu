@@ -15,6 +15,7 @@
 // with fewer groups) and larger inputs go there; keys of no window (hashed ids)
 // took 150 us through the two-pass path.
 #include <algorithm>
+#include "qg_cta_sort.cuh"
 #include "qg_internal.cuh"
 
 namespace {
@@ -22,7 +23,7 @@ namespace {
 constexpr int GS_THREADS = 1024;
 constexpr int GS_WARPS = GS_THREADS / 32;
 constexpr int GS_SLOTS = 8192;      // at most; a power of two
-constexpr int GS_ITEMS = GS_SLOTS / GS_THREADS;  // sorted keys per thread
+static_assert(GS_THREADS == QG_CS_THREADS && GS_SLOTS <= QG_CS_MAX, "the distinct keys are sorted by qg_cta_sort");
 constexpr uint32_t GS_PROBES = 32;  // slots looked at before the table counts as full
 // Distinct keys among the first 4096 rows, and among the rows of any later
 // round, above which the table is given up: it is likely to fill, and the
@@ -49,7 +50,7 @@ k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
                    reinterpret_cast<uint32_t *>(ord + slots) + 2 * pitch,
                    reinterpret_cast<uint32_t *>(ord + slots) + 3 * pitch};
     uint32_t(*whist)[256] = reinterpret_cast<uint32_t(*)[256]>(T.hi + pitch);  // [GS_WARPS] the sort's counters
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
     // the first vectors in flight while the table is cleared
     const int nv = n >> 2;
     const int4 *k4 = reinterpret_cast<const int4 *>(key), *v4 = reinterpret_cast<const int4 *>(val),
@@ -137,68 +138,7 @@ k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
     }
     __syncthreads();
     const uint32_t g = s_n, top = T.cnt[slots] ? 1u : 0u;  // key 0xffffffff comes last
-    // Stable LSD radix sort of the g keys, 8 bits a pass, each warp 256 of them;
-    // a digit that all keys share is skipped.  (A bitonic sort of 4096 keys
-    // took 40 us here, 78 dependent steps; this takes 8.)
-    const uint32_t warps = (g + 255) / 256;
-    const uint32_t lt = qg_lanemask_lt();
-    for (int shift = 32; shift < 64; shift += 8) {
-        unsigned long long it[GS_ITEMS];
-        uint32_t rank[GS_ITEMS];
-        if (warp < (int)warps) {
-            for (int i = lane; i < 256; i += 32) whist[warp][i] = 0;
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < GS_ITEMS; i++) {
-                const uint32_t at = warp * 256 + i * 32 + lane;
-                it[i] = at < g ? ord[at] : ~0ull;
-            }
-#pragma unroll
-            for (int i = 0; i < GS_ITEMS; i++) {
-                const bool valid = warp * 256 + i * 32 + lane < g;
-                const uint32_t d = (uint32_t)(it[i] >> shift) & 255u;
-                uint32_t peers = __ballot_sync(QG_FULL_MASK, valid);
-#pragma unroll
-                for (int b = 0; b < 8; b++) {
-                    const uint32_t bal = __ballot_sync(QG_FULL_MASK, (d >> b) & 1u);
-                    peers &= ((d >> b) & 1u) ? bal : ~bal;
-                }
-                rank[i] = valid ? whist[warp][d] + __popc(peers & lt) : 0u;
-                __syncwarp();
-                if (valid && lane == 31 - __clz(peers)) whist[warp][d] = rank[i] + 1u;
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        uint32_t tot = 0, inc = 0;
-        if (tid < 256) {
-            for (uint32_t w = 0; w < warps; w++) tot += whist[w][tid];
-            inc = tot;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t x = __shfl_up_sync(QG_FULL_MASK, inc, d);
-                if (lane >= d) inc += x;
-            }
-            if (lane == 31) s_dsum[warp] = inc;
-        }
-        if (__syncthreads_or(tid < 256 && tot == g)) continue;  // one digit value: in place already
-        if (tid < 256) {
-            uint32_t run = inc - tot;
-            for (int w = 0; w < warp; w++) run += s_dsum[w];
-            for (uint32_t w = 0; w < warps; w++) {
-                const uint32_t c = whist[w][tid];
-                whist[w][tid] = run;
-                run += c;
-            }
-        }
-        __syncthreads();
-        if (warp < (int)warps) {
-#pragma unroll
-            for (int i = 0; i < GS_ITEMS; i++)
-                if (warp * 256 + i * 32 + lane < g) ord[whist[warp][(uint32_t)(it[i] >> shift) & 255u] + rank[i]] = it[i];
-        }
-        __syncthreads();
-    }
+    qg_cta_sort(ord, whist, s_dsum, g);
     for (uint32_t r = tid; r < g + top && r < cap; r += GS_THREADS) {
         const uint32_t i = r < g ? (uint32_t)ord[r] : slots;
         gkey[r] = r < g ? (int32_t)(ord[r] >> 32) : -1;

@@ -20,6 +20,8 @@ struct qg_control {
     uint32_t gbd[48];               // per-call state of the dense-window group-by (qg_gbdense.cu)
     uint32_t ghist[4 * 256];        // digit counts of emitted group keys (group-by in key order)
     uint32_t shist[4 * 256];        // a record sort's digit counts, zero between sorts
+    uint32_t jd[12];                // state of the counting join (qg_jdirect.cu)
+    uint32_t jd_arrived, jd_pad;    // its scan's tiles that are done (wraps to zero)
     // Address of the context's host error word (0: none), written with the
     // first error only: a call that met no error reads it after its
     // synchronisation instead of copying this block back.
@@ -66,6 +68,7 @@ struct qg_ctx {
     uint32_t gb_kbase;      // first key of the next dense-order window (from the last call's keys)
     bool sort_odd_passes;   // the last in-place record sort took an odd number of passes
     uint32_t pj_stats[8];   // last qg_join_filter_sort (see qg_join_stats)
+    bool pj_sparse;         // the last join's R keys had no dense span: look before launching the counting path
     char *pj_tmp;           // the join's sort-merge arrays (grow-only)
     size_t pj_tmp_bytes;
     void *pin_join;         // host pinned bucket bounds and group plan of the join (allocated on first use)
@@ -141,6 +144,8 @@ void qg_steer_free(qg_ctx *ctx);
 qg_status qg_scratch(qg_ctx *ctx, size_t bytes, char **out);
 // Ensure the operator-temporary arena holds at least `bytes` (not zeroed).
 qg_status qg_aux(qg_ctx *ctx, size_t bytes, char **out);
+// Ensure the join's spare arena (pj_tmp) holds at least `bytes` (not zeroed).
+qg_status qg_spare(qg_ctx *ctx, size_t bytes, char **out);
 // Ensure the hash-table arena holds at least `bytes` of zeroed memory.
 qg_status qg_table(qg_ctx *ctx, size_t bytes, char **out);
 // Look-back descriptor for a single-pass kernel of `tiles` tiles.  Its status

@@ -1,0 +1,28 @@
+// qg_join.cuh -- the join paths that qg_join_filter_sort and batches share.
+#pragma once
+#include "qg_internal.cuh"
+
+// Dense build side by counting (qg_jdirect.cu): six launches on the context's
+// stream, no read back.  `work`: qg_jd_bytes(nR, nS) bytes, 256-byte aligned.
+// Afterwards ctl->jd[QG_JD_OK] (also *result, when set) is QG_JD_DONE when the
+// outputs hold the result, *d_count then the match count (the first cap rows
+// are written); else what stood against it, and the outputs hold nothing valid.
+enum { QG_JD_OK = 4 };
+enum qg_jd_result : uint32_t {
+    QG_JD_SPARSE = 0,  // R's keys spread over more than 2 nR values
+    QG_JD_DONE = 1,
+    QG_JD_OTHER = 2,   // dense span, but a build key twice or a probe key with too many rows
+};
+size_t qg_jd_bytes(int64_t nR, int64_t nS);
+qg_status qg_jd_launch(qg_ctx *ctx, char *work, const int32_t *rkey, const int32_t *rpay, int64_t nR,
+                       const int32_t *skey, const int32_t *spay, int64_t nS, int32_t slo, int32_t shi, uint32_t *out_key,
+                       uint32_t *out_rpay, uint32_t *out_spay, int64_t cap, long long *d_count, volatile uint32_t *result);
+
+// Hash join + sort of the matches (qg_join.cu).  most_probes > 0: give up
+// (*crowded) when a build row needs more slots than that, as it does where a
+// build key repeats often; nothing valid is written then.  *span: R's largest
+// key minus its smallest.
+qg_status qg_join_hash_sort(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpay, int64_t nR, const int32_t *skey,
+                            const int32_t *spay, int64_t nS, int32_t slo, int32_t shi, int32_t *out_key,
+                            int32_t *out_rpay, int32_t *out_spay, int64_t cap, int64_t *out_n, uint32_t most_probes = 0,
+                            bool *crowded = nullptr, uint32_t *span = nullptr);

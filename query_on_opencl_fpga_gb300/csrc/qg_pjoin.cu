@@ -49,6 +49,7 @@
 #include <string.h>
 #include <vector>
 #include "qg_internal.cuh"
+#include "qg_join.cuh"
 #include "qg_part.cuh"
 #include "qg_sort.cuh"
 
@@ -1564,11 +1565,6 @@ k_pj_minmax(const PjCross *__restrict__ list, uint32_t nlist, const unsigned lon
 // ===========================================================================
 // host
 // ===========================================================================
-qg_status qg_join_hash_sort(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpay, int64_t nR,
-                            const int32_t *skey, const int32_t *spay, int64_t nS, int32_t slo,
-                            int32_t shi, int32_t *out_key, int32_t *out_rpay, int32_t *out_spay,
-                            int64_t cap, int64_t *out_n);
-
 namespace {
 
 int g_pj_variant = 0;  // 0 auto (radix; learned when a key sample shows that it spreads the rows better), 1 radix, 2 learned, 3 hash join + sort
@@ -1655,25 +1651,6 @@ void pj_level_carve(char *p, uint32_t nb, bool learned, PjLevel *L) {
         L->smp = (unsigned long long *)take((size_t)CDF_SAMPLE * 8);
         L->smp2 = (unsigned long long *)take((size_t)CDF_SAMPLE * 8);
     }
-}
-
-// Grow-only device buffer of the context (the sort-merge arrays).
-qg_status pj_pool_get(qg_ctx *ctx, char **slot, size_t *slot_bytes, size_t bytes, char **out) {
-    bytes = qg_align_up(bytes ? bytes : 256, 256);
-    if (bytes > *slot_bytes) {
-        QG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "sync");
-        if (*slot) cudaFree(*slot);
-        *slot = nullptr;
-        *slot_bytes = 0;
-        if (cudaMalloc((void **)slot, bytes + bytes / 4) != cudaSuccess) {
-            cudaGetLastError();
-            *slot = nullptr;
-            return QG_ERR_OOM;
-        }
-        *slot_bytes = bytes + bytes / 4;
-    }
-    *out = *slot;
-    return QG_OK;
 }
 
 int g_pd_ctas_per_sm = 1;  // resident CTAs of k_pj_join_dense per SM
@@ -1892,7 +1869,7 @@ qg_status pj_core(qg_ctx *ctx, const PjLevel &L, PjPin *pin, uint32_t nb, int lb
     if (use_learned) {
         const size_t rb2 = qg_align_up((size_t)nR * 2, 256), sb2 = qg_align_up((size_t)nS * 2, 256);
         char *side;
-        QG_TRY(pj_pool_get(ctx, &ctx->pj_tmp, &ctx->pj_tmp_bytes, 2 * rb2 + 2 * sb2, &side));
+        QG_TRY(qg_spare(ctx, 2 * rb2 + 2 * sb2, &side));
         bidr[0] = (uint16_t *)side;
         bidr[1] = (uint16_t *)(side + rb2);
         bids[0] = (uint16_t *)(side + 2 * rb2);
@@ -2040,7 +2017,7 @@ qg_status pj_core(qg_ctx *ctx, const PjLevel &L, PjPin *pin, uint32_t nb, int lb
         const size_t rbb = qg_align_up((size_t)nrb * 8, 256), sbb = qg_align_up((size_t)nsb * 8, 256),
                      cb = qg_align_up((size_t)nsb * 4, 256);
         char *tmp;
-        QG_TRY(pj_pool_get(ctx, &ctx->pj_tmp, &ctx->pj_tmp_bytes, 2 * rbb + 2 * sbb + 3 * cb, &tmp));
+        QG_TRY(qg_spare(ctx, 2 * rbb + 2 * sbb + 3 * cb, &tmp));
         Rb = (unsigned long long *)tmp;
         unsigned long long *Rt = (unsigned long long *)(tmp + rbb);
         Sb = (unsigned long long *)(tmp + 2 * rbb);
@@ -2157,6 +2134,38 @@ extern "C" QG_API qg_status qg_join_filter_sort(qg_ctx *ctx, const int32_t *rkey
     return st;
 }
 
+// Largest S of the counting path (qg_jdirect.cu).  Both paths, R = S / 16, 24 %
+// of the rows joined: 4K rows 61 / 126 us, 1M 72 / 149, 16M 182 / 280, 32M 315 /
+// 380, 64M 608 / 583: from there the scattered accesses leave L2.
+constexpr int64_t PJ_DIRECT_S = 40'000'000;
+// Build rows of the hash join, whose table (16 to 32 bytes a row) stays in L2.
+// Against the partitioned path (radix, or learned where that spreads better),
+// skewed keys: 64K rows 92 / 156 us, 1M 107 / 415, 16M 303 / 925, 64M 910 /
+// 1665; random 32-bit keys: 1M 158 / 249, 16M 402 / 666, 64M 1316 / 1880.
+constexpr int64_t PJ_HASH_R = 1 << 23;
+// Slots a build row may look at: unique keys at load 1/2 need a few dozen.
+constexpr uint32_t PJ_HASH_PROBES = 256;
+
+// The counting path, waited for: pj_stats[0] = 4 and the output count when it
+// answered, else pj_sparse or *other says why not.
+static qg_status join_direct(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpay, int64_t nR, const int32_t *skey,
+                             const int32_t *spay, int64_t nS, int32_t slo, int32_t shi, int32_t *out_key,
+                             int32_t *out_rpay, int32_t *out_spay, int64_t cap, int64_t *out_n, bool *other) {
+    char *work;
+    QG_TRY(qg_aux(ctx, qg_jd_bytes(nR, nS), &work));
+    QG_TRY(qg_jd_launch(ctx, work, rkey, rpay, nR, skey, spay, nS, slo, shi, (uint32_t *)out_key, (uint32_t *)out_rpay,
+                        (uint32_t *)out_spay, cap, (long long *)&ctx->hres->count, &ctx->hres->aux));
+    long long M = 0;
+    QG_TRY(qg_host_count(ctx, &M));
+    ctx->pj_sparse = ctx->hres->aux == QG_JD_SPARSE;
+    *other = ctx->hres->aux == QG_JD_OTHER;
+    if (ctx->hres->aux == QG_JD_DONE) {
+        ctx->pj_stats[0] = 4;
+        *out_n = M;
+    }
+    return QG_OK;
+}
+
 static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpay, int64_t nR,
                                        const int32_t *skey, const int32_t *spay, int64_t nS, int32_t slo,
                                        int32_t shi, int32_t *out_key, int32_t *out_rpay, int32_t *out_spay,
@@ -2174,6 +2183,36 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     *out_n = 0;
     memset(ctx->pj_stats, 0, sizeof(ctx->pj_stats));
     if (nR == 0 || nS == 0) return QG_OK;
+    // With the default knobs: the counting path for small and middling inputs
+    // whose R keys are unique over a dense span, the hash join for R keys of no
+    // dense span.  Which of the two is launched first is what the context's last
+    // such call found; each sees R's span and hands over to the other.
+    const bool dflt = variant == 0 && g_pj_dense && g_pj_blog2 == 0 && g_pj_smax == PB_SMAX && g_pj_rmax == PB_RMAX;
+    if (dflt && nR <= PJ_HASH_R) {
+        const bool direct = nS <= PJ_DIRECT_S;
+        bool other = false;  // a dense span, but not for the counting path
+        if (direct && !ctx->pj_sparse) QG_TRY(join_direct(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key,
+                                                          out_rpay, out_spay, cap, out_n, &other));
+        if (ctx->pj_stats[0]) return *out_n > cap ? QG_ERR_CAPACITY : QG_OK;
+        if (ctx->pj_sparse && !other) {
+            bool crowded = false;
+            uint32_t span = 0;
+            const qg_status st = qg_join_hash_sort(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay,
+                                                   out_spay, cap, out_n, PJ_HASH_PROBES, &crowded, &span);
+            if (st != QG_OK && st != QG_ERR_CAPACITY) return st;
+            ctx->pj_sparse = crowded || (unsigned long long)span + 1ull > 2ull * (unsigned long long)nR;
+            if (!crowded && (ctx->pj_sparse || !direct)) {
+                ctx->pj_stats[0] = 3;
+                return st;
+            }
+            if (!ctx->pj_sparse) {  // dense after all
+                QG_TRY(join_direct(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay, out_spay, cap, out_n,
+                                   &other));
+                if (ctx->pj_stats[0]) return *out_n > cap ? QG_ERR_CAPACITY : QG_OK;
+            }
+        }
+        *out_n = 0;
+    }
     // aux: R records + spare (the spare doubles as the dense build side's
     // payload table), S' records + spare, the presence bitmap, level-0 arrays
     const size_t rb = qg_align_up((size_t)nR * 8, 256), sb = qg_align_up((size_t)nS * 8, 256);
@@ -2231,6 +2270,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
                pin->dflags[PJ_F_DENSE] != 0u && distinct == (unsigned long long)nR && g_pj_dense,
                pin->dflags[PJ_F_SENT_OK] != 0u, pin->dflags[PJ_F_SENT],
                bitmap, T};
+    if (dflt) ctx->pj_sparse = rs.rec_ready;
     long long M = 0;
     // pj_core ends with a read of the output count and the error word
     QG_TRY(pj_core(ctx, L, pin, nb, lb2, rs, R, Rsp, nR, S, Ssp, ns1, hr.kmin, hr.kmax, variant,

@@ -302,3 +302,84 @@ def test_join_dense_capacity_error(ctx, orc, full):
     assert ctx.join_stats()["path"] == "dense"
     assert all(int((o[small:] != 7).sum()) == 0 for o in out), "a row was written past cap"
     check_join(ctx.join_filter_sort(r, rp, s, sp, -(2 ** 31), 299), exp)
+
+
+def _join_case(ctx, orc, rkey, rpay, skey, spay, path, hi=299, extra=16):
+    exp = orc.join_filter_sort(rkey, rpay, skey, spay, -(2 ** 31), hi, cap=skey.size * extra, mt=True)
+    args = [dev(a) for a in (rkey, rpay, skey, spay)]
+    for _ in range(2):  # the second call knows what the first one found
+        check_join(ctx.join_filter_sort(*args, -(2 ** 31), hi, cap=max(len(exp[0]), 1)), exp)
+        assert ctx.join_stats()["path"] == path
+    return len(exp[0])
+
+
+# The counting path around its tiles (2 and 16 table entries per lane, 4096 probe
+# rows), spans of nR, 2 nR and 2 nR + 1 values, keys at the ends of the range,
+# build payloads of every value, a key with the most rows it takes and one more.
+@pytest.mark.parametrize("nR,nS,gap", [(1, 1, 1), (255, 4095, 1), (256, 4096, 2), (257, 4097, 1), (1 << 18, 9000, 1),
+                                       ((1 << 18) + 1, 50_001, 2), (5000, 300_003, 1)])
+@pytest.mark.parametrize("base", [0, -(2 ** 31), 2 ** 31 - 600_000])
+def test_join_counting_path_edges(ctx, orc, nR, nS, gap, base):
+    rng = np.random.default_rng(nR + nS)
+    off = rng.permutation(nR).astype(np.int64) * gap
+    if gap == 2:
+        off[np.argmax(off)] = 2 * nR - 1  # the widest dense span
+    rkey = (base + off).astype(np.int64)
+    rkey = ((rkey + 2 ** 31) % 2 ** 32 - 2 ** 31).astype(np.int32)
+    rpay = rng.choice(np.array([-(2 ** 31), 2 ** 31 - 1, -1, 0, 7]), nR).astype(np.int32)
+    skey = ((base + rng.integers(-3, nR * gap + 3, nS) + 2 ** 31) % 2 ** 32 - 2 ** 31).astype(np.int32)
+    spay = rng.integers(0, 1000, nS).astype(np.int32)
+    _join_case(ctx, orc, rkey, rpay, skey, spay, "dense")
+
+
+def test_join_counting_path_limits(ctx, orc):
+    rng = np.random.default_rng(3)
+    n = 1000
+    rpay = rng.integers(0, 1000, n).astype(np.int32)
+    rkey = rng.permutation(n).astype(np.int32)
+    skey = np.concatenate([rng.integers(0, n, 20_000), np.full(4000, n + 5)]).astype(np.int32)
+    spay = np.full(skey.size, 5, np.int32)
+    for rows, path in ((4096, "dense"), (4098, "radix")):  # rows of one key
+        s = np.concatenate([skey[skey != 77], np.full(rows, 77, np.int32)])
+        _join_case(ctx, orc, rkey, rpay, s, np.full(s.size, 5, np.int32), path)
+    wide = rkey.astype(np.int64) * 2
+    wide[np.argmax(wide)] = 2 * n  # one value too wide
+    _join_case(ctx, orc, wide.astype(np.int32), rpay, skey, spay, "hash_sort")
+    _join_case(ctx, orc, rkey, rpay, skey, spay, "dense")  # and back
+
+
+# The hash join behind the default: 8192 and 8193 matches (one-CTA sort), key
+# ranges of 1 to 4 digits, build keys twice, the key and payload that mark free
+# slots, no match at all.
+@pytest.mark.parametrize("bits", [14, 20, 27, 32])
+@pytest.mark.parametrize("m", [0, 1, 8192, 8193, 60_000])
+@pytest.mark.parametrize("twice", [False, True])
+def test_join_sparse_keys_take_the_hash_join(ctx, orc, bits, m, twice):
+    rng = np.random.default_rng(bits + m)
+    nR = 3000
+    keys = np.unique(np.concatenate([[0, 2 ** bits - 1], rng.integers(0, 2 ** bits, 2 * nR)]))[:nR].astype(np.int64)
+    keys[-1] = 2 ** bits - 1
+    gone = np.setdiff1d(rng.integers(0, 2 ** bits, 4000), keys)
+    rkey = np.concatenate([keys, keys[:50]]) if twice else keys
+    rpay = rng.integers(-5, 5, rkey.size).astype(np.int64)
+    rpay[keys.size - 1] = -1
+    hits = keys[rng.integers(50 if twice else 0, keys.size, m)]
+    if twice:
+        hits = np.concatenate([hits, keys[:50]])
+    skey = np.concatenate([hits, gone])
+    spay = np.zeros(skey.size, np.int64)
+    p = rng.permutation(skey.size)
+    as32 = lambda x: ((x + 2 ** 31) % 2 ** 32 - 2 ** 31).astype(np.int32)  # noqa: E731
+    got = _join_case(ctx, orc, as32(rkey), as32(rpay), as32(skey[p]), as32(spay[p]), "hash_sort")
+    assert got == m + (100 if twice else 0)
+
+
+def test_join_sparse_crowded_key_takes_general_path(ctx, orc):
+    # one build key 2000 times: more slots than a row may look at
+    rng = np.random.default_rng(8)
+    rkey = np.concatenate([rng.integers(-(2 ** 31), 2 ** 31, 5000), np.full(2000, 123)]).astype(np.int32)
+    rpay = rng.integers(0, 9, rkey.size).astype(np.int32)
+    skey = np.concatenate([rng.choice(rkey[:5000], 20_000), np.full(3, 123)]).astype(np.int32)
+    spay = rng.integers(0, 400, skey.size).astype(np.int32)
+    spay[-3:] = 1
+    _join_case(ctx, orc, rkey, rpay, skey, spay, "radix")
