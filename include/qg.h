@@ -330,7 +330,7 @@ QG_API qg_status qg_batch_check(qg_batch *b, void *stream);
 QG_API qg_status qg_batch_info(const qg_batch *b, int32_t *out4);
 QG_API qg_status qg_batch_destroy(qg_batch *b);
 /* Lanes of the batches created after this call (process-wide, 1..16; default
- * 8): the queries are spread over that many streams, each with a private
+ * 12): the queries are spread over that many streams, each with a private
  * context, and the graph runs the lanes side by side. */
 QG_API qg_status qg_batch_set_lanes(int lanes);
 /* Form of the batches created after this call (process-wide): 1

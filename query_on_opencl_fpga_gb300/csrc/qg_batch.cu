@@ -45,7 +45,9 @@ void qg_bpersist_destroy(qg_bpersist *p);
 // forks into the lanes and joins them, so that small queries run beside
 // large ones instead of one after another.
 constexpr int QG_BATCH_MAX_LANES = 16;
-static int g_batch_lanes = 8;
+// 4 / 8 / 12 / 16 lanes: 24 queries of 4K to 16M rows 713 / 797 / 676 / 670 us, 128
+// of 4K to 4M rows 1491 / 1316 / 1204 / 1261, 16 of 20K to 16M 249 / 227 / 188 / 207.
+static int g_batch_lanes = 12;
 // Measured on config 3 (512 mixed queries): lanes 18 ms, persistent 28 ms.
 // The persistent kernel's group-by tables are touched at about one random
 // sector per group, and Zipf keys over 1M groups give nearly as many groups
@@ -61,6 +63,7 @@ struct qg_batch {
     cudaStream_t stream = nullptr;  // == ls[0]
     std::vector<qg_query> q;
     std::vector<int> lane;  // lane of each query
+    std::vector<int> order; // the order in which the queries are enqueued
     cudaGraphExec_t exec = nullptr;
     int32_t info[4] = {0, 0, 0, 0};  // hot slots / group tile log2, table factor, best replay us, graph nodes
     bool persistent = false;
@@ -79,7 +82,8 @@ struct BatchCfg {
 qg_status enqueue(qg_batch *b, const BatchCfg &c, qg_bpersist *bp) {
     qg_status st = QG_OK;
     if (b->persistent && bp) st = qg_bpersist_launch(b->own[0], bp);
-    for (size_t i = 0; i < b->q.size() && st == QG_OK; i++) {
+    for (size_t o = 0; o < b->q.size() && st == QG_OK; o++) {
+        const size_t i = (size_t)b->order[o];
         const qg_query &q = b->q[i];
         if (b->persistent && q.op != QG_OP_JOIN) continue;  // in the persistent kernel
         qg_ctx *ctx = b->own[b->lane[i]];
@@ -201,14 +205,21 @@ QG_API qg_status qg_batch_create(const qg_query *queries, int nq, int autotune, 
     b->persistent = g_batch_persistent != 0;
     for (int i = 0; i < nq && b->persistent; i++)
         if (b->q[i].op != QG_OP_JOIN) b->pq.push_back(i);
-    // Largest queries first, each to the lane with the fewest rows so far
+    // Longest queries first, each to the lane with the least work so far
     // (persistent form: lane 0 runs the persistent kernel, the joins share
     // the other lanes).
     {
         std::vector<int> order;
         for (int i = 0; i < nq; i++)
             if (!b->persistent || b->q[i].op == QG_OP_JOIN) order.push_back(i);
-        auto rows = [&](int i) { return b->q[i].n + (b->q[i].op == QG_OP_JOIN ? b->q[i].n2 : 0); };
+        // a query's time alone, in ns (measured, 4K to 16M rows): its launches and its rows
+        auto rows = [&](int i) -> long long {
+            const qg_query &q = b->q[i];
+            return q.op == QG_OP_FILTER ? 6000 + 2 * q.n
+                 : q.op == QG_OP_JOIN   ? 45000 + 13 * (q.n + q.n2)
+                 : q.n < 8192           ? 10000
+                                        : 20000 + 4 * q.n;
+        };
         std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return rows(x) > rows(y); });
         const int first = b->persistent && b->lanes > 1 ? 1 : 0;
         std::vector<long long> load(b->lanes, 0);
@@ -220,6 +231,12 @@ QG_API qg_status qg_batch_create(const qg_query *queries, int nq, int autotune, 
             b->lane[i] = best;
             load[best] += rows(i);
         }
+        // Shortest first in every lane: the lanes' long queries then overlap
+        // (24 mixed queries on 8 / 12 lanes: longest first 851 / 711 us,
+        // shortest first 783 / 673, as listed 798 / 676).
+        b->order.assign(order.rbegin(), order.rend());
+        for (int i = 0; i < nq; i++)
+            if (b->persistent && b->q[i].op != QG_OP_JOIN) b->order.push_back(i);
     }
     // Lanes: a group-by query on the default variant (dense window first) is
     // run once on the dense-window path; when every row fell in the window the
@@ -356,7 +373,7 @@ QG_API qg_status qg_batch_set_persistent(int on) {
     return QG_OK;
 }
 
-// Lanes of the batches created after this call (1..16; default 8).
+// Lanes of the batches created after this call (1..16; default 12).
 QG_API qg_status qg_batch_set_lanes(int lanes) {
     if (lanes < 1 || lanes > QG_BATCH_MAX_LANES) return QG_ERR_INVALID;
     g_batch_lanes = lanes;

@@ -42,6 +42,8 @@ __global__ void __launch_bounds__(GS_THREADS, 1)
 k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, const int32_t *__restrict__ val2,
            int32_t lo2, int32_t hi2, int n, uint32_t slots, int32_t *__restrict__ gkey, long long *__restrict__ gsum,
            long long *__restrict__ gcnt, long long cap, volatile long long *d_num, volatile uint32_t *full) {
+    // with more slots than rows a row always finds its slot
+    const uint32_t probes = (uint32_t)n < slots ? slots : GS_PROBES;
     extern __shared__ __align__(16) unsigned char gs_raw[];
     __shared__ uint32_t s_full, s_n, s_dsum[8];  // s_n: distinct keys of the whole rounds, then of the table
     unsigned long long *ord = reinterpret_cast<unsigned long long *>(gs_raw);  // [slots] key << 32 | slot
@@ -80,7 +82,7 @@ k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
                     fresh += cur == GS_FREE;
                     if (cur == GS_FREE || cur == k) break;
                 }
-                if (p == GS_PROBES) {
+                if (p == probes) {
                     s_full = 1;
                     return;
                 }
@@ -122,7 +124,7 @@ k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
     }
     __syncthreads();
     if (s_full) {
-        if (tid == 0) *full = 1;
+        if (tid == 0 && full) *full = 1;
         return;
     }
     __syncthreads();
@@ -147,7 +149,7 @@ k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
     }
     if (tid == 0) {
         *d_num = g + top;
-        *full = 0;
+        if (full) *full = 0;
     }
 }
 
@@ -155,11 +157,13 @@ k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
 
 // Launches the small form (1 <= n <= QG_GBS_MAX_ROWS) on the context's stream;
 // after the stream is synchronised *full tells whether the table filled up
-// (nothing valid was written), else *d_num holds the group count.
+// (nothing valid was written; never below QG_GBS_SURE_ROWS rows, where full may
+// be null), else *d_num holds the group count.
 qg_status qg_gbs_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, const int32_t *val2, int32_t lo2,
                         int32_t hi2, int64_t n, int32_t *gkey, int64_t *gsum, int64_t *gcnt, int64_t cap,
                         volatile long long *d_num, volatile uint32_t *full) {
     static_assert(QG_GBS_MAX_ROWS <= 65536, "the sums' words");
+    static_assert(QG_GBS_SURE_ROWS <= GS_SLOTS, "more slots than rows, and no checked round");
     uint32_t slots = 1024;
     while (slots < GS_SLOTS && slots < 2 * (uint32_t)n) slots <<= 1;
     auto bytes = [](uint32_t s) { return (size_t)s * 8 + 4 * (s + 4) * 4 + (size_t)std::min<uint32_t>(GS_WARPS, s / 256) * 1024; };

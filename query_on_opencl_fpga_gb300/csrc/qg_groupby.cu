@@ -1518,6 +1518,8 @@ extern "C" QG_API qg_status qg_groupby_cols_async(qg_ctx *ctx, const int32_t *ke
     if (order == QG_ORDER_KEY && (gb_mode(ctx) == 1 || cap >= (1LL << 30))) return QG_ERR_UNSUPPORTED;
     if ((((uintptr_t)key) | ((uintptr_t)val) | ((uintptr_t)val2)) & 15) return QG_ERR_INVALID;
     if (n >= (1LL << 32)) return QG_ERR_UNSUPPORTED;
+    if (gb_mode(ctx) == 0 && n > 0 && n < QG_GBS_SURE_ROWS)  // one launch, key order either way
+        return qg_gbs_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, (long long *)d_num, nullptr);
     GbOut o;
     QG_TRY(gb_outputs(ctx, gkey, gsum, gcnt, cap, order, &o));
     if (gb_mode(ctx) == 1)
@@ -1548,7 +1550,7 @@ qg_status qg_groupby_dense_async(qg_ctx *ctx, const int32_t *key, const int32_t 
                                  int64_t cap, int64_t *d_num) {
     if (!ctx || n < 0 || cap < 0 || !d_num || (n > 0 && (!key || !val))) return QG_ERR_INVALID;
     if ((((uintptr_t)key) | ((uintptr_t)val) | ((uintptr_t)val2)) & 15) return QG_ERR_INVALID;
-    if (n == 0 || n >= (1LL << 32))
+    if (n < QG_GBS_SURE_ROWS || n >= (1LL << 32))
         return qg_groupby_cols_async(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, QG_ORDER_NONE, d_num);
     QG_TRY(qg_gbd_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, (long long *)d_num, nullptr));
     qg_pre_launch(ctx);

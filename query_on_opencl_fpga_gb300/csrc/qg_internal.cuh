@@ -107,7 +107,7 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
                         int64_t cap, long long *d_num, volatile uint32_t *outside);
 enum { QG_GBD_OUTSIDE = 6 };
 // Small column group-by in one launch (qg_gbsmall.cu).
-constexpr int64_t QG_GBS_MAX_ROWS = 16384;
+constexpr int64_t QG_GBS_MAX_ROWS = 16384, QG_GBS_SURE_ROWS = 8192;
 qg_status qg_gbs_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, const int32_t *val2, int32_t lo2,
                         int32_t hi2, int64_t n, int32_t *gkey, int64_t *gsum, int64_t *gcnt, int64_t cap,
                         volatile long long *d_num, volatile uint32_t *full);

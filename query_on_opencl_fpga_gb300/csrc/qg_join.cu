@@ -41,6 +41,7 @@ struct JoinCtl {
     unsigned long long sortn;      // rows the device-planned sort orders (0 when over capacity)
     uint32_t crowded;              // 1: a build row met more slots than it may
     uint32_t twice;                // 1: some build key occurs more than once
+    qg_sort_range range;           // the device-planned sort's positions and key offset
     uint32_t hist[4][QG_RADIX];
 };
 
@@ -151,12 +152,13 @@ struct ProbeOut {
 // where they lay and emitting step by step left two thirds of the lanes idle
 // behind votes, one row's slots at a time: 16M rows on a 1M-row table 494 us,
 // 115 now; 190 with the slots walked one by one.
-// The sort digits of (key - key_off) are counted (npos positions; key_off is
-// R's smallest key when from_kmin).
+// The sort digits of key - (R's smallest key) are counted (npos positions).
+// odd: where the matches go instead when that key range has an odd number of
+// digits (unless null).
 __global__ void __launch_bounds__(PJ_THREADS, 4)
 k_join_probe(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, long long nS,
              int32_t slo, int32_t shi, const unsigned long long *__restrict__ tab, uint32_t mask,
-             JoinCtl *jc, ProbeOut out, long long cap, bool from_kmin, int npos) {
+             JoinCtl *jc, ProbeOut out, ProbeOut odd, long long cap, int npos) {
     extern __shared__ __align__(16) unsigned char pj_raw[];
     PjSmem &S = *reinterpret_cast<PjSmem *>(pj_raw);
     if (jc->crowded) return;
@@ -165,7 +167,9 @@ k_join_probe(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay,
     const long long ntiles = (nS + PJ_TILE - 1) / PJ_TILE;
     const unsigned long long nspec = jc->n_special;
     const uint32_t kmin = jc->kmin, kspan = jc->kmax - kmin;  // rows outside cannot match
-    const uint32_t key_off = from_kmin ? kmin : 0u;
+    const uint32_t key_off = kmin;
+    // a sort of an odd number of positions starts from the other columns
+    if (odd.k && (qg_sort_npos(kmin, jc->kmax) & 1u)) out = odd;
     const bool once = jc->twice == 0 && nspec == 0;
     for (int i = tid; i < 4 * QG_RADIX; i += PJ_THREADS) (&S.hist[0][0])[i] = 0;
     if (tid < 2) S.cnt[tid] = 0;
@@ -411,6 +415,7 @@ namespace {
 // sort run only when the output fits.
 __global__ void k_join_finish_async(JoinCtl *jc, long long cap, unsigned long long *d_count, qg_control *ctl) {
     const unsigned long long m = jc->cursor;
+    jc->range = qg_sort_range{qg_sort_npos(jc->kmin, jc->kmax), jc->kmin};
     *d_count = m;
     if (m > (unsigned long long)cap) {
         jc->sortn = 0;
@@ -474,8 +479,8 @@ k_join_sort_small(qg_sort_bufs in, qg_sort_bufs out, uint32_t n) {
 
 // Launch of k_join_probe.
 static qg_status join_probe(qg_ctx *ctx, const int32_t *skey, const int32_t *spay, int64_t nS, int32_t slo, int32_t shi,
-                            const unsigned long long *tab, uint32_t mask, JoinCtl *jc, const ProbeOut &po, int64_t cap,
-                            bool from_kmin) {
+                            const unsigned long long *tab, uint32_t mask, JoinCtl *jc, const ProbeOut &po,
+                            const ProbeOut &odd, int64_t cap) {
     const size_t smem = sizeof(PjSmem);
     static bool attr = false;
     if (!attr) {
@@ -485,7 +490,7 @@ static qg_status join_probe(qg_ctx *ctx, const int32_t *skey, const int32_t *spa
     const long long ntiles = (nS + PJ_TILE - 1) / PJ_TILE;
     const int blocks = (int)(ntiles < (long long)ctx->sm_count * 4 ? ntiles : (long long)ctx->sm_count * 4);
     qg_pre_launch(ctx);
-    k_join_probe<<<blocks, PJ_THREADS, smem, ctx->stream>>>(skey, spay, nS, slo, shi, tab, mask, jc, po, cap, from_kmin, 4);
+    k_join_probe<<<blocks, PJ_THREADS, smem, ctx->stream>>>(skey, spay, nS, slo, shi, tab, mask, jc, po, odd, cap, 4);
     return qg_check_launch(ctx, "k_join_probe");
 }
 
@@ -512,7 +517,7 @@ qg_status qg_join_hash_sort(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpa
     QG_TRY(join_build(ctx, rkey, rpay, 1, nR, 3 * colbytes, most_probes, &tab, &mask, &jc, &tail));
     qg_sort_bufs A{nullptr, (uint32_t *)tail, (uint32_t *)(tail + colbytes), (uint32_t *)(tail + 2 * colbytes)};
     const qg_sort_bufs B{nullptr, (uint32_t *)out_key, (uint32_t *)out_rpay, (uint32_t *)out_spay};
-    QG_TRY(join_probe(ctx, skey, spay, nS, slo, shi, tab, mask, jc, ProbeOut{A.k, A.a, A.b}, cap, true));
+    QG_TRY(join_probe(ctx, skey, spay, nS, slo, shi, tab, mask, jc, ProbeOut{A.k, A.a, A.b}, ProbeOut{}, cap));
     JoinCtl *hjc = reinterpret_cast<JoinCtl *>(ctx->pin_ctl);
     static_assert(sizeof(JoinCtl) <= sizeof(qg_control), "read back into the pinned control block");
     QG_TRY_CUDA(ctx, cudaMemcpyAsync(hjc, jc, sizeof(JoinCtl), cudaMemcpyDeviceToHost, ctx->stream), "ctl d2h");
@@ -568,8 +573,8 @@ qg_status qg_join_hash_sort(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpa
 }
 
 // The hash join + filter + sort with no host round trip (for CUDA graph
-// capture, e.g. by qg_batch): the sort always takes all four key digits and
-// is planned on the device from the probe's digit counts.  d_count (device
+// capture, e.g. by qg_batch): the sort is planned on the device from the build's
+// key range and the probe's digit counts.  d_count (device
 // int64) receives the match count; more matches than cap records
 // QG_ERR_CAPACITY in the context's error word and leaves the output unsorted.
 qg_status qg_join_hash_sort_async(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpay, int64_t nR,
@@ -595,14 +600,12 @@ qg_status qg_join_hash_sort_async(qg_ctx *ctx, const int32_t *rkey, const int32_
     QG_TRY(join_build(ctx, rkey, rpay, 1, nR, 3 * colbytes + work, 0u, &tab, &mask, &jc, &tail));
     qg_sort_bufs A{nullptr, (uint32_t *)out_key, (uint32_t *)out_rpay, (uint32_t *)out_spay};
     qg_sort_bufs B{nullptr, (uint32_t *)tail, (uint32_t *)(tail + colbytes), (uint32_t *)(tail + 2 * colbytes)};
-    QG_TRY(join_probe(ctx, skey, spay, nS, slo, shi, tab, mask, jc, ProbeOut{A.k, A.a, A.b}, cap, false));
+    QG_TRY(join_probe(ctx, skey, spay, nS, slo, shi, tab, mask, jc, ProbeOut{A.k, A.a, A.b}, ProbeOut{B.k, B.a, B.b},
+                      cap));
     qg_pre_launch(ctx);
     k_join_finish_async<<<1, 1, 0, ctx->stream>>>(jc, cap, (unsigned long long *)d_count, ctx->ctl);
     QG_TRY(qg_check_launch(ctx, "k_join_finish_async"));
-    bool in_b = false;
-    QG_TRY(qg_radix_passes_dev(ctx, true, A, B, cap, &jc->sortn, &jc->hist[0][0], 4, 0u,
-                               tail + 3 * colbytes, &in_b));
-    return in_b ? QG_ERR_INVALID : QG_OK;  // four passes end where they began
+    return qg_radix_passes_range(ctx, A, B, cap, &jc->sortn, &jc->hist[0][0], &jc->range, tail + 3 * colbytes);
 }
 
 // ---------------------------------------------------------------------------

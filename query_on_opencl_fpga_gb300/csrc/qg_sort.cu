@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS)
 k_radix_pass(qg_sort_bufs src, qg_sort_bufs dst, long long n, int shift, uint32_t key_off,
              const uint32_t *__restrict__ dbase, uint32_t *__restrict__ status, qg_control *ctl, uint32_t spin_limit,
              const unsigned long long *__restrict__ d_n, const uint32_t *__restrict__ trivial,
-             const RsPass *__restrict__ plan) {
+             const RsPass *__restrict__ plan, const qg_sort_range *__restrict__ range) {
     extern __shared__ __align__(16) unsigned char rs_raw[];
     static_assert(!(KV3 && SIDE), "no sidecar with three columns");
     RsSmem<KV3, SIDE> &S = *reinterpret_cast<RsSmem<KV3, SIDE> *>(rs_raw);
@@ -404,6 +404,16 @@ k_radix_pass(qg_sort_bufs src, qg_sort_bufs dst, long long n, int shift, uint32_
         dst.rec = plan->dst;
         status = plan->status;
         if (plan->clear) plan->clear[(size_t)blockIdx.x * QG_RADIX + threadIdx.x] = 0;
+    }
+    if (range) {  // three columns: the pass runs or not, and reads a or b, by the key range's positions
+        const int left = (int)range->npos - shift / 8;
+        if (left <= 0) return;
+        key_off = range->key_off;
+        if (left & 1) {
+            const qg_sort_bufs t = src;
+            src = dst;
+            dst = t;
+        }
     }
     if (copy) {  // one digit value holds every item: a stable pass is the identity
         rs_copy_tile<KV3, SIDE>(src, dst, n);
@@ -458,7 +468,8 @@ int qg_sort_plan(const uint32_t *h_hist, int npos, long long n, int *passes, uin
 }
 
 using rs_kernel = void (*)(qg_sort_bufs, qg_sort_bufs, long long, int, uint32_t, const uint32_t *, uint32_t *,
-                           qg_control *, uint32_t, const unsigned long long *, const uint32_t *, const RsPass *);
+                           qg_control *, uint32_t, const unsigned long long *, const uint32_t *, const RsPass *,
+                           const qg_sort_range *);
 
 // The pass kernel of a ranking form (see k_radix_pass); form 2 for records only.
 template <bool KV3, bool SIDE>
@@ -548,7 +559,7 @@ qg_status qg_radix_passes_pf(qg_ctx *ctx, bool kv3, qg_sort_bufs a, qg_sort_bufs
         qg_pre_launch(ctx);
         kern<<<(unsigned)tiles, RS_THREADS, smem, ctx->stream>>>(s, d, n, shift, side ? 0u : pf.kmin,
                                                                  dbase + p * QG_RADIX, status, ctx->ctl, ctx->spin_limit,
-                                                                 nullptr, nullptr, nullptr);
+                                                                 nullptr, nullptr, nullptr, nullptr);
         QG_TRY(qg_check_launch(ctx, "k_radix_pass"));
         in_a = !in_a;
     }
@@ -617,11 +628,37 @@ qg_status qg_radix_passes_dev(qg_ctx *ctx, bool kv3, qg_sort_bufs a, qg_sort_buf
         qg_pre_launch(ctx);
         const rs_kernel kern = kv3 ? rs_pick<true, false>(3) : rs_pick<false, false>(3);
         kern<<<(unsigned)tiles, RS_THREADS, smem, ctx->stream>>>(s, d, n_bound, 8 * p, key_off, dbase + p * QG_RADIX, stp,
-                                                                 ctx->ctl, ctx->spin_limit, d_n, trivial + p, nullptr);
+                                                                 ctx->ctl, ctx->spin_limit, d_n, trivial + p, nullptr, nullptr);
         QG_TRY(qg_check_launch(ctx, "k_radix_pass"));
         in_a = !in_a;
     }
     *result_in_b = !in_a;
+    return QG_OK;
+}
+
+qg_status qg_radix_passes_range(qg_ctx *ctx, qg_sort_bufs a, qg_sort_bufs b, long long n_bound,
+                                const unsigned long long *d_n, const uint32_t *d_hist, const qg_sort_range *range,
+                                char *work) {
+    if (n_bound <= 1) return QG_OK;
+    if (n_bound >= (1LL << 30)) return QG_ERR_UNSUPPORTED;
+    const long long tiles = (n_bound + RS_TILE - 1) / RS_TILE;
+    uint32_t *dbase = (uint32_t *)work;
+    uint32_t *trivial = dbase + 4 * QG_RADIX;  // (not used: a pass whose digits are all equal is an ordinary one)
+    uint32_t *status = trivial + 64;           // [4][tiles][256]
+    const size_t st_words = (size_t)tiles * QG_RADIX;
+    QG_TRY((rs_set_attr<true, false>(ctx)));
+    qg_pre_launch(ctx);
+    k_radix_bases<<<1, QG_RADIX, 0, ctx->stream>>>(d_hist, 4, dbase, trivial);
+    QG_TRY(qg_check_launch(ctx, "k_radix_bases"));
+    QG_TRY_CUDA(ctx, cudaMemsetAsync(status, 0, 4 * st_words * 4, ctx->stream), "memset status");
+    const rs_kernel kern = rs_pick<true, false>(3);
+    for (int p = 0; p < 4; p++) {
+        qg_pre_launch(ctx);
+        kern<<<(unsigned)tiles, RS_THREADS, sizeof(RsSmem<true>), ctx->stream>>>(
+            a, b, n_bound, 8 * p, 0u, dbase + p * QG_RADIX, status + (size_t)p * st_words, ctx->ctl, ctx->spin_limit, d_n,
+            nullptr, nullptr, range);
+        QG_TRY(qg_check_launch(ctx, "k_radix_pass"));
+    }
     return QG_OK;
 }
 
@@ -738,7 +775,7 @@ qg_status qg_sort_rec(qg_ctx *ctx, const unsigned long long *in, unsigned long l
         qg_pre_launch(ctx);
         kern<<<(unsigned)tiles, RS_THREADS, sizeof(RsSmem<false>), ctx->stream>>>(
             qg_sort_bufs{}, qg_sort_bufs{}, n, 8 * p, 0u, plan->base + (p & 3) * QG_RADIX, nullptr, ctx->ctl,
-            ctx->spin_limit, nullptr, nullptr, &plan->pass[p]);
+            ctx->spin_limit, nullptr, nullptr, &plan->pass[p], nullptr);
         QG_TRY(qg_check_launch(ctx, "k_radix_pass"));
     }
     return QG_OK;

@@ -49,6 +49,19 @@ qg_status qg_radix_passes_pf(qg_ctx *ctx, bool kv3, qg_sort_bufs a, qg_sort_bufs
 qg_status qg_radix_passes_dev(qg_ctx *ctx, bool kv3, qg_sort_bufs a, qg_sort_bufs b, long long n_bound,
                               const unsigned long long *d_n, const uint32_t *d_hist, int npos, uint32_t key_off,
                               char *work, bool *result_in_b);
+// Three columns whose key range is known on the device only: `range` says how
+// many positions the keys (minus its key_off) have and thereby where the items
+// start, so that they end in `a`: in `b` for an odd number, else in `a`.
+struct qg_sort_range {
+    uint32_t npos, key_off;
+};
+__host__ __device__ inline uint32_t qg_sort_npos(uint32_t kmin, uint32_t kmax) {
+    const uint32_t r = kmax - kmin;
+    return (uint32_t)(r != 0) + (r >> 8 != 0) + (r >> 16 != 0) + (r >> 24 != 0);
+}
+qg_status qg_radix_passes_range(qg_ctx *ctx, qg_sort_bufs a, qg_sort_bufs b, long long n_bound,
+                                const unsigned long long *d_n, const uint32_t *d_hist, const qg_sort_range *range,
+                                char *work);
 size_t qg_radix_dev_work_bytes(long long n_bound);
 // Sort REC items of `in` into `out` (may be `in`) with `tmp` as the second
 // buffer, planned on the device (no synchronisation, nothing read back).
