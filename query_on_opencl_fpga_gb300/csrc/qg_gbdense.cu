@@ -64,6 +64,7 @@ namespace {
 
 constexpr int GBD_WLOG2 = 22;
 constexpr uint32_t GBD_W = 1u << GBD_WLOG2;       // window keys (dense table entries)
+static_assert(GBD_W == QG_GBD_WINDOW, "the window");
 constexpr int GBD_SLOG2 = 14;
 constexpr int GBD_S = 1 << GBD_SLOG2;             // heavy-key slots (direct-mapped)
 constexpr int GBD_TLOG2 = 19;                     // counters per row of the sample's count sketch
@@ -842,6 +843,13 @@ k_gbd_single(const int32_t *__restrict__ key, const int32_t *__restrict__ val, c
 
 }  // namespace
 
+qg_status qg_gbd_range(qg_ctx *ctx, const int32_t *key, int64_t n) {
+    const unsigned grid = (unsigned)std::min<long long>(qg_ceil_div(n, 4 * 256), 4LL * ctx->sm_count);
+    qg_pre_launch(ctx);
+    k_gbd_range<<<grid, 256, 0, ctx->stream>>>(key, n, ctx->ctl->gbd);
+    return qg_check_launch(ctx, "k_gbd_range");
+}
+
 static int g_gbd_single = 0;  // 1: the four steps in one cooperative launch where it fits
 
 extern "C" QG_API qg_status qg_groupby_set_single_launch(int enable) {
@@ -939,10 +947,7 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
         }
     }
     if (n > 0 && n <= GBM_MAX_ROWS) {
-        const unsigned rg = (unsigned)std::min<long long>(qg_ceil_div(n, 4 * 256), 4LL * C);
-        qg_pre_launch(ctx);
-        k_gbd_range<<<rg, 256, 0, ctx->stream>>>(key, n, st);
-        s = qg_check_launch(ctx, "k_gbd_range");
+        s = qg_gbd_range(ctx, key, n);
         if (s == QG_OK) {
             const unsigned mg = (unsigned)std::min<long long>(qg_ceil_div(n, GBM_ROWS), 2LL * C);
             const size_t sm = (size_t)GBM_SLOTS * 12;

@@ -10,13 +10,14 @@
 // keys are sorted there.  A table that fills up (more distinct keys than it
 // takes) is reported and the caller takes the general paths.
 //
-// A 10K-row call 57 -> 46 us.  One SM adds about 4K rows a microsecond, so at
-// 16K rows (4096 groups) the call meets the dense-window path's 58 us (46 to 50
-// with fewer groups) and larger inputs go there; keys of no window (hashed ids)
-// took 150 us through the two-pass path.
+// A 10K-row call in 500 groups 57 -> 43 us, hashed ids (keys of no window) 150
+// -> 46.  One SM adds 2K to 4K rows a microsecond: at 16K rows a call takes 46
+// (64 groups) to 59 us (4096), the dense-window path's three launches 48 whatever
+// the groups and hashed ids 64 on theirs, so larger inputs go there.
 #include <algorithm>
 #include "qg_cta_sort.cuh"
 #include "qg_internal.cuh"
+#include "qg_keytable.cuh"
 
 namespace {
 
@@ -29,7 +30,6 @@ constexpr uint32_t GS_PROBES = 32;  // slots looked at before the table counts a
 // round, above which the table is given up: it is likely to fill, and the
 // general paths should not wait for that.
 constexpr uint32_t GS_FIRST_MOST = 3000, GS_MOST = 5000;
-constexpr uint32_t GS_FREE = 0xffffffffu;
 
 // A sum is kept as two 32-bit words: the values' low halves and (signed) high
 // halves, each exact for up to GS_MAX_ROWS rows, so an add needs no carry.
@@ -45,7 +45,7 @@ k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
     // with more slots than rows a row always finds its slot
     const uint32_t probes = (uint32_t)n < slots ? slots : GS_PROBES;
     extern __shared__ __align__(16) unsigned char gs_raw[];
-    __shared__ uint32_t s_full, s_n, s_dsum[8];  // s_n: distinct keys of the whole rounds, then of the table
+    __shared__ uint32_t s_full, s_n;  // s_n: distinct keys of the whole rounds, then of the table
     unsigned long long *ord = reinterpret_cast<unsigned long long *>(gs_raw);  // [slots] key << 32 | slot
     const uint32_t pitch = slots + 4;  // entry `slots`: key 0xffffffff, the free mark
     const GsSlot T{reinterpret_cast<uint32_t *>(ord + slots), reinterpret_cast<uint32_t *>(ord + slots) + pitch,
@@ -64,31 +64,13 @@ k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
         if (PRED) wn = w4[tid];
     }
     uint4 *kz = reinterpret_cast<uint4 *>(T.key), *cz = reinterpret_cast<uint4 *>(T.cnt);
-    for (uint32_t i = tid; i < pitch / 4; i += GS_THREADS) kz[i] = make_uint4(GS_FREE, GS_FREE, GS_FREE, GS_FREE);
+    for (uint32_t i = tid; i < pitch / 4; i += GS_THREADS) kz[i] = make_uint4(QG_KT_FREE, QG_KT_FREE, QG_KT_FREE, QG_KT_FREE);
     for (uint32_t i = tid; i < 3 * (pitch / 4); i += GS_THREADS) cz[i] = make_uint4(0, 0, 0, 0);
     if (tid == 0) s_full = s_n = 0;
     __syncthreads();
     const uint32_t mask = slots - 1;
     uint32_t fresh = 0;  // keys this thread was the first to see
-    auto row = [&](uint32_t k, int32_t v) {
-        uint32_t h = slots;
-        if (k != GS_FREE) {
-            h = qg_hash32(k) & mask;
-            for (uint32_t p = 0;; p++) {
-                uint32_t cur = T.key[h];
-                if (cur == k) break;
-                if (cur == GS_FREE) {
-                    cur = atomicCAS(&T.key[h], GS_FREE, k);
-                    fresh += cur == GS_FREE;
-                    if (cur == GS_FREE || cur == k) break;
-                }
-                if (p == probes) {
-                    s_full = 1;
-                    return;
-                }
-                h = (h + 1) & mask;
-            }
-        }
+    auto add = [&](uint32_t h, int32_t v) {
         atomicAdd(&T.cnt[h], 1u);
         atomicAdd(&T.lo[h], (uint32_t)v & 0xffffu);
         const int32_t up = v >> 16;
@@ -101,10 +83,19 @@ k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
             vn = v4[q + GS_THREADS];
             if (PRED) wn = w4[q + GS_THREADS];
         }
-        const int32_t ks[4] = {kk.x, kk.y, kk.z, kk.w}, vs[4] = {vv.x, vv.y, vv.z, vv.w}, ws[4] = {ww.x, ww.y, ww.z, ww.w};
+        const int32_t vs[4] = {vv.x, vv.y, vv.z, vv.w}, ws[4] = {ww.x, ww.y, ww.z, ww.w};
+        const uint32_t ks[4] = {(uint32_t)kk.x, (uint32_t)kk.y, (uint32_t)kk.z, (uint32_t)kk.w};
+        uint32_t h[4], live = 0;
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            if (!PRED || ((ws[j] >= lo2) & (ws[j] <= hi2))) row((uint32_t)ks[j], vs[j]);
+            if (!PRED || ((ws[j] >= lo2) & (ws[j] <= hi2))) live |= 1u << j;
+        if (qg_kt_find<4>(T.key, mask, ks, live, h, probes, fresh)) {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if ((live >> j) & 1u) add(h[j], vs[j]);
+        } else {
+            s_full = 1;
+        }
         if (q - tid + 2 * GS_THREADS <= nv) {  // every thread has this round and the next
             const uint32_t f = __reduce_add_sync(QG_FULL_MASK, fresh);
             if (lane == 0 && f) atomicAdd(&s_n, f);
@@ -120,7 +111,12 @@ k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
     }
     if (tid < (n & 3)) {
         const int i = nv * 4 + tid;
-        if (!PRED || ((val2[i] >= lo2) & (val2[i] <= hi2))) row((uint32_t)key[i], val[i]);
+        if (!PRED || ((val2[i] >= lo2) & (val2[i] <= hi2))) {
+            const uint32_t k[1] = {(uint32_t)key[i]};
+            uint32_t h[1];
+            if (qg_kt_find<1>(T.key, mask, k, 1u, h, probes, fresh)) add(h[0], val[i]);
+            else s_full = 1;
+        }
     }
     __syncthreads();
     if (s_full) {
@@ -140,7 +136,7 @@ k_gb_small(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
     }
     __syncthreads();
     const uint32_t g = s_n, top = T.cnt[slots] ? 1u : 0u;  // key 0xffffffff comes last
-    qg_cta_sort(ord, whist, s_dsum, g);
+    qg_cta_sort(ord, whist, g);
     for (uint32_t r = tid; r < g + top && r < cap; r += GS_THREADS) {
         const uint32_t i = r < g ? (uint32_t)ord[r] : slots;
         gkey[r] = r < g ? (int32_t)(ord[r] >> 32) : -1;
@@ -166,7 +162,7 @@ qg_status qg_gbs_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
     static_assert(QG_GBS_SURE_ROWS <= GS_SLOTS, "more slots than rows, and no checked round");
     uint32_t slots = 1024;
     while (slots < GS_SLOTS && slots < 2 * (uint32_t)n) slots <<= 1;
-    auto bytes = [](uint32_t s) { return (size_t)s * 8 + 4 * (s + 4) * 4 + (size_t)std::min<uint32_t>(GS_WARPS, s / 256) * 1024; };
+    auto bytes = [](uint32_t s) { return (size_t)s * 8 + 4 * (s + 4) * 4 + (size_t)GS_WARPS * 1024; };
     const size_t most = bytes(GS_SLOTS), smem = bytes(slots);
     static bool attr[2] = {false, false};
     const bool pred = val2 != nullptr;

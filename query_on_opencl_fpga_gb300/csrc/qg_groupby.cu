@@ -1631,7 +1631,38 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
         }
         // more distinct keys than the small table takes: the general paths
     }
-    if (gm == 0 && !global && n > 0) {
+    // Wide keys: partitioned by key range, else the two-pass path below.  What
+    // the context's last such call took is launched first; a narrow range or a
+    // verdict against it leads to the others, so the path depends on the input.
+    bool wide_tried = false;
+    auto wide = [&](uint32_t *verdict) -> qg_status {
+        wide_tried = true;
+        const qg_status ws = qg_gbw_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, &ctx->hres->count,
+                                           &ctx->hres->aux);
+        if (ws == QG_ERR_OOM) {  // no room for two copies of the rows (nothing was launched)
+            *verdict = QG_GBW_OTHER;
+            return QG_OK;
+        }
+        QG_TRY(ws);
+        QG_TRY(qg_host_count(ctx, &g));
+        *verdict = ctx->hres->aux;
+        if (*verdict == QG_GBW_DONE) {
+            ctx->gb_stats[0] = 0u;
+            ctx->gb_stats[1] = ctx->gb_stats[2] = ctx->gb_stats[3] = 0;
+            *num_groups = g;
+        }
+        return QG_OK;
+    };
+    const bool may_wide = gm == 0 && qg_gbw_applies(n, cap);
+    bool narrow = true;
+    if (may_wide && ctx->gb_first == 1) {
+        uint32_t v;
+        QG_TRY(wide(&v));
+        if (v == QG_GBW_DONE) return g > cap ? QG_ERR_CAPACITY : QG_OK;
+        narrow = v == QG_GBW_NARROW;
+        if (!narrow) ctx->gb_first = 2;
+    }
+    if (gm == 0 && !global && n > 0 && narrow) {
         // Dense-window path: output in key order whatever `order` asks for;
         // its last kernel stores the group count and the rows outside the
         // window in host memory.
@@ -1639,14 +1670,22 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
                              (long long *)&ctx->hres->count, &ctx->hres->aux));
         QG_TRY(qg_host_count(ctx, &g));
         if (ctx->hres->aux == 0) {
+            ctx->gb_first = 0;
             ctx->gb_stats[0] = 2u;
             ctx->gb_stats[1] = ctx->gb_stats[2] = ctx->gb_stats[3] = 0;
             *num_groups = g;
             return g > cap ? QG_ERR_CAPACITY : QG_OK;
         }
         // some key fell outside the sampled window (or the sample spread too
-        // wide for one): the two-pass path below writes the output instead
+        // wide for one)
+        if (may_wide && !wide_tried && ctx->gb_first != 2) {
+            uint32_t v;
+            QG_TRY(wide(&v));
+            ctx->gb_first = v == QG_GBW_DONE ? 1 : 2;
+            if (v == QG_GBW_DONE) return g > cap ? QG_ERR_CAPACITY : QG_OK;
+        }
     }
+    if (wide_tried) QG_TRY(gb_outputs(ctx, gkey, gsum, gcnt, cap, order, &o));  // the arena may have moved
     const bool dense = o.rec && !ctx->gb_wide_keys;
     const bool dev_order = o.rec && !dense && cap < (1LL << 30);
     uint32_t *mm = (uint32_t *)&ctx->ctl->counter[4];

@@ -462,12 +462,11 @@ namespace {
 __global__ void __launch_bounds__(QG_CS_THREADS, 1)
 k_join_sort_small(qg_sort_bufs in, qg_sort_bufs out, uint32_t n) {
     extern __shared__ __align__(16) unsigned char js_raw[];
-    __shared__ uint32_t s_dsum[8];
-    unsigned long long *ord = reinterpret_cast<unsigned long long *>(js_raw);
-    uint32_t(*whist)[256] = reinterpret_cast<uint32_t(*)[256]>(ord + n);
+    uint32_t(*whist)[256] = reinterpret_cast<uint32_t(*)[256]>(js_raw);
+    unsigned long long *ord = reinterpret_cast<unsigned long long *>(whist + 32);
     for (uint32_t i = threadIdx.x; i < n; i += QG_CS_THREADS) ord[i] = (unsigned long long)in.k[i] << 32 | i;
     __syncthreads();
-    qg_cta_sort(ord, whist, s_dsum, n);
+    qg_cta_sort(ord, whist, n);
     for (uint32_t i = threadIdx.x; i < n; i += QG_CS_THREADS) {
         const uint32_t j = (uint32_t)ord[i];
         out.k[i] = (uint32_t)(ord[i] >> 32);
@@ -535,7 +534,7 @@ qg_status qg_join_hash_sort(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpa
     const int npos = range ? qg_sort_positions(32 - __builtin_clz(range)) : 0;
     // Up to 8192 matches: one launch (4 radix passes took 45 us for 4K of them)
     if (m <= QG_CS_MAX) {
-        const size_t most = QG_CS_MAX * 8 + QG_CS_MAX / 256 * 1024, smem = (size_t)m * 8 + (size_t)(m + 255) / 256 * 1024;
+        const size_t most = QG_CS_MAX * 8 + 32 * 1024, smem = (size_t)m * 8 + 32 * 1024;
         static bool attr = false;
         if (!attr) {
             QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_join_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most), "attr");

@@ -96,13 +96,6 @@ k_radix_hist(const uint32_t *__restrict__ kin, const unsigned long long *__restr
 
 // A record sort planned on the device: per key position its digit bases and
 // what its pass does.
-struct RsPass {
-    const unsigned long long *src;
-    unsigned long long *dst;
-    uint32_t *status, *clear;  // the pass's status words, and the next pass's to clear
-    uint32_t mode;             // 0 nothing, 1 a pass, 2 a copy
-    uint32_t pad;
-};
 struct RsPlan {
     RsPass pass[5];  // the four positions, and the copy back of an in-place sort
     uint32_t base[4 * QG_RADIX];
@@ -403,6 +396,8 @@ k_radix_pass(qg_sort_bufs src, qg_sort_bufs dst, long long n, int shift, uint32_
         src.rec = const_cast<unsigned long long *>(plan->src);
         dst.rec = plan->dst;
         status = plan->status;
+        shift = (int)plan->shift;
+        key_off = plan->key_off;
         if (plan->clear) plan->clear[(size_t)blockIdx.x * QG_RADIX + threadIdx.x] = 0;
     }
     if (range) {  // three columns: the pass runs or not, and reads a or b, by the key range's positions
@@ -721,7 +716,7 @@ k_radix_plan(uint32_t *__restrict__ hist, const unsigned long long *in, unsigned
 #pragma unroll
     for (int p = 0; p < 4; p++) {
         RsPass &P = plan->pass[p];
-        P = RsPass{nullptr, nullptr, nullptr, nullptr, 0u, 0u};
+        P = RsPass{nullptr, nullptr, nullptr, nullptr, 0u, 8u * p, 0u, 0u};
         if (!act[p]) continue;
         left--;
         unsigned long long *to = ((left & 1) != 0) == to_tmp ? out : tmp;
@@ -733,8 +728,8 @@ k_radix_plan(uint32_t *__restrict__ hist, const unsigned long long *in, unsigned
         from = to;
         q++;
     }
-    if (np == 0 && !same) plan->pass[0] = RsPass{in, out, nullptr, nullptr, 2u, 0u};
-    plan->pass[4] = RsPass{tmp, out, nullptr, nullptr, to_tmp ? 2u : 0u, 0u};
+    if (np == 0 && !same) plan->pass[0] = RsPass{in, out, nullptr, nullptr, 2u, 0u, 0u, 0u};
+    plan->pass[4] = RsPass{tmp, out, nullptr, nullptr, to_tmp ? 2u : 0u, 0u, 0u, 0u};
     *h_passes = (uint32_t)np;
 }
 
@@ -779,6 +774,18 @@ qg_status qg_sort_rec(qg_ctx *ctx, const unsigned long long *in, unsigned long l
         QG_TRY(qg_check_launch(ctx, "k_radix_pass"));
     }
     return QG_OK;
+}
+
+size_t qg_radix_status_words(long long n_bound) { return (size_t)((n_bound + RS_TILE - 1) / RS_TILE) * QG_RADIX; }
+
+qg_status qg_radix_pass_planned(qg_ctx *ctx, const RsPass *plan, const uint32_t *dbase, long long n_bound,
+                                const unsigned long long *d_n) {
+    if (n_bound >= (1LL << 30)) return QG_ERR_UNSUPPORTED;
+    QG_TRY((rs_set_attr<false, false>(ctx)));
+    qg_pre_launch(ctx);
+    k_radix_pass<false, false, 2><<<(unsigned)((n_bound + RS_TILE - 1) / RS_TILE), RS_THREADS, sizeof(RsSmem<false>), ctx->stream>>>(
+        qg_sort_bufs{}, qg_sort_bufs{}, n_bound, 0, 0u, dbase, nullptr, ctx->ctl, ctx->spin_limit, d_n, nullptr, plan, nullptr);
+    return qg_check_launch(ctx, "k_radix_pass");
 }
 
 // After the sort's stream has been waited for: remember the parity of an

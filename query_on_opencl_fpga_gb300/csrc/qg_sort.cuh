@@ -19,6 +19,21 @@ struct qg_sort_bufs {
     uint16_t *bid;
 };
 
+// One pass of a record sort whose plan is in device memory.
+struct RsPass {
+    const unsigned long long *src;
+    unsigned long long *dst;
+    uint32_t *status, *clear;  // the pass's status words, and the next pass's to clear
+    uint32_t mode;             // 0 nothing, 1 a pass, 2 a copy
+    uint32_t shift, key_off;   // the digit: ((key - key_off) >> shift) & 255
+    uint32_t pad;
+};
+// One unstable pass over at most n_bound items (*d_n of them): plan, digit bases
+// and cleared status words (qg_radix_status_words) in device memory.
+size_t qg_radix_status_words(long long n_bound);
+qg_status qg_radix_pass_planned(qg_ctx *ctx, const RsPass *plan, const uint32_t *dbase, long long n_bound,
+                                const unsigned long long *d_n);
+
 // Number of 8-bit digit positions covering `bits` key bits (1..4).
 int qg_sort_positions(int bits);
 // Device histogram of (key - key_off) digits for `npos` positions into

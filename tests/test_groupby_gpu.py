@@ -540,3 +540,71 @@ def test_groupby_small_capacity(ctx):
         ctx.groupby_cols(key, key, cap=2999)
     assert e.value.status == 3
     assert ctx.groupby_cols(key, key, cap=3000)[0].numel() == 3000
+
+
+# Three launches from the exact key range: the row after the small form, tiles of
+# 4096 rows, the largest input and the next one; a span that just fits the window
+# and one that does not, windows at both ends of the key space, sums that need
+# the carry into the high word.
+@pytest.mark.parametrize("n", [16_385, 20_479, 4096 * 304 + 3, 1 << 23, (1 << 23) + 1])
+@pytest.mark.parametrize("lo,span", [(0, 1 << 22), (2 ** 32 - (1 << 22), 1 << 22), (2 ** 31 - 7, 50), (5, (1 << 22) + 1)])
+def test_groupby_dense_exact_range(ctx, orc, n, lo, span):
+    rng = np.random.default_rng(n + span)
+    u = rng.integers(0, span, n)
+    u[::3] = rng.integers(0, 9, u[::3].size) * (span // 9)  # frequent ones
+    u[[7, n - 2]] = 0, span - 1
+    key = ((u + lo) % 2 ** 32).astype(np.uint32).view(np.int32)
+    val = rng.choice(np.array([-(2 ** 31), 2 ** 31 - 1, -1, 12345]), n).astype(np.int32)
+    val2 = rng.integers(0, 1000, n).astype(np.int32)
+    fits = (span <= 1 << 22) if n <= 1 << 23 else None
+    for v2 in (None, val2):
+        _dense_case(ctx, orc, key, val, v2, 0, 499, path={True: "dense", False: "two_pass", None: None}[fits])
+
+
+# Keys of no window, partitioned by range: one row more than the small form, tile
+# remainders, 128 and 256 parts, the key that marks free slots, parts of more
+# than 65536 rows (sums with a carry), few rows selected, none selected; inputs
+# it gives up: a few frequent keys (uneven parts), more distinct keys in a part
+# than its table takes.  In sequence on one context, with narrow keys between.
+def test_groupby_wide(ctx, orc):
+    rng = np.random.default_rng(77)
+    ids = rng.integers(-(2 ** 31), 2 ** 31, 1 << 20)
+
+    def keys(kind, n):
+        if kind == "ids":
+            return rng.choice(ids[: max(50, n // 5)], n)
+        if kind == "own":
+            return rng.permutation(n) * (2 ** 32 // n) - 2 ** 31
+        if kind == "many_rows":
+            return rng.choice(np.linspace(-(2 ** 31), 2 ** 31 - 1, 20).astype(np.int64), n)
+        if kind == "uneven":
+            return rng.choice(np.array([-(2 ** 31), 5, 2 ** 31 - 1]), n)
+        if kind == "crowded":
+            k = rng.choice(ids[:50], n)
+            k[:16_000] = rng.permutation(16_000)
+            return k
+        return rng.integers(0, 5000, n)  # narrow
+
+    for n, kind in [(16_385, "ids"), (4096 * 5, "ids"), (70_001, "narrow"), (4096 * 9 + 1, "own"), (300_003, "ids"),
+                    (1 << 20, "own"), (3_000_001, "many_rows"), (50_000, "uneven"), (100_003, "ids"),
+                    (120_000, "crowded"), (30_001, "narrow"), (4_000_002, "own"), (20_001, "ids")]:
+        key = keys(kind, n).astype(np.int32)
+        key[[3, n // 2]] = -1
+        val = rng.choice(np.array([-(2 ** 31), 2 ** 31 - 1, -1, 65535, 65536, 7]), n).astype(np.int32)
+        val2 = rng.integers(0, 1000, n).astype(np.int32)
+        for v2, hi in ((None, 0), (val2, 499), (val2, 3), (val2, -1)):
+            _dense_case(ctx, orc, key, val, v2, 0, hi, order=QG_ORDER_NONE if hi == 3 else QG_ORDER_KEY)
+
+
+def test_groupby_wide_capacity(ctx, orc):
+    from query_on_opencl_fpga_gb300 import QGError
+
+    rng = np.random.default_rng(78)
+    n = 100_000
+    key = rng.choice(rng.integers(-(2 ** 31), 2 ** 31, 20_000), n).astype(np.int32)
+    g = np.unique(key).size
+    for _ in range(2):
+        with pytest.raises(QGError) as e:
+            ctx.groupby_cols(dev(key), dev(key), cap=g - 1)
+        assert e.value.status == 3
+        _dense_case(ctx, orc, key, key, cap=g)
