@@ -26,3 +26,26 @@ qg_status qg_join_hash_sort(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpa
                             const int32_t *spay, int64_t nS, int32_t slo, int32_t shi, int32_t *out_key,
                             int32_t *out_rpay, int32_t *out_spay, int64_t cap, int64_t *out_n, uint32_t most_probes = 0,
                             bool *crowded = nullptr, uint32_t *span = nullptr);
+
+// flags of the dense build side (u32 words): [1] dense span, [2..3] distinct
+// keys (u64), [4] / [5] smallest / largest R payload (int32), [6] a sentinel
+// payload exists, [7] the sentinel.
+enum { PJ_F_DENSE = 1, PJ_F_DISTINCT = 2, PJ_F_PMIN = 4, PJ_F_PMAX = 5, PJ_F_SENT_OK = 6, PJ_F_SENT = 7, PJ_F_WORDS = 8 };
+
+// Dense build side, large probe inputs (qg_jpart.cu): four launches, no read
+// back.  r: R's payload table as k_pj_rtab leaves it.  rows: `room` rows of
+// scratch, 16-byte aligned.  Afterwards *result is 1 when the outputs hold the
+// result, *d_count then the match count, else 0; qg_jp_done() is the same word in
+// device memory for kernels that follow.  work: qg_jp_bytes(), 16-byte aligned.
+struct qg_jp_r {
+    const uint32_t *range;  // smallest and largest key
+    const uint32_t *flags;  // PJ_F_*
+    const uint32_t *bitmap, *T;
+    int64_t nR;
+};
+size_t qg_jp_bytes();
+const uint32_t *qg_jp_done(const char *work);
+qg_status qg_jp_launch(qg_ctx *ctx, char *work, const qg_jp_r &r, const int32_t *skey, const int32_t *spay, int64_t nS,
+                       int32_t slo, int32_t shi, unsigned long long *rows, int64_t room, uint32_t *out_key,
+                       uint32_t *out_rpay, uint32_t *out_spay, int64_t cap, volatile long long *d_count,
+                       volatile uint32_t *result);

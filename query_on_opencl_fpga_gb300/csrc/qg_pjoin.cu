@@ -96,11 +96,6 @@ struct PjPackOut {
     uint32_t most, pad;
 };
 
-// flags of the dense build side (u32 words): [1] dense span, [2..3] distinct
-// keys (u64), [4] / [5] smallest / largest R payload (int32), [6] a sentinel
-// payload exists, [7] the sentinel.
-enum { PJ_F_DENSE = 1, PJ_F_DISTINCT = 2, PJ_F_PMIN = 4, PJ_F_PMAX = 5, PJ_F_SENT_OK = 6, PJ_F_SENT = 7, PJ_F_WORDS = 8 };
-
 // One CTA: the head block (range, digit histograms, flags) of a new call.
 __global__ void k_pj_range_init(PjRange *r, uint32_t *dh, uint32_t *flags) {
     for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) dh[i] = 0;
@@ -133,10 +128,21 @@ k_pj_rrec(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, lo
     }
 }
 
-// R's key range and payload range (16-byte loads where aligned).
+// R's key range and payload range (16-byte loads where aligned).  One set of
+// atomics per CTA: with one per warp, 2M rows took 20 us, all of it in the queue
+// at four words.
 __global__ void __launch_bounds__(256)
 k_pj_rrange(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, long long nR, PjRange *range,
             uint32_t *flags) {
+    __shared__ uint32_t s_k[2];
+    __shared__ int s_p[2];
+    if (threadIdx.x == 0) {
+        s_k[0] = 0xffffffffu;
+        s_k[1] = 0;
+        s_p[0] = 0x7fffffff;
+        s_p[1] = (int)0x80000000;
+    }
+    __syncthreads();
     uint32_t lmin = 0xffffffffu, lmax = 0;
     int32_t pmin = 0x7fffffff, pmax = (int32_t)0x80000000;
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -164,10 +170,17 @@ k_pj_rrange(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, 
     pmin = __reduce_min_sync(QG_FULL_MASK, pmin);
     pmax = __reduce_max_sync(QG_FULL_MASK, pmax);
     if ((threadIdx.x & 31) == 0) {
-        atomicMin(&range->kmin, lmin);
-        atomicMax(&range->kmax, lmax);
-        atomicMin(reinterpret_cast<int *>(flags + PJ_F_PMIN), pmin);
-        atomicMax(reinterpret_cast<int *>(flags + PJ_F_PMAX), pmax);
+        atomicMin(&s_k[0], lmin);
+        atomicMax(&s_k[1], lmax);
+        atomicMin(&s_p[0], pmin);
+        atomicMax(&s_p[1], pmax);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicMin(&range->kmin, s_k[0]);
+        atomicMax(&range->kmax, s_k[1]);
+        atomicMin(reinterpret_cast<int *>(flags + PJ_F_PMIN), s_p[0]);
+        atomicMax(reinterpret_cast<int *>(flags + PJ_F_PMAX), s_p[1]);
     }
 }
 
@@ -288,8 +301,13 @@ k_pj_distinct(const uint32_t *__restrict__ bitmap, const uint32_t *__restrict__ 
     } else {
         for (unsigned long long i = t0; i < ((w + 31ull) >> 5); i += stride) c += __popc(__ldcg(bitmap + i));
     }
+    __shared__ uint32_t s_c;
+    if (threadIdx.x == 0) s_c = 0;
+    __syncthreads();
     c = __reduce_add_sync(QG_FULL_MASK, c);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, (unsigned long long)c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&s_c, c);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_c) atomicAdd(count, (unsigned long long)s_c);
 }
 
 // ---------------------------------------------------------------------------
@@ -314,7 +332,10 @@ __global__ void __launch_bounds__(SF_THREADS, 4)
 k_pj_sfilter(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, long long n,
                int32_t slo, int32_t shi, const PjRange *__restrict__ range,
                unsigned long long *__restrict__ out, unsigned long long *__restrict__ cursor,
-               qg_control *ctl, int lb2, uint32_t *__restrict__ hist) {
+               qg_control *ctl, int lb2, uint32_t *__restrict__ hist, const uint32_t *__restrict__ done,
+               const uint32_t *__restrict__ dense) {
+    if (done && *done == 1u) return;     // qg_jpart.cu has answered
+    if (dense && *dense == 0u) return;   // the hash join will
     constexpr int TILE = SF_THREADS * SF_ROUNDS * 4;
     __shared__ uint32_t s_woff[SF_ROUNDS * SF_WARPS];
     __shared__ unsigned long long s_base;
@@ -2134,10 +2155,12 @@ extern "C" QG_API qg_status qg_join_filter_sort(qg_ctx *ctx, const int32_t *rkey
     return st;
 }
 
-// Largest S of the counting path (qg_jdirect.cu).  Both paths, R = S / 16, 24 %
-// of the rows joined: 4K rows 61 / 126 us, 1M 72 / 149, 16M 182 / 280, 32M 315 /
-// 380, 64M 608 / 583: from there the scattered accesses leave L2.
-constexpr int64_t PJ_DIRECT_S = 40'000'000;
+// Largest S of the counting path (qg_jdirect.cu); above it the one partition step
+// (qg_jpart.cu).  R = S / 16, 24 % of the rows joined, counting / one step: 16M
+// rows 187 / 185 us, 32M 319 / 262; the scattered accesses of the first leave L2.
+// The partitioned form below took 4K rows 126 us, 16M 280, 64M 583, 256M 1764,
+// where one of the two takes 61, 185, 407 and 1357.
+constexpr int64_t PJ_DIRECT_S = 18'000'000;
 // Build rows of the hash join, whose table (16 to 32 bytes a row) stays in L2.
 // Against the partitioned path (radix, or learned where that spreads better),
 // skewed keys: 64K rows 92 / 156 us, 1M 107 / 415, 16M 303 / 925, 64M 910 /
@@ -2188,6 +2211,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     // dense span.  Which of the two is launched first is what the context's last
     // such call found; each sees R's span and hands over to the other.
     const bool dflt = variant == 0 && g_pj_dense && g_pj_blog2 == 0 && g_pj_smax == PB_SMAX && g_pj_rmax == PB_RMAX;
+    bool hash_tried = false;
     if (dflt && nR <= PJ_HASH_R) {
         const bool direct = nS <= PJ_DIRECT_S;
         bool other = false;  // a dense span, but not for the counting path
@@ -2197,6 +2221,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
         if (ctx->pj_sparse && !other) {
             bool crowded = false;
             uint32_t span = 0;
+            hash_tried = true;
             const qg_status st = qg_join_hash_sort(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay,
                                                    out_spay, cap, out_n, PJ_HASH_PROBES, &crowded, &span);
             if (st != QG_OK && st != QG_ERR_CAPACITY) return st;
@@ -2218,7 +2243,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     const size_t rb = qg_align_up((size_t)nR * 8, 256), sb = qg_align_up((size_t)nS * 8, 256);
     const size_t bmb = qg_align_up(((size_t)2 * nR + 63) / 32 * 4, 256);
     char *aux;
-    QG_TRY(qg_aux(ctx, 2 * rb + 2 * sb + bmb + pj_level_bytes(PJ_MAX_BUCKETS, true), &aux));
+    QG_TRY(qg_aux(ctx, 2 * rb + 2 * sb + bmb + pj_level_bytes(PJ_MAX_BUCKETS, true) + qg_jp_bytes(), &aux));
     PjPin *pin;
     QG_TRY(pj_pin(ctx, &pin));
     unsigned long long *R = (unsigned long long *)aux, *Rsp = (unsigned long long *)(aux + rb);
@@ -2250,18 +2275,38 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     k_pj_distinct<<<pj_grid(ctx, nR, 256, 8), 256, 0, ctx->stream>>>(
         bitmap, T, L.range, lb2, nR, L.dflags, reinterpret_cast<unsigned long long *>(L.dflags + PJ_F_DISTINCT));
     QG_TRY(qg_check_launch(ctx, "k_pj_distinct"));
+    // large probe inputs: one partition step, unless the build side is not dense or the rows spread unevenly
+    const bool jp = dflt && nS > PJ_DIRECT_S;
+    const bool may_hash = nR <= PJ_HASH_R && !hash_tried;
+    char *jp_work = aux + 2 * rb + 2 * sb + bmb + pj_level_bytes(PJ_MAX_BUCKETS, true);
+    if (jp) {
+        const qg_jp_r jr{&L.range->kmin, L.dflags, bitmap, T, nR};
+        QG_TRY(qg_jp_launch(ctx, jp_work, jr, skey, spay, nS, slo, shi, S, (int64_t)(2 * sb / 8), (uint32_t *)out_key,
+                            (uint32_t *)out_rpay, (uint32_t *)out_spay, cap, &ctx->hres->count, &ctx->hres->aux));
+    }
     // S filter with the S' digit histograms of the radix function
     constexpr int SF_TILE = SF_THREADS * SF_ROUNDS * 4;
     const long long tiles = (nS + SF_TILE - 1) / SF_TILE;
     qg_pre_launch(ctx);
     k_pj_sfilter<<<(unsigned)std::min<long long>(tiles, (long long)ctx->sm_count * 4), SF_THREADS, 0, ctx->stream>>>(
-        skey, spay, nS, slo, shi, L.range, S, &L.range->count, ctx->ctl, lb2, L.dh + 512);
+        skey, spay, nS, slo, shi, L.range, S, &L.range->count, ctx->ctl, lb2, L.dh + 512, jp ? qg_jp_done(jp_work) : nullptr,
+        jp && may_hash ? L.dflags + PJ_F_DENSE : nullptr);
     QG_TRY(qg_check_launch(ctx, "k_pj_sfilter"));
     // one copy brings R's key range, the S' count, the histograms and the dense flags
     constexpr size_t head = offsetof(PjPin, dflags) + PJ_F_WORDS * 4;
     static_assert(offsetof(PjPin, h) == 256 && offsetof(PjPin, dflags) == 256 + 4096, "as carved");
     QG_TRY_CUDA(ctx, cudaMemcpyAsync(pin, L.range, head, cudaMemcpyDeviceToHost, ctx->stream), "head d2h");
     QG_TRY(qg_collect_error(ctx));
+    if (jp && ctx->hres->aux) {
+        ctx->pj_stats[0] = 4;
+        ctx->pj_sparse = false;
+        *out_n = ctx->hres->count;
+        return *out_n > cap ? QG_ERR_CAPACITY : QG_OK;
+    }
+    if (jp && may_hash && pin->dflags[PJ_F_DENSE] == 0u) {  // sparse build keys: the hash join, then what follows it
+        ctx->pj_sparse = true;
+        return join_filter_sort_impl(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay, out_spay, cap, out_n);
+    }
     const PjRange hr = pin->range;
     const long long ns1 = (long long)hr.count;
     unsigned long long distinct;

@@ -383,3 +383,54 @@ def test_join_sparse_crowded_key_takes_general_path(ctx, orc):
     spay = rng.integers(0, 400, skey.size).astype(np.int32)
     spay[-3:] = 1
     _join_case(ctx, orc, rkey, rpay, skey, spay, "radix")
+
+
+def _hash32(x):
+    x = x.astype(np.uint64)
+    for mul, sh in ((0x85EBCA6B, 16), (0xC2B2AE35, 13)):
+        x ^= x >> np.uint64(sh)
+        x = x * np.uint64(mul) & np.uint64(0xFFFFFFFF)
+    return x ^ (x >> np.uint64(16))
+
+
+# Large probe inputs with a dense build side (one partition step): every value of
+# R's span present, half of it (with a payload that leaves no sentinel), every row
+# selected, few, none; a frequent key that the sample shows (another path), and
+# rows off the sampled ones that overflow a bucket's room.
+@pytest.mark.parametrize("kind", ["full", "half", "all", "few", "none", "hot", "missed"])
+def test_join_large_dense(ctx, kind):
+    nS = 20_000_003
+    nR = 1_300_000
+    step = 2 if kind == "half" else 1
+    base = -(2 ** 31) + 5 if kind == "half" else 2 ** 31 - 1_000_000 if kind == "few" else 0
+    g = torch.Generator(device="cuda")
+    g.manual_seed(11)
+    ints = lambda lo, hi, n: torch.randint(lo, hi, (n,), generator=g, device="cuda")  # noqa: E731
+    roff = torch.randperm(nR, generator=g, device="cuda") * step
+    rpay = ints(-(2 ** 31), 2 ** 31, nR) if kind != "half" else ints(0, 2, nR) * (2 ** 32 - 1) - 2 ** 31
+    soff = ints(0, nR * step, nS) if kind in ("all", "missed") else ints(-nR, 3 * nR * step, nS)
+    spay = ints(0, 1000, nS)
+    row = np.arange(nS // 1024 * 1024)
+    sampled = (row % 1024) // 16 == (_hash32(row // 1024) & np.uint64(63)).astype(np.int64)
+    off = torch.from_numpy(np.flatnonzero(~sampled)).cuda()  # rows that the sample does not see
+    hi = {"all": 999, "few": 3, "none": -1}.get(kind, 299)
+    if kind == "hot":
+        soff[::200] = 12_345
+    elif kind == "missed":
+        soff[off] = soff[off] % (nR // 3)
+    i32 = lambda t: (((t + base + 2 ** 31) & 0xFFFFFFFF) - 2 ** 31).to(torch.int32)  # noqa: E731
+    skey = i32(soff)
+    for _ in range(2):  # the first call may follow one with sparse keys
+        got = ctx.join_filter_sort(i32(roff), rpay.to(torch.int32), skey, spay.to(torch.int32), 0, hi, cap=nS)
+    if kind not in ("hot", "missed"):
+        assert ctx.join_stats()["path"] == "dense"
+    table = torch.full((nR * step,), 2 ** 40, dtype=torch.int64, device="cuda")
+    table[roff] = rpay
+    sel = (spay <= hi) & (soff >= 0) & (soff < nR * step)
+    so, sp = soff[sel], spay[sel]
+    here = table[so] < 2 ** 40
+    exp = (((so[here] + base) & 0xFFFFFFFF) * 1000 + sp[here]).sort().values
+    uk = got[0].to(torch.int64) & 0xFFFFFFFF
+    assert bool((uk[1:] >= uk[:-1]).all())
+    assert torch.equal((uk * 1000 + got[2]).sort().values, exp)
+    assert torch.equal(got[1].to(torch.int64), table[(uk - base) & 0xFFFFFFFF])
