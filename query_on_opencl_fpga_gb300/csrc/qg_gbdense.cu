@@ -384,10 +384,44 @@ k_gbd_main(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
 // and the grid grows with the input.  Calls with
 // Zipf keys, groups = rows / 16: 64K rows 64 -> 51 us, 1M 69 -> 55, 4M 80 -> 71,
 // 8M 96 -> 89; at 16M 125 / 130, the sampled table's better hit rate wins.
+// SAMPLE: the last CTA counts the distinct keys of 4096 rows instead (1024 vectors
+// spread over the column), while the others read it all.
+template <bool SAMPLE>
 __global__ void __launch_bounds__(256)
-k_gbd_range(const int32_t *__restrict__ key, long long n, uint32_t *__restrict__ st) {
+k_gbd_range(const int32_t *__restrict__ key, long long n, uint32_t *__restrict__ st, uint32_t few_limit,
+            uint32_t *__restrict__ few) {
     __shared__ uint32_t s[2];
     if (threadIdx.x < 2) s[threadIdx.x] = 0;
+    if (SAMPLE && blockIdx.x == gridDim.x - 1) {
+        // hashed to 64K bits: one in thirty of 4096 distinct keys finds its bit set
+        // (a hash table of the keys took 15 us longer than the other CTAs)
+        constexpr int WORDS = 2048;
+        __shared__ uint32_t bits[SAMPLE ? WORDS : 1];
+        int4 v[4];
+        const long long nv = n >> 2;
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = __ldg(reinterpret_cast<const int4 *>(key) + (nv * (j * 256 + (int)threadIdx.x) >> 10));
+        for (int i = threadIdx.x; i < WORDS; i += 256) bits[i] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t k[4] = {(uint32_t)v[j].x, (uint32_t)v[j].y, (uint32_t)v[j].z, (uint32_t)v[j].w};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const uint32_t h = qg_hash32(k[e]) >> 16;
+                atomicOr(&bits[h >> 5], 1u << (h & 31u));
+            }
+        }
+        __syncthreads();
+        uint32_t fresh = 0;
+        for (int i = threadIdx.x; i < WORDS; i += 256) fresh += __popc(bits[i]);
+        fresh = __reduce_add_sync(QG_FULL_MASK, fresh);
+        if ((threadIdx.x & 31) == 0 && fresh) atomicAdd(&s[0], fresh);
+        __syncthreads();
+        if (threadIdx.x == 0) *few = s[0] <= few_limit;
+        return;
+    }
+    const uint32_t ctas = gridDim.x - (SAMPLE ? 1u : 0u);
     if (blockIdx.x == 0 && threadIdx.x == 0) st[G_EXTRA] = 0;  // k_gbd_mid sets the call's other words
     __syncthreads();
     uint32_t lo = 0, hi = 0;  // the smallest key as the largest complement
@@ -395,7 +429,7 @@ k_gbd_range(const int32_t *__restrict__ key, long long n, uint32_t *__restrict__
         lo = max(lo, ~(uint32_t)k);
         hi = max(hi, (uint32_t)k);
     };
-    const long long nv = n >> 2, stride = (long long)gridDim.x * 256, t0 = (long long)blockIdx.x * 256 + threadIdx.x;
+    const long long nv = n >> 2, stride = (long long)ctas * 256, t0 = (long long)blockIdx.x * 256 + threadIdx.x;
     for (long long i = t0; i < nv; i += stride) {
         const int4 k = __ldg(reinterpret_cast<const int4 *>(key) + i);
         row(k.x);
@@ -843,10 +877,13 @@ k_gbd_single(const int32_t *__restrict__ key, const int32_t *__restrict__ val, c
 
 }  // namespace
 
-qg_status qg_gbd_range(qg_ctx *ctx, const int32_t *key, int64_t n) {
+qg_status qg_gbd_range(qg_ctx *ctx, const int32_t *key, int64_t n, uint32_t few_limit) {
     const unsigned grid = (unsigned)std::min<long long>(qg_ceil_div(n, 4 * 256), 4LL * ctx->sm_count);
     qg_pre_launch(ctx);
-    k_gbd_range<<<grid, 256, 0, ctx->stream>>>(key, n, ctx->ctl->gbd);
+    if (few_limit)
+        k_gbd_range<true><<<grid + 1, 256, 0, ctx->stream>>>(key, n, ctx->ctl->gbd, few_limit, &ctx->ctl->gbw_few);
+    else
+        k_gbd_range<false><<<grid, 256, 0, ctx->stream>>>(key, n, ctx->ctl->gbd, 0u, nullptr);
     return qg_check_launch(ctx, "k_gbd_range");
 }
 

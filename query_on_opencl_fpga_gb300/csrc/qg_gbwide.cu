@@ -57,14 +57,14 @@ template <bool PRED>
 __global__ void __launch_bounds__(GW_THREADS, 4)
 k_gbw_rows(const int32_t *__restrict__ key, const int32_t *__restrict__ val, const int32_t *__restrict__ val2,
            int32_t lo2, int32_t hi2, long long n, const uint32_t *__restrict__ range, uint32_t window, int parts_log2,
-           unsigned long long *__restrict__ rec, uint32_t *__restrict__ hist, unsigned long long *__restrict__ rows,
-           uint4 *__restrict__ clear, long long clear_n) {
+           const uint32_t *__restrict__ few, unsigned long long *__restrict__ rec, uint32_t *__restrict__ hist,
+           unsigned long long *__restrict__ rows, uint4 *__restrict__ clear, long long clear_n) {
     __shared__ uint32_t s_h[GW_PARTS], s_woff[32], s_cnt;
     __shared__ unsigned long long s_base;
     __shared__ unsigned long long s_row[PRED ? GW_TILE : 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t kmin = ~range[0], span = range[1] - kmin, lt = qg_lanemask_lt();
-    if (span < window) return;  // a window holds the keys
+    if (span < window || (few && *few)) return;  // a window holds the keys; few groups
     const int shift = gw_shift(span, parts_log2);
     for (long long j = (long long)blockIdx.x * GW_THREADS + tid; j < clear_n; j += (long long)gridDim.x * GW_THREADS)
         clear[j] = make_uint4(0, 0, 0, 0);  // the radix pass's status words
@@ -174,8 +174,8 @@ k_gbw_rows(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
 // One CTA of GW_PARTS threads.  The histogram and the row counter are cleared
 // for their next user.
 __global__ void __launch_bounds__(GW_PARTS)
-k_gbw_plan(const uint32_t *__restrict__ range, uint32_t window, int parts_log2, uint32_t *__restrict__ hist,
-           unsigned long long *__restrict__ rows, GwState *__restrict__ W, const unsigned long long *r0,
+k_gbw_plan(const uint32_t *__restrict__ range, uint32_t window, int parts_log2, const uint32_t *__restrict__ few,
+           uint32_t *__restrict__ hist, unsigned long long *__restrict__ rows, GwState *__restrict__ W, const unsigned long long *r0,
            unsigned long long *r1, uint32_t *status) {
     __shared__ uint32_t ws[GW_PARTS / 32], wm[GW_PARTS / 32];
     const int d = threadIdx.x, lane = d & 31, w = d >> 5;
@@ -205,7 +205,7 @@ k_gbw_plan(const uint32_t *__restrict__ range, uint32_t window, int parts_log2, 
     W->full = 0;
     *rows = 0;
     const bool even = most <= 16384u || ((unsigned long long)most << parts_log2) <= (unsigned long long)GW_UNEVEN * all;
-    const uint32_t verdict = span < window ? QG_GBW_NARROW : even ? QG_GBW_DONE : QG_GBW_OTHER;
+    const uint32_t verdict = span < window ? QG_GBW_NARROW : few && *few ? QG_GBW_FEW : even ? QG_GBW_DONE : QG_GBW_OTHER;
     W->verdict = verdict;
     W->pass = RsPass{r0, r1, status, nullptr, verdict == QG_GBW_DONE ? 1u : 0u, (uint32_t)gw_shift(span, parts_log2), kmin, 0u};
 }
@@ -326,6 +326,18 @@ size_t gw_smem(uint32_t slots) { return (size_t)slots * 8 + 4 * (slots + 4) * 4 
 // Distinct keys a part of 2^parts_log2 may expect, for the tables' sizes.
 static int64_t gw_expected(int64_t n, int64_t cap, int parts_log2) { return std::min(n, cap) >> parts_log2; }
 
+// Few groups among many rows stay in the two-pass path's per-SM tables, and its one
+// pass over the rows wins; here each part's CTA meets its rows one a clock.  Hashed
+// ids, two-pass / this path: 4M rows in 64 groups 168 / 133 us; 8M in 64 178 / 201,
+// in 512 190 / 161; 16M in 512 213 / 277, in 2048 251 / 255, in 8192 413 / 249; 32M in
+// 2048 314 / 461, in 8192 582 / 446.  The line in distinct keys of a 4096-row sample
+// (5000 equally frequent keys show 2800):
+static uint32_t gw_few_limit(int64_t n) {
+    return n < 6'000'000 ? 0u : (uint32_t)std::min<int64_t>((n - 6'000'000) / 5500, 2700);
+}
+
+bool qg_gbw_few(int64_t n, int64_t groups) { return groups <= gw_few_limit(n) * 3 / 2; }
+
 bool qg_gbw_applies(int64_t n, int64_t cap) {
     return n > QG_GBS_MAX_ROWS && n < (1LL << 30) && gw_expected(n, cap, 8) <= GW_SLOTS * 5 / 8;
 }
@@ -354,15 +366,16 @@ qg_status qg_gbw_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
     }
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, GW_PARTS, QG_SITE_GROUPBY, &lb));
-    QG_TRY(qg_gbd_range(ctx, key, n));
+    const uint32_t limit = gw_few_limit(n), *few = limit ? &ctx->ctl->gbw_few : nullptr;
+    QG_TRY(qg_gbd_range(ctx, key, n, limit));
     const unsigned grid = (unsigned)std::min<long long>(qg_ceil_div(n, GW_TILE), 4LL * ctx->sm_count);
     qg_pre_launch(ctx);
     (pred ? k_gbw_rows<true> : k_gbw_rows<false>)<<<grid, GW_THREADS, 0, ctx->stream>>>(
-        key, val, val2, lo2, hi2, n, range, window, plog2, r0, hist, &ctx->ctl->gbw_rows, (uint4 *)status,
+        key, val, val2, lo2, hi2, n, range, window, plog2, few, r0, hist, &ctx->ctl->gbw_rows, (uint4 *)status,
         (long long)(words / 4));
     QG_TRY(qg_check_launch(ctx, "k_gbw_rows"));
     qg_pre_launch(ctx);
-    k_gbw_plan<<<1, GW_PARTS, 0, ctx->stream>>>(range, window, plog2, hist, &ctx->ctl->gbw_rows, W, r0, r1, status);
+    k_gbw_plan<<<1, GW_PARTS, 0, ctx->stream>>>(range, window, plog2, few, hist, &ctx->ctl->gbw_rows, W, r0, r1, status);
     QG_TRY(qg_check_launch(ctx, "k_gbw_plan"));
     QG_TRY(qg_radix_pass_planned(ctx, &W->pass, W->base, n, &W->rows));
     qg_pre_launch(ctx);

@@ -1595,6 +1595,7 @@ extern "C" QG_API qg_status qg_groupby_cols(qg_ctx *ctx, const int32_t *key, con
                    fused ? ((double)hi2 - (double)lo2 + 1.0) / 4294967296.0 : 1.0, &sc);
     const qg_status st = groupby_cols_impl(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, order,
                                            num_groups);
+    if (ctx && st == QG_OK && ctx->gb_first == 3 && !qg_gbw_few(n, *num_groups)) ctx->gb_first = 1;  // many groups by now
     qg_steer_end(ctx, &sc, st);
     return st;
 }
@@ -1632,8 +1633,9 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
         // more distinct keys than the small table takes: the general paths
     }
     // Wide keys: partitioned by key range, else the two-pass path below.  What
-    // the context's last such call took is launched first; a narrow range or a
-    // verdict against it leads to the others, so the path depends on the input.
+    // the context's last such call found says which is launched first (after an
+    // uneven or few-grouped input the dense window, then the two-pass path); each
+    // hands over by the input's own keys.
     bool wide_tried = false;
     auto wide = [&](uint32_t *verdict) -> qg_status {
         wide_tried = true;
@@ -1660,7 +1662,7 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
         QG_TRY(wide(&v));
         if (v == QG_GBW_DONE) return g > cap ? QG_ERR_CAPACITY : QG_OK;
         narrow = v == QG_GBW_NARROW;
-        if (!narrow) ctx->gb_first = 2;
+        if (!narrow) ctx->gb_first = v == QG_GBW_FEW ? 3 : 2;
     }
     if (gm == 0 && !global && n > 0 && narrow) {
         // Dense-window path: output in key order whatever `order` asks for;
@@ -1678,10 +1680,10 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
         }
         // some key fell outside the sampled window (or the sample spread too
         // wide for one)
-        if (may_wide && !wide_tried && ctx->gb_first != 2) {
+        if (may_wide && !wide_tried && ctx->gb_first < 2) {
             uint32_t v;
             QG_TRY(wide(&v));
-            ctx->gb_first = v == QG_GBW_DONE ? 1 : 2;
+            ctx->gb_first = v == QG_GBW_DONE ? 1 : v == QG_GBW_FEW ? 3 : 2;
             if (v == QG_GBW_DONE) return g > cap ? QG_ERR_CAPACITY : QG_OK;
         }
     }

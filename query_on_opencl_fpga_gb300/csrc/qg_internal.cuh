@@ -20,6 +20,7 @@ struct qg_control {
     uint32_t gbd[48];               // per-call state of the dense-window group-by (qg_gbdense.cu)
     uint32_t ghist[4 * 256];        // digit counts of emitted group keys (group-by in key order)
     uint32_t shist[4 * 256];        // a record sort's digit counts, zero between sorts
+    unsigned int gbw_few;           // the group-by's key sample shows few groups (written before it is read)
     unsigned long long gbw_rows;    // records appended by the wide-key group-by, zero between calls
     uint32_t jd[12];                // state of the counting join (qg_jdirect.cu)
     uint32_t jd_arrived, jd_pad;    // its scan's tiles that are done (wraps to zero)
@@ -65,7 +66,7 @@ struct qg_ctx {
     uint64_t launches;
     bool table_dirty;       // group-by table must be cleared before next use
     uint32_t gb_stats[4];   // last qg_groupby_cols: path, flags, fullest bucket, bucket cap
-    int gb_first;           // what the next default group-by launches first: 0 dense window, 1 wide keys
+    int gb_first;           // what the last default group-by found (qg_groupby.cu): 0 narrow keys, 1 wide ones, 2 uneven, 3 few
                             //   (qg_gbwide.cu), 2 dense window and no attempt at the wide keys' path after it
     bool gb_wide_keys;      // last key-ordered group-by's keys spanned too wide a range for the dense order
     uint32_t gb_kbase;      // first key of the next dense-order window (from the last call's keys)
@@ -129,13 +130,18 @@ enum qg_gbw_result : uint32_t {
     QG_GBW_NARROW = 0,  // the keys fit the dense window
     QG_GBW_DONE = 1,
     QG_GBW_OTHER = 2,   // parts too uneven, or with too many distinct keys
+    QG_GBW_FEW = 3,     // few groups among many rows: the two-pass path's tables hold them
 };
 bool qg_gbw_applies(int64_t n, int64_t cap);
 qg_status qg_gbw_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, const int32_t *val2, int32_t lo2,
                         int32_t hi2, int64_t n, int32_t *gkey, int64_t *gsum, int64_t *gcnt, int64_t cap,
                         volatile long long *d_num, volatile uint32_t *result);
 // Key range into ctl->gbd[0] (largest complement) and [1] (qg_gbdense.cu).
-qg_status qg_gbd_range(qg_ctx *ctx, const int32_t *key, int64_t n);
+// Key range into ctl->gbd; few_limit > 0: ctl->gbw_few = whether a sample of 4096
+// rows (n at least that) has at most that many distinct keys.
+qg_status qg_gbd_range(qg_ctx *ctx, const int32_t *key, int64_t n, uint32_t few_limit = 0);
+bool qg_gbw_few(int64_t n, int64_t groups);  // too few groups for the wide path
+
 
 // Operators the learned variant choice covers (the batch's OP_* order).
 enum { QG_STEER_FILTER = 0, QG_STEER_GROUPBY = 1, QG_STEER_FUSED = 2, QG_STEER_JOIN = 3, QG_STEER_OPS = 4 };

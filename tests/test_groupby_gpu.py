@@ -565,7 +565,7 @@ def test_groupby_dense_exact_range(ctx, orc, n, lo, span):
 # remainders, 128 and 256 parts, the key that marks free slots, parts of more
 # than 65536 rows (sums with a carry), few rows selected, none selected; inputs
 # it gives up: a few frequent keys (uneven parts), more distinct keys in a part
-# than its table takes.  In sequence on one context, with narrow keys between.
+# than its table takes, few groups among many rows.  In sequence on one context, with narrow keys between.
 def test_groupby_wide(ctx, orc):
     rng = np.random.default_rng(77)
     ids = rng.integers(-(2 ** 31), 2 ** 31, 1 << 20)
@@ -577,6 +577,8 @@ def test_groupby_wide(ctx, orc):
             return rng.permutation(n) * (2 ** 32 // n) - 2 ** 31
         if kind == "many_rows":
             return rng.choice(np.linspace(-(2 ** 31), 2 ** 31 - 1, 20).astype(np.int64), n)
+        if kind == "few":
+            return rng.choice(ids[:60], n)
         if kind == "uneven":
             return rng.choice(np.array([-(2 ** 31), 5, 2 ** 31 - 1]), n)
         if kind == "crowded":
@@ -587,7 +589,8 @@ def test_groupby_wide(ctx, orc):
 
     for n, kind in [(16_385, "ids"), (4096 * 5, "ids"), (70_001, "narrow"), (4096 * 9 + 1, "own"), (300_003, "ids"),
                     (1 << 20, "own"), (3_000_001, "many_rows"), (50_000, "uneven"), (100_003, "ids"),
-                    (120_000, "crowded"), (30_001, "narrow"), (4_000_002, "own"), (20_001, "ids")]:
+                    (120_000, "crowded"), (30_001, "narrow"), (4_000_002, "own"), (8_000_001, "few"),
+                    (6_100_000, "few"), (6_100_000, "ids"), (20_001, "ids")]:
         key = keys(kind, n).astype(np.int32)
         key[[3, n // 2]] = -1
         val = rng.choice(np.array([-(2 ** 31), 2 ** 31 - 1, -1, 65535, 65536, 7]), n).astype(np.int32)
