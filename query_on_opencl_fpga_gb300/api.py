@@ -18,10 +18,15 @@ INT32_MIN = -(2 ** 31)
 INT32_MAX = 2 ** 31 - 1
 
 
-def _ptr(t: torch.Tensor | None) -> c_void_p:
-    if t is None:
-        return c_void_p(0)
-    return c_void_p(t.data_ptr())
+def _ptr(t: torch.Tensor | None) -> int:
+    return 0 if t is None else t.data_ptr()
+
+
+def _first(t: torch.Tensor, n: int) -> torch.Tensor:
+    """The first n rows of a buffer allocated by the call, which it ends up as.
+
+    Shrinking it takes 0.3 us, a view of it 1 us and 4 right after a wait."""
+    return t.resize_(n, *t.shape[1:])
 
 
 def _check_dev(*ts: torch.Tensor | None) -> None:
@@ -146,7 +151,7 @@ class Context:
         cnt = c_int64()
         st = self.lib.qg_filter_range_rec(self.handle, _ptr(rec), n, lo, hi, _ptr(out), cap, byref(cnt))
         self.check(st, "qg_filter_range_rec")
-        return out[: cnt.value]
+        return _first(out, cnt.value)
 
     def filter_cols(self, key: torch.Tensor, pay: torch.Tensor, lo: int, hi: int,
                     cap: int | None = None, out: torch.Tensor | None = None):
@@ -157,7 +162,8 @@ class Context:
         _check_dev(key, pay)
         n = key.numel()
         cap = n if cap is None else cap
-        if out is None:
+        own = out is None
+        if own:
             out = torch.empty((max(cap, 1), 2), dtype=torch.int32, device=key.device)
         elif (out.dtype != torch.int32 or not out.is_cuda or not out.is_contiguous() or out.dim() != 2
               or out.shape[1] != 2 or out.shape[0] < max(cap, 1)):
@@ -166,7 +172,7 @@ class Context:
         st = self.lib.qg_filter_cols(self.handle, _ptr(key), _ptr(pay), n, lo, hi, _ptr(out), cap,
                                      byref(cnt))
         self.check(st, "qg_filter_cols")
-        return out[: cnt.value]
+        return _first(out, cnt.value) if own else out[: cnt.value]
 
     # ---- scan / sort ------------------------------------------------------
     def scan_excl(self, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -191,7 +197,7 @@ class Context:
         g = c_int64()
         st = self.lib.qg_groupby_rec(self.handle, _ptr(rec), n, _ptr(sorted_out), _ptr(sp), n, byref(g))
         self.check(st, "qg_groupby_rec")
-        return sorted_out, sp[: g.value]
+        return sorted_out, _first(sp, g.value)
 
     def aggregate_groups(self, sorted_rec: torch.Tensor, start_pos: torch.Tensor, op: int):
         _check_dev(sorted_rec, start_pos)
@@ -200,7 +206,7 @@ class Context:
         st = self.lib.qg_aggregate_groups(self.handle, _ptr(sorted_rec), sorted_rec.shape[0],
                                           _ptr(start_pos), g, op, _ptr(agg))
         self.check(st, "qg_aggregate_groups")
-        return agg[:g]
+        return _first(agg, g)
 
     def groupby_cols(self, key, val, val2=None, lo2: int = INT32_MIN, hi2: int = INT32_MAX,
                      cap: int = 1 << 20, order: int = QG_ORDER_KEY, out=None):
@@ -239,7 +245,7 @@ class Context:
                     ent[3].clear()
                 ent[3][m] = views
             return views
-        return gk[:m], gs[:m], gc[:m]
+        return _first(gk, m), _first(gs, m), _first(gc, m)
 
     def _out_entry(self, out, cap):
         """Validated (key, sum, count) output buffers, remembered for the last
@@ -286,7 +292,7 @@ class Context:
                 cap = m.value
                 continue
             self.check(st, "qg_join_filter_sort")
-            return ok[: m.value], orp[: m.value], osp[: m.value]
+            return _first(ok, m.value), _first(orp, m.value), _first(osp, m.value)
 
     def reduce_rec(self, rec: torch.Tensor, op: int) -> int:
         """SUM / MAX / MIN / AVERAGE (QG_REDUCE_*) of Record.y, unsigned 32-bit as the reference checks it."""
