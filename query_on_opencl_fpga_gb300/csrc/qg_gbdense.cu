@@ -390,6 +390,7 @@ template <bool SAMPLE>
 __global__ void __launch_bounds__(256)
 k_gbd_range(const int32_t *__restrict__ key, long long n, uint32_t *__restrict__ st, uint32_t few_limit,
             uint32_t *__restrict__ few) {
+    qg_chain();
     __shared__ uint32_t s[2];
     if (threadIdx.x < 2) s[threadIdx.x] = 0;
     if (SAMPLE && blockIdx.x == gridDim.x - 1) {
@@ -453,6 +454,7 @@ __global__ void __launch_bounds__(GBM_THREADS, 2)
 k_gbd_mid(const int32_t *__restrict__ key, const int32_t *__restrict__ val, const int32_t *__restrict__ val2,
           int32_t lo2, int32_t hi2, long long n, uint32_t *__restrict__ st, unsigned long long *__restrict__ dense,
           long long *__restrict__ extra, uint32_t shift, uint32_t fast_max) {
+    qg_chain();
     extern __shared__ __align__(16) unsigned char gbm_raw[];
     uint32_t *hk = reinterpret_cast<uint32_t *>(gbm_raw), *hc = hk + GBM_SLOTS, *hl = hc + GBM_SLOTS;
     const int tid = threadIdx.x;
@@ -657,6 +659,7 @@ k_gbd_emit(unsigned long long *__restrict__ dense, long long *__restrict__ extra
            unsigned long long *__restrict__ img, uint32_t *__restrict__ sketch, uint32_t *__restrict__ st,
            uint32_t shift, int32_t *__restrict__ gkey, long long *__restrict__ gsum, long long *__restrict__ gcnt,
            long long cap, long long *__restrict__ d_num, volatile uint32_t *outside, qg_lookback lb) {
+    qg_chain();
     __shared__ uint32_t s_tile, s_epoch, s_tot, s_wsum[GBD_ENW], s_off[GBD_EPER * GBD_ENW], s_tmp[2 * 8];
     if (img) gbd_clear_sample(img, sketch, blockIdx.x, gridDim.x);
     else if (blockIdx.x == 0 && threadIdx.x < 2) st[threadIdx.x == 0 ? G_NSMIN : G_SMAX] = 0;  // k_gbd_mid has read them
@@ -994,15 +997,12 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
                 QG_TRY_CUDA(ctx, cudaFuncSetAttribute(midf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm), "attr");
                 attr_mid[pred] = true;
             }
-            qg_pre_launch(ctx);
-            midf<<<mg, GBM_THREADS, sm, ctx->stream>>>(key, val, val2, lo2, hi2, n, st, dense, extra, shift, fast_max_mid);
-            s = qg_check_launch(ctx, "k_gbd_mid");
+            s = qg_launch_chained(ctx, "k_gbd_mid", midf, mg, GBM_THREADS, sm, key, val, val2, lo2, hi2, n, st, dense, extra,
+                                  shift, fast_max_mid);
         }
         if (s == QG_OK) {
-            qg_pre_launch(ctx);
-            k_gbd_emit<<<C, GBD_THREADS, 0, ctx->stream>>>(dense, extra, nullptr, nullptr, st, shift, gkey,
-                                                           (long long *)gsum, (long long *)gcnt, cap, d_num, outside, lb);
-            s = qg_check_launch(ctx, "k_gbd_emit");
+            s = qg_launch_chained(ctx, "k_gbd_emit", k_gbd_emit, C, GBD_THREADS, 0, dense, extra, nullptr, nullptr, st, shift,
+                                  gkey, (long long *)gsum, (long long *)gcnt, cap, d_num, outside, lb);
         }
         if (s != QG_OK) ctx->table_dirty = true;
         return s;

@@ -93,6 +93,35 @@ struct qg_ctx {
 // Record the start event of the next launch (no-op unless timing is on).
 void qg_pre_launch(qg_ctx *ctx);
 
+// Chained launches.  A kernel that calls qg_chain() before it touches memory may be
+// launched with qg_launch_chained: its CTAs are then set up while the kernel before
+// it in the stream ends, and wait in qg_chain() until that one's results are in.
+// (Whatever else runs before or after it is ordered as usual.)  A boundary between
+// two short kernels costs about CHAINNOTE.
+__device__ __forceinline__ void qg_chain() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+qg_status qg_check_launch(qg_ctx *ctx, const char *what);
+template <class... P, class... A>
+inline qg_status qg_launch_chained(qg_ctx *ctx, const char *what, void (*kern)(P...), unsigned grid, unsigned block,
+                                   size_t smem, A... args) {
+    qg_pre_launch(ctx);
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    return qg_check_launch(ctx, what);
+}
+
 // Site tags for the error word.
 enum {
     QG_SITE_FILTER = 1, QG_SITE_SCAN = 2, QG_SITE_SORT = 3, QG_SITE_GROUPBY = 4,

@@ -48,6 +48,7 @@ constexpr uint32_t JD_HERE = 0x80000000u;  // in an entry's count: R has the key
 
 __global__ void __launch_bounds__(JD_THREADS)
 k_jd_range(const int32_t *__restrict__ rkey, long long nR, uint32_t *jd) {
+    qg_chain();
     __shared__ uint32_t s[2];
     if (threadIdx.x < 2) s[threadIdx.x] = 0;
     __syncthreads();
@@ -78,6 +79,7 @@ k_jd_range(const int32_t *__restrict__ rkey, long long nR, uint32_t *jd) {
 
 __global__ void __launch_bounds__(JD_THREADS)
 k_jd_fill(unsigned long long *__restrict__ E, long long nR, uint32_t *__restrict__ jd) {
+    qg_chain();
     const uint32_t kmin = ~jd[JD_NKMIN], kmax = jd[JD_KMAX];
     const unsigned long long w = (unsigned long long)(kmax - kmin) + 1ull;
     const bool ok = w <= 2ull * (unsigned long long)nR;
@@ -98,6 +100,7 @@ k_jd_fill(unsigned long long *__restrict__ E, long long nR, uint32_t *__restrict
 __global__ void __launch_bounds__(JD_THREADS)
 k_jd_table(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, long long nR,
            unsigned long long *__restrict__ E, uint32_t *__restrict__ jd) {
+    qg_chain();
     if (blockIdx.x == 0 && threadIdx.x < 2) jd[JD_NKMIN + threadIdx.x] = 0;  // k_jd_fill has read them
     if (jd[JD_OK] != QG_JD_DONE) return;
     const uint32_t kmin = jd[JD_KMIN];
@@ -131,6 +134,7 @@ __global__ void __launch_bounds__(JD_THREADS, 4)
 k_jd_count(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, long long n, int32_t slo, int32_t shi,
            unsigned long long *__restrict__ E, uint32_t *__restrict__ jd, uint32_t *__restrict__ ak,
            uint32_t *__restrict__ ap, uint32_t *__restrict__ an) {
+    qg_chain();
     __shared__ uint32_t s_woff[JD_ROUNDS * JD_WARPS], s_base, s_cnt, s_stop;
     __shared__ unsigned long long s_row[JD_TILE];
     if (jd[JD_OK] != QG_JD_DONE) return;
@@ -233,6 +237,7 @@ __global__ void __launch_bounds__(JD_THREADS)
 k_jd_scan(unsigned long long *__restrict__ E, long long nR, uint32_t *__restrict__ jd, uint32_t *__restrict__ ok,
           uint32_t *__restrict__ oa, long long cap, long long *__restrict__ d_count, volatile uint32_t *result,
           uint32_t *__restrict__ arrived, qg_lookback lb) {
+    qg_chain();
     __shared__ uint32_t s_tile, s_epoch, s_excl, s_w[JD_WARPS], s_d[JD_WARPS], s_tmp[2 * JD_WARPS];
     qg_lb_begin_dyn(lb, &s_tile, &s_epoch);
     const uint32_t tile = s_tile, kmin = jd[JD_KMIN];
@@ -318,6 +323,7 @@ k_jd_scan(unsigned long long *__restrict__ E, long long nR, uint32_t *__restrict
 __global__ void __launch_bounds__(JD_THREADS)
 k_jd_write(const unsigned long long *__restrict__ E, const uint32_t *__restrict__ jd, const uint32_t *__restrict__ ak,
            const uint32_t *__restrict__ ap, const uint32_t *__restrict__ an, uint32_t *__restrict__ ob, long long cap) {
+    qg_chain();
     if (jd[JD_OK] != QG_JD_DONE) return;
     const long long n = jd[JD_ROWS], stride = (long long)gridDim.x * JD_THREADS;
     constexpr int U = 4;
@@ -360,25 +366,14 @@ qg_status qg_jd_launch(qg_ctx *ctx, char *work, const int32_t *rkey, const int32
     qg_pre_launch(ctx);
     k_jd_range<<<jd_grid(ctx, nR, 4 * JD_THREADS, 4), JD_THREADS, 0, ctx->stream>>>(rkey, nR, jd);
     QG_TRY(qg_check_launch(ctx, "k_jd_range"));
-    qg_pre_launch(ctx);
-    k_jd_fill<<<jd_grid(ctx, nR, 2 * JD_THREADS, 8), JD_THREADS, 0, ctx->stream>>>(E, nR, jd);
-    QG_TRY(qg_check_launch(ctx, "k_jd_fill"));
-    qg_pre_launch(ctx);
-    k_jd_table<<<jd_grid(ctx, nR, JD_THREADS, 8), JD_THREADS, 0, ctx->stream>>>(rkey, rpay, nR, E, jd);
-    QG_TRY(qg_check_launch(ctx, "k_jd_table"));
-    qg_pre_launch(ctx);
-    k_jd_count<<<jd_grid(ctx, nS, JD_TILE, 4), JD_THREADS, 0, ctx->stream>>>(skey, spay, nS, slo, shi, E, jd, ak, ap, an);
-    QG_TRY(qg_check_launch(ctx, "k_jd_count"));
+    QG_TRY(qg_launch_chained(ctx, "k_jd_fill", k_jd_fill, jd_grid(ctx, nR, 2 * JD_THREADS, 8), JD_THREADS, 0, E, nR, jd));
+    QG_TRY(qg_launch_chained(ctx, "k_jd_table", k_jd_table, jd_grid(ctx, nR, JD_THREADS, 8), JD_THREADS, 0, rkey, rpay, nR, E, jd));
+    QG_TRY(qg_launch_chained(ctx, "k_jd_count", k_jd_count, jd_grid(ctx, nS, JD_TILE, 4), JD_THREADS, 0, skey, spay, nS, slo, shi, E, jd, ak, ap, an));
     // few entries: more, smaller tiles (2K build rows 15 us with 16 entries per lane)
     const int per = nR <= (1 << 18) ? 2 : 16;
     const long long tiles = qg_ceil_div(2 * nR, per * JD_THREADS);
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, tiles, QG_SITE_JOIN_PROBE, &lb));
-    qg_pre_launch(ctx);
-    (per == 2 ? k_jd_scan<2> : k_jd_scan<16>)<<<(unsigned)tiles, JD_THREADS, 0, ctx->stream>>>(
-        E, nR, jd, out_key, out_rpay, cap, d_count, result, &ctx->ctl->jd_arrived, lb);
-    QG_TRY(qg_check_launch(ctx, "k_jd_scan"));
-    qg_pre_launch(ctx);
-    k_jd_write<<<jd_grid(ctx, nS / 4, JD_THREADS, 8), JD_THREADS, 0, ctx->stream>>>(E, jd, ak, ap, an, out_spay, cap);
-    return qg_check_launch(ctx, "k_jd_write");
+    QG_TRY(qg_launch_chained(ctx, "k_jd_scan", per == 2 ? k_jd_scan<2> : k_jd_scan<16>, (unsigned)tiles, JD_THREADS, 0, E, nR, jd, out_key, out_rpay, cap, d_count, result, &ctx->ctl->jd_arrived, lb));
+    return qg_launch_chained(ctx, "k_jd_write", k_jd_write, jd_grid(ctx, nS / 4, JD_THREADS, 8), JD_THREADS, 0, E, jd, ak, ap, an, out_spay, cap);
 }
