@@ -195,6 +195,7 @@ QG_API qg_status qg_batch_create(const qg_query *queries, int nq, int autotune, 
             cudaEventCreateWithFlags(&b->join[l], cudaEventDisableTiming) != cudaSuccess)
             st = QG_ERR_CUDA;
         if (st == QG_OK) st = qg_ctx_create(&b->own[l], b->ls[l]);
+        if (st == QG_OK) b->own[l]->unchained = true;
     }
     if (st != QG_OK) {
         cudaGetLastError();

@@ -92,7 +92,7 @@ enum {
     G_KBASE = 3,   // first key of the window
     G_NUMIN = 4,   // ~(smallest window offset of a counted row), by atomicMax
     G_UMAX = 5,    // largest window offset of a counted row
-    G_OUTSIDE = QG_GBD_OUTSIDE,  // rows outside the window (or 1 when no window)
+    G_OUTSIDE = QG_GBD_OUTSIDE, // rows outside the window (or 1 when no window)
     G_EXTRA = 7,   // 1: some value went to the extra (int64) table
     G_BAR = 8,     // k_gbd_single: grid barrier arrivals
     G_WORDS = 9
@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(GBD_SAMPLE_THREADS)
 k_gbd_sample(const int32_t *__restrict__ key, long long n, int runs, bool every_row,
              uint32_t *__restrict__ sketch, uint32_t *__restrict__ lst, uint32_t *__restrict__ lcnt,
              uint32_t *__restrict__ st) {
+    qg_chain();
     __shared__ uint32_t tkey[GBD_SSLOTS], tcnt[GBD_SSLOTS], s_n, s_mm[2];
     for (int i = threadIdx.x; i < GBD_SSLOTS; i += GBD_SAMPLE_THREADS) {
         tkey[i] = GBD_EMPTY;
@@ -220,6 +221,7 @@ __global__ void __launch_bounds__(GBD_CANDS_THREADS)
 k_gbd_cands(const uint32_t *__restrict__ sketch, const uint32_t *__restrict__ lst,
             const uint32_t *__restrict__ lcnt, unsigned long long *__restrict__ img, uint32_t min_count,
             uint32_t *__restrict__ st) {
+    qg_chain();
     const uint32_t m = lcnt[blockIdx.x];
     const uint32_t *mine = lst + (size_t)blockIdx.x * GBD_LIST;
     constexpr int PER = GBD_LIST / GBD_CANDS_THREADS;
@@ -366,6 +368,7 @@ k_gbd_main(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
            int32_t lo2, int32_t hi2, long long n, const unsigned long long *__restrict__ img,
            uint32_t *__restrict__ st, unsigned long long *__restrict__ dense, long long *__restrict__ extra,
            uint32_t shift, uint32_t fast_max) {
+    qg_chain();
     extern __shared__ __align__(16) unsigned char gbd_main_raw[];
     __shared__ uint32_t s_red[4];
     if (!st[G_OK]) {  // no window: the caller takes the two-pass path
@@ -997,12 +1000,12 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
                 QG_TRY_CUDA(ctx, cudaFuncSetAttribute(midf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm), "attr");
                 attr_mid[pred] = true;
             }
-            s = qg_launch_chained(ctx, "k_gbd_mid", midf, mg, GBM_THREADS, sm, key, val, val2, lo2, hi2, n, st, dense, extra,
-                                  shift, fast_max_mid);
+            s = qg_launch_chained(ctx, "k_gbd_mid", midf, mg, GBM_THREADS, sm, key, val, val2, lo2, hi2, n, st, dense,
+                                  extra, shift, fast_max_mid);
         }
         if (s == QG_OK) {
-            s = qg_launch_chained(ctx, "k_gbd_emit", k_gbd_emit, C, GBD_THREADS, 0, dense, extra, nullptr, nullptr, st, shift,
-                                  gkey, (long long *)gsum, (long long *)gcnt, cap, d_num, outside, lb);
+            s = qg_launch_chained(ctx, "k_gbd_emit", k_gbd_emit, C, GBD_THREADS, 0, dense, extra, nullptr, nullptr, st,
+                                  shift, gkey, (long long *)gsum, (long long *)gcnt, cap, d_num, outside, lb);
         }
         if (s != QG_OK) ctx->table_dirty = true;
         return s;
@@ -1012,22 +1015,16 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
                                                                           st);
     s = qg_check_launch(ctx, "k_gbd_sample");
     if (s == QG_OK) {
-        qg_pre_launch(ctx);
-        k_gbd_cands<<<GBD_SAMPLE_CTAS, GBD_CANDS_THREADS, 0, ctx->stream>>>(sketch, lst, lcnt, img,
-                                                                            every_row ? 1u : 2u, st);
-        s = qg_check_launch(ctx, "k_gbd_cands");
+        s = qg_launch_chained(ctx, "k_gbd_cands", k_gbd_cands, GBD_SAMPLE_CTAS, GBD_CANDS_THREADS, 0, sketch, lst,
+                              lcnt, img, every_row ? 1u : 2u, st);
     }
     if (s == QG_OK && n > 0) {
-        qg_pre_launch(ctx);
-        mainf<<<C, GBD_THREADS, smem_main, ctx->stream>>>(key, val, val2, lo2, hi2, n, img, st, dense, extra,
-                                                          shift, fast_max);
-        s = qg_check_launch(ctx, pred ? "k_gbd_main_fused" : "k_gbd_main");
+        s = qg_launch_chained(ctx, pred ? "k_gbd_main_fused" : "k_gbd_main", mainf, C, GBD_THREADS, smem_main, key,
+                              val, val2, lo2, hi2, n, img, st, dense, extra, shift, fast_max);
     }
     if (s == QG_OK) {
-        qg_pre_launch(ctx);
-        k_gbd_emit<<<C, GBD_THREADS, 0, ctx->stream>>>(dense, extra, img, sketch, st, shift, gkey, (long long *)gsum,
-                                                       (long long *)gcnt, cap, d_num, outside, lb);
-        s = qg_check_launch(ctx, "k_gbd_emit");
+        s = qg_launch_chained(ctx, "k_gbd_emit", k_gbd_emit, C, GBD_THREADS, 0, dense, extra, img, sketch, st, shift,
+                              gkey, (long long *)gsum, (long long *)gcnt, cap, d_num, outside, lb);
     }
     if (s != QG_OK) ctx->table_dirty = true;  // the dense table may hold partial sums
     return s;

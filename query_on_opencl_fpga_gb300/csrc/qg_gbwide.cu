@@ -59,6 +59,7 @@ k_gbw_rows(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
            int32_t lo2, int32_t hi2, long long n, const uint32_t *__restrict__ range, uint32_t window, int parts_log2,
            const uint32_t *__restrict__ few, unsigned long long *__restrict__ rec, uint32_t *__restrict__ hist,
            unsigned long long *__restrict__ rows, uint4 *__restrict__ clear, long long clear_n) {
+    qg_chain();
     __shared__ uint32_t s_h[GW_PARTS], s_woff[32], s_cnt;
     __shared__ unsigned long long s_base;
     __shared__ unsigned long long s_row[PRED ? GW_TILE : 1];
@@ -177,6 +178,7 @@ __global__ void __launch_bounds__(GW_PARTS)
 k_gbw_plan(const uint32_t *__restrict__ range, uint32_t window, int parts_log2, const uint32_t *__restrict__ few,
            uint32_t *__restrict__ hist, unsigned long long *__restrict__ rows, GwState *__restrict__ W, const unsigned long long *r0,
            unsigned long long *r1, uint32_t *status) {
+    qg_chain();
     __shared__ uint32_t ws[GW_PARTS / 32], wm[GW_PARTS / 32];
     const int d = threadIdx.x, lane = d & 31, w = d >> 5;
     const uint32_t kmin = ~range[0], span = range[1] - kmin;
@@ -217,6 +219,7 @@ __global__ void __launch_bounds__(QG_CS_THREADS, 1)
 k_gbw_merge(GwState *__restrict__ W, const unsigned long long *__restrict__ rec, uint32_t slots,
             int32_t *__restrict__ gkey, long long *__restrict__ gsum, long long *__restrict__ gcnt, long long cap,
             uint32_t *__restrict__ range, volatile long long *d_num, volatile uint32_t *result, qg_lookback lb) {
+    qg_chain();
     extern __shared__ __align__(16) unsigned char gw_raw[];
     __shared__ uint32_t s_tile, s_epoch, s_full, s_n, s_excl, s_tmp[16];
     const int tid = threadIdx.x, lane = tid & 31;
@@ -369,17 +372,12 @@ qg_status qg_gbw_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
     const uint32_t limit = gw_few_limit(n), *few = limit ? &ctx->ctl->gbw_few : nullptr;
     QG_TRY(qg_gbd_range(ctx, key, n, limit));
     const unsigned grid = (unsigned)std::min<long long>(qg_ceil_div(n, GW_TILE), 4LL * ctx->sm_count);
-    qg_pre_launch(ctx);
-    (pred ? k_gbw_rows<true> : k_gbw_rows<false>)<<<grid, GW_THREADS, 0, ctx->stream>>>(
-        key, val, val2, lo2, hi2, n, range, window, plog2, few, r0, hist, &ctx->ctl->gbw_rows, (uint4 *)status,
-        (long long)(words / 4));
-    QG_TRY(qg_check_launch(ctx, "k_gbw_rows"));
-    qg_pre_launch(ctx);
-    k_gbw_plan<<<1, GW_PARTS, 0, ctx->stream>>>(range, window, plog2, few, hist, &ctx->ctl->gbw_rows, W, r0, r1, status);
-    QG_TRY(qg_check_launch(ctx, "k_gbw_plan"));
+    QG_TRY(qg_launch_chained(ctx, "k_gbw_rows", (pred ? k_gbw_rows<true> : k_gbw_rows<false>), grid, GW_THREADS, 0,
+                             key, val, val2, lo2, hi2, n, range, window, plog2, few, r0, hist, &ctx->ctl->gbw_rows,
+                             (uint4 *)status, (long long)(words / 4)));
+    QG_TRY(qg_launch_chained(ctx, "k_gbw_plan", k_gbw_plan, 1, GW_PARTS, 0, range, window, plog2, few, hist,
+                             &ctx->ctl->gbw_rows, W, r0, r1, status));
     QG_TRY(qg_radix_pass_planned(ctx, &W->pass, W->base, n, &W->rows));
-    qg_pre_launch(ctx);
-    k_gbw_merge<<<1u << plog2, QG_CS_THREADS, gw_smem(slots), ctx->stream>>>(
-        W, r1, slots, gkey, (long long *)gsum, (long long *)gcnt, cap, range, d_num, result, lb);
-    return qg_check_launch(ctx, "k_gbw_merge");
+    return qg_launch_chained(ctx, "k_gbw_merge", k_gbw_merge, 1u << plog2, QG_CS_THREADS, gw_smem(slots), W, r1, slots,
+                             gkey, (long long *)gsum, (long long *)gcnt, cap, range, d_num, result, lb);
 }

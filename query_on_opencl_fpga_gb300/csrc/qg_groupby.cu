@@ -49,6 +49,7 @@ constexpr int GH_SUNITS = 32;                       // units of a warp whose hea
 __global__ void __launch_bounds__(32 * GH_MAX_WARPS, 1)
 k_group_bounds(const uint2 *__restrict__ in, long long n, long long units, int32_t *__restrict__ startPos,
                long long cap, long long *__restrict__ d_count, uint8_t *__restrict__ spill, qg_lookback lb) {
+    qg_chain();
     extern __shared__ __align__(16) unsigned char gh_raw[];
     __shared__ uint32_t s_tile, s_epoch, s_excl, s_cnt[GH_MAX_WARPS], s_tmp[2 * GH_MIN_WARPS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -144,6 +145,7 @@ __device__ __forceinline__ int32_t agg_op(int32_t a, int32_t b) {
 }
 
 __global__ void k_agg_init(int32_t *agg, long long g0, long long g1, int op) {
+    qg_chain();
     long long stride = (long long)gridDim.x * blockDim.x;
     int32_t id = agg_identity(op);
     for (long long i = g0 + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < g1; i += stride)
@@ -162,6 +164,7 @@ template <int OP, bool AVG, bool VEC>
 __global__ void __launch_bounds__(32 * AGG_WARPS, 4)
 k_agg_chunks(const uint2 *__restrict__ rec, long long n, const int32_t *__restrict__ startPos, long long G,
              long long g0, long long g1, int32_t *__restrict__ agg) {
+    qg_chain();
     __shared__ int32_t s_x[AGG_WARPS][AGG_PAD];
     __shared__ uint32_t s_head[AGG_WARPS][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -305,6 +308,7 @@ k_agg_chunks(const uint2 *__restrict__ rec, long long n, const int32_t *__restri
 // AVG of groups that spanned chunks: the atomics left the wrapped sum.
 __global__ void k_agg_avg_finish(const int32_t *__restrict__ startPos, long long n, long long G,
                                  long long g0, long long g1, int32_t *__restrict__ agg) {
+    qg_chain();
     long long stride = (long long)gridDim.x * blockDim.x;
     for (long long g = g0 + (long long)blockIdx.x * blockDim.x + threadIdx.x; g < g1; g += stride) {
         long long gs = startPos[g], ge = (g == G - 1) ? n : startPos[g + 1];
@@ -473,6 +477,7 @@ __global__ void k_groupby_gather(const unsigned long long *__restrict__ rec, lon
                                  const long long *__restrict__ tsum, const long long *__restrict__ tcnt,
                                  int32_t *__restrict__ gkey, long long *__restrict__ gsum,
                                  long long *__restrict__ gcnt, const long long *__restrict__ d_n) {
+    qg_chain();
     if (d_n && *d_n < g) g = *d_n;
     long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < g; i += stride) {
@@ -777,6 +782,7 @@ k_gb_merge(GbSpill sp, int C, int32_t *__restrict__ gkey, long long *__restrict_
            unsigned long long *__restrict__ rec, unsigned int *__restrict__ flags,
            unsigned int *__restrict__ work, uint32_t *__restrict__ ghist, uint32_t *__restrict__ mm,
            uint32_t *__restrict__ bits, uint32_t kbase) {
+    qg_chain();
     constexpr int T = 1 << P2_TLOG2;
     constexpr int NB = T / 4;
     constexpr int W = P2_THREADS / 32;
@@ -1043,6 +1049,7 @@ __host__ __device__ __forceinline__ bool gb_dense_fits(uint32_t lo, uint32_t hi,
 __global__ void __launch_bounds__(DN_THREADS)
 k_gb_dense_scan(uint32_t *__restrict__ bits, uint2 *__restrict__ pre, const uint32_t *__restrict__ mm,
                 uint32_t kbase, qg_lookback lb) {
+    qg_chain();
     constexpr int NW = DN_THREADS / 32;
     constexpr uint32_t ROUND = DN_THREADS * DN_WPT;
     __shared__ uint32_t s_tile, s_epoch, s_excl;
@@ -1129,6 +1136,7 @@ k_gb_dense_place(const unsigned long long *__restrict__ rec, long long cap, cons
                  const uint32_t *__restrict__ mm, uint32_t kbase, const uint2 *__restrict__ pre,
                  const long long *__restrict__ tsum, const long long *__restrict__ tcnt,
                  int32_t *__restrict__ gkey, long long *__restrict__ gsum, long long *__restrict__ gcnt) {
+    qg_chain();
     uint32_t w0, w1;
     if (!gb_dense_fits(~mm[0], mm[1], kbase, &w0, &w1)) return;
     const long long g = *d_n < cap ? *d_n : cap;
@@ -1190,10 +1198,9 @@ extern "C" QG_API qg_status qg_groupby_rec(qg_ctx *ctx, const void *in, int64_t 
     }
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, grid, QG_SITE_GROUPBY, &lb));
-    qg_pre_launch(ctx);
-    k_group_bounds<<<(unsigned)grid, (unsigned)(32 * warps), smem, ctx->stream>>>(
-        (const uint2 *)sorted_out, n, units, startPos, cap_groups, (long long *)&ctx->hres->count, spill, lb);
-    QG_TRY(qg_check_launch(ctx, "k_group_bounds"));
+    QG_TRY(qg_launch_chained(ctx, "k_group_bounds", k_group_bounds, (unsigned)grid, (unsigned)(32 * warps), smem,
+                             (const uint2 *)sorted_out, n, units, startPos, cap_groups, (long long *)&ctx->hres->count,
+                             spill, lb));
     long long h = 0;
     QG_TRY(qg_host_count(ctx, &h));
     if (in == sorted_out) qg_sort_remember(ctx);
@@ -1222,13 +1229,10 @@ extern "C" QG_API qg_status qg_aggregate_group_range(qg_ctx *ctx, const void *so
                 : op == QG_REDUCE_MIN     ? (vec ? k_agg_chunks<QG_REDUCE_MIN, false, true> : k_agg_chunks<QG_REDUCE_MIN, false, false>)
                 : op == QG_REDUCE_AVERAGE ? (vec ? k_agg_chunks<QG_REDUCE_SUM, true, true> : k_agg_chunks<QG_REDUCE_SUM, true, false>)
                                           : (vec ? k_agg_chunks<QG_REDUCE_SUM, false, true> : k_agg_chunks<QG_REDUCE_SUM, false, false>);
-    qg_pre_launch(ctx);
-    kern<<<blocks, 32 * AGG_WARPS, 0, ctx->stream>>>((const uint2 *)sorted, n, startPos, G, g0, g1, agg);
-    QG_TRY(qg_check_launch(ctx, "k_agg_chunks"));
+    QG_TRY(qg_launch_chained(ctx, "k_agg_chunks", kern, blocks, 32 * AGG_WARPS, 0, (const uint2 *)sorted, n, startPos,
+                             G, g0, g1, agg));
     if (op == QG_REDUCE_AVERAGE) {
-        qg_pre_launch(ctx);
-        k_agg_avg_finish<<<ib, 256, 0, ctx->stream>>>(startPos, n, G, g0, g1, agg);
-        QG_TRY(qg_check_launch(ctx, "k_agg_avg_finish"));
+        QG_TRY(qg_launch_chained(ctx, "k_agg_avg_finish", k_agg_avg_finish, ib, 256, 0, startPos, n, G, g0, g1, agg));
     }
     return qg_ctx_check(ctx);
 }
@@ -1467,10 +1471,8 @@ static qg_status gb_key_order_dev(qg_ctx *ctx, const GbOut &o, int64_t cap, long
                                work, &in_b));
     if (in_b) return QG_ERR_INVALID;  // four passes end where they began
     const int gb = grid_for(ctx, cap, 256, 8);
-    qg_pre_launch(ctx);
-    k_groupby_gather<<<gb, 256, 0, ctx->stream>>>(o.rec, cap, o.s, o.c, gkey, (long long *)gsum,
-                                                  (long long *)gcnt, d_num);
-    return qg_check_launch(ctx, "k_groupby_gather");
+    return qg_launch_chained(ctx, "k_groupby_gather", k_groupby_gather, gb, 256, 0, o.rec, cap, o.s, o.c, gkey,
+                             (long long *)gsum, (long long *)gcnt, d_num);
 }
 
 // Dense key order after a merge that set the window's bits (see
@@ -1494,10 +1496,8 @@ static qg_status gb_key_order_dense(qg_ctx *ctx, const GbOut &o, int64_t cap, co
     }
     if (cap <= 0) return QG_OK;
     const int gb = grid_for(ctx, cap, 256, 8);
-    qg_pre_launch(ctx);
-    k_gb_dense_place<<<gb, 256, 0, ctx->stream>>>(o.rec, cap, d_num, mm, kbase, (const uint2 *)prep, o.s, o.c,
-                                                  gkey, (long long *)gsum, (long long *)gcnt);
-    return qg_check_launch(ctx, "k_gb_dense_place");
+    return qg_launch_chained(ctx, "k_gb_dense_place", k_gb_dense_place, gb, 256, 0, o.rec, cap, d_num, mm, kbase,
+                             (const uint2 *)prep, o.s, o.c, gkey, (long long *)gsum, (long long *)gcnt);
 }
 
 // The next call's window: centred on this call's keys (so that a range that
@@ -1745,10 +1745,8 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
         unsigned long long *tmp = (unsigned long long *)(o.c + (cap > 0 ? cap : 1));
         QG_TRY(qg_sort_rec(ctx, o.rec, o.rec, tmp, g));
         int gb = grid_for(ctx, g, 256, 8);
-        qg_pre_launch(ctx);
-        k_groupby_gather<<<gb, 256, 0, ctx->stream>>>(o.rec, g, o.s, o.c, gkey, (long long *)gsum,
-                                                      (long long *)gcnt, nullptr);
-        QG_TRY(qg_check_launch(ctx, "k_groupby_gather"));
+        QG_TRY(qg_launch_chained(ctx, "k_groupby_gather", k_groupby_gather, gb, 256, 0, o.rec, g, o.s, o.c, gkey,
+                                 (long long *)gsum, (long long *)gcnt, nullptr));
         return qg_ctx_check(ctx);
     } else if (order == QG_ORDER_KEY && g == 1) {
         QG_TRY_CUDA(ctx, cudaMemcpyAsync(gsum, o.s, 8, cudaMemcpyDeviceToDevice, ctx->stream), "copy");

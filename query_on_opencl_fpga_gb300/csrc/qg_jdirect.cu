@@ -35,7 +35,7 @@ namespace {
 // Words of ctl->jd.  The first two are zero between calls: the smallest key is
 // kept as the largest complement.
 enum {
-    JD_NKMIN = 0, JD_KMAX = 1,  // ~(smallest key), largest key (unsigned)
+    JD_NKMIN = 0, JD_KMAX = 1, // ~(smallest key), largest key (unsigned)
     JD_OK = QG_JD_OK,           // a qg_jd_result: QG_JD_DONE while nothing speaks against the path
     JD_KMIN = 5, JD_SPAN = 6,   // first key and number of key values of the table
     JD_DISTINCT = 8,            // table entries of R's keys

@@ -63,6 +63,7 @@ constexpr size_t REF_HASH_HDR = (sizeof(RefHashHdr) + 255) / 256 * 256;
 __device__ __forceinline__ uint32_t join_group(uint32_t k, uint32_t mask) { return qg_hash32(k) & mask & ~3u; }
 
 __global__ void k_join_ctl_init(JoinCtl *jc) {
+    qg_chain();
     int t = threadIdx.x;
     if (t == 0) {
         jc->kmin = 0xffffffffu;
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(256)
 k_join_build(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, long long stride_el,
              long long nR, unsigned long long *__restrict__ tab, uint32_t mask, JoinCtl *jc,
              qg_control *ctl, uint32_t most_probes) {
+    qg_chain();
     uint32_t lmin = 0xffffffffu, lmax = 0;
     unsigned long long nspec = 0;
     bool twice = false;
@@ -159,6 +161,7 @@ __global__ void __launch_bounds__(PJ_THREADS, 4)
 k_join_probe(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, long long nS,
              int32_t slo, int32_t shi, const unsigned long long *__restrict__ tab, uint32_t mask,
              JoinCtl *jc, ProbeOut out, ProbeOut odd, long long cap, int npos) {
+    qg_chain();
     extern __shared__ __align__(16) unsigned char pj_raw[];
     PjSmem &S = *reinterpret_cast<PjSmem *>(pj_raw);
     if (jc->crowded) return;
@@ -445,10 +448,8 @@ static qg_status join_build(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpa
     QG_TRY(qg_check_launch(ctx, "k_join_ctl_init"));
     if (nR > 0) {
         int blocks = grid_cap(ctx, nR, 256, 8);
-        qg_pre_launch(ctx);
-        k_join_build<<<blocks, 256, 0, ctx->stream>>>(rkey, rpay, stride, nR, tab, slots - 1, jc,
-                                                      ctx->ctl, most_probes);
-        QG_TRY(qg_check_launch(ctx, "k_join_build"));
+        QG_TRY(qg_launch_chained(ctx, "k_join_build", k_join_build, blocks, 256, 0, rkey, rpay, stride, nR, tab,
+                                 slots - 1, jc, ctx->ctl, most_probes));
     }
     *tab_out = tab;
     *mask_out = slots - 1;
@@ -461,6 +462,7 @@ namespace {
 // A few matches: sorted by key by one CTA and written to the output columns.
 __global__ void __launch_bounds__(QG_CS_THREADS, 1)
 k_join_sort_small(qg_sort_bufs in, qg_sort_bufs out, uint32_t n) {
+    qg_chain();
     extern __shared__ __align__(16) unsigned char js_raw[];
     uint32_t(*whist)[256] = reinterpret_cast<uint32_t(*)[256]>(js_raw);
     unsigned long long *ord = reinterpret_cast<unsigned long long *>(whist + 32);
@@ -488,9 +490,8 @@ static qg_status join_probe(qg_ctx *ctx, const int32_t *skey, const int32_t *spa
     }
     const long long ntiles = (nS + PJ_TILE - 1) / PJ_TILE;
     const int blocks = (int)(ntiles < (long long)ctx->sm_count * 4 ? ntiles : (long long)ctx->sm_count * 4);
-    qg_pre_launch(ctx);
-    k_join_probe<<<blocks, PJ_THREADS, smem, ctx->stream>>>(skey, spay, nS, slo, shi, tab, mask, jc, po, odd, cap, 4);
-    return qg_check_launch(ctx, "k_join_probe");
+    return qg_launch_chained(ctx, "k_join_probe", k_join_probe, blocks, PJ_THREADS, smem, skey, spay, nS, slo, shi,
+                             tab, mask, jc, po, odd, cap, 4);
 }
 
 // Hash join + filter + radix sort of the output: the variant of
@@ -653,10 +654,8 @@ extern "C" QG_API qg_status qg_hash_build_ref(qg_ctx *ctx, const uint32_t *r, in
     QG_TRY(qg_check_launch(ctx, "k_ref_hash_hdr_init"));
     if (nR > 0) {
         int blocks = grid_cap(ctx, nR, 256, 8);
-        qg_pre_launch(ctx);
-        k_join_build<<<blocks, 256, 0, ctx->stream>>>((const int32_t *)r, (const int32_t *)r + 1, 2, nR, tab,
-                                                      slots - 1, &hdr->jc, ctx->ctl, 0u);
-        QG_TRY(qg_check_launch(ctx, "k_join_build"));
+        QG_TRY(qg_launch_chained(ctx, "k_join_build", k_join_build, blocks, 256, 0, (const int32_t *)r,
+                                 (const int32_t *)r + 1, 2, nR, tab, slots - 1, &hdr->jc, ctx->ctl, 0u));
     }
     // a table that fills up (cannot happen at 2 slots per row) reports TABLE_FULL
     return qg_ctx_check(ctx);

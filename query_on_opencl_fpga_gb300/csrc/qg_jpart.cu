@@ -81,6 +81,7 @@ __device__ __forceinline__ bool jp_dense(const qg_jp_r &r, uint32_t *kmin, uint3
 __global__ void __launch_bounds__(1024)
 k_jp_sample(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, long long chunks, int32_t slo,
             int32_t shi, qg_jp_r r, JpPlan *__restrict__ P) {
+    qg_chain();
     __shared__ uint32_t h[JP_BINS];
     uint32_t kmin, span;
     if (!jp_dense(r, &kmin, &span)) return;
@@ -106,6 +107,7 @@ k_jp_sample(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, 
 // One CTA.  room: rows that the buckets may take together.
 __global__ void __launch_bounds__(1024)
 k_jp_plan(long long nS, long long chunks, long long room, qg_jp_r r, JpPlan *__restrict__ P) {
+    qg_chain();
     __shared__ uint32_t cum[JP_BINS + 1], ws[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t kmin, span;
@@ -175,6 +177,7 @@ struct JpTile {
 __global__ void __launch_bounds__(JPP_THREADS, 1)
 k_jp_part(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, uint32_t n, int32_t slo, int32_t shi,
           JpPlan *__restrict__ P, unsigned long long *__restrict__ out) {
+    qg_chain();
     extern __shared__ __align__(16) unsigned char jp_raw[];
     JpTile &S = *reinterpret_cast<JpTile *>(jp_raw);
     __shared__ uint32_t s_rows, s_w[JPP_WARPS];
@@ -319,6 +322,7 @@ __global__ void __launch_bounds__(JP_THREADS, 2)
 k_jp_join(JpPlan *__restrict__ P, const unsigned long long *__restrict__ rows, qg_jp_r r, uint32_t *__restrict__ ok,
           uint32_t *__restrict__ oa, uint32_t *__restrict__ ob, long long cap, volatile long long *d_count,
           volatile uint32_t *result, qg_lookback lb) {
+    qg_chain();
     extern __shared__ __align__(16) unsigned char jp_raw[];
     JpBucket &S = *reinterpret_cast<JpBucket *>(jp_raw);
     __shared__ uint32_t s_tile, s_epoch, s_excl, s_w[JP_WARPS];
@@ -478,14 +482,9 @@ qg_status qg_jp_launch(qg_ctx *ctx, char *work, const qg_jp_r &r, const int32_t 
     qg_pre_launch(ctx);
     k_jp_sample<<<(unsigned)ctx->sm_count, 1024, 0, ctx->stream>>>(skey, spay, chunks, slo, shi, r, P);
     QG_TRY(qg_check_launch(ctx, "k_jp_sample"));
-    qg_pre_launch(ctx);
-    k_jp_plan<<<1, 1024, 0, ctx->stream>>>(nS, chunks, room, r, P);
-    QG_TRY(qg_check_launch(ctx, "k_jp_plan"));
-    qg_pre_launch(ctx);
-    k_jp_part<<<(unsigned)ctx->sm_count, JPP_THREADS, sizeof(JpTile), ctx->stream>>>(skey, spay, (uint32_t)nS, slo, shi, P, rows);
-    QG_TRY(qg_check_launch(ctx, "k_jp_part"));
-    qg_pre_launch(ctx);
-    k_jp_join<<<2 * (unsigned)ctx->sm_count, JP_THREADS, sizeof(JpBucket), ctx->stream>>>(P, rows, r, out_key, out_rpay, out_spay, cap,
-                                                                          d_count, result, lb);
-    return qg_check_launch(ctx, "k_jp_join");
+    QG_TRY(qg_launch_chained(ctx, "k_jp_plan", k_jp_plan, 1, 1024, 0, nS, chunks, room, r, P));
+    QG_TRY(qg_launch_chained(ctx, "k_jp_part", k_jp_part, (unsigned)ctx->sm_count, JPP_THREADS, sizeof(JpTile), skey,
+                             spay, (uint32_t)nS, slo, shi, P, rows));
+    return qg_launch_chained(ctx, "k_jp_join", k_jp_join, 2 * (unsigned)ctx->sm_count, JP_THREADS, sizeof(JpBucket), P,
+                             rows, r, out_key, out_rpay, out_spay, cap, d_count, result, lb);
 }

@@ -98,6 +98,7 @@ struct PjPackOut {
 
 // One CTA: the head block (range, digit histograms, flags) of a new call.
 __global__ void k_pj_range_init(PjRange *r, uint32_t *dh, uint32_t *flags) {
+    qg_chain();
     for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) dh[i] = 0;
     if (threadIdx.x != 0) return;
     r->kmin = 0xffffffffu;
@@ -134,6 +135,7 @@ k_pj_rrec(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, lo
 __global__ void __launch_bounds__(256)
 k_pj_rrange(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, long long nR, PjRange *range,
             uint32_t *flags) {
+    qg_chain();
     __shared__ uint32_t s_k[2];
     __shared__ int s_p[2];
     if (threadIdx.x == 0) {
@@ -203,6 +205,7 @@ __device__ __forceinline__ bool pj_sentinel(int32_t pmin, int32_t pmax, uint32_t
 __global__ void __launch_bounds__(256)
 k_pj_tfill(uint32_t *__restrict__ T, uint32_t *__restrict__ bitmap, const PjRange *__restrict__ range, int lb2,
            long long nR, uint32_t *flags) {
+    qg_chain();
     const uint32_t kmin = range->kmin, kmax = range->kmax;
     if (!pj_dense_span(kmin, kmax, lb2, nR)) return;
     uint32_t sent;
@@ -238,6 +241,7 @@ __global__ void __launch_bounds__(256)
 k_pj_rtab(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, long long nR,
           const PjRange *__restrict__ range, int lb2, uint32_t *__restrict__ bitmap, uint32_t *__restrict__ T,
           uint32_t *__restrict__ flags, unsigned long long *__restrict__ rec, uint32_t *__restrict__ hist) {
+    qg_chain();
     __shared__ uint32_t h[2][256];
     const uint32_t kmin = range->kmin, kmax = range->kmax;
     const bool dense = pj_dense_span(kmin, kmax, lb2, nR);
@@ -284,6 +288,7 @@ k_pj_rtab(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, lo
 __global__ void __launch_bounds__(256)
 k_pj_distinct(const uint32_t *__restrict__ bitmap, const uint32_t *__restrict__ T, const PjRange *__restrict__ range,
               int lb2, long long nR, const uint32_t *__restrict__ flags, unsigned long long *__restrict__ count) {
+    qg_chain();
     const uint32_t kmin = range->kmin, kmax = range->kmax;
     if (!pj_dense_span(kmin, kmax, lb2, nR)) return;
     const unsigned long long w = (unsigned long long)(kmax - kmin) + 1ull;
@@ -334,6 +339,7 @@ k_pj_sfilter(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay,
                unsigned long long *__restrict__ out, unsigned long long *__restrict__ cursor,
                qg_control *ctl, int lb2, uint32_t *__restrict__ hist, const uint32_t *__restrict__ done,
                const uint32_t *__restrict__ dense) {
+    qg_chain();
     if (done && *done == 1u) return;     // qg_jpart.cu has answered
     if (dense && *dense == 0u) return;   // the hash join will
     constexpr int TILE = SF_THREADS * SF_ROUNDS * 4;
@@ -2260,21 +2266,15 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     qg_pre_launch(ctx);
     k_pj_range_init<<<1, 1024, 0, ctx->stream>>>(L.range, L.dh, L.dflags);
     QG_TRY(qg_check_launch(ctx, "k_pj_range_init"));
-    qg_pre_launch(ctx);
-    k_pj_rrange<<<pj_grid(ctx, nR, 256, 8), 256, 0, ctx->stream>>>(rkey, rpay, nR, L.range, L.dflags);
-    QG_TRY(qg_check_launch(ctx, "k_pj_rrange"));
+    QG_TRY(qg_launch_chained(ctx, "k_pj_rrange", k_pj_rrange, pj_grid(ctx, nR, 256, 8), 256, 0, rkey, rpay, nR,
+                             L.range, L.dflags));
     // R: payload table (+ presence bitmap without a sentinel) on a dense span, else records + digit histograms
-    qg_pre_launch(ctx);
-    k_pj_tfill<<<pj_grid(ctx, nR / 2, 256, 8), 256, 0, ctx->stream>>>(T, bitmap, L.range, lb2, nR, L.dflags);
-    QG_TRY(qg_check_launch(ctx, "k_pj_tfill"));
-    qg_pre_launch(ctx);
-    k_pj_rtab<<<pj_grid(ctx, nR, 256, 8), 256, 0, ctx->stream>>>(rkey, rpay, nR, L.range, lb2, bitmap, T,
-                                                                 L.dflags, R, L.dh);
-    QG_TRY(qg_check_launch(ctx, "k_pj_rtab"));
-    qg_pre_launch(ctx);
-    k_pj_distinct<<<pj_grid(ctx, nR, 256, 8), 256, 0, ctx->stream>>>(
-        bitmap, T, L.range, lb2, nR, L.dflags, reinterpret_cast<unsigned long long *>(L.dflags + PJ_F_DISTINCT));
-    QG_TRY(qg_check_launch(ctx, "k_pj_distinct"));
+    QG_TRY(qg_launch_chained(ctx, "k_pj_tfill", k_pj_tfill, pj_grid(ctx, nR / 2, 256, 8), 256, 0, T, bitmap, L.range,
+                             lb2, nR, L.dflags));
+    QG_TRY(qg_launch_chained(ctx, "k_pj_rtab", k_pj_rtab, pj_grid(ctx, nR, 256, 8), 256, 0, rkey, rpay, nR, L.range,
+                             lb2, bitmap, T, L.dflags, R, L.dh));
+    QG_TRY(qg_launch_chained(ctx, "k_pj_distinct", k_pj_distinct, pj_grid(ctx, nR, 256, 8), 256, 0, bitmap, T, L.range,
+                             lb2, nR, L.dflags, reinterpret_cast<unsigned long long *>(L.dflags + PJ_F_DISTINCT)));
     // large probe inputs: one partition step, unless the build side is not dense or the rows spread unevenly
     const bool jp = dflt && nS > PJ_DIRECT_S;
     const bool may_hash = nR <= PJ_HASH_R && !hash_tried;
@@ -2287,11 +2287,10 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     // S filter with the S' digit histograms of the radix function
     constexpr int SF_TILE = SF_THREADS * SF_ROUNDS * 4;
     const long long tiles = (nS + SF_TILE - 1) / SF_TILE;
-    qg_pre_launch(ctx);
-    k_pj_sfilter<<<(unsigned)std::min<long long>(tiles, (long long)ctx->sm_count * 4), SF_THREADS, 0, ctx->stream>>>(
-        skey, spay, nS, slo, shi, L.range, S, &L.range->count, ctx->ctl, lb2, L.dh + 512, jp ? qg_jp_done(jp_work) : nullptr,
-        jp && may_hash ? L.dflags + PJ_F_DENSE : nullptr);
-    QG_TRY(qg_check_launch(ctx, "k_pj_sfilter"));
+    QG_TRY(qg_launch_chained(ctx, "k_pj_sfilter", k_pj_sfilter, (unsigned)std::min<long long>(tiles,
+                             (long long)ctx->sm_count * 4), SF_THREADS, 0, skey, spay, nS, slo, shi, L.range, S,
+                             &L.range->count, ctx->ctl, lb2, L.dh + 512, jp ? qg_jp_done(jp_work) : nullptr,
+                             jp && may_hash ? L.dflags + PJ_F_DENSE : nullptr));
     // one copy brings R's key range, the S' count, the histograms and the dense flags
     constexpr size_t head = offsetof(PjPin, dflags) + PJ_F_WORDS * 4;
     static_assert(offsetof(PjPin, h) == 256 && offsetof(PjPin, dflags) == 256 + 4096, "as carved");

@@ -45,6 +45,7 @@ __global__ void __launch_bounds__(256)
 k_radix_hist(const uint32_t *__restrict__ kin, const unsigned long long *__restrict__ rin,
              long long n, uint32_t key_off, int npos, uint32_t *__restrict__ ghist,
              unsigned long long *__restrict__ copy, uint4 *__restrict__ clear, long long clear_n) {
+    qg_chain();
     __shared__ uint32_t sh[4][QG_RADIX];
     for (int i = threadIdx.x; i < 4 * QG_RADIX; i += blockDim.x) (&sh[0][0])[i] = 0;
     __syncthreads();
@@ -379,6 +380,7 @@ k_radix_pass(qg_sort_bufs src, qg_sort_bufs dst, long long n, int shift, uint32_
              const uint32_t *__restrict__ dbase, uint32_t *__restrict__ status, qg_control *ctl, uint32_t spin_limit,
              const unsigned long long *__restrict__ d_n, const uint32_t *__restrict__ trivial,
              const RsPass *__restrict__ plan, const qg_sort_range *__restrict__ range) {
+    qg_chain();
     extern __shared__ __align__(16) unsigned char rs_raw[];
     static_assert(!(KV3 && SIDE), "no sidecar with three columns");
     RsSmem<KV3, SIDE> &S = *reinterpret_cast<RsSmem<KV3, SIDE> *>(rs_raw);
@@ -551,11 +553,9 @@ qg_status qg_radix_passes_pf(qg_ctx *ctx, bool kv3, qg_sort_bufs a, qg_sort_bufs
         const int sr = g_rs_stable_rank >= 0 ? g_rs_stable_rank : 3;
         const int rk = (first_unstable && i == 0 && !kv3) ? 2 : (m ? 1 : sr);
         const rs_kernel kern = kv3 ? rs_pick<true, false>(rk) : side ? rs_pick<false, true>(rk) : rs_pick<false, false>(rk);
-        qg_pre_launch(ctx);
-        kern<<<(unsigned)tiles, RS_THREADS, smem, ctx->stream>>>(s, d, n, shift, side ? 0u : pf.kmin,
-                                                                 dbase + p * QG_RADIX, status, ctx->ctl, ctx->spin_limit,
-                                                                 nullptr, nullptr, nullptr, nullptr);
-        QG_TRY(qg_check_launch(ctx, "k_radix_pass"));
+        QG_TRY(qg_launch_chained(ctx, "k_radix_pass", kern, (unsigned)tiles, RS_THREADS, smem, s, d, n, shift,
+                                 side ? 0u : pf.kmin, dbase + p * QG_RADIX, status, ctx->ctl, ctx->spin_limit, nullptr,
+                                 nullptr, nullptr, nullptr));
         in_a = !in_a;
     }
     *result_in_b = !in_a;
@@ -567,6 +567,7 @@ qg_status qg_radix_passes_pf(qg_ctx *ctx, bool kv3, qg_sort_bufs a, qg_sort_bufs
 // pass is then a copy).
 __global__ void k_radix_bases(const uint32_t *__restrict__ hist, int npos, uint32_t *__restrict__ bases,
                               uint32_t *__restrict__ trivial) {
+    qg_chain();
     __shared__ uint32_t ws[QG_RADIX / 32], wm[QG_RADIX / 32];
     const int d = threadIdx.x, lane = d & 31, w = d >> 5;
     for (int p = 0; p < npos; p++) {
@@ -611,20 +612,17 @@ qg_status qg_radix_passes_dev(qg_ctx *ctx, bool kv3, qg_sort_bufs a, qg_sort_buf
     const size_t smem = kv3 ? sizeof(RsSmem<true>) : sizeof(RsSmem<false>);
     if (kv3) QG_TRY((rs_set_attr<true, false>(ctx)));
     else QG_TRY((rs_set_attr<false, false>(ctx)));
-    qg_pre_launch(ctx);
-    k_radix_bases<<<1, QG_RADIX, 0, ctx->stream>>>(d_hist, npos, dbase, trivial);
-    QG_TRY(qg_check_launch(ctx, "k_radix_bases"));
+    QG_TRY(qg_launch_chained(ctx, "k_radix_bases", k_radix_bases, 1, QG_RADIX, 0, d_hist, npos, dbase, trivial));
     QG_TRY_CUDA(ctx, cudaMemsetAsync(status, 0, (size_t)npos * st_words * 4, ctx->stream), "memset status");
     bool in_a = true;
     for (int p = 0; p < npos; p++) {
         const qg_sort_bufs &s = in_a ? a : b;
         const qg_sort_bufs &d = in_a ? b : a;
         uint32_t *stp = status + (size_t)p * st_words;
-        qg_pre_launch(ctx);
         const rs_kernel kern = kv3 ? rs_pick<true, false>(3) : rs_pick<false, false>(3);
-        kern<<<(unsigned)tiles, RS_THREADS, smem, ctx->stream>>>(s, d, n_bound, 8 * p, key_off, dbase + p * QG_RADIX, stp,
-                                                                 ctx->ctl, ctx->spin_limit, d_n, trivial + p, nullptr, nullptr);
-        QG_TRY(qg_check_launch(ctx, "k_radix_pass"));
+        QG_TRY(qg_launch_chained(ctx, "k_radix_pass", kern, (unsigned)tiles, RS_THREADS, smem, s, d, n_bound, 8 * p,
+                                 key_off, dbase + p * QG_RADIX, stp, ctx->ctl, ctx->spin_limit, d_n, trivial + p,
+                                 nullptr, nullptr));
         in_a = !in_a;
     }
     *result_in_b = !in_a;
@@ -642,17 +640,13 @@ qg_status qg_radix_passes_range(qg_ctx *ctx, qg_sort_bufs a, qg_sort_bufs b, lon
     uint32_t *status = trivial + 64;           // [4][tiles][256]
     const size_t st_words = (size_t)tiles * QG_RADIX;
     QG_TRY((rs_set_attr<true, false>(ctx)));
-    qg_pre_launch(ctx);
-    k_radix_bases<<<1, QG_RADIX, 0, ctx->stream>>>(d_hist, 4, dbase, trivial);
-    QG_TRY(qg_check_launch(ctx, "k_radix_bases"));
+    QG_TRY(qg_launch_chained(ctx, "k_radix_bases", k_radix_bases, 1, QG_RADIX, 0, d_hist, 4, dbase, trivial));
     QG_TRY_CUDA(ctx, cudaMemsetAsync(status, 0, 4 * st_words * 4, ctx->stream), "memset status");
     const rs_kernel kern = rs_pick<true, false>(3);
     for (int p = 0; p < 4; p++) {
-        qg_pre_launch(ctx);
-        kern<<<(unsigned)tiles, RS_THREADS, sizeof(RsSmem<true>), ctx->stream>>>(
-            a, b, n_bound, 8 * p, 0u, dbase + p * QG_RADIX, status + (size_t)p * st_words, ctx->ctl, ctx->spin_limit, d_n,
-            nullptr, nullptr, range);
-        QG_TRY(qg_check_launch(ctx, "k_radix_pass"));
+        QG_TRY(qg_launch_chained(ctx, "k_radix_pass", kern, (unsigned)tiles, RS_THREADS, sizeof(RsSmem<true>), a, b,
+                                 n_bound, 8 * p, 0u, dbase + p * QG_RADIX, status + (size_t)p * st_words, ctx->ctl,
+                                 ctx->spin_limit, d_n, nullptr, nullptr, range));
     }
     return QG_OK;
 }
@@ -677,6 +671,7 @@ __global__ void __launch_bounds__(QG_RADIX)
 k_radix_plan(uint32_t *__restrict__ hist, const unsigned long long *in, unsigned long long *out,
              unsigned long long *tmp, bool pre_copy, uint32_t *status, size_t status_words, long long n, RsPlan *plan,
              volatile uint32_t *h_passes) {
+    qg_chain();
     __shared__ uint32_t ws[4][QG_RADIX / 32], wm[4][QG_RADIX / 32];
     const int d = threadIdx.x, lane = d & 31, w = d >> 5;
     uint32_t c[4], inc[4];
@@ -761,17 +756,13 @@ qg_status qg_sort_rec(qg_ctx *ctx, const unsigned long long *in, unsigned long l
                                                                 pre_copy ? tmp : nullptr, (uint4 *)status,
                                                                 (long long)(words / 4));
     QG_TRY(qg_check_launch(ctx, "k_radix_hist"));
-    qg_pre_launch(ctx);
-    k_radix_plan<<<1, QG_RADIX, 0, ctx->stream>>>(ctx->ctl->shist, in, out, tmp, pre_copy, status, words, n, plan,
-                                                  &ctx->hres->passes);
-    QG_TRY(qg_check_launch(ctx, "k_radix_plan"));
+    QG_TRY(qg_launch_chained(ctx, "k_radix_plan", k_radix_plan, 1, QG_RADIX, 0, ctx->ctl->shist, in, out, tmp,
+                             pre_copy, status, words, n, plan, &ctx->hres->passes));
     const rs_kernel kern = rs_pick<false, false>(g_rs_stable_rank >= 0 ? g_rs_stable_rank : 3);
     for (int p = 0; p < (same && !pre_copy ? 5 : 4); p++) {
-        qg_pre_launch(ctx);
-        kern<<<(unsigned)tiles, RS_THREADS, sizeof(RsSmem<false>), ctx->stream>>>(
-            qg_sort_bufs{}, qg_sort_bufs{}, n, 8 * p, 0u, plan->base + (p & 3) * QG_RADIX, nullptr, ctx->ctl,
-            ctx->spin_limit, nullptr, nullptr, &plan->pass[p], nullptr);
-        QG_TRY(qg_check_launch(ctx, "k_radix_pass"));
+        QG_TRY(qg_launch_chained(ctx, "k_radix_pass", kern, (unsigned)tiles, RS_THREADS, sizeof(RsSmem<false>),
+                                 qg_sort_bufs{}, qg_sort_bufs{}, n, 8 * p, 0u, plan->base + (p & 3) * QG_RADIX,
+                                 nullptr, ctx->ctl, ctx->spin_limit, nullptr, nullptr, &plan->pass[p], nullptr));
     }
     return QG_OK;
 }
@@ -782,10 +773,10 @@ qg_status qg_radix_pass_planned(qg_ctx *ctx, const RsPass *plan, const uint32_t 
                                 const unsigned long long *d_n) {
     if (n_bound >= (1LL << 30)) return QG_ERR_UNSUPPORTED;
     QG_TRY((rs_set_attr<false, false>(ctx)));
-    qg_pre_launch(ctx);
-    k_radix_pass<false, false, 2><<<(unsigned)((n_bound + RS_TILE - 1) / RS_TILE), RS_THREADS, sizeof(RsSmem<false>), ctx->stream>>>(
-        qg_sort_bufs{}, qg_sort_bufs{}, n_bound, 0, 0u, dbase, nullptr, ctx->ctl, ctx->spin_limit, d_n, nullptr, plan, nullptr);
-    return qg_check_launch(ctx, "k_radix_pass");
+    return qg_launch_chained(ctx, "k_radix_pass", k_radix_pass<false, false, 2>,
+                             (unsigned)((n_bound + RS_TILE - 1) / RS_TILE), RS_THREADS, sizeof(RsSmem<false>),
+                             qg_sort_bufs{}, qg_sort_bufs{}, n_bound, 0, 0u, dbase, nullptr, ctx->ctl, ctx->spin_limit,
+                             d_n, nullptr, plan, nullptr);
 }
 
 // After the sort's stream has been waited for: remember the parity of an
