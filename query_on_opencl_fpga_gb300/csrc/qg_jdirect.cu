@@ -20,9 +20,8 @@
 //   5. k_jd_scan   counts -> first places; every key and its R payload are
 //                  written as often as counted; the distinct keys are counted
 //   6. k_jd_write  every appended row's S payload to its place
-// Six launches and one wait.  The partitioned form (qg_pjoin.cu) takes twelve
-// launches and three waits, 120 us before it reads anything, and stays the
-// better one where the scattered accesses leave L2.  A key with
+// Six launches (four for a small build side, k_jd_build) and one wait.  Where the
+// scattered accesses leave L2, the rows are partitioned first (qg_jpart.cu).  A key with
 // more than JD_KEY_ROWS rows ends the attempt: its atomics would queue at one
 // word, and the partitioned form treats such keys apart.
 #include <algorithm>
@@ -118,6 +117,58 @@ k_jd_table(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, l
         for (int u = 0; u < U; u++)
             if (i0 + u * stride < nR) E[k[u]] = (unsigned long long)p[u] << 32 | JD_HERE;
     }
+}
+
+// The three steps above in one CTA: with so few rows the launches are what costs.
+// Joins with 256 to 2048 build rows 53 -> 48 us; with 4096 one SM takes as long as
+// the three launches (52), with 8192 longer (55 / 52).
+constexpr int JD_ONE_THREADS = 1024, JD_ONE_PER = 2;
+constexpr int64_t JD_ONE_R = JD_ONE_THREADS * JD_ONE_PER;
+__global__ void __launch_bounds__(JD_ONE_THREADS, 1)
+k_jd_build(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, uint32_t nR,
+           unsigned long long *__restrict__ E, uint32_t *__restrict__ jd) {
+    qg_chain();
+    __shared__ uint32_t s[2];
+    const uint32_t tid = threadIdx.x;
+    uint32_t k[JD_ONE_PER], p[JD_ONE_PER], lo = 0xffffffffu, hi = 0;
+    if (tid == 0) {
+        s[0] = 0xffffffffu;
+        s[1] = 0;
+    }
+#pragma unroll
+    for (int j = 0; j < JD_ONE_PER; j++) {
+        const uint32_t i = j * JD_ONE_THREADS + tid;
+        if (i >= nR) break;
+        k[j] = (uint32_t)__ldg(rkey + i);
+        p[j] = (uint32_t)__ldg(rpay + i);
+        lo = min(lo, k[j]);
+        hi = max(hi, k[j]);
+    }
+    __syncthreads();
+    lo = __reduce_min_sync(QG_FULL_MASK, lo);
+    hi = __reduce_max_sync(QG_FULL_MASK, hi);
+    if ((tid & 31) == 0) {
+        atomicMin(&s[0], lo);
+        atomicMax(&s[1], hi);
+    }
+    __syncthreads();
+    const uint32_t kmin = s[0];
+    const unsigned long long w = (unsigned long long)(s[1] - kmin) + 1ull;
+    const bool ok = w <= 2ull * nR;
+    if (tid == 0) {
+        jd[JD_OK] = ok ? QG_JD_DONE : QG_JD_SPARSE;
+        jd[JD_KMIN] = kmin;
+        jd[JD_SPAN] = ok ? (uint32_t)w : 0u;
+        jd[JD_DISTINCT] = 0;
+        jd[JD_ROWS] = 0;
+    }
+    if (!ok) return;
+    ulonglong2 *E2 = reinterpret_cast<ulonglong2 *>(E);  // one entry past an odd span is part of the buffer
+    for (uint32_t i = tid; i < ((uint32_t)w + 1) / 2; i += JD_ONE_THREADS) E2[i] = make_ulonglong2(0ull, 0ull);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < JD_ONE_PER; j++)
+        if (j * JD_ONE_THREADS + tid < nR) E[k[j] - kmin] = (unsigned long long)p[j] << 32 | JD_HERE;
 }
 
 // S rows, 4096 per tile (persistent CTAs): the rows that pass the filter and
@@ -363,17 +414,28 @@ qg_status qg_jd_launch(qg_ctx *ctx, char *work, const int32_t *rkey, const int32
     const size_t eb = qg_align_up(((size_t)2 * nR + 2) * 8, 256), ab = qg_align_up((size_t)nS * 4, 256);
     uint32_t *ak = (uint32_t *)(work + eb), *ap = (uint32_t *)(work + eb + ab), *an = (uint32_t *)(work + eb + 2 * ab);
     uint32_t *jd = ctx->ctl->jd;
-    qg_pre_launch(ctx);
-    k_jd_range<<<jd_grid(ctx, nR, 4 * JD_THREADS, 4), JD_THREADS, 0, ctx->stream>>>(rkey, nR, jd);
-    QG_TRY(qg_check_launch(ctx, "k_jd_range"));
-    QG_TRY(qg_launch_chained(ctx, "k_jd_fill", k_jd_fill, jd_grid(ctx, nR, 2 * JD_THREADS, 8), JD_THREADS, 0, E, nR, jd));
-    QG_TRY(qg_launch_chained(ctx, "k_jd_table", k_jd_table, jd_grid(ctx, nR, JD_THREADS, 8), JD_THREADS, 0, rkey, rpay, nR, E, jd));
-    QG_TRY(qg_launch_chained(ctx, "k_jd_count", k_jd_count, jd_grid(ctx, nS, JD_TILE, 4), JD_THREADS, 0, skey, spay, nS, slo, shi, E, jd, ak, ap, an));
+    if (nR <= JD_ONE_R) {
+        qg_pre_launch(ctx);
+        k_jd_build<<<1, JD_ONE_THREADS, 0, ctx->stream>>>(rkey, rpay, (uint32_t)nR, E, jd);
+        QG_TRY(qg_check_launch(ctx, "k_jd_build"));
+    } else {
+        qg_pre_launch(ctx);
+        k_jd_range<<<jd_grid(ctx, nR, 4 * JD_THREADS, 4), JD_THREADS, 0, ctx->stream>>>(rkey, nR, jd);
+        QG_TRY(qg_check_launch(ctx, "k_jd_range"));
+        QG_TRY(qg_launch_chained(ctx, "k_jd_fill", k_jd_fill, jd_grid(ctx, nR, 2 * JD_THREADS, 8), JD_THREADS, 0, E,
+                                 nR, jd));
+        QG_TRY(qg_launch_chained(ctx, "k_jd_table", k_jd_table, jd_grid(ctx, nR, JD_THREADS, 8), JD_THREADS, 0, rkey,
+                                 rpay, nR, E, jd));
+    }
+    QG_TRY(qg_launch_chained(ctx, "k_jd_count", k_jd_count, jd_grid(ctx, nS, JD_TILE, 4), JD_THREADS, 0, skey, spay,
+                             nS, slo, shi, E, jd, ak, ap, an));
     // few entries: more, smaller tiles (2K build rows 15 us with 16 entries per lane)
     const int per = nR <= (1 << 18) ? 2 : 16;
     const long long tiles = qg_ceil_div(2 * nR, per * JD_THREADS);
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, tiles, QG_SITE_JOIN_PROBE, &lb));
-    QG_TRY(qg_launch_chained(ctx, "k_jd_scan", per == 2 ? k_jd_scan<2> : k_jd_scan<16>, (unsigned)tiles, JD_THREADS, 0, E, nR, jd, out_key, out_rpay, cap, d_count, result, &ctx->ctl->jd_arrived, lb));
-    return qg_launch_chained(ctx, "k_jd_write", k_jd_write, jd_grid(ctx, nS / 4, JD_THREADS, 8), JD_THREADS, 0, E, jd, ak, ap, an, out_spay, cap);
+    QG_TRY(qg_launch_chained(ctx, "k_jd_scan", per == 2 ? k_jd_scan<2> : k_jd_scan<16>, (unsigned)tiles, JD_THREADS, 0,
+                             E, nR, jd, out_key, out_rpay, cap, d_count, result, &ctx->ctl->jd_arrived, lb));
+    return qg_launch_chained(ctx, "k_jd_write", k_jd_write, jd_grid(ctx, nS / 4, JD_THREADS, 8), JD_THREADS, 0, E, jd,
+                             ak, ap, an, out_spay, cap);
 }

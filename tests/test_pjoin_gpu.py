@@ -314,9 +314,10 @@ def _join_case(ctx, orc, rkey, rpay, skey, spay, path, hi=299, extra=16):
 
 
 # The counting path around its tiles (2 and 16 table entries per lane, 4096 probe
-# rows), spans of nR, 2 nR and 2 nR + 1 values, keys at the ends of the range,
+# rows, the most build rows that one CTA takes), spans of nR, 2 nR and 2 nR + 1 values, keys at the ends of the range,
 # build payloads of every value, a key with the most rows it takes and one more.
-@pytest.mark.parametrize("nR,nS,gap", [(1, 1, 1), (255, 4095, 1), (256, 4096, 2), (257, 4097, 1), (1 << 18, 9000, 1),
+@pytest.mark.parametrize("nR,nS,gap", [(1, 1, 1), (255, 4095, 1), (256, 4096, 2), (257, 4097, 1), (1025, 3000, 2),
+                                       (2048, 70_000, 2), (2049, 70_000, 2), (1 << 18, 9000, 1),
                                        ((1 << 18) + 1, 50_001, 2), (5000, 300_003, 1)])
 @pytest.mark.parametrize("base", [0, -(2 ** 31), 2 ** 31 - 600_000])
 def test_join_counting_path_edges(ctx, orc, nR, nS, gap, base):
