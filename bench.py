@@ -500,7 +500,8 @@ def operator_lines(ctx, args, peak, stream):
                            "op_frac_of_peak": alg / (ms * 1e-3) / 1e9 / peak,
                            "kernels_ms": {k: v[1] / steps for k, v in kern.items()},
                            "path": ctx.join_stats()["path"],
-                           "roofline_sfilter": roofline(kern, "k_pj_sfilter", nS * 8 + sp * 8, peak)}
+                           "roofline_sfilter": roofline(kern, "k_jp_part", nS * 8 + sp * 8, peak)
+                           or roofline(kern, "k_pj_sfilter", nS * 8 + sp * 8, peak)}
     del j, res
     torch.cuda.empty_cache()
     out["sort_64M"] = sort_line(ctx, steps, peak, stream)
@@ -545,13 +546,16 @@ def sort_line(ctx, steps, peak, stream):
     torch.cuda.synchronize()
     kern = ctx.timing_report()
     ctx.enable_timing(False)
-    passes = kern.get("k_radix_pass", (0, 0.0))[0] // steps
+    # four passes are launched, planned on the device: the one over the keys' high
+    # zero byte ends at once and moves nothing
+    launches = kern.get("k_radix_pass", (0, 0.0))[0] // steps
+    passes = 3
     alg = ns * 16 * passes  # one read and one write of the records per key pass
     del base, rec
     return {"rows_per_s": ns / (ms * 1e-3), "ms_per_op": ms, "rows": ns, "passes": passes, "sorted": ok,
             "op_frac_of_peak": alg / (ms * 1e-3) / 1e9 / peak,
             "kernels_ms": {k: v[1] / steps for k, v in kern.items()},
-            "roofline": roofline(kern, "k_radix_pass", ns * 16, peak)}
+            "roofline": roofline(kern, "k_radix_pass", alg / max(launches, 1), peak)}
 
 
 def skew_line(ctx, stream):

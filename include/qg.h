@@ -187,11 +187,14 @@ QG_API qg_status qg_scatter_rec(qg_ctx *ctx, const void *R, int64_t rLen, const 
  * QG_ORDER_KEY (ascending unsigned key, the reference's sorted order) or
  * QG_ORDER_NONE.  By default up to 16384 rows are aggregated by one CTA in
  * shared memory (key order either way).  Larger inputs, and small ones with
- * too many distinct keys for that, are first aggregated in a direct-indexed
- * window of 2^22 keys placed on a sample's key range (output in key order
- * either way); when the sample spans more than 2^21 keys or any row's key
- * falls outside the window, the call runs the two-pass hash path instead.
- * There `cap` also sizes the spill partitions (about 1024 groups each), so a
+ * too many distinct keys for that, are aggregated in a direct-indexed window of
+ * 2^22 keys (output in key order either way): up to 2^23 rows it lies on the
+ * exact key range, beyond on a sample's (at most 2^21 keys wide).  When the keys
+ * do not fit, the rows are partitioned by key range and aggregated in key order
+ * (rows < 2^30, cap up to 1.3M groups), or, where the partitions would be
+ * uneven, hold too many groups or few groups meet many rows, the call runs the
+ * two-pass hash path; which of these is launched first is what the context's
+ * last call found.  On the two-pass path `cap` also sizes the spill partitions (about 1024 groups each), so a
  * cap near the true group count is fastest, and for key order the context
  * remembers the key range of its previous call and ranks keys in a bitmap
  * window placed there; results never depend on either, only the path does
@@ -225,12 +228,15 @@ QG_API qg_status qg_groupby_set_knobs(int mode, int hot_slots_log2, int partitio
 /* The dense-window path's four steps (sample, candidates, main pass, emit)
  * as one cooperative launch with grid barriers between them (enable = 1), or
  * as four launches (0, the default; also what runs while the stream is being
- * captured into a graph).  Process-wide; results are identical. */
+ * captured into a graph).  With 0, up to 2^23 rows take three launches (key
+ * range, main pass, emit).  Process-wide; results are identical. */
 QG_API qg_status qg_groupby_set_single_launch(int enable);
 /* Diagnostics of the context's last qg_groupby_cols call: out[0] = path
- * (0 two-pass, 1 global table, 2 dense window or a small input's one launch), out[1] = overflow flags
+ * (0 two-pass or partitioned by key range, 1 global table, 2 dense window or a
+ * small input's one launch), out[1] = overflow flags
  * (bit 0 spill bucket, bit 1 pass-2 table), out[2] = fullest spill bucket,
- * out[3] = bucket capacity (the last three 0 on the dense-window path). */
+ * out[3] = bucket capacity (the last three 0 on the dense-window path and when
+ * partitioned by key range). */
 QG_API qg_status qg_groupby_stats(qg_ctx *ctx, uint32_t *out4);
 
 /* ---- hash join + filter + sort (config 2; kernel/hj_filter_sort/1/hj_filter_sort_op.cl)
@@ -244,9 +250,10 @@ QG_API qg_status qg_join_filter_sort(qg_ctx *ctx, const int32_t *rkey, const int
                                      int32_t *out_rpay, int32_t *out_spay, int64_t cap,
                                      int64_t *out_n);
 /* Join algorithm knobs (process-wide).  variant: 0 auto -- with the other
- * knobs at their defaults, a counting join when R's keys are unique over a
- * dense span (at most 2 nR values) and S has up to 40M rows, the hash join (3)
- * when R has up to 2^23 keys of no dense span; else range partitioning by
+ * knobs at their defaults, when R's keys are unique over a dense span (at most
+ * 2 nR values): a counting join for S up to 18M rows, beyond it one partition
+ * step fused with the filter if the rows spread evenly; the hash join (3) when R
+ * has up to 2^23 keys of no dense span; else range partitioning by
  * radix over the key, switching to the learned CDF partition function when
  * radix leaves more than 2% of the rows in buckets too large for shared memory
  * and the model does better on the same counts; 1 radix
@@ -266,8 +273,8 @@ QG_API qg_status qg_join_set_knobs(int variant, int buckets_log2, uint32_t bucke
  * general path.  Results are identical. */
 QG_API qg_status qg_join_set_dense(int enable);
 /* Diagnostics of the context's last qg_join_filter_sort: out[0] path
- * (1 radix, 2 learned, 3 hash join + sort, 4 dense build side: counting or radix,
- * 0 nothing to join), out[1]
+ * (1 radix, 2 learned, 3 hash join + sort, 4 dense build side: counting, one
+ * partition step or radix, 0 nothing to join), out[1]
  * buckets, out[2] buckets handled outside the bucket kernel, out[3] their
  * rows, out[4] those of them with several keys (joined together by the
  * sort-merge path; the others are single-key cross products), out[5] knots

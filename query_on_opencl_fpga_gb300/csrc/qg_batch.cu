@@ -22,7 +22,9 @@
 // qg_batch_run then replays that graph on the caller's stream: the whole
 // batch costs one graph launch and no host round trip.  Each query's kernel
 // variant comes from the query (chosen by the caller, e.g. by the learned
-// cost model) or is the default.  The batch owns a private context, so its
+// cost model) or is the default.  A group-by of up to 8192 rows is one launch
+// (qg_gbsmall.cu).  Queries go to the lane with the least measured time so far and
+// start shortest first.  The batch owns a private context, so its
 // arenas are never moved by other calls.
 #include <algorithm>
 #include <vector>

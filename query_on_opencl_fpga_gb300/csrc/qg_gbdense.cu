@@ -9,7 +9,9 @@
 // value column.  Here the key order comes from the table's index order, so no
 // sort pass exists.
 //
-// Four launches, no host round trip until the caller's one read at the end:
+// Up to 2^23 rows take three launches (k_gbd_range, k_gbd_mid, k_gbd_emit, further
+// down).  Larger inputs take four, no host round trip until the caller's one read at
+// the end:
 //  1. k_gbd_sample -- 2^18 keys (1024 runs of 256 consecutive rows spread over
 //                     the column, or every row of a smaller input) are counted
 //                     per CTA in shared memory; each CTA adds its distinct

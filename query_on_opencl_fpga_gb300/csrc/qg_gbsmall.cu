@@ -10,10 +10,10 @@
 // keys are sorted there.  A table that fills up (more distinct keys than it
 // takes) is reported and the caller takes the general paths.
 //
-// A 10K-row call in 500 groups 57 -> 43 us, hashed ids (keys of no window) 150
-// -> 46.  One SM adds 2K to 4K rows a microsecond: at 16K rows a call takes 46
-// (64 groups) to 59 us (4096), the dense-window path's three launches 48 whatever
-// the groups and hashed ids 64 on theirs, so larger inputs go there.
+// A 10K-row call in 500 groups 57 -> 40 us, hashed ids (keys of no window) 150
+// -> 40.  One SM adds 2K to 4K rows a microsecond: at 16K rows a call takes 41
+// (64 groups) to 54 us (4096), the dense-window path's three launches 41 whatever
+// the groups and hashed ids 51 on theirs, so larger inputs go there.
 #include <algorithm>
 #include "qg_cta_sort.cuh"
 #include "qg_internal.cuh"

@@ -14,10 +14,10 @@
 //                   keys sorted there, their place from a look-back over the
 //                   parts, written in ascending key order
 // The two-pass path (qg_groupby.cu) spills misses into 1024 buckets per SM and
-// sorts the groups in four passes afterwards: calls of 64K rows took 160 us (64
-// here), of 1M rows 150 to 220 (74 to 82), of 8M rows in 1M groups 390 (199).  It
+// sorts the groups in four passes afterwards: calls of 64K rows took 160 us (52
+// here), of 1M rows 150 to 220 (64 to 72), of 8M rows in 1M groups 390 (190).  It
 // stays for keys that fill the parts unevenly (a frequent key, clusters) and for
-// more groups than the parts' tables hold.  Of the 199 us the range takes 14, the
+// more groups than the parts' tables hold.  Of the 190 us the range takes 14, the
 // rows 27, the plan 6, the pass 37 (bandwidth) and the merge 92: 1.9 clocks a row
 // and SM of shared-memory probes and atomics, in two waves of 152 CTAs.
 #include <algorithm>

@@ -7,8 +7,8 @@
 //    boundaries (scanGroupLabel_kernel, kernel/aggregation/1/
 //    group_by_cu_op_dp.cl:293-327), scan the labels and write startPos
 //    (:505-528), then aggregate .x per group (parallelAggregate_kernel,
-//    :547-716).  Here the label + scan + outSize + write chain is one
-//    single-pass compaction kernel, and the per-group aggregation runs over
+//    :547-716).  Here the label + scan + outSize + write chain is one launch
+//    (count, one exchange, write), and the per-group aggregation runs over
 //    fixed row chunks (a group spanning chunks combines with atomics) instead
 //    of one work-group per group in chunks of 512 launches.
 //
@@ -16,9 +16,11 @@
 //    predicate on a second column (configs 1 / 1-fused; the fused
 //    filter_aggregation image, kernel/filter_aggregation/
 //    filter_aggregation_cu_op_dp.cl).  Instead of sort -> label -> scan ->
-//    aggregate, rows are aggregated in tables: the default path is the
-//    dense-window kernels of qg_gbdense.cu (keys within a 2^22-key window,
-//    emitted in key order).  Keys that do not fit a window take two passes
+//    aggregate, rows are aggregated in tables: small inputs by one CTA
+//    (qg_gbsmall.cu), others by the dense-window kernels of qg_gbdense.cu (keys
+//    within a 2^22-key window, emitted in key order).  Keys that do not fit a
+//    window are partitioned by key range (qg_gbwide.cu), or, with few groups or
+//    uneven ranges, take two passes
 //    (k_gb_part, k_gb_merge, section 2' below) -- per-SM shared-memory tables
 //    absorb the heavy hitters, the remaining rows are spilled into hash
 //    partitions and each partition is summed by one CTA in shared memory.

@@ -1,5 +1,8 @@
-// qg_pjoin.cu -- range-partitioned join + filter + sort (the default path of
-// qg_join_filter_sort).
+// qg_pjoin.cu -- range-partitioned join + filter + sort, and the choice among the
+// paths of qg_join_filter_sort: counting (qg_jdirect.cu) for dense build keys and
+// up to 18M probe rows, one partition step (qg_jpart.cu, after steps 1 here) beyond,
+// the hash join (qg_join.cu) for up to 2^23 build keys of no dense span, and the
+// pipeline below for the rest and for what those hand over.
 //
 // Reference operators this replaces: buildHashTable / probeHashTable and the
 // filter + bitonic sort of the matches (kernel/hj_filter_sort/1/
