@@ -21,20 +21,24 @@ constexpr int FT_LB_WARPS = 4;  // warps doing the look-back: 128 predecessors p
 // Two phases in one launch (records, and the default column form).  The rows
 // are cut into units of four 128-bit loads per lane of a warp, and every warp
 // owns a contiguous range of units:
-//   phase 1: the warp reads its keys (or records), keeps each row's predicate
-//            bit and counts them, with no exchange between warps;
+//   phase 1: the warp reads its keys (or records) and counts the selected rows,
+//            with no exchange between warps; it keeps each row's predicate bit,
+//            and the selected records themselves as far as they fit;
 //   exchange: one count per CTA, a wide look-back over the CTAs before it
 //            (CTAs are numbered as they start, so they are running);
-//   phase 2: the warp walks its units backwards from its end position and
-//            writes the selected rows in input order.  Columns read payloads
-//            of lanes with a selected row only; records are read again, the
-//            last unit from registers and the most recent ones from L2.
+//   phase 2: the warp writes the kept records, then walks the other units
+//            backwards from its end position, all in input order.  Columns read
+//            payloads of lanes with a selected row only; records are read again,
+//            the last unit from registers and the most recent ones from L2.
 // What bounds it is the memory's pace in both phases plus one exchange per
 // launch: neither a chain of look-backs, tile by tile (what records had:
-// 5M of them, 40 % kept, 30.8 us, now 23), nor a second launch (what columns
+// 5M of them, 40 % kept, 30.8 us, now 21), nor a second launch (what columns
 // had: 16M rows, 10 % kept, 45.6 us in two launches, now 36.9; 4096-row tiles
 // with a look-back each 67).  One CTA per SM: with four to eight smaller ones
 // the exchange took longer (49 us with six).  Loading a unit ahead did not help.
+// Keeping records spares their second read (16M, 10 % selected: 48.8 -> 34.1 us),
+// unless most would not fit anyway (40M, 90 %: 161 -> 170).  A column's payloads
+// would be waited for after its keys: 2 % selected 36.7 -> 34.0, but 25 % 38.3 -> 41.7.
 // The selected rows pass through shared memory so that a warp's stores are
 // consecutive (16M rows, 90 % kept: 87 -> 53 us).
 constexpr int F2_MAX_WARPS = 32;  // one CTA of up to 1024 threads per SM
@@ -47,6 +51,7 @@ struct F2 {
     static constexpr int PER = REC ? 2 : 4;                      // rows per 128-bit load
     static constexpr int UNIT = 32 * F2_LOADS * PER;             // rows per unit
     static constexpr uint32_t FM = (1u << PER) - 1u;             // predicate bits of one load
+    static constexpr int SEG = 512;  // rows of a warp's shared memory: a unit's, or selected records kept
 };
 
 // Lane's load r of unit u: rows [idx, idx + PER), zero past the end.
@@ -77,12 +82,12 @@ k_filter_two(const int32_t *__restrict__ src, const int32_t *__restrict__ pay, l
              int32_t lo, int32_t hi, int2 *__restrict__ out, long long cap, long long *__restrict__ d_count,
              uint16_t *__restrict__ spill, qg_lookback lb) {
     constexpr int PER = F2<REC>::PER, UNIT = F2<REC>::UNIT;
-    // per warp: the unit's selected rows on their way out; per thread: predicate bits
+    // per warp: a unit's selected rows on their way out, or records kept; per thread: predicate bits
     extern __shared__ __align__(16) unsigned char f2_raw[];
     __shared__ uint32_t s_tile, s_epoch, s_excl, s_cnt[F2_MAX_WARPS], s_tmp[2 * F2_MIN_WARPS];
     const uint32_t nw = blockDim.x >> 5;
-    int2 *stage = reinterpret_cast<int2 *>(f2_raw) + (size_t)(threadIdx.x >> 5) * UNIT;
-    uint16_t *s_mask = reinterpret_cast<uint16_t *>(reinterpret_cast<int2 *>(f2_raw) + (size_t)nw * UNIT);
+    int2 *stage = reinterpret_cast<int2 *>(f2_raw) + (size_t)(threadIdx.x >> 5) * F2<REC>::SEG;
+    uint16_t *s_mask = reinterpret_cast<uint16_t *>(reinterpret_cast<int2 *>(f2_raw) + (size_t)nw * F2<REC>::SEG);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t lt = qg_lanemask_lt();
     qg_lb_begin_dyn(lb, &s_tile, &s_epoch);
@@ -90,8 +95,36 @@ k_filter_two(const int32_t *__restrict__ src, const int32_t *__restrict__ pay, l
     const long long W = (long long)gridDim.x * nw, gw = (long long)tile * nw + warp;
     const long long ub = units * gw / W, ue = units * (gw + 1) / W;
     int4 v[F2_LOADS];
-    uint32_t cnt = 0, fl = 0;
-    for (long long u = ub; u < ue; u++) {
+    uint32_t cnt = 0, fl = 0, kept = 0;
+    long long ur = ub;  // the rows of units [ub, ur) are kept, the others' counted
+    if (REC) {
+        const long long most = 4 * F2<REC>::SEG / max(ue - ub, 1ll);
+        for (; ur < ue; ur++) {
+            const long long r0 = ur * UNIT + lane * PER;
+#pragma unroll
+            for (int r = 0; r < F2_LOADS; r++) v[r] = f2_load<REC>(src, r0 + r * 32 * PER, n);
+            fl = 0;
+#pragma unroll
+            for (int r = 0; r < F2_LOADS; r++) fl |= f2_flags<REC>(v[r], r0 + r * 32 * PER, n, lo, hi) << (PER * r);
+            uint32_t pre[F2_LOADS * PER], tot = 0;
+#pragma unroll
+            for (int j = 0; j < F2_LOADS * PER; j++) {
+                const uint32_t b = __ballot_sync(QG_FULL_MASK, (fl >> j) & 1u);
+                if (j % PER == 0) pre[j] = tot + __popc(b & lt);
+                else pre[j - j % PER] += __popc(b & lt);
+                tot += __popc(b);
+            }
+            if (kept + tot > (uint32_t)F2<REC>::SEG || (ur == ub && tot > most)) break;
+#pragma unroll
+            for (int r = 0; r < F2_LOADS; r++) {
+                uint32_t pos = kept + pre[r * PER];
+                if ((fl >> (PER * r)) & 1u) stage[pos++] = make_int2(v[r].x, v[r].y);
+                if ((fl >> (PER * r)) & 2u) stage[pos] = make_int2(v[r].z, v[r].w);
+            }
+            kept += tot;
+        }
+    }
+    for (long long u = ur; u < ue; u++) {
         const long long r0 = u * UNIT + lane * PER;
 #pragma unroll
         for (int r = 0; r < F2_LOADS; r++) v[r] = f2_load<REC>(src, r0 + r * 32 * PER, n);
@@ -103,7 +136,7 @@ k_filter_two(const int32_t *__restrict__ src, const int32_t *__restrict__ pay, l
         if (u - ub < F2_SUNITS) s_mask[(u - ub) * blockDim.x + tid] = (uint16_t)fl;
         else spill[u * 32 + lane] = (uint16_t)fl;
     }
-    cnt = __reduce_add_sync(QG_FULL_MASK, cnt);
+    cnt = __reduce_add_sync(QG_FULL_MASK, cnt) + kept;
     if (lane == 0) s_cnt[warp] = cnt;
     __syncthreads();
     const uint32_t wc = lane < (int)nw ? s_cnt[lane] : 0u;
@@ -118,7 +151,14 @@ k_filter_two(const int32_t *__restrict__ src, const int32_t *__restrict__ pay, l
     }
     __syncthreads();
     long long end = (long long)s_excl + before + cnt;  // one past the warp's last output row
-    for (long long u = ue - 1; u >= ub; u--) {
+    if (REC) {
+        const long long start = end - cnt;
+        const uint32_t lim = start >= cap ? 0u : (uint32_t)min((long long)kept, cap - start);
+        __syncwarp();
+        for (uint32_t i = lane; i < lim; i += 32) out[start + i] = stage[i];
+        __syncwarp();
+    }
+    for (long long u = ue - 1; u >= ur; u--) {
         const long long r0 = u * UNIT + lane * PER;
         if (u < ue - 1) {
             fl = u - ub < F2_SUNITS ? (uint32_t)s_mask[(u - ub) * blockDim.x + tid] : (uint32_t)spill[u * 32 + lane];
@@ -421,11 +461,11 @@ static qg_status f2_launch(qg_ctx *ctx, const int32_t *src, const int32_t *pay, 
         QG_TRY(qg_scratch(ctx, (size_t)units * 64, &scr));
         spill = (uint16_t *)scr;
     }
-    const size_t smem = (size_t)warps * (F2<REC>::UNIT * 8 + std::min<long long>(per_warp, F2_SUNITS) * 64);
+    const size_t smem = (size_t)warps * (F2<REC>::SEG * 8 + std::min<long long>(per_warp, F2_SUNITS) * 64);
     static bool attr = false;
     if (!attr) {
         QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_filter_two<REC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              F2_MAX_WARPS * (F2<REC>::UNIT * 8 + F2_SUNITS * 64)), "attr");
+                                              F2_MAX_WARPS * (F2<REC>::SEG * 8 + F2_SUNITS * 64)), "attr");
         attr = true;
     }
     qg_pre_launch(ctx);

@@ -169,3 +169,25 @@ def test_filter_rec_into_its_input(ctx, orc):
     st = ctx.lib.qg_filter_range_rec(ctx.handle, buf.data_ptr(), n, 0, 400, buf.data_ptr(), n, ctypes.byref(cnt))
     exp = orc.filter_rec(r, 0, 400)
     assert st == 0 and np.array_equal(buf[: cnt.value].cpu().numpy(), exp)
+
+
+# Records kept in shared memory (512 a warp, units of 256): none and all selected,
+# kept to the last one, run full in the middle of a warp's units or at once, and
+# not kept at all (one unit, several, many per warp; a capacity among the kept).
+@pytest.mark.parametrize("units", [1, 2, 5, 40])
+@pytest.mark.parametrize("sel", [0.0, 0.004, 0.3, 0.45, 0.9, 1.0])
+def test_filter_rec_kept_rows(ctx, orc, units, sel):
+    from query_on_opencl_fpga_gb300 import QGError
+
+    n = 152 * 32 * 256 * units - 77
+    g = torch.Generator(device="cuda")
+    g.manual_seed(units)
+    key = torch.where(torch.rand(n, generator=g, device="cuda") < sel, 5, 900).to(torch.int32)
+    key[: 256 * units] = 5  # the first warp's rows are all selected
+    rec = torch.stack([torch.arange(n, dtype=torch.int32, device="cuda"), key], 1)
+    got = ctx.filter_range_rec(rec, -3, 5)
+    exp = rec[(key == 5).nonzero().flatten()]
+    assert torch.equal(got, exp)
+    with pytest.raises(QGError) as e:
+        ctx.filter_range_rec(rec, -3, 5, cap=exp.shape[0] - 1)
+    assert e.value.status == 3
