@@ -76,6 +76,34 @@ __device__ __forceinline__ uint32_t f2_flags(const int4 &k, long long idx, long 
            ((uint32_t)((k.w >= lo) & (k.w <= hi) & (idx + 3 < n)) << 3);
 }
 
+// A unit's selected rows before this lane's load r; returns the unit's total.  One
+// scan over the lanes of the four loads' counts, a byte each: a ballot and two
+// population counts per row took 37.4 us instead of 34.2 (16M rows, 10 % selected).
+template <bool REC>
+__device__ __forceinline__ uint32_t f2_places(uint32_t fl, uint32_t (&pre)[F2_LOADS]) {
+    constexpr int PER = F2<REC>::PER;
+    static_assert(F2_LOADS == 4 && 32 * PER < 256, "a byte per load");
+    const int lane = threadIdx.x & 31;
+    uint32_t c = 0;
+#pragma unroll
+    for (int r = 0; r < F2_LOADS; r++) c |= (uint32_t)__popc((fl >> (PER * r)) & F2<REC>::FM) << (8 * r);
+    uint32_t inc = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t x = __shfl_up_sync(QG_FULL_MASK, inc, d);
+        if (lane >= d) inc += x;
+    }
+    const uint32_t all = __shfl_sync(QG_FULL_MASK, inc, 31);
+    inc -= c;
+    uint32_t tot = 0;
+#pragma unroll
+    for (int r = 0; r < F2_LOADS; r++) {
+        pre[r] = tot + ((inc >> (8 * r)) & 255u);
+        tot += (all >> (8 * r)) & 255u;
+    }
+    return tot;
+}
+
 template <bool REC>
 __global__ void __launch_bounds__(32 * F2_MAX_WARPS, 1)
 k_filter_two(const int32_t *__restrict__ src, const int32_t *__restrict__ pay, long long n, long long units,
@@ -106,18 +134,12 @@ k_filter_two(const int32_t *__restrict__ src, const int32_t *__restrict__ pay, l
             fl = 0;
 #pragma unroll
             for (int r = 0; r < F2_LOADS; r++) fl |= f2_flags<REC>(v[r], r0 + r * 32 * PER, n, lo, hi) << (PER * r);
-            uint32_t pre[F2_LOADS * PER], tot = 0;
-#pragma unroll
-            for (int j = 0; j < F2_LOADS * PER; j++) {
-                const uint32_t b = __ballot_sync(QG_FULL_MASK, (fl >> j) & 1u);
-                if (j % PER == 0) pre[j] = tot + __popc(b & lt);
-                else pre[j - j % PER] += __popc(b & lt);
-                tot += __popc(b);
-            }
+            uint32_t pre[F2_LOADS];
+            const uint32_t tot = f2_places<REC>(fl, pre);
             if (kept + tot > (uint32_t)F2<REC>::SEG || (ur == ub && tot > most)) break;
 #pragma unroll
             for (int r = 0; r < F2_LOADS; r++) {
-                uint32_t pos = kept + pre[r * PER];
+                uint32_t pos = kept + pre[r];
                 if ((fl >> (PER * r)) & 1u) stage[pos++] = make_int2(v[r].x, v[r].y);
                 if ((fl >> (PER * r)) & 2u) stage[pos] = make_int2(v[r].z, v[r].w);
             }
@@ -171,17 +193,8 @@ k_filter_two(const int32_t *__restrict__ src, const int32_t *__restrict__ pay, l
                 if ((fl >> (PER * r)) & F2<REC>::FM) v[r] = f2_load<REC>(REC ? src : pay, r0 + r * 32 * PER, n);
             }
         }
-        uint32_t pre[F2_LOADS], tot = 0;  // selected rows of the unit before this lane's load r
-#pragma unroll
-        for (int r = 0; r < F2_LOADS; r++) {
-            pre[r] = tot;
-#pragma unroll
-            for (int j = 0; j < PER; j++) {
-                const uint32_t b = __ballot_sync(QG_FULL_MASK, (fl >> (PER * r + j)) & 1u);
-                pre[r] += __popc(b & lt);
-                tot += __popc(b);
-            }
-        }
+        uint32_t pre[F2_LOADS];
+        const uint32_t tot = f2_places<REC>(fl, pre);
         // through shared memory, so that the warp's stores are consecutive
 #pragma unroll
         for (int r = 0; r < F2_LOADS; r++) {
