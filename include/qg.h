@@ -253,7 +253,8 @@ QG_API qg_status qg_join_filter_sort(qg_ctx *ctx, const int32_t *rkey, const int
  * knobs at their defaults, when R's keys are unique over a dense span (at most
  * 2 nR values): a counting join for S up to 18M rows, beyond it one partition
  * step fused with the filter if the rows spread evenly; the hash join (3) when R
- * has up to 2^23 keys of no dense span; else range partitioning by
+ * has up to 2^23 keys of no dense span (over 40M S rows: of a span above half
+ * of them); else range partitioning by
  * radix over the key, switching to the learned CDF partition function when
  * radix leaves more than 2% of the rows in buckets too large for shared memory
  * and the model does better on the same counts; 1 radix

@@ -2175,6 +2175,11 @@ constexpr int64_t PJ_DIRECT_S = 18'000'000;
 // skewed keys: 64K rows 92 / 156 us, 1M 107 / 415, 16M 303 / 925, 64M 910 /
 // 1665; random 32-bit keys: 1M 158 / 249, 16M 402 / 666, 64M 1316 / 1880.
 constexpr int64_t PJ_HASH_R = 1 << 23;
+// ... except with many probe rows and build keys close enough for the bucket
+// kernel's counting sort (4096 rows, 8192 key values, about a third of S joined):
+// 50M rows on keys three apart 960 us hashed, 658 partitioned; twenty apart 1091 / 1571.
+constexpr int64_t PJ_NEAR_S = 40'000'000;
+static bool pj_near(int64_t nS, unsigned long long span) { return nS > PJ_NEAR_S && span <= (unsigned long long)nS / 2; }
 // Slots a build row may look at: unique keys at load 1/2 need a few dozen.
 constexpr uint32_t PJ_HASH_PROBES = 256;
 
@@ -2236,6 +2241,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
             if (st != QG_OK && st != QG_ERR_CAPACITY) return st;
             ctx->pj_sparse = crowded || (unsigned long long)span + 1ull > 2ull * (unsigned long long)nR;
             if (!crowded && (ctx->pj_sparse || !direct)) {
+                if (pj_near(nS, (unsigned long long)span + 1ull)) ctx->pj_sparse = false;  // the next call looks at the span first
                 ctx->pj_stats[0] = 3;
                 return st;
             }
@@ -2281,6 +2287,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     // large probe inputs: one partition step, unless the build side is not dense or the rows spread unevenly
     const bool jp = dflt && nS > PJ_DIRECT_S;
     const bool may_hash = nR <= PJ_HASH_R && !hash_tried;
+    const bool filter_later = may_hash && nS <= PJ_NEAR_S;  // with sparse build keys, if the hash join hands back
     char *jp_work = aux + 2 * rb + 2 * sb + bmb + pj_level_bytes(PJ_MAX_BUCKETS, true);
     if (jp) {
         const qg_jp_r jr{&L.range->kmin, L.dflags, bitmap, T, nR};
@@ -2293,7 +2300,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     QG_TRY(qg_launch_chained(ctx, "k_pj_sfilter", k_pj_sfilter, (unsigned)std::min<long long>(tiles,
                              (long long)ctx->sm_count * 4), SF_THREADS, 0, skey, spay, nS, slo, shi, L.range, S,
                              &L.range->count, ctx->ctl, lb2, L.dh + 512, jp ? qg_jp_done(jp_work) : nullptr,
-                             jp && may_hash ? L.dflags + PJ_F_DENSE : nullptr));
+                             jp && filter_later ? L.dflags + PJ_F_DENSE : nullptr));
     // one copy brings R's key range, the S' count, the histograms and the dense flags
     constexpr size_t head = offsetof(PjPin, dflags) + PJ_F_WORDS * 4;
     static_assert(offsetof(PjPin, h) == 256 && offsetof(PjPin, dflags) == 256 + 4096, "as carved");
@@ -2305,7 +2312,8 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
         *out_n = ctx->hres->count;
         return *out_n > cap ? QG_ERR_CAPACITY : QG_OK;
     }
-    if (jp && may_hash && pin->dflags[PJ_F_DENSE] == 0u) {  // sparse build keys: the hash join, then what follows it
+    const bool near = pj_near(nS, (unsigned long long)(pin->range.kmax - pin->range.kmin) + 1ull);
+    if (jp && may_hash && !near && pin->dflags[PJ_F_DENSE] == 0u) {  // sparse build keys: the hash join, then what follows it
         ctx->pj_sparse = true;
         return join_filter_sort_impl(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay, out_spay, cap, out_n);
     }
@@ -2317,7 +2325,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
                pin->dflags[PJ_F_DENSE] != 0u && distinct == (unsigned long long)nR && g_pj_dense,
                pin->dflags[PJ_F_SENT_OK] != 0u, pin->dflags[PJ_F_SENT],
                bitmap, T};
-    if (dflt) ctx->pj_sparse = rs.rec_ready;
+    if (dflt) ctx->pj_sparse = rs.rec_ready && !near;
     long long M = 0;
     // pj_core ends with a read of the output count and the error word
     QG_TRY(pj_core(ctx, L, pin, nb, lb2, rs, R, Rsp, nR, S, Ssp, ns1, hr.kmin, hr.kmax, variant,

@@ -435,3 +435,28 @@ def test_join_large_dense(ctx, kind):
     assert bool((uk[1:] >= uk[:-1]).all())
     assert torch.equal((uk * 1000 + got[2]).sort().values, exp)
     assert torch.equal(got[1].to(torch.int64), table[(uk - base) & 0xFFFFFFFF])
+
+
+# Many probe rows on build keys three apart: partitioned, whichever path the last
+# call took (keys three hundred apart are hashed).
+def test_join_large_near_keys(ctx):
+    nS, nR = 40_000_003, 700_000
+    g = torch.Generator(device="cuda")
+    g.manual_seed(12)
+    ints = lambda lo, hi, n: torch.randint(lo, hi, (n,), generator=g, device="cuda")  # noqa: E731
+    r = torch.randperm(nR, generator=g, device="cuda")
+    rpay, soff, spay = ints(0, 1 << 20, nR), ints(0, 4 * nR, nS), ints(0, 1000, nS)
+    hit = (soff % 3 == 0) & (soff < 3 * nR) & (spay <= 99)
+    table = torch.empty(nR, dtype=torch.int64, device="cuda")
+    table[r] = rpay
+    exp = (soff[hit] // 3 * 1000 + spay[hit]).sort().values
+    for stride in (3, 300, 3, 3):
+        # rows that match no key lie between two of them
+        key = torch.where(soff % 3 == 0, soff // 3 * stride, soff // 3 * stride + 1)
+        got = ctx.join_filter_sort((r * stride).to(torch.int32), rpay.to(torch.int32), key.to(torch.int32),
+                                   spay.to(torch.int32), 0, 99, cap=nS)
+        k = got[0].to(torch.int64) // stride
+        assert bool((k[1:] >= k[:-1]).all())
+        assert torch.equal((k * 1000 + got[2]).sort().values, exp)
+        assert torch.equal(got[1].to(torch.int64), table[k])
+    assert ctx.join_stats()["path"] == "radix"
