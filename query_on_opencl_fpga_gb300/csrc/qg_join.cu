@@ -600,8 +600,9 @@ qg_status qg_join_hash_sort_async(qg_ctx *ctx, const int32_t *rkey, const int32_
     QG_TRY(join_build(ctx, rkey, rpay, 1, nR, 3 * colbytes + work, 0u, &tab, &mask, &jc, &tail));
     qg_sort_bufs A{nullptr, (uint32_t *)out_key, (uint32_t *)out_rpay, (uint32_t *)out_spay};
     qg_sort_bufs B{nullptr, (uint32_t *)tail, (uint32_t *)(tail + colbytes), (uint32_t *)(tail + 2 * colbytes)};
-    QG_TRY(join_probe(ctx, skey, spay, nS, slo, shi, tab, mask, jc, ProbeOut{A.k, A.a, A.b}, ProbeOut{B.k, B.a, B.b},
-                      cap));
+    // (with room for one row no sort follows, so it has to land in the output)
+    QG_TRY(join_probe(ctx, skey, spay, nS, slo, shi, tab, mask, jc, ProbeOut{A.k, A.a, A.b},
+                      cap > 1 ? ProbeOut{B.k, B.a, B.b} : ProbeOut{}, cap));
     qg_pre_launch(ctx);
     k_join_finish_async<<<1, 1, 0, ctx->stream>>>(jc, cap, (unsigned long long *)d_count, ctx->ctl);
     QG_TRY(qg_check_launch(ctx, "k_join_finish_async"));

@@ -66,7 +66,8 @@ qg_status qg_radix_passes_dev(qg_ctx *ctx, bool kv3, qg_sort_bufs a, qg_sort_buf
                               char *work, bool *result_in_b);
 // Three columns whose key range is known on the device only: `range` says how
 // many positions the keys (minus its key_off) have and thereby where the items
-// start, so that they end in `a`: in `b` for an odd number, else in `a`.
+// start, so that they end in `a`: in `b` for an odd number, else in `a`.  With
+// n_bound below 2 nothing runs, and an item has to be in `a` to begin with.
 struct qg_sort_range {
     uint32_t npos, key_off;
 };

@@ -243,3 +243,27 @@ def test_batch_dense_window_group_bys(ctx):
         assert ei.value.status == 7  # QG_ERR_UNSUPPORTED
     finally:
         b.close()
+
+
+# One and two output rows, key ranges around the ends of 0 to 4 digits: the sort's
+# passes end in the output whatever their number, and with one row there are none.
+@pytest.mark.parametrize("span", [1, 2, 256, 257, 1 << 16, (1 << 16) + 1, 1 << 24, (1 << 24) + 1, 1 << 32])
+@pytest.mark.parametrize("cap", [1, 2])
+def test_batch_join_small_capacity(ctx, orc, span, cap):
+    rkey = np.unique(np.array([0, span // 2, span - 1], np.int64)).astype(np.uint32).view(np.int32)
+    rpay = np.arange(rkey.size, dtype=np.int32) + 50
+    skey = rkey[::-1][:cap].copy()
+    spay = np.arange(skey.size, dtype=np.int32) + 7
+    inp = [torch.from_numpy(x).cuda() for x in (rkey, rpay, skey, spay)]
+    q = {"op": qb.OP_JOIN, "n": skey.size, "n2": rkey.size, "variant": -1, "inp": inp, "lo": 0, "hi": 100, "cap": cap,
+         "out": [torch.full((cap,), -77, dtype=torch.int32, device="cuda") for _ in range(3)],
+         "count": torch.zeros(1, dtype=torch.int64, device="cuda")}
+    b = qb.Batch([q], autotune=False)
+    try:
+        b.run()
+        b.check()
+        assert int(q["count"].item()) == skey.size
+        exp = orc.join_filter_sort(rkey, rpay, skey, spay, 0, 100, cap=4)
+        _same(qb.OP_JOIN, tuple(t[:skey.size] for t in q["out"]), tuple(torch.from_numpy(x) for x in exp))
+    finally:
+        b.close()
