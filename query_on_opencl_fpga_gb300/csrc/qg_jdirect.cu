@@ -188,8 +188,12 @@ k_jd_count(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, l
     qg_chain();
     __shared__ uint32_t s_woff[JD_ROUNDS * JD_WARPS], s_base, s_cnt, s_stop;
     __shared__ unsigned long long s_row[JD_TILE];
-    if (jd[JD_OK] != QG_JD_DONE) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // Other CTAs may store to the verdict meanwhile, so one thread reads it for all:
+    // a CTA leaves whole, here and in the loop, or not at all.
+    if (tid == 0) s_stop = qg_ld_relaxed_u32(&jd[JD_OK]) != QG_JD_DONE;
+    __syncthreads();
+    if (s_stop) return;
     const uint32_t lt = qg_lanemask_lt(), kmin = jd[JD_KMIN], span = jd[JD_SPAN];
     const long long ntiles = (n + JD_TILE - 1) / JD_TILE;
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -243,6 +247,7 @@ k_jd_count(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, l
             }
         }
         __syncthreads();
+        if (s_stop) return;  // a key with too many rows was met
 #pragma unroll
         for (int r = 0; r < JD_ROUNDS; r++) {
             uint32_t pos = s_woff[r * JD_WARPS + warp] + lpre[r];
@@ -253,7 +258,6 @@ k_jd_count(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, l
         }
         __syncthreads();
         const uint32_t cnt = s_cnt, at = s_base;
-        if (s_stop) return;  // a key with too many rows was met
         constexpr int U = 4;
         bool heavy = false;
         for (uint32_t i0 = tid; i0 < cnt; i0 += U * JD_THREADS) {

@@ -460,3 +460,38 @@ def test_join_large_near_keys(ctx):
         assert torch.equal((k * 1000 + got[2]).sort().values, exp)
         assert torch.equal(got[1].to(torch.int64), table[k])
     assert ctx.join_stats()["path"] == "radix"
+
+
+# Probe keys with far too many rows, met by some CTAs while others still start or
+# wait for an SM that another stream's kernels hold: the attempt ends everywhere.
+def test_join_counting_path_hot_keys_beside_other_work():
+    from query_on_opencl_fpga_gb300.api import Context
+
+    nR, nS = 30_000, 3_000_003
+    g = torch.Generator(device="cuda")
+    g.manual_seed(17)
+    ints = lambda lo, hi, n: torch.randint(lo, hi, (n,), generator=g, device="cuda")  # noqa: E731
+    roff, rpay = torch.randperm(nR, generator=g, device="cuda"), ints(0, 1000, nR)
+    soff, spay = ints(0, 2 * nR, nS), ints(0, 1000, nS)
+    soff[nS // 2:: 3] = 5 + ints(0, 3, soff[nS // 2:: 3].numel())
+    sel = (spay <= 299) & (soff < nR)
+    table = torch.empty(nR, dtype=torch.int64, device="cuda")
+    table[roff] = rpay
+    exp = (soff[sel] * 1000 + spay[sel]).sort().values
+    args = [t.to(torch.int32) for t in (roff, rpay, soff, spay)]
+    side, busy = torch.cuda.Stream(), torch.empty(1 << 26, dtype=torch.int32, device="cuda")
+    for rep in range(6):
+        c = Context()
+        try:
+            with torch.cuda.stream(side):
+                for _ in range(rep * 3):
+                    busy.add_(1)
+            got = c.join_filter_sort(*args, 0, 299, cap=nS)
+            assert c.join_stats()["path"] == "radix"
+        finally:
+            c.close()
+        k = got[0].to(torch.int64)
+        assert bool((k[1:] >= k[:-1]).all())
+        assert torch.equal((k * 1000 + got[2]).sort().values, exp)
+        assert torch.equal(got[1].to(torch.int64), table[k])
+    torch.cuda.synchronize()
