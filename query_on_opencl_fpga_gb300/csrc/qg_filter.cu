@@ -18,8 +18,8 @@ constexpr int FT_THREADS = 256;
 constexpr int FT_WARPS = FT_THREADS / 32;
 constexpr int FT_LB_WARPS = 4;  // warps doing the look-back: 128 predecessors per round
 
-// Two phases in one launch (records, and the default column form).  The rows
-// are cut into units of four 128-bit loads per lane of a warp, and every warp
+// Two phases in one launch (records, and the default column form below 2^22 rows).
+// The rows are cut into units of four 128-bit loads per lane of a warp, and every warp
 // owns a contiguous range of units:
 //   phase 1: the warp reads its keys (or records) and counts the selected rows,
 //            with no exchange between warps; it keeps each row's predicate bit,
@@ -32,9 +32,9 @@ constexpr int FT_LB_WARPS = 4;  // warps doing the look-back: 128 predecessors p
 //            the last unit from registers and the most recent ones from L2.
 // What bounds it is the memory's pace in both phases plus one exchange per
 // launch: neither a chain of look-backs, tile by tile (what records had:
-// 5M of them, 40 % kept, 30.8 us, now 21), nor a second launch (what columns
-// had: 16M rows, 10 % kept, 45.6 us in two launches, now 36.9; 4096-row tiles
-// with a look-back each 67).  One CTA per SM: with four to eight smaller ones
+// 5M of them, 40 % kept, 30.8 us, now 21; columns of 16M rows in 4096-row tiles
+// with a look-back each 67, now 34), nor a second launch (columns of 300K rows 18 us
+// in two, 13).  One CTA per SM: with four to eight smaller ones
 // the exchange took longer (49 us with six).  Loading a unit ahead did not help.
 // Keeping records spares their second read (16M, 10 % selected: 48.8 -> 34.1 us),
 // unless most would not fit anyway (40M, 90 %: 161 -> 170).  A column's payloads
@@ -117,7 +117,6 @@ k_filter_two(const int32_t *__restrict__ src, const int32_t *__restrict__ pay, l
     int2 *stage = reinterpret_cast<int2 *>(f2_raw) + (size_t)(threadIdx.x >> 5) * F2<REC>::SEG;
     uint16_t *s_mask = reinterpret_cast<uint16_t *>(reinterpret_cast<int2 *>(f2_raw) + (size_t)nw * F2<REC>::SEG);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t lt = qg_lanemask_lt();
     qg_lb_begin_dyn(lb, &s_tile, &s_epoch);
     const uint32_t tile = s_tile;
     const long long W = (long long)gridDim.x * nw, gw = (long long)tile * nw + warp;
@@ -213,6 +212,147 @@ k_filter_two(const int32_t *__restrict__ src, const int32_t *__restrict__ pay, l
         __syncwarp();
     }
     qg_lb_finish_dyn(lb, tile, gridDim.x - 1, s_epoch);
+}
+
+// The default column filter of larger inputs: the two phases in two launches, the
+// launch boundary being their exchange.  In k_filter_two a warp writes the rows it
+// has counted, so rows selected close together (a time range of a sorted table) are
+// written by a few SMs: 40M sorted rows, 1 % selected 109 us a call, 59 here (16M 60
+// / 40, 4M 32 / 30).  Here the write phase deals the units out one by one to all
+// warps; it reads the predicate bits (64 bytes per unit) instead of the keys.  For
+// rows selected evenly both take the same (16M rows, 10 %: 46 / 45 us; 40M 74 / 75,
+// 1 % 69 / 72); below 4M rows one launch is 1 to 2 us faster.  As the keys are not
+// read again, the output may lie over them.
+//   per: units per range, which one warp of the count phase takes;
+//   upre: selected rows of the range before the unit; rtot: of the range.
+constexpr int FC_WARPS = 32;  // k_filter_count, one CTA per SM
+constexpr int FW_WARPS = 28;  // k_filter_write: 72 registers; 24 warps take 48 us instead of 42, 32 spill
+constexpr int FW_EACH = 12;   // ranges per thread, at most
+constexpr int64_t F2_TWO_ROWS = 1 << 22;
+
+__global__ void __launch_bounds__(32 * FC_WARPS, 1)
+k_filter_count(const int32_t *__restrict__ key, long long n, uint32_t units, uint32_t per, int32_t lo, int32_t hi,
+               uint16_t *__restrict__ mask, uint32_t *__restrict__ upre, uint32_t *__restrict__ rtot) {
+    constexpr int PER = F2<false>::PER, UNIT = F2<false>::UNIT;
+    qg_chain();
+    const int lane = threadIdx.x & 31;
+    const uint32_t range = blockIdx.x * FC_WARPS + (threadIdx.x >> 5);
+    const long long ub = (long long)range * per, ue = min(ub + per, (long long)units);
+    uint32_t run = 0;
+    for (long long u = ub; u < ue; u++) {
+        const long long r0 = u * UNIT + lane * PER;
+        int4 v[F2_LOADS];
+#pragma unroll
+        for (int r = 0; r < F2_LOADS; r++) v[r] = f2_load<false>(key, r0 + r * 32 * PER, n);
+        uint32_t fl = 0;
+#pragma unroll
+        for (int r = 0; r < F2_LOADS; r++) fl |= f2_flags<false>(v[r], r0 + r * 32 * PER, n, lo, hi) << (PER * r);
+        mask[u * 32 + lane] = (uint16_t)fl;
+        if (lane == 0) upre[u] = run;
+        run += __reduce_add_sync(QG_FULL_MASK, __popc(fl));
+    }
+    if (lane == 0) rtot[range] = run;
+}
+
+__global__ void __launch_bounds__(32 * FW_WARPS, 1)
+k_filter_write(const uint16_t *__restrict__ mask, const uint32_t *__restrict__ upre, const uint32_t *__restrict__ rtot,
+               uint32_t ranges, const int32_t *__restrict__ pay, long long n, uint32_t units, uint32_t per,
+               int2 *__restrict__ out, long long cap, long long *__restrict__ d_count) {
+    constexpr int PER = F2<false>::PER, UNIT = F2<false>::UNIT;
+    qg_chain();
+    extern __shared__ __align__(16) unsigned char f2_raw[];
+    __shared__ uint32_t s_w[FW_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int2 *stage = reinterpret_cast<int2 *>(f2_raw) + (size_t)warp * F2<false>::SEG;
+    uint32_t *s_base = reinterpret_cast<uint32_t *>(reinterpret_cast<int2 *>(f2_raw) + (size_t)FW_WARPS * F2<false>::SEG);
+    const uint32_t W = gridDim.x * FW_WARPS;
+    uint32_t u = blockIdx.x * FW_WARPS + warp;
+    // the bits two units ahead, the payloads of lanes with a selected row one unit
+    // ahead (16M rows, 10 %: 46.5 us without the payloads, 45)
+    uint32_t fl = 0, up = 0, fn = 0, pn = 0;
+    if (u < units) {
+        fl = mask[(size_t)u * 32 + lane];
+        up = upre[u];
+    }
+    {  // the ranges' first output rows
+        uint32_t c[FW_EACH], sum = 0;
+        const uint32_t b0 = tid * FW_EACH;
+#pragma unroll
+        for (int i = 0; i < FW_EACH; i += 4) {  // (ranges is a multiple of four)
+            const uint4 x = b0 + i < ranges ? __ldg(reinterpret_cast<const uint4 *>(rtot + b0 + i)) : make_uint4(0, 0, 0, 0);
+            c[i] = x.x;
+            c[i + 1] = x.y;
+            c[i + 2] = x.z;
+            c[i + 3] = x.w;
+        }
+#pragma unroll
+        for (int i = 0; i < FW_EACH; i++) {
+            const uint32_t x = c[i];
+            c[i] = sum;
+            sum += x;
+        }
+        uint32_t inc = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t x = __shfl_up_sync(QG_FULL_MASK, inc, d);
+            if (lane >= d) inc += x;
+        }
+        if (lane == 31) s_w[warp] = inc;
+        __syncthreads();
+        const uint32_t at = __reduce_add_sync(QG_FULL_MASK, lane < warp ? s_w[lane] : 0u) + inc - sum;
+#pragma unroll
+        for (int i = 0; i < FW_EACH; i++)
+            if (b0 + i < ranges) s_base[b0 + i] = at + c[i];
+        if (blockIdx.x == 0 && tid == 32 * FW_WARPS - 1) *d_count = (long long)at + sum;
+        __syncthreads();
+    }
+    auto load = [&](int4 (&v)[F2_LOADS], uint32_t unit, uint32_t f) {
+        const long long r0 = (long long)unit * UNIT + lane * PER;
+#pragma unroll
+        for (int r = 0; r < F2_LOADS; r++) {
+            v[r] = make_int4(0, 0, 0, 0);
+            if ((f >> (PER * r)) & F2<false>::FM) v[r] = f2_load<false>(pay, r0 + r * 32 * PER, n);
+        }
+    };
+    int4 vn[F2_LOADS];
+    load(vn, u, fl);
+    if (u + W < units) {
+        fn = mask[(size_t)(u + W) * 32 + lane];
+        pn = upre[u + W];
+    }
+    while (u < units) {
+        const uint32_t f = fl, p = up, next = u + W;
+        int4 v[F2_LOADS];
+#pragma unroll
+        for (int r = 0; r < F2_LOADS; r++) v[r] = vn[r];
+        fl = fn;
+        up = pn;
+        if (next < units) load(vn, next, fl);
+        fn = 0;
+        if (next + W < units) {
+            fn = mask[(size_t)(next + W) * 32 + lane];
+            pn = upre[next + W];
+        }
+        if (__any_sync(QG_FULL_MASK, f != 0u)) {
+            const long long r0 = (long long)u * UNIT + lane * PER;
+            uint32_t pre[F2_LOADS];
+            const uint32_t tot = f2_places<false>(f, pre);
+#pragma unroll
+            for (int r = 0; r < F2_LOADS; r++) {
+                uint32_t pos = pre[r];
+                const int x[4] = {v[r].x, v[r].y, v[r].z, v[r].w};
+#pragma unroll
+                for (int j = 0; j < PER; j++)
+                    if ((f >> (PER * r + j)) & 1u) stage[pos++] = make_int2((int)(r0 + r * 32 * PER + j), x[j]);
+            }
+            __syncwarp();
+            const long long at = (long long)s_base[u / per] + p;
+            const uint32_t lim = at >= cap ? 0u : (uint32_t)min((long long)tot, cap - at);
+            for (uint32_t i = lane; i < lim; i += 32) out[at + i] = stage[i];
+            __syncwarp();
+        }
+        u = next;
+    }
 }
 
 // Columns: int32 key and payload, four rows per 128-bit load.  Output is the
@@ -458,7 +598,7 @@ static qg_status finish_count(qg_ctx *ctx, int64_t cap, int64_t *out_n) {
 
 // Launch of k_filter_two: a warp per unit until every SM is full, then
 // contiguous ranges.  `spill` holds the predicate bits of a warp's units past
-// the 16 it keeps in shared memory (inputs above about 60M column rows).
+// the 16 it keeps in shared memory (above 20M records on 152 SMs, or 40M column rows).
 template <bool REC>
 static qg_status f2_launch(qg_ctx *ctx, const int32_t *src, const int32_t *pay, int64_t n, int32_t lo, int32_t hi,
                            void *out, int64_t cap, long long *d_count) {
@@ -487,6 +627,41 @@ static qg_status f2_launch(qg_ctx *ctx, const int32_t *src, const int32_t *pay, 
     return qg_check_launch(ctx, REC ? "k_filter_rec" : "k_filter_two");
 }
 
+static size_t f2_two_bytes(qg_ctx *ctx, int64_t n) {
+    return (size_t)qg_ceil_div(n, F2<false>::UNIT) * 68 + 512 + (size_t)ctx->sm_count * FC_WARPS * 4;
+}
+// Whether the scratch arena holds the bits, or may grow (not while a graph is captured).
+static bool f2_two_fits(qg_ctx *ctx, int64_t n) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    return f2_two_bytes(ctx, n) <= ctx->scratch_bytes ||
+           (cudaStreamIsCapturing(ctx->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone);
+}
+
+static qg_status f2_launch_two(qg_ctx *ctx, const int32_t *key, const int32_t *pay, int64_t n, int32_t lo, int32_t hi,
+                               void *out, int64_t cap, long long *d_count) {
+    const uint32_t units = (uint32_t)qg_ceil_div(n, F2<false>::UNIT);
+    const long long sms = std::min<long long>(ctx->sm_count, FW_EACH * FW_WARPS);  // ranges fit the write phase's threads
+    const uint32_t gc = (uint32_t)std::min<long long>(qg_ceil_div(units, FC_WARPS), sms), ranges = gc * FC_WARPS;
+    const uint32_t gw = (uint32_t)std::min<long long>(qg_ceil_div(units, FW_WARPS), ctx->sm_count);
+    const uint32_t per = (uint32_t)qg_ceil_div(units, ranges);
+    const size_t mb = qg_align_up((size_t)units * 64, 256), ub = qg_align_up((size_t)units * 4, 256);
+    char *scr;
+    QG_TRY(qg_scratch(ctx, f2_two_bytes(ctx, n), &scr));
+    uint16_t *mask = (uint16_t *)scr;
+    uint32_t *upre = (uint32_t *)(scr + mb), *rtot = (uint32_t *)(scr + mb + ub);
+    const size_t smem = (size_t)FW_WARPS * F2<false>::SEG * 8 + (size_t)ranges * 4;
+    static size_t attr = 0;
+    if (attr < smem) {
+        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_filter_write, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "attr");
+        attr = smem;
+    }
+    qg_pre_launch(ctx);
+    k_filter_count<<<gc, 32 * FC_WARPS, 0, ctx->stream>>>(key, n, units, per, lo, hi, mask, upre, rtot);
+    QG_TRY(qg_check_launch(ctx, "k_filter_count"));
+    return qg_launch_chained(ctx, "k_filter_write", k_filter_write, gw, 32 * FW_WARPS, smem, mask, upre, rtot, ranges, pay,
+                             n, units, per, (int2 *)out, cap, d_count);
+}
+
 // The count of an empty input: the host word directly, a device word in stream order.
 static qg_status qg_zero_count(qg_ctx *ctx, long long *d_count) {
     if (d_count == (long long *)&ctx->hres->count) ctx->hres->count = 0;
@@ -502,8 +677,7 @@ qg_status qg_filter_rec_launch(qg_ctx *ctx, const void *in, int64_t n, int32_t l
     if (((uintptr_t)in & 15) != 0 || ((uintptr_t)out & 7) != 0) return QG_ERR_INVALID;
     // Phase 2 reads rows that other warps' writes may have reached by then
     // when the output overlaps the input: such a call filters a copy.
-    const uintptr_t ib = (uintptr_t)in, ob = (uintptr_t)out;
-    if (ib < ob + (size_t)std::min(cap, n) * 8 && ob < ib + (size_t)n * 8) {
+    if (qg_overlap(out, (size_t)std::min(cap, n) * 8, in, (size_t)n * 8)) {
         char *tmp;
         QG_TRY(qg_aux(ctx, (size_t)n * 8, &tmp));
         QG_TRY_CUDA(ctx, cudaMemcpyAsync(tmp, in, (size_t)n * 8, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
@@ -526,7 +700,13 @@ qg_status qg_filter_cols_launch(qg_ctx *ctx, const int32_t *key, const int32_t *
     int64_t tiles = qg_ceil_div(n, TILE);
     if (tiles > 0x7fffffff || n > 0x7fffffffLL) return QG_ERR_UNSUPPORTED;
     const int variant = qg_effective_variant(ctx, QG_STEER_FILTER, g_filter_variant);
-    if (variant == 2) return f2_launch<false>(ctx, key, pay, n, lo, hi, out, cap, d_count);
+    if (variant == 2) {
+        // k_filter_two writes rows while other CTAs still read keys
+        const bool over = qg_overlap(out, (size_t)std::min(cap, n) * 8, key, (size_t)n * 4);
+        if (over || (n >= F2_TWO_ROWS && f2_two_fits(ctx, n)))
+            return f2_launch_two(ctx, key, pay, n, lo, hi, out, cap, d_count);
+        return f2_launch<false>(ctx, key, pay, n, lo, hi, out, cap, d_count);
+    }
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, tiles, QG_SITE_FILTER, &lb));
     if (variant == 1) {

@@ -238,6 +238,10 @@ qg_status qg_read_count(qg_ctx *ctx, const long long *d, long long *h);
     } while (0)
 
 static inline size_t qg_align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
+// Whether [a, a + an) and [b, b + bn) share a byte.
+static inline bool qg_overlap(const void *a, size_t an, const void *b, size_t bn) {
+    return (uintptr_t)a < (uintptr_t)b + bn && (uintptr_t)b < (uintptr_t)a + an;
+}
 static inline int64_t qg_ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // ---------------------------------------------------------------------------

@@ -191,3 +191,45 @@ def test_filter_rec_kept_rows(ctx, orc, units, sel):
     with pytest.raises(QGError) as e:
         ctx.filter_range_rec(rec, -3, 5, cap=exp.shape[0] - 1)
     assert e.value.status == 3
+
+
+# Two launches from 2^22 rows on: the line and beside it, sorted keys (the selected
+# rows close together) and others, none, some and all selected, a capacity among them.
+@pytest.mark.parametrize("n", [(1 << 22) - 1, 1 << 22, (1 << 22) + 513, 152 * 32 * 512 * 3 + 5])
+@pytest.mark.parametrize("sorted_keys", [True, False])
+def test_filter_cols_two_launches(ctx, n, sorted_keys):
+    from query_on_opencl_fpga_gb300 import QGError
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    key = torch.randint(-(2 ** 31), 2 ** 31, (n,), generator=g, device="cuda")
+    key = (key.sort().values if sorted_keys else key).to(torch.int32)
+    pay = torch.randint(-(2 ** 31), 2 ** 31, (n,), generator=g, device="cuda").to(torch.int32)
+    for lo, hi in [(0, 30_000_000), (-(2 ** 31), 2 ** 31 - 1), (5, 4), (-(2 ** 31), 0)]:
+        at = ((key >= lo) & (key <= hi)).nonzero().flatten()
+        exp = torch.stack([at.to(torch.int32), pay[at]], 1)
+        assert torch.equal(ctx.filter_cols(key, pay, lo, hi), exp)
+        m = exp.shape[0]
+        if m > 1:
+            out = torch.full((m + 64, 2), 7, dtype=torch.int32, device="cuda")
+            with pytest.raises(QGError) as e:
+                ctx.filter_cols(key, pay, lo, hi, cap=m - 1, out=out)
+            assert e.value.status == 3
+            assert torch.equal(out[: m - 1], exp[:-1]) and bool((out[m - 1:] == 7).all())
+
+
+@pytest.mark.parametrize("n", [1, 5, 4097, 300_007, 5_000_003])
+@pytest.mark.parametrize("sel", [0.1, 1.0])
+def test_filter_cols_over_its_keys(ctx, n, sel):
+    # the output lies over the key column: every key is read before a row is written
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    for _ in range(3):
+        key = torch.randint(0, 1000, (n,), generator=g, device="cuda").to(torch.int32)
+        pay = torch.randint(0, 1000, (n,), generator=g, device="cuda").to(torch.int32)
+        hi = int(1000 * sel) - 1
+        at = (key <= hi).nonzero().flatten()
+        exp = torch.stack([at.to(torch.int32), pay[at]], 1)
+        buf = torch.empty((n, 2), dtype=torch.int32, device="cuda")
+        keys = buf.view(-1)[:n].copy_(key)
+        assert torch.equal(ctx.filter_cols(keys, pay, 0, hi, out=buf), exp)
