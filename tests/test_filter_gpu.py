@@ -233,3 +233,26 @@ def test_filter_cols_over_its_keys(ctx, n, sel):
         buf = torch.empty((n, 2), dtype=torch.int32, device="cuda")
         keys = buf.view(-1)[:n].copy_(key)
         assert torch.equal(ctx.filter_cols(keys, pay, 0, hi, out=buf), exp)
+
+
+# The output over the input: at its start, before it (records that its rows have
+# left behind) and inside it; one tile of 4096 records, its edges, many tiles.
+@pytest.mark.parametrize("n", [1, 4095, 4096, 4097, 300_007, 5_000_001])
+@pytest.mark.parametrize("shift", [0, -3000, 3000])
+@pytest.mark.parametrize("sel", [0.02, 1.0])
+def test_filter_rec_over_its_input(ctx, n, shift, sel):
+    import ctypes
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    rec = torch.stack([torch.arange(n, device="cuda"), torch.randint(0, 1000, (n,), generator=g, device="cuda")], 1)
+    rec = rec.to(torch.int32)
+    hi = int(1000 * sel) - 1
+    exp = rec[rec[:, 1] <= hi]
+    buf = torch.full((n + 6000, 2), -9, dtype=torch.int32, device="cuda")
+    buf[3000: 3000 + n] = rec
+    cnt = ctypes.c_int64()
+    out = buf[3000 + shift: 3000 + shift + n]
+    st = ctx.lib.qg_filter_range_rec(ctx.handle, buf[3000:].data_ptr(), n, -5, hi, out.data_ptr(), n, ctypes.byref(cnt))
+    assert st == 0 and cnt.value == exp.shape[0]
+    assert torch.equal(out[: cnt.value], exp)
