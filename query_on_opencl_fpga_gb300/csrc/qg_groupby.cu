@@ -1657,7 +1657,14 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
         }
         return QG_OK;
     };
-    const bool may_wide = gm == 0 && qg_gbw_applies(n, cap);
+    // The partitions' groups are written before it is known whether all of them have a
+    // place: not over a column that the path after it would read.
+    auto over = [&](const void *out, size_t bytes) {
+        return qg_overlap(out, bytes, key, (size_t)n * 4) || qg_overlap(out, bytes, val, (size_t)n * 4) ||
+               (val2 && qg_overlap(out, bytes, val2, (size_t)n * 4));
+    };
+    const bool may_wide = gm == 0 && qg_gbw_applies(n, cap) && !over(gkey, (size_t)cap * 4) &&
+                          !over(gsum, (size_t)cap * 8) && !over(gcnt, (size_t)cap * 8);
     bool narrow = true;
     if (may_wide && ctx->gb_first == 1) {
         uint32_t v;

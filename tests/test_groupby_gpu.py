@@ -611,3 +611,28 @@ def test_groupby_wide_capacity(ctx, orc):
             ctx.groupby_cols(dev(key), dev(key), cap=g - 1)
         assert e.value.status == 3
         _dense_case(ctx, orc, key, key, cap=g)
+
+
+# Outputs over an input column, keys that the partitioned path gives up after it has
+# written groups (more distinct keys in a part than its table takes).
+@pytest.mark.parametrize("which", ["key", "val"])
+def test_groupby_outputs_over_inputs(orc, which):
+    rng = np.random.default_rng(32)
+    n = 120_000
+    key = rng.choice(rng.integers(-(2 ** 31), 2 ** 31, 50), n).astype(np.int32)
+    key[n - 16_000:] = rng.permutation(16_000)
+    val = rng.integers(0, 1000, n).astype(np.int32)
+    from query_on_opencl_fpga_gb300.api import Context
+
+    c = Context()
+    try:
+        exp = orc.groupby_cols(key, val)
+        for _ in range(2):
+            k, v = dev(key), dev(val)
+            over = k if which == "key" else v
+            out = (over, torch.empty(n, dtype=torch.int64, device="cuda"), torch.empty(n, dtype=torch.int64, device="cuda"))
+            got = c.groupby_cols(k, v, cap=n, out=out)
+            for g, e in zip(got, exp):
+                assert np.array_equal(g.cpu().numpy(), e)
+    finally:
+        c.close()
