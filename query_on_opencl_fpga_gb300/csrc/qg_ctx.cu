@@ -367,7 +367,6 @@ static qg_status map_error(qg_ctx *ctx, const int32_t *h) {
     cudaMemsetAsync(ctx->ctl->gbd, 0, sizeof(ctx->ctl->gbd), ctx->stream);  // dense group-by state words
     cudaMemsetAsync(ctx->ctl->shist, 0, sizeof(ctx->ctl->shist), ctx->stream);
     cudaMemsetAsync(ctx->ctl->jd, 0, sizeof(ctx->ctl->jd), ctx->stream);
-    cudaMemsetAsync(&ctx->ctl->jd_arrived, 0, sizeof(uint32_t), ctx->stream);
     cudaMemsetAsync(&ctx->ctl->gbw_rows, 0, sizeof(unsigned long long), ctx->stream);
     cudaStreamSynchronize(ctx->stream);  // done before any later stream of this context runs
     ctx->table_dirty = true;

@@ -22,8 +22,7 @@ struct qg_control {
     uint32_t shist[4 * 256];        // a record sort's digit counts, zero between sorts
     unsigned int gbw_few;           // the group-by's key sample shows few groups (written before it is read)
     unsigned long long gbw_rows;    // records appended by the wide-key group-by, zero between calls
-    uint32_t jd[12];                // state of the counting join (qg_jdirect.cu)
-    uint32_t jd_arrived, jd_pad;    // its scan's tiles that are done (wraps to zero)
+    uint32_t jd[8];                 // state of the counting join (qg_jdirect.cu)
     // Address of the context's host error word (0: none), written with the
     // first error only: a call that met no error reads it after its
     // synchronisation instead of copying this block back.

@@ -12,13 +12,14 @@
 // rows of that key counted before it, so nothing is partitioned or sorted:
 //   1. k_jd_range  R's key range
 //   2. k_jd_fill   entries = 0
-//   3. k_jd_table  entries of R's keys = (payload, JD_HERE)
+//   3. k_jd_table  entries of R's keys = (payload, JD_HERE); a key met twice ends
+//                  the attempt, before S is read
 //   4. k_jd_count  S rows that pass the filter: one 64-bit atomic on the key's
 //                  entry returns R's payload (does the key match?) and the
 //                  row's number among its key's rows; (key, payload, number)
 //                  are appended
 //   5. k_jd_scan   counts -> first places; every key and its R payload are
-//                  written as often as counted; the distinct keys are counted
+//                  written as often as counted
 //   6. k_jd_write  every appended row's S payload to its place
 // Six launches (four for a small build side, k_jd_build) and one wait.  Where the
 // scattered accesses leave L2, the rows are partitioned first (qg_jpart.cu).  A key with
@@ -37,8 +38,7 @@ enum {
     JD_NKMIN = 0, JD_KMAX = 1, // ~(smallest key), largest key (unsigned)
     JD_OK = QG_JD_OK,           // a qg_jd_result: QG_JD_DONE while nothing speaks against the path
     JD_KMIN = 5, JD_SPAN = 6,   // first key and number of key values of the table
-    JD_DISTINCT = 8,            // table entries of R's keys
-    JD_ROWS = 9,                // appended rows
+    JD_ROWS = 7,                // appended rows
 };
 
 constexpr int JD_THREADS = 256;
@@ -86,7 +86,6 @@ k_jd_fill(unsigned long long *__restrict__ E, long long nR, uint32_t *__restrict
         jd[JD_OK] = ok ? QG_JD_DONE : QG_JD_SPARSE;
         jd[JD_KMIN] = kmin;
         jd[JD_SPAN] = ok ? (uint32_t)w : 0u;
-        jd[JD_DISTINCT] = 0;
         jd[JD_ROWS] = 0;
     }
     if (!ok) return;
@@ -94,6 +93,14 @@ k_jd_fill(unsigned long long *__restrict__ E, long long nR, uint32_t *__restrict
     for (unsigned long long i = (unsigned long long)blockIdx.x * JD_THREADS + threadIdx.x; i < (w + 1) / 2;
          i += (unsigned long long)gridDim.x * JD_THREADS)
         E2[i] = make_ulonglong2(0ull, 0ull);
+}
+
+// R's payload into its key's entry; true: another row of the key was there before.
+// (An exchange costs what the store did: tables of 1M rows 11 us.  Counting the
+// entries afterwards found duplicates only when all of S had been counted, 16M rows
+// 60 us in vain.)
+__device__ __forceinline__ bool jd_put(unsigned long long *e, uint32_t pay) {
+    return (uint32_t)atomicExch(e, (unsigned long long)pay << 32 | JD_HERE) & JD_HERE;
 }
 
 __global__ void __launch_bounds__(JD_THREADS)
@@ -105,6 +112,7 @@ k_jd_table(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, l
     const uint32_t kmin = jd[JD_KMIN];
     constexpr int U = 4;  // rows in flight per thread
     const long long stride = (long long)gridDim.x * JD_THREADS;
+    bool twice = false;
     for (long long i0 = (long long)blockIdx.x * JD_THREADS + threadIdx.x; i0 < nR; i0 += U * stride) {
         uint32_t k[U], p[U];
 #pragma unroll
@@ -115,8 +123,9 @@ k_jd_table(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, l
         }
 #pragma unroll
         for (int u = 0; u < U; u++)
-            if (i0 + u * stride < nR) E[k[u]] = (unsigned long long)p[u] << 32 | JD_HERE;
+            if (i0 + u * stride < nR) twice |= jd_put(E + k[u], p[u]);
     }
+    if (twice) jd[JD_OK] = QG_JD_OTHER;
 }
 
 // The three steps above in one CTA: with so few rows the launches are what costs.
@@ -159,7 +168,6 @@ k_jd_build(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, u
         jd[JD_OK] = ok ? QG_JD_DONE : QG_JD_SPARSE;
         jd[JD_KMIN] = kmin;
         jd[JD_SPAN] = ok ? (uint32_t)w : 0u;
-        jd[JD_DISTINCT] = 0;
         jd[JD_ROWS] = 0;
     }
     if (!ok) return;
@@ -168,7 +176,7 @@ k_jd_build(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, u
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < JD_ONE_PER; j++)
-        if (j * JD_ONE_THREADS + tid < nR) E[k[j] - kmin] = (unsigned long long)p[j] << 32 | JD_HERE;
+        if (j * JD_ONE_THREADS + tid < nR && jd_put(E + (k[j] - kmin), p[j])) jd[JD_OK] = QG_JD_OTHER;
 }
 
 // S rows, 4096 per tile (persistent CTAs): the rows that pass the filter and
@@ -285,18 +293,17 @@ k_jd_count(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, l
 
 // Counts of the table's entries -> first places (in the entries' low words),
 // 256 * PER entries per tile with a look-back over the tiles; a warp writes the keys
-// and R payloads of 32 entries at a time, consecutively.  The last tile to end
-// stores the verdict.
+// and R payloads of 32 entries at a time, consecutively.
 template <int PER>
 __global__ void __launch_bounds__(JD_THREADS)
-k_jd_scan(unsigned long long *__restrict__ E, long long nR, uint32_t *__restrict__ jd, uint32_t *__restrict__ ok,
+k_jd_scan(unsigned long long *__restrict__ E, const uint32_t *__restrict__ jd, uint32_t *__restrict__ ok,
           uint32_t *__restrict__ oa, long long cap, long long *__restrict__ d_count, volatile uint32_t *result,
-          uint32_t *__restrict__ arrived, qg_lookback lb) {
+          qg_lookback lb) {
     qg_chain();
-    __shared__ uint32_t s_tile, s_epoch, s_excl, s_w[JD_WARPS], s_d[JD_WARPS], s_tmp[2 * JD_WARPS];
+    __shared__ uint32_t s_tile, s_epoch, s_w[JD_WARPS], s_tmp[2 * JD_WARPS];
     qg_lb_begin_dyn(lb, &s_tile, &s_epoch);
-    const uint32_t tile = s_tile, kmin = jd[JD_KMIN];
-    const uint32_t span = jd[JD_OK] == QG_JD_DONE ? jd[JD_SPAN] : 0u;
+    const uint32_t tile = s_tile, kmin = jd[JD_KMIN], verdict = jd[JD_OK];
+    const uint32_t span = verdict == QG_JD_DONE ? jd[JD_SPAN] : 0u;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t base = tile * (PER * JD_THREADS) + warp * (PER * 32);
     unsigned long long e[PER];
@@ -305,12 +312,10 @@ k_jd_scan(unsigned long long *__restrict__ E, long long nR, uint32_t *__restrict
         const uint32_t i = base + j * 32 + lane;
         e[j] = i < span ? __ldcg(E + i) : 0ull;
     }
-    uint32_t pre[PER], sum = 0, have = 0;  // counted rows before the entry, among the warp's
+    uint32_t pre[PER], sum = 0;  // counted rows before the entry, among the warp's
 #pragma unroll
     for (int j = 0; j < PER; j++) {
-        const bool in = (uint32_t)e[j] & JD_HERE;
-        have += in;
-        const uint32_t c = in ? (uint32_t)e[j] & ~JD_HERE : 0u;
+        const uint32_t c = (uint32_t)e[j] & JD_HERE ? (uint32_t)e[j] & ~JD_HERE : 0u;
         uint32_t inc = c;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -320,18 +325,13 @@ k_jd_scan(unsigned long long *__restrict__ E, long long nR, uint32_t *__restrict
         pre[j] = sum + inc - c;
         sum += __shfl_sync(QG_FULL_MASK, inc, 31);
     }
-    have = __reduce_add_sync(QG_FULL_MASK, have);
-    if (lane == 0) {
-        s_w[warp] = sum;
-        s_d[warp] = have;
-    }
+    if (lane == 0) s_w[warp] = sum;
     __syncthreads();
-    uint32_t before = 0, total = 0, mine = 0;
+    uint32_t before = 0, total = 0;
 #pragma unroll
     for (int w = 0; w < JD_WARPS; w++) {
         before += w < warp ? s_w[w] : 0u;
         total += s_w[w];
-        mine += s_d[w];
     }
     const uint32_t excl = qg_lb_wide_exclusive<JD_WARPS>(lb, tile, s_epoch, total, s_tmp);
 #pragma unroll
@@ -359,18 +359,9 @@ k_jd_scan(unsigned long long *__restrict__ E, long long nR, uint32_t *__restrict
             }
         }
     }
-    if (tid == 0) {
-        if (tile == gridDim.x - 1) *d_count = (long long)excl + total;
-        if (mine) atomicAdd(&jd[JD_DISTINCT], mine);
-        __threadfence();
-        // the last tile to get here has every tile's distinct keys
-        if (atomicInc(arrived, gridDim.x - 1) == gridDim.x - 1) {
-            __threadfence();
-            uint32_t v = __ldcg(&jd[JD_OK]);
-            if (v == QG_JD_DONE && (long long)__ldcg(&jd[JD_DISTINCT]) != nR) v = QG_JD_OTHER;
-            jd[JD_OK] = v;
-            if (result) *result = v;
-        }
+    if (tid == 0 && tile == gridDim.x - 1) {
+        *d_count = (long long)excl + total;
+        if (result) *result = verdict;
     }
     qg_lb_finish_dyn(lb, tile, gridDim.x - 1, s_epoch);
 }
@@ -439,7 +430,7 @@ qg_status qg_jd_launch(qg_ctx *ctx, char *work, const int32_t *rkey, const int32
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, tiles, QG_SITE_JOIN_PROBE, &lb));
     QG_TRY(qg_launch_chained(ctx, "k_jd_scan", per == 2 ? k_jd_scan<2> : k_jd_scan<16>, (unsigned)tiles, JD_THREADS, 0,
-                             E, nR, jd, out_key, out_rpay, cap, d_count, result, &ctx->ctl->jd_arrived, lb));
+                             E, jd, out_key, out_rpay, cap, d_count, result, lb));
     return qg_launch_chained(ctx, "k_jd_write", k_jd_write, jd_grid(ctx, nS / 4, JD_THREADS, 8), JD_THREADS, 0, E, jd,
                              ak, ap, an, out_spay, cap);
 }

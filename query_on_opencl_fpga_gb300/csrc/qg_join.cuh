@@ -6,7 +6,7 @@
 // stream, no read back.  `work`: qg_jd_bytes(nR, nS) bytes, 256-byte aligned.
 // Afterwards ctl->jd[QG_JD_OK] (also *result, when set) is QG_JD_DONE when the
 // outputs hold the result, *d_count then the match count (the first cap rows
-// are written); else what stood against it, and the outputs hold nothing valid.
+// are written); else what stood against it, and nothing was written.
 enum { QG_JD_OK = 4 };
 enum qg_jd_result : uint32_t {
     QG_JD_SPARSE = 0,  // R's keys spread over more than 2 nR values

@@ -495,3 +495,36 @@ def test_join_counting_path_hot_keys_beside_other_work():
         assert torch.equal((k * 1000 + got[2]).sort().values, exp)
         assert torch.equal(got[1].to(torch.int64), table[k])
     torch.cuda.synchronize()
+
+
+# Outputs over the probe columns: an attempt that is given up has written nothing
+# when the next path reads them.
+@pytest.mark.parametrize("kind", ["dup", "hot"])
+def test_join_outputs_over_inputs(orc, kind):
+    import ctypes
+
+    from query_on_opencl_fpga_gb300.api import Context
+
+    rng = np.random.default_rng(31)
+    nR, nS = 20_000, 300_000
+    rkey = rng.permutation(nR).astype(np.int32)
+    if kind == "dup":
+        rkey[5] = rkey[6]
+    rpay = rng.integers(0, 1000, nR).astype(np.int32)
+    skey = rng.integers(-10, nR + 10, nS).astype(np.int32)
+    if kind == "hot":
+        skey[:6000] = 77
+    spay = rng.integers(0, 1000, nS).astype(np.int32)
+    c = Context()
+    try:
+        exp = orc.join_filter_sort(rkey, rpay, skey, spay, -(2 ** 31), 299, cap=nS, mt=True)
+        r, rp, s, sp = (dev(a) for a in (rkey, rpay, skey, spay))
+        o = torch.empty_like(s)
+        m = ctypes.c_int64()
+        p = lambda t: t.data_ptr()  # noqa: E731
+        st = c.lib.qg_join_filter_sort(c.handle, p(r), p(rp), nR, p(s), p(sp), nS, -(2 ** 31), 299, p(s), p(o), p(sp),
+                                       nS, ctypes.byref(m))
+        assert st == 0
+        check_join([t[: m.value] for t in (s, o, sp)], exp)
+    finally:
+        c.close()
