@@ -96,9 +96,9 @@ k_jd_fill(unsigned long long *__restrict__ E, long long nR, uint32_t *__restrict
 }
 
 // R's payload into its key's entry; true: another row of the key was there before.
-// (An exchange costs what the store did: tables of 1M rows 11 us.  Counting the
-// entries afterwards found duplicates only when all of S had been counted, 16M rows
-// 60 us in vain.)
+// (With an exchange instead of a store a table of 1M rows takes 14 us, 12 before.
+// Counting the entries afterwards found duplicates only when all of S had been
+// counted, 16M rows 60 us in vain.)
 __device__ __forceinline__ bool jd_put(unsigned long long *e, uint32_t pay) {
     return (uint32_t)atomicExch(e, (unsigned long long)pay << 32 | JD_HERE) & JD_HERE;
 }
@@ -429,8 +429,17 @@ qg_status qg_jd_launch(qg_ctx *ctx, char *work, const int32_t *rkey, const int32
     const long long tiles = qg_ceil_div(2 * nR, per * JD_THREADS);
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, tiles, QG_SITE_JOIN_PROBE, &lb));
-    QG_TRY(qg_launch_chained(ctx, "k_jd_scan", per == 2 ? k_jd_scan<2> : k_jd_scan<16>, (unsigned)tiles, JD_THREADS, 0,
-                             E, jd, out_key, out_rpay, cap, d_count, result, lb));
+    if (per == 2) {
+        QG_TRY(qg_launch_chained(ctx, "k_jd_scan", k_jd_scan<2>, (unsigned)tiles, JD_THREADS, 0, E, jd, out_key,
+                                 out_rpay, cap, d_count, result, lb));
+    } else {
+        // Not chained: CTAs that wait for the count are placed wherever its first CTAs end,
+        // several to an SM, and then run there (265K build rows, 17M probe rows: 186 us a
+        // call, chained 199 to 215).
+        qg_pre_launch(ctx);
+        k_jd_scan<16><<<(unsigned)tiles, JD_THREADS, 0, ctx->stream>>>(E, jd, out_key, out_rpay, cap, d_count, result, lb);
+        QG_TRY(qg_check_launch(ctx, "k_jd_scan"));
+    }
     return qg_launch_chained(ctx, "k_jd_write", k_jd_write, jd_grid(ctx, nS / 4, JD_THREADS, 8), JD_THREADS, 0, E, jd,
                              ak, ap, an, out_spay, cap);
 }
