@@ -42,6 +42,7 @@ struct qg_hostres {
 };
 
 #define QG_MAX_TIMED 4096
+#define QG_PJ_LEAVE_OUT 31
 struct qg_ctx {
     cudaStream_t stream;
     int device;
@@ -73,6 +74,9 @@ struct qg_ctx {
     bool sort_odd_passes;   // the last in-place record sort took an odd number of passes
     uint32_t pj_stats[8];   // last qg_join_filter_sort (see qg_join_stats)
     bool pj_sparse;         // the last join's R keys had no dense span: look before launching the counting path
+    // Joins that leave out an attempt which was given up at some cost, so that a stream
+    // of such inputs pays for it once in QG_PJ_LEAVE_OUT + 1 calls.
+    uint8_t pj_no_hash;
     char *pj_tmp;           // the join's sort-merge arrays (grow-only)
     size_t pj_tmp_bytes;
     void *pin_join;         // host pinned bucket bounds and group plan of the join (allocated on first use)

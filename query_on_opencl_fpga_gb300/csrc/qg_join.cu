@@ -23,6 +23,7 @@
 //   sort   -- LSD radix passes over (key - min_key) on the three output
 //             columns (qg_sort.cu), the last one into the caller's output; a
 //             few thousand matches are sorted by one CTA.
+#include <math.h>
 #include <string.h>
 #include <vector>
 #include "qg_cta_sort.cuh"
@@ -39,8 +40,8 @@ struct JoinCtl {
     unsigned long long n_special;  // build rows equal to EMPTY_SLOT (key -1, payload -1)
     unsigned long long cursor;     // output rows produced
     unsigned long long sortn;      // rows the device-planned sort orders (0 when over capacity)
-    uint32_t crowded;              // 1: a build row met more slots than it may
-    uint32_t twice;                // 1: some build key occurs more than once
+    uint32_t crowded;              // 1: build keys repeat more than they may
+    uint32_t twice;                // not 0: some build key occurs more than once
     qg_sort_range range;           // the device-planned sort's positions and key offset
     uint32_t hist[4][QG_RADIX];
 };
@@ -77,25 +78,42 @@ __global__ void k_join_ctl_init(JoinCtl *jc) {
     for (int i = t; i < 4 * QG_RADIX; i += blockDim.x) (&jc->hist[0][0])[i] = 0;
 }
 
-// Build: rows i of R at rkey[i * stride], rpay[i * stride].
-__global__ void __launch_bounds__(256)
-k_join_build(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, long long stride_el,
-             long long nR, unsigned long long *__restrict__ tab, uint32_t mask, JoinCtl *jc,
-             qg_control *ctl, uint32_t most_probes) {
+// Build: rows i of R at rkey[i * stride], rpay[i * stride].  LIMIT: the build is given
+// up when its keys repeat more than the probe can bear, as far as a CTA sees: the squares
+// of how many rows of its own key each row meets add up to more than `most`, a row has
+// looked at JB_PROBES slots or met JB_SAME by itself, JB_SAME rows equal the free slots'
+// mark.
+// A CTA stops at what it has seen itself: one word that all of them add to or look at is
+// a queue in L2 (0.3 % of 4M rows in pairs: 320 -> 540 us a call).
+// Eight CTAs per SM: with six a build of 8M rows takes 50 us longer.
+constexpr uint32_t JB_PROBES = 256;  // unique keys at load 1/2 need a few dozen
+constexpr uint32_t JB_SAME = 16;
+constexpr int JB_CTAS = 8;
+
+template <bool LIMIT>
+__global__ void __launch_bounds__(256, JB_CTAS)
+k_join_build(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, uint32_t stride_el,
+             uint32_t nR, unsigned long long *__restrict__ tab, uint32_t mask, JoinCtl *jc,
+             qg_control *ctl, uint32_t most) {
     qg_chain();
-    uint32_t lmin = 0xffffffffu, lmax = 0;
-    unsigned long long nspec = 0;
+    __shared__ uint32_t s_met;
+    if (LIMIT) {
+        if (threadIdx.x == 0) s_met = 0;
+        __syncthreads();
+    }
+    uint32_t lmin = 0xffffffffu, lmax = 0, nspec = 0;
     bool twice = false;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nR; i += stride) {
-        const uint32_t k = (uint32_t)__ldg(rkey + i * stride_el);
-        const uint32_t p = (uint32_t)__ldg(rpay + i * stride_el);
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nR; i += stride) {  // nR < 2^30
+        if (LIMIT && *(volatile uint32_t *)&s_met > most) break;
+        const uint32_t k = (uint32_t)__ldg(rkey + (size_t)i * stride_el);
+        const uint32_t p = (uint32_t)__ldg(rpay + (size_t)i * stride_el);
         lmin = min(lmin, k);
         lmax = max(lmax, k);
         const unsigned long long packed = ((unsigned long long)k << 32) | p;
         if (packed == EMPTY_SLOT) { nspec++; continue; }
-        uint32_t g = join_group(k, mask), probes = 0;
-        bool placed = false;
+        uint32_t g = join_group(k, mask), probes = 0, same = 0;
+        bool placed = false, over = false;
         while (!placed) {
             const ulonglong2 lo = __ldcg(reinterpret_cast<const ulonglong2 *>(tab + g)),
                              hi = __ldcg(reinterpret_cast<const ulonglong2 *>(tab + g + 2));
@@ -107,26 +125,34 @@ k_join_build(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay,
                 if (old == EMPTY_SLOT) old = atomicCAS(&tab[g + j], EMPTY_SLOT, packed);
                 // an equal key inserted before lies on this row's way to its slot
                 if (old == EMPTY_SLOT) placed = true;
-                else if ((uint32_t)(old >> 32) == k) twice = true;
+                else if ((uint32_t)(old >> 32) == k) same++;
             }
             if (placed) break;
             g = (g + 4) & mask;
             probes += 4;
-            if (most_probes && (probes > most_probes || ((probes & 31) == 0 && *(volatile uint32_t *)&jc->crowded))) {
-                jc->crowded = 1;
+            if (LIMIT && (probes > JB_PROBES || same > JB_SAME)) {
+                over = true;
                 break;
             }
             if (probes > mask) { qg_record_error(ctl, QG_ERR_TABLE_FULL, QG_SITE_JOIN_BUILD); break; }
         }
+        if (same || over) {
+            twice = true;
+            if (LIMIT) atomicAdd(&s_met, over ? most + 1 : same * same);
+        }
     }
+    __syncwarp();
     lmin = __reduce_min_sync(QG_FULL_MASK, lmin);
     lmax = __reduce_max_sync(QG_FULL_MASK, lmax);
     if ((threadIdx.x & 31) == 0) {
         if (lmin != 0xffffffffu) atomicMin(&jc->kmin, lmin);
         if (lmax != 0) atomicMax(&jc->kmax, lmax);
     }
-    if (twice) jc->twice = 1;
-    if (nspec) atomicAdd(&jc->n_special, nspec);
+    if (twice) {
+        jc->twice = 1;
+        if (LIMIT && *(volatile uint32_t *)&s_met > most) jc->crowded = 1;
+    }
+    if (nspec && atomicAdd(&jc->n_special, (unsigned long long)nspec) + nspec > JB_SAME && LIMIT) jc->crowded = 1;
 }
 
 constexpr int PJ_THREADS = 256;
@@ -160,11 +186,11 @@ struct ProbeOut {
 __global__ void __launch_bounds__(PJ_THREADS, 4)
 k_join_probe(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, long long nS,
              int32_t slo, int32_t shi, const unsigned long long *__restrict__ tab, uint32_t mask,
-             JoinCtl *jc, ProbeOut out, ProbeOut odd, long long cap, int npos) {
+             JoinCtl *jc, ProbeOut out, ProbeOut odd, long long cap, int npos, unsigned long long least) {
     qg_chain();
     extern __shared__ __align__(16) unsigned char pj_raw[];
     PjSmem &S = *reinterpret_cast<PjSmem *>(pj_raw);
-    if (jc->crowded) return;
+    if (jc->crowded || (unsigned long long)(jc->kmax - jc->kmin) < least) return;  // the caller has another path
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t lt = qg_lanemask_lt();
     const long long ntiles = (nS + PJ_TILE - 1) / PJ_TILE;
@@ -431,7 +457,7 @@ __global__ void k_join_finish_async(JoinCtl *jc, long long cap, unsigned long lo
 
 // Build the table in aux; returns the control block (in scratch) and mask.
 static qg_status join_build(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpay, long long stride,
-                            long long nR, size_t extra_aux, uint32_t most_probes, unsigned long long **tab_out,
+                            long long nR, size_t extra_aux, bool limit, unsigned long long **tab_out,
                             uint32_t *mask_out, JoinCtl **jc_out, char **aux_tail) {
     if (nR >= (1LL << 30)) return QG_ERR_UNSUPPORTED;
     const uint32_t slots = table_slots(nR);
@@ -447,9 +473,16 @@ static qg_status join_build(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpa
     k_join_ctl_init<<<1, 256, 0, ctx->stream>>>(jc);
     QG_TRY(qg_check_launch(ctx, "k_join_ctl_init"));
     if (nR > 0) {
-        int blocks = grid_cap(ctx, nR, 256, 8);
-        QG_TRY(qg_launch_chained(ctx, "k_join_build", k_join_build, blocks, 256, 0, rkey, rpay, stride, nR, tab,
-                                 slots - 1, jc, ctx->ctl, most_probes));
+        // What the probe bears (it then walks slot by slot, and clusters of equal keys
+        // lengthen every row's way), hashed / partitioned: 4M build rows and 8M probe rows 430
+        // / 500 us with unique keys, 490 / 500 with 25 % in pairs (an eighth of the rows), 520 /
+        // 500 with 3 % in eights (half), 884 / 530 with 12 %; 200K and 100K rows all in pairs
+        // (half) 145 / 217; 10K and 5K all in eights (17 times) 116 / 162, in thirty-twos 217 / 164.
+        const int blocks = grid_cap(ctx, nR, 256, JB_CTAS);
+        const float each = nR <= 16384 ? 30.f : nR <= (1 << 19) ? 1.f : 0.4f, share = each * (float)nR / (float)blocks;
+        QG_TRY(qg_launch_chained(ctx, "k_join_build", limit ? k_join_build<true> : k_join_build<false>, blocks, 256, 0,
+                                 rkey, rpay, (uint32_t)stride, (uint32_t)nR, tab, slots - 1, jc, ctx->ctl,
+                                 (uint32_t)(share + 4.f * sqrtf(share) + 1.f)));
     }
     *tab_out = tab;
     *mask_out = slots - 1;
@@ -481,7 +514,7 @@ k_join_sort_small(qg_sort_bufs in, qg_sort_bufs out, uint32_t n) {
 // Launch of k_join_probe.
 static qg_status join_probe(qg_ctx *ctx, const int32_t *skey, const int32_t *spay, int64_t nS, int32_t slo, int32_t shi,
                             const unsigned long long *tab, uint32_t mask, JoinCtl *jc, const ProbeOut &po,
-                            const ProbeOut &odd, int64_t cap) {
+                            const ProbeOut &odd, int64_t cap, uint64_t least = 0) {
     const size_t smem = sizeof(PjSmem);
     static bool attr = false;
     if (!attr) {
@@ -491,7 +524,7 @@ static qg_status join_probe(qg_ctx *ctx, const int32_t *skey, const int32_t *spa
     const long long ntiles = (nS + PJ_TILE - 1) / PJ_TILE;
     const int blocks = (int)(ntiles < (long long)ctx->sm_count * 4 ? ntiles : (long long)ctx->sm_count * 4);
     return qg_launch_chained(ctx, "k_join_probe", k_join_probe, blocks, PJ_THREADS, smem, skey, spay, nS, slo, shi,
-                             tab, mask, jc, po, odd, cap, 4);
+                             tab, mask, jc, po, odd, cap, 4, (unsigned long long)least);
 }
 
 // Hash join + filter + radix sort of the output: the variant of
@@ -500,7 +533,7 @@ static qg_status join_probe(qg_ctx *ctx, const int32_t *skey, const int32_t *spa
 qg_status qg_join_hash_sort(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpay, int64_t nR,
                             const int32_t *skey, const int32_t *spay, int64_t nS, int32_t slo,
                             int32_t shi, int32_t *out_key, int32_t *out_rpay, int32_t *out_spay,
-                            int64_t cap, int64_t *out_n, uint32_t most_probes, bool *crowded, uint32_t *span) {
+                            int64_t cap, int64_t *out_n, uint64_t least, qg_join_hash_end *end) {
     if (!ctx || nR < 0 || nS < 0 || cap < 0 || !out_n) return QG_ERR_INVALID;
     if ((nR > 0 && (!rkey || !rpay)) || (nS > 0 && (!skey || !spay)) ||
         (cap > 0 && (!out_key || !out_rpay || !out_spay)))
@@ -514,21 +547,21 @@ qg_status qg_join_hash_sort(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpa
     JoinCtl *jc;
     char *tail;
     const size_t colbytes = qg_align_up((size_t)(cap > 0 ? cap : 1) * 4, 256);
-    QG_TRY(join_build(ctx, rkey, rpay, 1, nR, 3 * colbytes, most_probes, &tab, &mask, &jc, &tail));
+    QG_TRY(join_build(ctx, rkey, rpay, 1, nR, 3 * colbytes, end != nullptr, &tab, &mask, &jc, &tail));
     qg_sort_bufs A{nullptr, (uint32_t *)tail, (uint32_t *)(tail + colbytes), (uint32_t *)(tail + 2 * colbytes)};
     const qg_sort_bufs B{nullptr, (uint32_t *)out_key, (uint32_t *)out_rpay, (uint32_t *)out_spay};
-    QG_TRY(join_probe(ctx, skey, spay, nS, slo, shi, tab, mask, jc, ProbeOut{A.k, A.a, A.b}, ProbeOut{}, cap));
+    QG_TRY(join_probe(ctx, skey, spay, nS, slo, shi, tab, mask, jc, ProbeOut{A.k, A.a, A.b}, ProbeOut{}, cap,
+                      least));
     JoinCtl *hjc = reinterpret_cast<JoinCtl *>(ctx->pin_ctl);
     static_assert(sizeof(JoinCtl) <= sizeof(qg_control), "read back into the pinned control block");
     QG_TRY_CUDA(ctx, cudaMemcpyAsync(hjc, jc, sizeof(JoinCtl), cudaMemcpyDeviceToHost, ctx->stream), "ctl d2h");
     QG_TRY(qg_collect_error(ctx));
-    if (hjc->crowded) {
-        if (crowded) *crowded = true;
-        return QG_OK;
+    const uint32_t range = hjc->kmax - hjc->kmin;
+    if (end) {
+        *end = hjc->crowded ? QG_JH_CROWDED : range < least ? QG_JH_CLOSE : QG_JH_DONE;
+        if (*end != QG_JH_DONE) return QG_OK;
     }
     const long long m = (long long)hjc->cursor;
-    const uint32_t range = hjc->kmax - hjc->kmin;
-    if (span) *span = range;
     *out_n = m;
     if (m > cap) return QG_ERR_CAPACITY;
     if (m == 0) return QG_OK;
@@ -597,7 +630,7 @@ qg_status qg_join_hash_sort_async(qg_ctx *ctx, const int32_t *rkey, const int32_
     uint32_t mask;
     JoinCtl *jc;
     char *tail;
-    QG_TRY(join_build(ctx, rkey, rpay, 1, nR, 3 * colbytes + work, 0u, &tab, &mask, &jc, &tail));
+    QG_TRY(join_build(ctx, rkey, rpay, 1, nR, 3 * colbytes + work, false, &tab, &mask, &jc, &tail));
     qg_sort_bufs A{nullptr, (uint32_t *)out_key, (uint32_t *)out_rpay, (uint32_t *)out_spay};
     qg_sort_bufs B{nullptr, (uint32_t *)tail, (uint32_t *)(tail + colbytes), (uint32_t *)(tail + 2 * colbytes)};
     // (with room for one row no sort follows, so it has to land in the output)
@@ -654,9 +687,9 @@ extern "C" QG_API qg_status qg_hash_build_ref(qg_ctx *ctx, const uint32_t *r, in
     k_ref_hash_hdr_init<<<1, 32, 0, ctx->stream>>>(hdr, slots);
     QG_TRY(qg_check_launch(ctx, "k_ref_hash_hdr_init"));
     if (nR > 0) {
-        int blocks = grid_cap(ctx, nR, 256, 8);
-        QG_TRY(qg_launch_chained(ctx, "k_join_build", k_join_build, blocks, 256, 0, (const int32_t *)r,
-                                 (const int32_t *)r + 1, 2, nR, tab, slots - 1, &hdr->jc, ctx->ctl, 0u));
+        int blocks = grid_cap(ctx, nR, 256, JB_CTAS);
+        QG_TRY(qg_launch_chained(ctx, "k_join_build", k_join_build<false>, blocks, 256, 0, (const int32_t *)r,
+                                 (const int32_t *)r + 1, 2u, (uint32_t)nR, tab, slots - 1, &hdr->jc, ctx->ctl, 0u));
     }
     // a table that fills up (cannot happen at 2 slots per row) reports TABLE_FULL
     return qg_ctx_check(ctx);

@@ -18,14 +18,18 @@ qg_status qg_jd_launch(qg_ctx *ctx, char *work, const int32_t *rkey, const int32
                        const int32_t *skey, const int32_t *spay, int64_t nS, int32_t slo, int32_t shi, uint32_t *out_key,
                        uint32_t *out_rpay, uint32_t *out_spay, int64_t cap, long long *d_count, volatile uint32_t *result);
 
-// Hash join + sort of the matches (qg_join.cu).  most_probes > 0: give up
-// (*crowded) when a build row needs more slots than that, as it does where a
-// build key repeats often; nothing valid is written then.  *span: R's largest
-// key minus its smallest.
+// Hash join + sort of the matches (qg_join.cu).  With `end` set it may be given up (*end
+// says so, and nothing was written): build keys that repeat often, or that lie within
+// fewer than `least` values.
+enum qg_join_hash_end {
+    QG_JH_DONE,
+    QG_JH_CROWDED,  // build keys repeat too often
+    QG_JH_CLOSE,    // too small a span
+};
 qg_status qg_join_hash_sort(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpay, int64_t nR, const int32_t *skey,
                             const int32_t *spay, int64_t nS, int32_t slo, int32_t shi, int32_t *out_key,
-                            int32_t *out_rpay, int32_t *out_spay, int64_t cap, int64_t *out_n, uint32_t most_probes = 0,
-                            bool *crowded = nullptr, uint32_t *span = nullptr);
+                            int32_t *out_rpay, int32_t *out_spay, int64_t cap, int64_t *out_n,
+                            uint64_t least = 0, qg_join_hash_end *end = nullptr);
 
 // flags of the dense build side (u32 words): [1] dense span, [2..3] distinct
 // keys (u64), [4] / [5] smallest / largest R payload (int32), [6] a sentinel

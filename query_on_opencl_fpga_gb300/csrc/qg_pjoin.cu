@@ -2170,7 +2170,7 @@ extern "C" QG_API qg_status qg_join_filter_sort(qg_ctx *ctx, const int32_t *rkey
 // The partitioned form below took 4K rows 126 us, 16M 280, 64M 583, 256M 1764,
 // where one of the two takes 61, 185, 407 and 1357.
 constexpr int64_t PJ_DIRECT_S = 18'000'000;
-// Build rows of the hash join, whose table (16 to 32 bytes a row) stays in L2.
+// Build rows of the hash join, whose table has 16 to 32 bytes a row.
 // Against the partitioned path (radix, or learned where that spreads better),
 // skewed keys: 64K rows 92 / 156 us, 1M 107 / 415, 16M 303 / 925, 64M 910 /
 // 1665; random 32-bit keys: 1M 158 / 249, 16M 402 / 666, 64M 1316 / 1880.
@@ -2178,16 +2178,14 @@ constexpr int64_t PJ_HASH_R = 1 << 23;
 // ... except with many probe rows and build keys close enough for the bucket
 // kernel's counting sort (4096 rows, 8192 key values, about a third of S joined):
 // 50M rows on keys three apart 960 us hashed, 658 partitioned; twenty apart 1091 / 1571.
-constexpr int64_t PJ_NEAR_S = 40'000'000;
-static bool pj_near(int64_t nS, unsigned long long span) { return nS > PJ_NEAR_S && span <= (unsigned long long)nS / 2; }
-// Slots a build row may look at: unique keys at load 1/2 need a few dozen.
-constexpr uint32_t PJ_HASH_PROBES = 256;
+static bool pj_near_size(int64_t nS, int64_t nR) { return nS > 40'000'000; }
+static uint64_t pj_near_span(int64_t nS, int64_t nR) { return pj_near_size(nS, nR) ? (uint64_t)nS / 2 : 0; }
 
 // The counting path, waited for: pj_stats[0] = 4 and the output count when it
-// answered, else pj_sparse or *other says why not.
+// answered, else pj_sparse says whether R's keys spread too widely for it.
 static qg_status join_direct(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpay, int64_t nR, const int32_t *skey,
                              const int32_t *spay, int64_t nS, int32_t slo, int32_t shi, int32_t *out_key,
-                             int32_t *out_rpay, int32_t *out_spay, int64_t cap, int64_t *out_n, bool *other) {
+                             int32_t *out_rpay, int32_t *out_spay, int64_t cap, int64_t *out_n) {
     char *work;
     QG_TRY(qg_aux(ctx, qg_jd_bytes(nR, nS), &work));
     QG_TRY(qg_jd_launch(ctx, work, rkey, rpay, nR, skey, spay, nS, slo, shi, (uint32_t *)out_key, (uint32_t *)out_rpay,
@@ -2195,7 +2193,6 @@ static qg_status join_direct(qg_ctx *ctx, const int32_t *rkey, const int32_t *rp
     long long M = 0;
     QG_TRY(qg_host_count(ctx, &M));
     ctx->pj_sparse = ctx->hres->aux == QG_JD_SPARSE;
-    *other = ctx->hres->aux == QG_JD_OTHER;
     if (ctx->hres->aux == QG_JD_DONE) {
         ctx->pj_stats[0] = 4;
         *out_n = M;
@@ -2223,36 +2220,37 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     // With the default knobs: the counting path for small and middling inputs
     // whose R keys are unique over a dense span, the hash join for R keys of no
     // dense span.  Which of the two is launched first is what the context's last
-    // such call found; each sees R's span and hands over to the other.
+    // such call found; each sees R's span and hands over.
     const bool dflt = variant == 0 && g_pj_dense && g_pj_blog2 == 0 && g_pj_smax == PB_SMAX && g_pj_rmax == PB_RMAX;
-    bool hash_tried = false;
-    if (dflt && nR <= PJ_HASH_R) {
-        const bool direct = nS <= PJ_DIRECT_S;
-        bool other = false;  // a dense span, but not for the counting path
-        if (direct && !ctx->pj_sparse) QG_TRY(join_direct(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key,
-                                                          out_rpay, out_spay, cap, out_n, &other));
-        if (ctx->pj_stats[0]) return *out_n > cap ? QG_ERR_CAPACITY : QG_OK;
-        if (ctx->pj_sparse && !other) {
-            bool crowded = false;
-            uint32_t span = 0;
-            hash_tried = true;
-            const qg_status st = qg_join_hash_sort(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay,
-                                                   out_spay, cap, out_n, PJ_HASH_PROBES, &crowded, &span);
-            if (st != QG_OK && st != QG_ERR_CAPACITY) return st;
-            ctx->pj_sparse = crowded || (unsigned long long)span + 1ull > 2ull * (unsigned long long)nR;
-            if (!crowded && (ctx->pj_sparse || !direct)) {
-                if (pj_near(nS, (unsigned long long)span + 1ull)) ctx->pj_sparse = false;  // the next call looks at the span first
-                ctx->pj_stats[0] = 3;
-                return st;
-            }
-            if (!ctx->pj_sparse) {  // dense after all
-                QG_TRY(join_direct(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay, out_spay, cap, out_n,
-                                   &other));
-                if (ctx->pj_stats[0]) return *out_n > cap ? QG_ERR_CAPACITY : QG_OK;
-            }
-        }
-        *out_n = 0;
+    const bool direct = dflt && nR <= PJ_HASH_R && nS <= PJ_DIRECT_S;
+    bool may_hash = dflt && nR <= PJ_HASH_R;
+    if (may_hash && ctx->pj_no_hash) {
+        ctx->pj_no_hash--;
+        may_hash = false;
     }
+    if (direct && !ctx->pj_sparse) {
+        QG_TRY(join_direct(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay, out_spay, cap, out_n));
+        if (ctx->pj_stats[0]) return *out_n > cap ? QG_ERR_CAPACITY : QG_OK;
+        if (!ctx->pj_sparse) may_hash = false;  // a dense span, but not for the counting path
+    }
+    if (may_hash && ctx->pj_sparse) {
+        may_hash = false;
+        qg_join_hash_end end = QG_JH_DONE;
+        const qg_status st = qg_join_hash_sort(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay,
+                                               out_spay, cap, out_n, std::max(2 * (uint64_t)nR, pj_near_span(nS, nR)), &end);
+        if (st != QG_OK && st != QG_ERR_CAPACITY) return st;
+        if (end == QG_JH_DONE) {
+            ctx->pj_stats[0] = 3;
+            return st;
+        }
+        if (end == QG_JH_CROWDED) ctx->pj_no_hash = QG_PJ_LEAVE_OUT;
+        ctx->pj_sparse = end == QG_JH_CROWDED;
+        if (direct && end == QG_JH_CLOSE) {  // dense after all
+            QG_TRY(join_direct(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay, out_spay, cap, out_n));
+            if (ctx->pj_stats[0]) return *out_n > cap ? QG_ERR_CAPACITY : QG_OK;
+        }
+    }
+    *out_n = 0;
     // aux: R records + spare (the spare doubles as the dense build side's
     // payload table), S' records + spare, the presence bitmap, level-0 arrays
     const size_t rb = qg_align_up((size_t)nR * 8, 256), sb = qg_align_up((size_t)nS * 8, 256);
@@ -2286,8 +2284,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
                              lb2, nR, L.dflags, reinterpret_cast<unsigned long long *>(L.dflags + PJ_F_DISTINCT)));
     // large probe inputs: one partition step, unless the build side is not dense or the rows spread unevenly
     const bool jp = dflt && nS > PJ_DIRECT_S;
-    const bool may_hash = nR <= PJ_HASH_R && !hash_tried;
-    const bool filter_later = may_hash && nS <= PJ_NEAR_S;  // with sparse build keys, if the hash join hands back
+    const bool filter_later = may_hash && !pj_near_size(nS, nR);  // with sparse build keys, if the hash join hands back
     char *jp_work = aux + 2 * rb + 2 * sb + bmb + pj_level_bytes(PJ_MAX_BUCKETS, true);
     if (jp) {
         const qg_jp_r jr{&L.range->kmin, L.dflags, bitmap, T, nR};
@@ -2312,7 +2309,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
         *out_n = ctx->hres->count;
         return *out_n > cap ? QG_ERR_CAPACITY : QG_OK;
     }
-    const bool near = pj_near(nS, (unsigned long long)(pin->range.kmax - pin->range.kmin) + 1ull);
+    const bool near = (unsigned long long)(pin->range.kmax - pin->range.kmin) + 1ull <= pj_near_span(nS, nR);
     if (jp && may_hash && !near && pin->dflags[PJ_F_DENSE] == 0u) {  // sparse build keys: the hash join, then what follows it
         ctx->pj_sparse = true;
         return join_filter_sort_impl(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay, out_spay, cap, out_n);

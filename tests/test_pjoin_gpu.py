@@ -499,7 +499,7 @@ def test_join_counting_path_hot_keys_beside_other_work():
 
 # Outputs over the probe columns: an attempt that is given up has written nothing
 # when the next path reads them.
-@pytest.mark.parametrize("kind", ["dup", "hot"])
+@pytest.mark.parametrize("kind", ["dup", "hot", "after_sparse"])
 def test_join_outputs_over_inputs(orc, kind):
     import ctypes
 
@@ -517,6 +517,9 @@ def test_join_outputs_over_inputs(orc, kind):
     spay = rng.integers(0, 1000, nS).astype(np.int32)
     c = Context()
     try:
+        if kind == "after_sparse":  # the hash join is launched first, and meets a dense span
+            c.join_filter_sort(dev(rkey * 100), dev(rpay), dev(skey), dev(spay))
+            assert c.join_stats()["path"] == "hash_sort"
         exp = orc.join_filter_sort(rkey, rpay, skey, spay, -(2 ** 31), 299, cap=nS, mt=True)
         r, rp, s, sp = (dev(a) for a in (rkey, rpay, skey, spay))
         o = torch.empty_like(s)
@@ -528,3 +531,91 @@ def test_join_outputs_over_inputs(orc, kind):
         check_join([t[: m.value] for t in (s, o, sp)], exp)
     finally:
         c.close()
+
+
+def launched(c, call):
+    """Names of the kernels that a call launches."""
+    c.timing_report()
+    c.enable_timing(True)
+    try:
+        call()
+        return set(c.timing_report())
+    finally:
+        c.enable_timing(False)
+
+
+def _join_rows(rng, kind):
+    nR, nS = 20_000, 300_000
+    rkey = rng.permutation(nR).astype(np.int32)
+    skey = rng.integers(-10, nR + 10, nS).astype(np.int32)
+    if kind == "crowded":
+        rkey = np.concatenate([rng.integers(-(2 ** 31), 2 ** 31, 5000), np.full(2000, 123)]).astype(np.int32)
+        skey = np.concatenate([rng.choice(rkey[:5000], 20_000), np.full(3, 123)]).astype(np.int32)
+    if kind == "marks":
+        rkey = np.concatenate([rng.integers(-(2 ** 31), 2 ** 31, 5000), np.full(2000, -1)]).astype(np.int32)
+        skey = np.concatenate([rng.choice(rkey[:5000], 20_000), np.full(3, -1)]).astype(np.int32)
+    rpay = rng.integers(0, 1000, rkey.size).astype(np.int32)
+    if kind == "marks":
+        rpay[5000:] = -1
+    return rkey, rpay, skey, rng.integers(0, 300, skey.size).astype(np.int32)
+
+
+# Build keys that repeat (one of them, and the key and payload that mark free slots):
+# given up by the hash join, and not tried again by the next calls; unique dense keys
+# are counted all the same.
+@pytest.mark.parametrize("kind,left_out", [("crowded", "k_join_build"), ("marks", "k_join_build")])
+def test_join_failed_attempt_is_not_repeated(orc, kind, left_out):
+    from query_on_opencl_fpga_gb300.api import Context
+
+    rng = np.random.default_rng(33)
+    a = _join_rows(rng, kind)
+    exp = orc.join_filter_sort(*a, 0, 299, cap=a[2].size * 4 + 10_000, mt=True)
+    c = Context()
+    try:
+        d = [dev(x) for x in a]
+        for i in range(2):
+            got = []
+            names = launched(c, lambda: got.extend(c.join_filter_sort(*d, 0, 299, cap=len(exp[0]))))
+            check_join(got, exp)
+            assert c.join_stats()["path"] == "radix"
+            if i:
+                assert left_out not in names, names
+        u = [dev(x) for x in _join_rows(rng, "unique")]
+        for i in range(2):
+            names = launched(c, lambda: c.join_filter_sort(*u, 0, 299))
+            assert c.join_stats()["path"] == "dense"
+        assert "k_jd_count" in names
+    finally:
+        c.close()
+
+
+# Many build keys twice or more, in the sizes' three ranges, just below and far above
+# what the hash join bears: the same rows whichever path answers.
+@pytest.mark.parametrize("nR", [900, 40_000, 700_000])
+@pytest.mark.parametrize("times,share", [(2, 0.1), (2, 1.0), (8, 0.02), (8, 1.0), (40, 1.0)])
+def test_join_sparse_repeated_keys(ctx, nR, times, share):
+    nS = 3 * nR
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nR + times)
+    rk = torch.randint(-(2 ** 31), 2 ** 31, (nR,), generator=g, device="cuda")
+    many = int(nR * share) // times * times
+    rk[:many] = rk[: many // times].repeat(times)
+    rk = rk[torch.randperm(nR, generator=g, device="cuda")]
+    sk = torch.where(torch.rand(nS, generator=g, device="cuda") < 0.3, rk[torch.randint(0, nR, (nS,), generator=g, device="cuda")],
+                     torch.randint(-(2 ** 31), 2 ** 31, (nS,), generator=g, device="cuda"))
+    rp, sp = torch.arange(nR, device="cuda"), torch.randint(0, 1000, (nS,), generator=g, device="cuda")
+    order = torch.argsort(rk)
+    rs = rk[order]
+    sel = sp <= 299
+    a, n = torch.searchsorted(rs, sk[sel]), torch.searchsorted(rs, sk[sel], right=True)
+    n -= a
+    row = torch.repeat_interleave(torch.arange(n.numel(), device="cuda"), n)
+    at = a[row] + torch.arange(row.numel(), device="cuda") - (n.cumsum(0) - n)[row]
+    exp = ((rp[order][at] << 10) | sp[sel][row]).sort().values  # a build row's payload tells its key
+    for _ in range(2):
+        got = ctx.join_filter_sort(rk.to(torch.int32), rp.to(torch.int32), sk.to(torch.int32), sp.to(torch.int32), 0, 299,
+                                   cap=max(exp.numel(), 1))
+        u = got[0].to(torch.int64) & 0xFFFFFFFF
+        assert bool((u[1:] >= u[:-1]).all())
+        assert torch.equal(((got[1].to(torch.int64) << 10) | got[2]).sort().values, exp)
+        assert torch.equal(got[0].to(torch.int64), rk[got[1].to(torch.int64)])
