@@ -2175,12 +2175,18 @@ constexpr int64_t PJ_DIRECT_S = 18'000'000;
 // skewed keys: 64K rows 92 / 156 us, 1M 107 / 415, 16M 303 / 925, 64M 910 /
 // 1665; random 32-bit keys: 1M 158 / 249, 16M 402 / 666, 64M 1316 / 1880.
 constexpr int64_t PJ_HASH_R = 1 << 23;
-// ... except with many probe rows and build keys close enough for the bucket
-// kernel's counting sort (4096 rows, 8192 key values, about a third of S joined):
-// 50M rows on keys three apart 960 us hashed, 658 partitioned; twenty apart 1091 / 1571.
-static bool pj_near_size(int64_t nS, int64_t nR) { return nS > 40'000'000; }
-static uint64_t pj_near_span(int64_t nS, int64_t nR) { return pj_near_size(nS, nR) ? (uint64_t)nS / 2 : 0; }
-
+// ... except where the bucket kernel's counting sort takes the partitioned path's
+// buckets (8192 key values: with 4096 rows, 30 % of S joined, a span of 0.6 nS; with
+// 2048 build rows, keys four apart) and the inputs are large.  Hashed / partitioned,
+// all rows matching: keys three apart, 4M build rows and 30M probe rows 677 / 560 us,
+// 2M and 30M 555 / 480, 6M and 17M 619 / 545; 1M thirty apart and 50M 876 / 730.  With a
+// fifth of the rows matching 516 / 500, 404 / 450, 500 / 565 and 558 / 706.
+static bool pj_near_size(int64_t nS, int64_t nR) { return nS > 40'000'000 || (nS > 24'000'000 && nR > 2'500'000); }
+static uint64_t pj_near_span(int64_t nS, int64_t nR) {  // key values; 0: none
+    if (!pj_near_size(nS, nR)) return 0;
+    const int64_t by_s = nR > (1 << 22) ? nS / 3 * 2 : nS / 8 * 5;  // a table beyond L2 loses a little earlier
+    return (uint64_t)std::max(by_s, 4 * nR);
+}
 // The counting path, waited for: pj_stats[0] = 4 and the output count when it
 // answered, else pj_sparse says whether R's keys spread too widely for it.
 static qg_status join_direct(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpay, int64_t nR, const int32_t *skey,

@@ -619,3 +619,31 @@ def test_join_sparse_repeated_keys(ctx, nR, times, share):
         assert bool((u[1:] >= u[:-1]).all())
         assert torch.equal(((got[1].to(torch.int64) << 10) | got[2]).sort().values, exp)
         assert torch.equal(got[0].to(torch.int64), rk[got[1].to(torch.int64)])
+
+
+# The line between hashing and partitioning close build keys: 24M probe rows and 2.5M
+# build rows, a span of 5/8 of the probe rows' number, keys four apart.
+@pytest.mark.parametrize("nS,nR,stride,path", [(24_000_001, 2_500_001, 5, "radix"), (24_000_001, 2_500_001, 7, "hash_sort"),
+                                               (24_000_001, 2_500_000, 5, "hash_sort"), (24_000_000, 2_500_001, 5, "hash_sort"),
+                                               (24_000_001, 5_000_000, 4, "radix")])
+def test_join_near_line(nS, nR, stride, path):
+    from query_on_opencl_fpga_gb300.api import Context
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nR + stride)
+    r = torch.randperm(nR, generator=g, device="cuda")
+    soff, spay = (torch.randint(0, m, (nS,), generator=g, device="cuda") for m in (2 * nR, 1000))
+    hit = (soff % 2 == 0) & (spay <= 99)
+    key = torch.where(soff % 2 == 0, soff // 2 * stride, soff // 2 * stride + 1)
+    exp = (soff[hit] // 2 * 1000 + spay[hit]).sort().values
+    args = [t.to(torch.int32) for t in (r * stride, r, key, spay)]
+    c = Context()
+    try:
+        for _ in range(2):
+            got = c.join_filter_sort(*args, 0, 99, cap=nS)
+            k = got[0].to(torch.int64) // stride
+            assert torch.equal(got[1].to(torch.int64), k) and bool((k[1:] >= k[:-1]).all())
+            assert torch.equal((k * 1000 + got[2]).sort().values, exp)
+            assert c.join_stats()["path"] == path
+    finally:
+        c.close()
