@@ -131,3 +131,30 @@ def test_hash_build_once_probe_three_batches(ctx, orc):
     st = ctx.lib.qg_hash_build_ref(ctx.handle, c_void_p(dev(r).data_ptr()), nR, c_void_p(table.data_ptr()),
                                    table.numel() - 8)
     assert st == 3
+
+
+# The probe's groups of four slots: keys repeated up to nine times (matches in one
+# group and over several), the key and payload that mark free slots and that key with
+# others, ragged last warps, a capacity among the matches.
+@pytest.mark.parametrize("nS", [1, 31, 33, 5000])
+def test_hash_probe_ref_groups(ctx, orc, nS):
+    from ctypes import byref, c_int64
+
+    rng = np.random.default_rng(nS)
+    keys = rng.integers(-(2 ** 31), 2 ** 31, 400)
+    rk = np.concatenate([np.repeat(keys[:100], rng.integers(1, 10, 100)), keys[100:], [-1] * 5])
+    rp = rng.integers(-3, 3, rk.size)
+    rp[-5:] = [-1, -1, -1, 7, 0]
+    r = np.stack([rk, rp], 1).astype(np.int32)[rng.permutation(rk.size)]
+    sk = np.concatenate([[-1], rng.choice(np.concatenate([keys, [-1, 5]]), nS - 1)])
+    s = np.stack([sk, rng.integers(-9, 9, nS)], 1).astype(np.int32)
+    exp = orc.hash_join_ref(r, s, cap=nS * 10)
+    table = ctx.hash_build_ref(dev(r))
+    got = ctx.hash_probe_ref(table, dev(s), cap=exp.shape[0]).cpu().numpy()
+    order = lambda a: a[np.lexsort(a.T)]  # noqa: E731
+    assert np.array_equal(order(got), order(exp))
+    out = torch.full((exp.shape[0] + 8, 2), 77, dtype=torch.int32, device="cuda")
+    m = c_int64()
+    small = exp.shape[0] - 1
+    st = ctx.lib.qg_hash_probe_ref(ctx.handle, table.data_ptr(), dev(s).data_ptr(), nS, out.data_ptr(), small, byref(m))
+    assert st == 3 and m.value == exp.shape[0] and bool((out[small:] == 77).all())
