@@ -61,6 +61,10 @@ QG_API const char *qg_last_error_message(qg_ctx *ctx);
 QG_API size_t qg_ctx_scratch_bytes(qg_ctx *ctx);
 /* Reserve scratch up front (so later calls allocate nothing). */
 QG_API qg_status qg_ctx_reserve(qg_ctx *ctx, size_t bytes);
+/* Largest size of one of the context's work arenas in bytes, 0 (the default) for
+ * none.  A call that would need more takes a path that needs less, where there is
+ * one, or returns QG_ERR_OOM, as it does when the device has no memory left. */
+QG_API qg_status qg_ctx_set_arena_limit(qg_ctx *ctx, size_t bytes);
 /* Number of kernels this context has launched (for launch accounting). */
 QG_API uint64_t qg_ctx_launch_count(qg_ctx *ctx);
 /* Per-kernel timing: with timing on, CUDA events on the context's stream

@@ -35,6 +35,7 @@ SIGNATURES: dict[str, tuple] = {
     "qg_last_error_message": (c_char_p, [c_void_p]),
     "qg_ctx_scratch_bytes": (c_size_t, [c_void_p]),
     "qg_ctx_reserve": (c_int, [c_void_p, c_size_t]),
+    "qg_ctx_set_arena_limit": (c_int, [c_void_p, c_size_t]),
     "qg_ctx_launch_count": (c_uint64, [c_void_p]),
     "qg_ctx_enable_timing": (c_int, [c_void_p, c_int]),
     "qg_ctx_timing_report": (c_int, [c_void_p, c_char_p, c_size_t]),

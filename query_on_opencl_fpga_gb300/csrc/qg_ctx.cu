@@ -115,6 +115,12 @@ QG_API const char *qg_last_error_message(qg_ctx *ctx) { return ctx ? ctx->msg : 
 
 QG_API size_t qg_ctx_scratch_bytes(qg_ctx *ctx) { return ctx ? ctx->scratch_bytes : 0; }
 
+QG_API qg_status qg_ctx_set_arena_limit(qg_ctx *ctx, size_t bytes) {
+    if (!ctx) return QG_ERR_INVALID;
+    ctx->arena_limit = bytes;
+    return QG_OK;
+}
+
 QG_API uint64_t qg_ctx_launch_count(qg_ctx *ctx) { return ctx ? ctx->launches : 0; }
 
 QG_API qg_status qg_ctx_reserve(qg_ctx *ctx, size_t bytes) {
@@ -223,6 +229,12 @@ QG_API int qg_ctx_timing_report(qg_ctx *ctx, char *buf, size_t len) {
 
 }  // extern "C"
 
+// Device memory of a work arena, within the context's limit.
+static cudaError_t arena_malloc(qg_ctx *ctx, void **p, size_t bytes) {
+    if (ctx->arena_limit && bytes > ctx->arena_limit) return cudaErrorMemoryAllocation;
+    return cudaMalloc(p, bytes);
+}
+
 qg_status qg_scratch(qg_ctx *ctx, size_t bytes, char **out) {
     bytes = qg_align_up(bytes ? bytes : 256, 256);
     if (bytes > ctx->scratch_bytes) {
@@ -232,7 +244,7 @@ qg_status qg_scratch(qg_ctx *ctx, size_t bytes, char **out) {
         if (ctx->scratch) cudaFree(ctx->scratch);
         ctx->scratch = nullptr;
         ctx->scratch_bytes = 0;
-        cudaError_t e = cudaMalloc((void **)&ctx->scratch, want);
+        cudaError_t e = arena_malloc(ctx, (void **)&ctx->scratch, want);
         if (e != cudaSuccess) {
             cudaGetLastError();
             snprintf(ctx->msg, sizeof(ctx->msg), "scratch cudaMalloc(%zu): %s", want,
@@ -278,7 +290,7 @@ qg_status qg_aux(qg_ctx *ctx, size_t bytes, char **out) {
         if (ctx->aux) cudaFree(ctx->aux);
         ctx->aux = nullptr;
         ctx->aux_bytes = 0;
-        cudaError_t e = cudaMalloc((void **)&ctx->aux, want);
+        cudaError_t e = arena_malloc(ctx, (void **)&ctx->aux, want);
         if (e != cudaSuccess) {
             cudaGetLastError();
             snprintf(ctx->msg, sizeof(ctx->msg), "aux cudaMalloc(%zu): %s", want,
@@ -298,7 +310,7 @@ qg_status qg_spare(qg_ctx *ctx, size_t bytes, char **out) {
         if (ctx->pj_tmp) cudaFree(ctx->pj_tmp);
         ctx->pj_tmp = nullptr;
         ctx->pj_tmp_bytes = 0;
-        if (cudaMalloc((void **)&ctx->pj_tmp, bytes + bytes / 4) != cudaSuccess) {
+        if (arena_malloc(ctx, (void **)&ctx->pj_tmp, bytes + bytes / 4) != cudaSuccess) {
             cudaGetLastError();
             ctx->pj_tmp = nullptr;
             return QG_ERR_OOM;

@@ -63,6 +63,7 @@ struct qg_ctx {
     cudaEvent_t pin_ev[8];  // a slot may be refilled once its copy (event) has completed
     int pin_next;
     uint32_t spin_limit;
+    size_t arena_limit;     // 0: none
     uint64_t launches;
     bool unchained;         // launches are not chained: the context shares the device with others (batch lanes)
     bool table_dirty;       // group-by table must be cleared before next use

@@ -595,21 +595,31 @@ qg_status qg_join_hash_sort(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpa
     uint32_t bases[4 * QG_RADIX];
     const int np = npos ? qg_sort_plan(&hjc->hist[0][0], npos, m, passes, bases) : 0;
     const uint32_t key_off = hjc->kmin;
-    if (np == 0) {  // one key: in order as it is
+    auto copy_out = [&]() -> qg_status {
         QG_TRY_CUDA(ctx, cudaMemcpyAsync(out_key, A.k, (size_t)m * 4, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
         QG_TRY_CUDA(ctx, cudaMemcpyAsync(out_rpay, A.a, (size_t)m * 4, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
         QG_TRY_CUDA(ctx, cudaMemcpyAsync(out_spay, A.b, (size_t)m * 4, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
+        return QG_OK;
+    };
+    if (np == 0) {  // one key: in order as it is
+        QG_TRY(copy_out());
         return qg_ctx_check(ctx);
     }
     // The last pass ends in the output: with an even number of them the first
-    // goes to a third set of columns (the table is not needed any more).
+    // goes to a third set of columns (the table is not needed any more), or, without
+    // memory for one, the last ends where the first began and is copied.
     bool other = false;
-    if (np & 1) {
+    const size_t mb = qg_align_up((size_t)m * 4, 256);
+    char *third = (char *)tab;
+    if (!(np & 1) && 3 * mb > ((size_t)mask + 1) * 8) {
+        const qg_status st = qg_spare(ctx, 3 * mb, &third);
+        if (st == QG_ERR_OOM) third = nullptr;
+        else QG_TRY(st);
+    }
+    if ((np & 1) || !third) {
         QG_TRY(qg_radix_passes(ctx, true, A, B, m, key_off, passes, np, bases, &other));
+        if (!(np & 1)) QG_TRY(copy_out());
     } else {
-        const size_t mb = qg_align_up((size_t)m * 4, 256);
-        char *third = (char *)tab;
-        if (3 * mb > ((size_t)mask + 1) * 8) QG_TRY(qg_spare(ctx, 3 * mb, &third));
         const qg_sort_bufs C{nullptr, (uint32_t *)third, (uint32_t *)(third + mb), (uint32_t *)(third + 2 * mb)};
         QG_TRY(qg_radix_passes(ctx, true, A, C, m, key_off, passes, 1, bases, &other));
         QG_TRY(qg_radix_passes(ctx, true, C, B, m, key_off, passes + 1, np - 1, bases, &other));

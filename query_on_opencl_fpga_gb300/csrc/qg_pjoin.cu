@@ -2244,7 +2244,8 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
         qg_join_hash_end end = QG_JH_DONE;
         const qg_status st = qg_join_hash_sort(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay,
                                                out_spay, cap, out_n, std::max(2 * (uint64_t)nR, pj_near_span(nS, nR)), &end);
-        if (st != QG_OK && st != QG_ERR_CAPACITY) return st;
+        if (st == QG_ERR_OOM) end = QG_JH_CROWDED;  // its columns are sized by cap, the arrays below are not
+        else if (st != QG_OK && st != QG_ERR_CAPACITY) return st;
         if (end == QG_JH_DONE) {
             ctx->pj_stats[0] = 3;
             return st;

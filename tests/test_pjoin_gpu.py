@@ -647,3 +647,58 @@ def test_join_near_line(nS, nR, stride, path):
             assert c.join_stats()["path"] == path
     finally:
         c.close()
+
+
+def _sparse_rows(g, nR, nS):
+    ints = lambda lo, hi, n: torch.randint(lo, hi, (n,), generator=g, device="cuda")  # noqa: E731
+    rk = torch.randperm(nR, generator=g, device="cuda") * (2 ** 32 // nR) - 2 ** 31
+    s = ints(0, nR, nS)
+    rp, sp = ints(0, 1000, nR), ints(0, 1000, nS)
+    exp = (((rk[s] & 0xFFFFFFFF) * 1000 + rp[s]) * 1000 + sp)[sp <= 299].sort().values
+    return [t.to(torch.int32) for t in (rk, rp, rk[s], sp)], exp
+
+
+def _check_sparse(got, exp):
+    u = got[0].to(torch.int64) & 0xFFFFFFFF
+    assert bool((u[1:] >= u[:-1]).all())
+    assert torch.equal(((u * 1000 + got[1]) * 1000 + got[2]).sort().values, exp)
+
+
+def test_join_without_room_for_the_hash_join():
+    # A generous capacity sizes the hash join's columns, not the partitioned path's
+    # arrays: without memory for the former the latter answers.
+    from query_on_opencl_fpga_gb300.api import Context
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(41)
+    args, exp = _sparse_rows(g, 50_000, 200_000)
+    c = Context()
+    try:
+        c.check(c.lib.qg_ctx_set_arena_limit(c.handle, 256 << 20), "limit")
+        for _ in range(3):
+            _check_sparse(c.join_filter_sort(*args, 0, 299, cap=40_000_000), exp)
+            assert c.join_stats()["path"] == "radix"
+        c.check(c.lib.qg_ctx_set_arena_limit(c.handle, 0), "limit")
+    finally:
+        c.close()
+
+
+def test_join_hash_without_room_for_a_third_set_of_columns():
+    # An even number of sort passes over more matches than the table's memory holds:
+    # without the spare columns they end in the first set and are copied.
+    from query_on_opencl_fpga_gb300.api import Context
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(42)
+    small, small_exp = _sparse_rows(g, 3000, 9000)
+    args, exp = _sparse_rows(g, 3000, 200_000)
+    c = Context()
+    try:
+        for _ in range(2):  # the other arenas have their size then
+            _check_sparse(c.join_filter_sort(*small, 0, 299, cap=2_000_000), small_exp)
+        c.check(c.lib.qg_ctx_set_arena_limit(c.handle, 100_000), "limit")
+        for _ in range(2):
+            _check_sparse(c.join_filter_sort(*args, 0, 299, cap=200_000), exp)
+            assert c.join_stats()["path"] == "hash_sort"
+    finally:
+        c.close()
