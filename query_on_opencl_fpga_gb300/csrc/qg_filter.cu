@@ -668,12 +668,8 @@ static qg_status f2_launch(qg_ctx *ctx, const int32_t *src, const int32_t *pay, 
         spill = (uint16_t *)scr;
     }
     const size_t smem = (size_t)warps * (F2<REC>::SEG * 8 + std::min<long long>(per_warp, F2_SUNITS) * 64);
-    static bool attr = false;
-    if (!attr) {
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_filter_two<REC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              F2_MAX_WARPS * (F2<REC>::SEG * 8 + F2_SUNITS * 64)), "attr");
-        attr = true;
-    }
+    static qg_per_device site;
+    QG_TRY(qg_allow_smem(ctx, site, k_filter_two<REC>, F2_MAX_WARPS * (F2<REC>::SEG * 8 + F2_SUNITS * 64)));
     qg_pre_launch(ctx);
     k_filter_two<REC><<<(unsigned)grid, (unsigned)(32 * warps), smem, ctx->stream>>>(src, pay, n, units, lo, hi,
                                                                                     (int2 *)out, cap, d_count, spill, lb);
@@ -703,11 +699,8 @@ static qg_status f2_launch_two(qg_ctx *ctx, const int32_t *key, const int32_t *p
     uint16_t *mask = (uint16_t *)scr;
     uint32_t *upre = (uint32_t *)(scr + mb), *rtot = (uint32_t *)(scr + mb + ub);
     const size_t smem = (size_t)FW_WARPS * F2<false>::SEG * 8 + (size_t)ranges * 4;
-    static size_t attr = 0;
-    if (attr < smem) {
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_filter_write, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "attr");
-        attr = smem;
-    }
+    static qg_per_device site;
+    QG_TRY(qg_allow_smem(ctx, site, k_filter_write, smem));
     qg_pre_launch(ctx);
     k_filter_count<<<gc, 32 * FC_WARPS, 0, ctx->stream>>>(key, n, units, per, lo, hi, mask, upre, rtot);
     QG_TRY(qg_check_launch(ctx, "k_filter_count"));
@@ -771,12 +764,8 @@ qg_status qg_filter_cols_launch(qg_ctx *ctx, const int32_t *key, const int32_t *
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, tiles, QG_SITE_FILTER, &lb));
     if (variant == 1) {
-        static bool attr = false;
-        if (!attr) {
-            QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_filter_cols_tma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)sizeof(FpSmem)), "attr");
-            attr = true;
-        }
+        static qg_per_device site;
+        QG_TRY(qg_allow_smem(ctx, site, k_filter_cols_tma, sizeof(FpSmem)));
         const long long ftiles = qg_ceil_div(n, FP_TILE);
         const int grid = (int)(ftiles < ctx->sm_count * 2LL ? ftiles : ctx->sm_count * 2LL);
         qg_pre_launch(ctx);

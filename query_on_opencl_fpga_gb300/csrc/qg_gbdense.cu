@@ -936,15 +936,11 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
     // k_gbd_mid's CTAs take at least GBM_ROWS + 8 and at most n / (2 C) + GBM_ROWS rows: the shared sums stay below 2^32
     const uint32_t fast_max_mid = (uint32_t)std::min<unsigned long long>(fast_max, 0xffffffffull / (2 * GBM_ROWS + n / C));
 
-    static size_t attr_main[2] = {0, 0};  // (the single launch's attribute is set with its occupancy check)
+    static qg_per_device site_main[2];
     const size_t smem_main = (size_t)GBD_S * 12;
     const bool pred = val2 != nullptr;
     auto mainf = pred ? k_gbd_main<true> : k_gbd_main<false>;
-    if (attr_main[pred] < smem_main) {
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(mainf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_main),
-                    "attr");
-        attr_main[pred] = smem_main;
-    }
+    QG_TRY(qg_allow_smem(ctx, site_main[pred], mainf, smem_main));
 
     const bool every_row = n <= (long long)GBD_SAMPLE_RUNS * GBD_RUN;
     const int runs = every_row ? (int)qg_ceil_div(n, GBD_RUN) : GBD_SAMPLE_RUNS;
@@ -954,19 +950,18 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
     // not being captured (graphs take the four launches below).
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (g_gbd_single) QG_TRY_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cs), "capture status");
-    static int single_fits[2] = {-1, -1};
+    static qg_per_device site_single[2], single_fits[2];  // the latter: 1 no, 2 yes
     if (g_gbd_single && n > 0 && cs == cudaStreamCaptureStatusNone && C >= 128 &&
         (long long)C * GBD1_MAX_RUNS >= runs) {
         auto singlef = pred ? k_gbd_single<true> : k_gbd_single<false>;
-        if (single_fits[pred] < 0) {
+        if (!single_fits[pred].covers(ctx->device, 1)) {
             int nb = 0;
-            QG_TRY_CUDA(ctx, cudaFuncSetAttribute(singlef, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_main),
-                        "attr");
+            QG_TRY(qg_allow_smem(ctx, site_single[pred], singlef, smem_main));
             QG_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, singlef, GBD_THREADS, smem_main),
                         "occupancy");
-            single_fits[pred] = nb >= 1;
+            single_fits[pred].set(ctx->device, nb >= 1 ? 2 : 1);
         }
-        if (single_fits[pred]) {
+        if (single_fits[pred].covers(ctx->device, 2)) {
             QG_TRY_CUDA(ctx, cudaMemsetAsync(st, 0, G_WORDS * 4, ctx->stream), "memset gbd state");
             uint32_t *counts = (uint32_t *)scr;  // [C] groups per emit chunk (the sample lists are unused)
             bool er = every_row;
@@ -996,12 +991,9 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
         if (s == QG_OK) {
             const unsigned mg = (unsigned)std::min<long long>(qg_ceil_div(n, GBM_ROWS), 2LL * C);
             const size_t sm = (size_t)GBM_SLOTS * 12;
-            static bool attr_mid[2] = {false, false};
+            static qg_per_device site_mid[2];
             auto midf = pred ? k_gbd_mid<true> : k_gbd_mid<false>;
-            if (!attr_mid[pred]) {
-                QG_TRY_CUDA(ctx, cudaFuncSetAttribute(midf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm), "attr");
-                attr_mid[pred] = true;
-            }
+            QG_TRY(qg_allow_smem(ctx, site_mid[pred], midf, sm));
             s = qg_launch_chained(ctx, "k_gbd_mid", midf, mg, GBM_THREADS, sm, key, val, val2, lo2, hi2, n, st, dense,
                                   extra, shift, fast_max_mid);
         }

@@ -164,13 +164,10 @@ qg_status qg_gbs_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
     while (slots < GS_SLOTS && slots < 2 * (uint32_t)n) slots <<= 1;
     auto bytes = [](uint32_t s) { return (size_t)s * 8 + 4 * (s + 4) * 4 + (size_t)GS_WARPS * 1024; };
     const size_t most = bytes(GS_SLOTS), smem = bytes(slots);
-    static bool attr[2] = {false, false};
+    static qg_per_device site[2];
     const bool pred = val2 != nullptr;
     auto kern = pred ? k_gb_small<true> : k_gb_small<false>;
-    if (!attr[pred]) {
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most), "attr");
-        attr[pred] = true;
-    }
+    QG_TRY(qg_allow_smem(ctx, site[pred], kern, most));
     qg_pre_launch(ctx);
     kern<<<1, GS_THREADS, smem, ctx->stream>>>(key, val, val2, lo2, hi2, (int)n, slots, gkey, (long long *)gsum,
                                                (long long *)gcnt, cap, d_num, full);

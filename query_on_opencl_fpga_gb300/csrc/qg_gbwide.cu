@@ -362,11 +362,8 @@ qg_status qg_gbw_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
     const uint32_t window = QG_GBD_WINDOW;
     const bool pred = val2 != nullptr;
     uint32_t *range = ctx->ctl->gbd, *hist = ctx->ctl->shist;
-    static bool attr = false;
-    if (!attr) {
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_gbw_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gw_smem(GW_SLOTS)), "attr");
-        attr = true;
-    }
+    static qg_per_device site;
+    QG_TRY(qg_allow_smem(ctx, site, k_gbw_merge, gw_smem(GW_SLOTS)));
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, GW_PARTS, QG_SITE_GROUPBY, &lb));
     const uint32_t limit = gw_few_limit(n), *few = limit ? &ctx->ctl->gbw_few : nullptr;

@@ -1192,12 +1192,8 @@ extern "C" QG_API qg_status qg_groupby_rec(qg_ctx *ctx, const void *in, int64_t 
         spill = (uint8_t *)scr;
     }
     const size_t smem = (size_t)warps * (GH_UNIT * 4 + std::min<long long>(per_warp, GH_SUNITS) * 32);
-    static bool attr = false;
-    if (!attr) {
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_group_bounds, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              GH_MAX_WARPS * (GH_UNIT * 4 + GH_SUNITS * 32)), "attr");
-        attr = true;
-    }
+    static qg_per_device site;
+    QG_TRY(qg_allow_smem(ctx, site, k_group_bounds, GH_MAX_WARPS * (GH_UNIT * 4 + GH_SUNITS * 32)));
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, grid, QG_SITE_GROUPBY, &lb));
     QG_TRY(qg_launch_chained(ctx, "k_group_bounds", k_group_bounds, (unsigned)grid, (unsigned)(32 * warps), smem,
@@ -1333,15 +1329,9 @@ static qg_status gb_launch_global(qg_ctx *ctx, const int32_t *key, const int32_t
     GSlot *tab = (GSlot *)tabp;
     const int slog2 = g_gb_slog2;
     const size_t smem = ((size_t)1 << slog2) * 16;
-    static bool attr[2] = {false, false};
+    static qg_per_device site[2];
     const bool pred = val2 != nullptr;
-    if (!attr[pred]) {
-        if (pred)
-            QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_groupby_hash<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "attr");
-        else
-            QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_groupby_hash<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "attr");
-        attr[pred] = true;
-    }
+    QG_TRY(qg_allow_smem(ctx, site[pred], pred ? k_groupby_hash<true> : k_groupby_hash<false>, smem));
     if (n > 0) {
         int blocks = grid_for(ctx, (n + 3) / 4, GB_THREADS, g_gb_blocks_per_sm);
         qg_pre_launch(ctx);
@@ -1410,12 +1400,8 @@ static qg_status gb_launch_twopass(qg_ctx *ctx, const int32_t *key, const int32_
     const bool s64 = gb_mode(ctx) == 2;
     auto part = pred ? (s64 ? k_gb_part<true, true> : k_gb_part<true, false>)
                      : (s64 ? k_gb_part<false, true> : k_gb_part<false, false>);
-    static size_t attr[4] = {0, 0, 0, 0};
-    const int ai = (pred ? 2 : 0) + (s64 ? 1 : 0);
-    if (attr[ai] < smem1) {
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(part, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1), "attr");
-        attr[ai] = smem1;
-    }
+    static qg_per_device site[4];
+    QG_TRY(qg_allow_smem(ctx, site[(pred ? 2 : 0) + (s64 ? 1 : 0)], part, smem1));
     // d_flags is the low word of one control counter; the pass-2 work counter
     // is the next counter (both cleared together).
     unsigned int *work = d_flags + 2;

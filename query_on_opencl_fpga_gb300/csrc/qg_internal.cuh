@@ -5,6 +5,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include "qg.h"
+#include "qg_perdev.h"
 
 // ---------------------------------------------------------------------------
 // Device-resident control block (one per context).
@@ -111,6 +112,20 @@ __device__ __forceinline__ void qg_chain() {
 }
 
 qg_status qg_check_launch(qg_ctx *ctx, const char *what);
+qg_status qg_cuda_fail(qg_ctx *ctx, cudaError_t e, const char *what);
+
+// Lets `kern` be launched on the context's device with up to `bytes` of dynamic shared
+// memory; `site` is the kernel's own (static).
+template <class K>
+inline qg_status qg_allow_smem(qg_ctx *ctx, qg_per_device &site, K kern, size_t bytes) {
+    if (site.covers(ctx->device, bytes)) return QG_OK;
+    const cudaError_t e =
+        cudaFuncSetAttribute(reinterpret_cast<const void *>(kern), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return qg_cuda_fail(ctx, e, "shared memory of a kernel");
+    site.set(ctx->device, bytes);
+    return QG_OK;
+}
+
 template <class... P, class... A>
 inline qg_status qg_launch_chained(qg_ctx *ctx, const char *what, void (*kern)(P...), unsigned grid, unsigned block,
                                    size_t smem, A... args) {
@@ -136,7 +151,6 @@ enum {
     QG_SITE_PJ_HIST = 9, QG_SITE_PJ_FILTER = 10, QG_SITE_PJ_BUCKET = 11
 };
 
-qg_status qg_cuda_fail(qg_ctx *ctx, cudaError_t e, const char *what);
 // Dense-window column group-by (qg_gbdense.cu): launches the whole path on the
 // context's stream, output in ascending unsigned key order; the caller reads
 // ctl->gbd[QG_GBD_OUTSIDE] (non-zero: the path did not apply, nothing valid

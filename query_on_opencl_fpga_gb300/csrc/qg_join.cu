@@ -528,11 +528,8 @@ static qg_status join_probe(qg_ctx *ctx, const int32_t *skey, const int32_t *spa
                             const unsigned long long *tab, uint32_t mask, JoinCtl *jc, const ProbeOut &po,
                             const ProbeOut &odd, int64_t cap, uint64_t least = 0) {
     const size_t smem = sizeof(PjSmem);
-    static bool attr = false;
-    if (!attr) {
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_join_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "attr");
-        attr = true;
-    }
+    static qg_per_device site;
+    QG_TRY(qg_allow_smem(ctx, site, k_join_probe, smem));
     const long long ntiles = (nS + PJ_TILE - 1) / PJ_TILE;
     const int blocks = (int)(ntiles < (long long)ctx->sm_count * 4 ? ntiles : (long long)ctx->sm_count * 4);
     return qg_launch_chained(ctx, "k_join_probe", k_join_probe, blocks, PJ_THREADS, smem, skey, spay, nS, slo, shi,
@@ -581,11 +578,8 @@ qg_status qg_join_hash_sort(qg_ctx *ctx, const int32_t *rkey, const int32_t *rpa
     // Up to 8192 matches: one launch (4 radix passes took 45 us for 4K of them)
     if (m <= QG_CS_MAX) {
         const size_t most = QG_CS_MAX * 8 + 32 * 1024, smem = (size_t)m * 8 + 32 * 1024;
-        static bool attr = false;
-        if (!attr) {
-            QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_join_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most), "attr");
-            attr = true;
-        }
+        static qg_per_device site;
+        QG_TRY(qg_allow_smem(ctx, site, k_join_sort_small, most));
         qg_pre_launch(ctx);
         k_join_sort_small<<<1, QG_CS_THREADS, smem, ctx->stream>>>(A, B, (uint32_t)m);
         QG_TRY(qg_check_launch(ctx, "k_join_sort_small"));

@@ -472,12 +472,9 @@ qg_status qg_jp_launch(qg_ctx *ctx, char *work, const qg_jp_r &r, const int32_t 
                        uint32_t *out_rpay, uint32_t *out_spay, int64_t cap, volatile long long *d_count,
                        volatile uint32_t *result) {
     JpPlan *P = (JpPlan *)work;
-    static bool attr = false;
-    if (!attr) {
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_jp_part, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JpTile)), "attr");
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_jp_join, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(JpBucket)), "attr");
-        attr = true;
-    }
+    static qg_per_device sites[2];
+    QG_TRY(qg_allow_smem(ctx, sites[0], k_jp_part, sizeof(JpTile)));
+    QG_TRY(qg_allow_smem(ctx, sites[1], k_jp_join, sizeof(JpBucket)));
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, JP_MAX_NB, QG_SITE_PJ_BUCKET, &lb));
     QG_TRY_CUDA(ctx, cudaMemsetAsync(P, 0, sizeof(JpPlan), ctx->stream), "plan");

@@ -1686,19 +1686,16 @@ void pj_level_carve(char *p, uint32_t nb, bool learned, PjLevel *L) {
 int g_pd_ctas_per_sm = 1;  // resident CTAs of k_pj_join_dense per SM
 
 qg_status pj_attrs(qg_ctx *ctx) {
-    static bool done = false;
-    if (!done) {
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_pj_join, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PbSmem)), "attr join");
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_pj_join_dense<PB_THREADS, PB_SMAX, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)sizeof(PdSmem<PB_SMAX, PB_WARPS>)), "attr join dense");
-        QG_TRY_CUDA(ctx, cudaFuncSetAttribute(k_pj_join_dense<PB_THREADS, PB_SMAX, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)sizeof(PdSmem<PB_SMAX, PB_WARPS>)), "attr join dense");
-        int occ = 0;
-        QG_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pj_join_dense<PB_THREADS, PB_SMAX, false>,
-                                                                       PB_THREADS, sizeof(PdSmem<PB_SMAX, PB_WARPS>)), "occupancy");
-        g_pd_ctas_per_sm = occ > 0 ? occ : 1;
-        done = true;
-    }
+    static qg_per_device sites[3];
+    const size_t dense = sizeof(PdSmem<PB_SMAX, PB_WARPS>);
+    if (sites[2].covers(ctx->device, dense)) return QG_OK;
+    QG_TRY(qg_allow_smem(ctx, sites[0], k_pj_join, sizeof(PbSmem)));
+    QG_TRY(qg_allow_smem(ctx, sites[1], k_pj_join_dense<PB_THREADS, PB_SMAX, true>, dense));
+    QG_TRY(qg_allow_smem(ctx, sites[2], k_pj_join_dense<PB_THREADS, PB_SMAX, false>, dense));
+    int occ = 0;
+    QG_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pj_join_dense<PB_THREADS, PB_SMAX, false>,
+                                                                   PB_THREADS, dense), "occupancy");
+    g_pd_ctas_per_sm = occ > 0 ? occ : 1;
     return QG_OK;
 }
 

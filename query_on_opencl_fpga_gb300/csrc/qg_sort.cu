@@ -479,13 +479,9 @@ static rs_kernel rs_pick(int rank) {
 
 template <bool KV3, bool SIDE>
 static qg_status rs_set_attr(qg_ctx *ctx) {
-    static bool done = false;
-    if (!done) {
-        for (int rank = 0; rank < 5; rank++)
-            QG_TRY_CUDA(ctx, cudaFuncSetAttribute(rs_pick<KV3, SIDE>(rank), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)sizeof(RsSmem<KV3, SIDE>)), "attr");
-        done = true;
-    }
+    static qg_per_device sites[5];
+    for (int rank = 0; rank < 5; rank++)
+        QG_TRY(qg_allow_smem(ctx, sites[rank], rs_pick<KV3, SIDE>(rank), sizeof(RsSmem<KV3, SIDE>)));
     return QG_OK;
 }
 
