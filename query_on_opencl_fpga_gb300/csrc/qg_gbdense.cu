@@ -394,7 +394,7 @@ k_gbd_main(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
 template <bool SAMPLE>
 __global__ void __launch_bounds__(256)
 k_gbd_range(const int32_t *__restrict__ key, long long n, uint32_t *__restrict__ st, uint32_t few_limit,
-            uint32_t *__restrict__ few) {
+            uint32_t many_limit, uint32_t *__restrict__ groups) {
     qg_chain();
     __shared__ uint32_t s[2];
     if (threadIdx.x < 2) s[threadIdx.x] = 0;
@@ -424,7 +424,7 @@ k_gbd_range(const int32_t *__restrict__ key, long long n, uint32_t *__restrict__
         fresh = __reduce_add_sync(QG_FULL_MASK, fresh);
         if ((threadIdx.x & 31) == 0 && fresh) atomicAdd(&s[0], fresh);
         __syncthreads();
-        if (threadIdx.x == 0) *few = s[0] <= few_limit;
+        if (threadIdx.x == 0) *groups = s[0] <= few_limit ? QG_GBW_SEEMS_FEW : s[0] > many_limit ? QG_GBW_SEEMS_MANY : 0u;
         return;
     }
     const uint32_t ctas = gridDim.x - (SAMPLE ? 1u : 0u);
@@ -885,13 +885,14 @@ k_gbd_single(const int32_t *__restrict__ key, const int32_t *__restrict__ val, c
 
 }  // namespace
 
-qg_status qg_gbd_range(qg_ctx *ctx, const int32_t *key, int64_t n, uint32_t few_limit) {
+qg_status qg_gbd_range(qg_ctx *ctx, const int32_t *key, int64_t n, uint32_t few_limit, uint32_t many_limit) {
     const unsigned grid = (unsigned)std::min<long long>(qg_ceil_div(n, 4 * 256), 4LL * ctx->sm_count);
     qg_pre_launch(ctx);
     if (few_limit)
-        k_gbd_range<true><<<grid + 1, 256, 0, ctx->stream>>>(key, n, ctx->ctl->gbd, few_limit, &ctx->ctl->gbw_few);
+        k_gbd_range<true><<<grid + 1, 256, 0, ctx->stream>>>(key, n, ctx->ctl->gbd, few_limit, many_limit,
+                                                                  &ctx->ctl->gbw_groups);
     else
-        k_gbd_range<false><<<grid, 256, 0, ctx->stream>>>(key, n, ctx->ctl->gbd, 0u, nullptr);
+        k_gbd_range<false><<<grid, 256, 0, ctx->stream>>>(key, n, ctx->ctl->gbd, 0u, 0u, nullptr);
     return qg_check_launch(ctx, "k_gbd_range");
 }
 

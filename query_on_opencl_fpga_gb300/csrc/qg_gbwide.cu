@@ -57,7 +57,7 @@ template <bool PRED>
 __global__ void __launch_bounds__(GW_THREADS, 4)
 k_gbw_rows(const int32_t *__restrict__ key, const int32_t *__restrict__ val, const int32_t *__restrict__ val2,
            int32_t lo2, int32_t hi2, long long n, const uint32_t *__restrict__ range, uint32_t window, int parts_log2,
-           const uint32_t *__restrict__ few, unsigned long long *__restrict__ rec, uint32_t *__restrict__ hist,
+           const uint32_t *__restrict__ seems, unsigned long long *__restrict__ rec, uint32_t *__restrict__ hist,
            unsigned long long *__restrict__ rows, uint4 *__restrict__ clear, long long clear_n) {
     qg_chain();
     __shared__ uint32_t s_h[GW_PARTS], s_woff[32], s_cnt;
@@ -65,7 +65,7 @@ k_gbw_rows(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
     __shared__ unsigned long long s_row[PRED ? GW_TILE : 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t kmin = ~range[0], span = range[1] - kmin, lt = qg_lanemask_lt();
-    if (span < window || (few && *few)) return;  // a window holds the keys; few groups
+    if (span < window || (seems && *seems)) return;  // a window holds the keys; too few groups or too many
     const int shift = gw_shift(span, parts_log2);
     for (long long j = (long long)blockIdx.x * GW_THREADS + tid; j < clear_n; j += (long long)gridDim.x * GW_THREADS)
         clear[j] = make_uint4(0, 0, 0, 0);  // the radix pass's status words
@@ -175,7 +175,7 @@ k_gbw_rows(const int32_t *__restrict__ key, const int32_t *__restrict__ val, con
 // One CTA of GW_PARTS threads.  The histogram and the row counter are cleared
 // for their next user.
 __global__ void __launch_bounds__(GW_PARTS)
-k_gbw_plan(const uint32_t *__restrict__ range, uint32_t window, int parts_log2, const uint32_t *__restrict__ few,
+k_gbw_plan(const uint32_t *__restrict__ range, uint32_t window, int parts_log2, const uint32_t *__restrict__ seems,
            uint32_t *__restrict__ hist, unsigned long long *__restrict__ rows, GwState *__restrict__ W, const unsigned long long *r0,
            unsigned long long *r1, uint32_t *status) {
     qg_chain();
@@ -207,7 +207,9 @@ k_gbw_plan(const uint32_t *__restrict__ range, uint32_t window, int parts_log2, 
     W->full = 0;
     *rows = 0;
     const bool even = most <= 16384u || ((unsigned long long)most << parts_log2) <= (unsigned long long)GW_UNEVEN * all;
-    const uint32_t verdict = span < window ? QG_GBW_NARROW : few && *few ? QG_GBW_FEW : even ? QG_GBW_DONE : QG_GBW_OTHER;
+    const uint32_t g = seems ? *seems : 0u;
+    const uint32_t verdict = span < window ? QG_GBW_NARROW : g == QG_GBW_SEEMS_FEW ? QG_GBW_FEW
+                             : even && g != QG_GBW_SEEMS_MANY ? QG_GBW_DONE : QG_GBW_OTHER;
     W->verdict = verdict;
     W->pass = RsPass{r0, r1, status, nullptr, verdict == QG_GBW_DONE ? 1u : 0u, (uint32_t)gw_shift(span, parts_log2), kmin, 0u};
 }
@@ -339,6 +341,15 @@ static uint32_t gw_few_limit(int64_t n) {
     return n < 6'000'000 ? 0u : (uint32_t)std::min<int64_t>((n - 6'000'000) / 5500, 2700);
 }
 
+// Many groups among very many rows: a part's table is half full and its CTA meets a row
+// in two clocks, where the two-pass path spills sequentially.  1M groups, two-pass /
+// this path: 45M rows 1017 / 919 us, 60M 1257 / 1275, 100M 1950 / 2336; 400K groups,
+// 100M rows 1697 / 1424.  The sample tells 100K groups (3890 bits) from 1M (3960), cap
+// has to say the rest.
+static uint32_t gw_many_limit(int64_t rows, int64_t cap) {
+    return rows > 56'000'000 && gw_expected(rows, cap, 8) > 2700 ? 3925u : 0xffffffffu;
+}
+
 bool qg_gbw_few(int64_t n, int64_t groups) { return groups <= gw_few_limit(n) * 3 / 2; }
 
 bool qg_gbw_applies(int64_t n, int64_t cap) {
@@ -366,13 +377,13 @@ qg_status qg_gbw_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
     QG_TRY(qg_allow_smem(ctx, site, k_gbw_merge, gw_smem(GW_SLOTS)));
     qg_lookback lb;
     QG_TRY(qg_lb_make(ctx, GW_PARTS, QG_SITE_GROUPBY, &lb));
-    const uint32_t limit = gw_few_limit(n), *few = limit ? &ctx->ctl->gbw_few : nullptr;
-    QG_TRY(qg_gbd_range(ctx, key, n, limit));
+    const uint32_t limit = gw_few_limit(n), *seems = limit ? &ctx->ctl->gbw_groups : nullptr;
+    QG_TRY(qg_gbd_range(ctx, key, n, limit, gw_many_limit(pred ? n / 2 : n, cap)));  // a predicate: half the rows, say
     const unsigned grid = (unsigned)std::min<long long>(qg_ceil_div(n, GW_TILE), 4LL * ctx->sm_count);
     QG_TRY(qg_launch_chained(ctx, "k_gbw_rows", (pred ? k_gbw_rows<true> : k_gbw_rows<false>), grid, GW_THREADS, 0,
-                             key, val, val2, lo2, hi2, n, range, window, plog2, few, r0, hist, &ctx->ctl->gbw_rows,
+                             key, val, val2, lo2, hi2, n, range, window, plog2, seems, r0, hist, &ctx->ctl->gbw_rows,
                              (uint4 *)status, (long long)(words / 4)));
-    QG_TRY(qg_launch_chained(ctx, "k_gbw_plan", k_gbw_plan, 1, GW_PARTS, 0, range, window, plog2, few, hist,
+    QG_TRY(qg_launch_chained(ctx, "k_gbw_plan", k_gbw_plan, 1, GW_PARTS, 0, range, window, plog2, seems, hist,
                              &ctx->ctl->gbw_rows, W, r0, r1, status));
     QG_TRY(qg_radix_pass_planned(ctx, &W->pass, W->base, n, &W->rows));
     return qg_launch_chained(ctx, "k_gbw_merge", k_gbw_merge, 1u << plog2, QG_CS_THREADS, gw_smem(slots), W, r1, slots,

@@ -21,7 +21,7 @@ struct qg_control {
     uint32_t gbd[48];               // per-call state of the dense-window group-by (qg_gbdense.cu)
     uint32_t ghist[4 * 256];        // digit counts of emitted group keys (group-by in key order)
     uint32_t shist[4 * 256];        // a record sort's digit counts, zero between sorts
-    unsigned int gbw_few;           // the group-by's key sample shows few groups (written before it is read)
+    unsigned int gbw_groups;        // what the group-by's key sample shows (QG_GBW_SEEMS_*, written before it is read)
     unsigned long long gbw_rows;    // records appended by the wide-key group-by, zero between calls
     uint32_t jd[8];                 // state of the counting join (qg_jdirect.cu)
     // Address of the context's host error word (0: none), written with the
@@ -179,7 +179,7 @@ constexpr uint32_t QG_GBD_WINDOW = 1u << 22;  // key values the dense window tak
 enum qg_gbw_result : uint32_t {
     QG_GBW_NARROW = 0,  // the keys fit the dense window
     QG_GBW_DONE = 1,
-    QG_GBW_OTHER = 2,   // parts too uneven, or with too many distinct keys
+    QG_GBW_OTHER = 2,   // parts too uneven, or with too many distinct keys, or many of them among very many rows
     QG_GBW_FEW = 3,     // few groups among many rows: the two-pass path's tables hold them
 };
 bool qg_gbw_applies(int64_t n, int64_t cap);
@@ -187,9 +187,10 @@ qg_status qg_gbw_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
                         int32_t hi2, int64_t n, int32_t *gkey, int64_t *gsum, int64_t *gcnt, int64_t cap,
                         volatile long long *d_num, volatile uint32_t *result);
 // Key range into ctl->gbd[0] (largest complement) and [1] (qg_gbdense.cu).
-// Key range into ctl->gbd; few_limit > 0: ctl->gbw_few = whether a sample of 4096
-// rows (n at least that) has at most that many distinct keys.
-qg_status qg_gbd_range(qg_ctx *ctx, const int32_t *key, int64_t n, uint32_t few_limit = 0);
+// few_limit > 0: ctl->gbw_groups tells whether a sample of 4096 rows (n at least that)
+// sets at most few_limit or more than many_limit of 64K bits by its keys' hashes.
+enum { QG_GBW_SEEMS_FEW = 1, QG_GBW_SEEMS_MANY = 2 };
+qg_status qg_gbd_range(qg_ctx *ctx, const int32_t *key, int64_t n, uint32_t few_limit = 0, uint32_t many_limit = 0);
 bool qg_gbw_few(int64_t n, int64_t groups);  // too few groups for the wide path
 
 

@@ -636,3 +636,30 @@ def test_groupby_outputs_over_inputs(orc, which):
                 assert np.array_equal(g.cpu().numpy(), e)
     finally:
         c.close()
+
+
+# Rows and capacity around the line above which many groups stay on the two-pass
+# path: the same groups on both sides, and with fewer groups than the capacity allows.
+@pytest.mark.parametrize("n,cap,groups", [(56_000_000, 1 << 20, 900_000), (56_000_001, 1 << 20, 900_000),
+                                          (56_000_001, 1 << 20, 60_000), (56_000_001, 691_000, 600_000)])
+def test_groupby_wide_many_rows(n, cap, groups):
+    from query_on_opencl_fpga_gb300.api import Context
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n % 1000 + groups)
+    ids = torch.randint(-(2 ** 31), 2 ** 31, (groups,), generator=g, device="cuda").unique()
+    pick = torch.randint(0, ids.numel(), (n,), generator=g, device="cuda")
+    val = torch.randint(-1000, 1000, (n,), generator=g, device="cuda").to(torch.int32)
+    key = ids[pick].to(torch.int32)
+    u, order = (ids & 0xFFFFFFFF).sort()
+    rank = torch.empty_like(order).scatter_(0, order, torch.arange(order.numel(), device="cuda"))[pick]
+    s = torch.zeros(u.numel(), dtype=torch.int64, device="cuda").index_add_(0, rank, val.to(torch.int64))
+    cnt = torch.bincount(rank, minlength=u.numel())
+    c = Context()
+    try:
+        for _ in range(2):
+            gk, gs, gc = c.groupby_cols(key, val, cap=cap)
+            assert torch.equal(gk.to(torch.int64) & 0xFFFFFFFF, u[cnt > 0])
+            assert torch.equal(gs, s[cnt > 0]) and torch.equal(gc, cnt[cnt > 0])
+    finally:
+        c.close()
