@@ -140,7 +140,7 @@ __device__ __forceinline__ int32_t agg_identity(int op) {
     return op == QG_REDUCE_MIN ? (1 << 30) : 0;
 }
 
-// OP: QG_REDUCE_SUM (also AVERAGE, which divides at the end), MAX or MIN.
+// OP: QG_REDUCE_SUM (also for AVERAGE, whose sums k_agg_avg_finish divides), MAX or MIN.
 template <int OP>
 __device__ __forceinline__ int32_t agg_op(int32_t a, int32_t b) {
     return OP == QG_REDUCE_MAX ? max(a, b) : OP == QG_REDUCE_MIN ? min(a, b) : (int32_t)((uint32_t)a + (uint32_t)b);
@@ -162,7 +162,7 @@ __global__ void k_agg_init(int32_t *agg, long long g0, long long g1, int op) {
 // with atomics (agg holds the identity).  One group at a time per warp took
 // 195 us for 16M records in 1M groups (16 of 32 lanes idle, a dependent load
 // per group); this takes 39 us (floor 20).
-template <int OP, bool AVG, bool VEC>
+template <int OP, bool VEC>
 __global__ void __launch_bounds__(32 * AGG_WARPS, 4)
 k_agg_chunks(const uint2 *__restrict__ rec, long long n, const int32_t *__restrict__ startPos, long long G,
              long long g0, long long g1, int32_t *__restrict__ agg) {
@@ -177,15 +177,16 @@ k_agg_chunks(const uint2 *__restrict__ rec, long long n, const int32_t *__restri
     if (rs < 0 || re > n || rs >= re) return;
     auto group_end = [&](long long g) { return g == G - 1 ? n : (long long)__ldg(&startPos[g + 1]); };
     // the result of the whole group g, and a part of it
-    auto put = [&](long long g, int32_t v) {
-        if (AVG) v = v / (int32_t)(group_end(g) - __ldg(&startPos[g]));
-        agg[g] = v;
-    };
+    auto put = [&](long long g, int32_t v) { agg[g] = v; };
     auto part = [&](long long g, int32_t v) {
         if (OP == QG_REDUCE_MAX) atomicMax(&agg[g], v);
         else if (OP == QG_REDUCE_MIN) atomicMin(&agg[g], v);
         else atomicAdd((unsigned int *)&agg[g], (unsigned int)v);
     };
+    // the group that reaches beyond a chunk, kept over the warp's chunks: one group of
+    // 64M records 121 us a call with an atomic per chunk, 99 so
+    long long open = -1;
+    int32_t open_v = id;
     for (long long c = rs / AGG_CHUNK + wid; c * AGG_CHUNK < re; c += nwarps) {
         const long long cs = c * AGG_CHUNK, lo = max(cs, rs), hi = min(cs + AGG_CHUNK, re);
         int32_t *x = s_x[warp];
@@ -285,8 +286,16 @@ k_agg_chunks(const uint2 *__restrict__ rec, long long n, const int32_t *__restri
             }
             if (lane == 31) {  // the chunk's last group
                 const long long gt = gl - ((long long)__ldg(&startPos[gl]) >= cs ? 1 : 0) + hb;
-                if (hb > 0 && group_end(gt) <= hi) put(gt, run);
-                else part(gt, run);
+                if (hb > 0 && group_end(gt) <= hi) {
+                    put(gt, run);
+                } else {
+                    if (gt != open) {
+                        if (open >= 0) part(open, open_v);
+                        open = gt;
+                        open_v = id;
+                    }
+                    open_v = agg_op<OP>(open_v, run);
+                }
             }
         } else {  // empty groups among these: one group at a time
             long long pos = lo;
@@ -305,17 +314,19 @@ k_agg_chunks(const uint2 *__restrict__ rec, long long n, const int32_t *__restri
         }
         __syncwarp();
     }
+    if (open >= 0) part(open, open_v);
 }
 
-// AVG of groups that spanned chunks: the atomics left the wrapped sum.
+// AVERAGE from the groups' wrapped sums.  (Dividing where a whole group ends, in
+// k_agg_chunks, made that kernel's unrolled fold larger: 64M records in 60K groups 141 us
+// a call, 120 so, in 21M 403 / 305.)
 __global__ void k_agg_avg_finish(const int32_t *__restrict__ startPos, long long n, long long G,
                                  long long g0, long long g1, int32_t *__restrict__ agg) {
     qg_chain();
     long long stride = (long long)gridDim.x * blockDim.x;
     for (long long g = g0 + (long long)blockIdx.x * blockDim.x + threadIdx.x; g < g1; g += stride) {
-        long long gs = startPos[g], ge = (g == G - 1) ? n : startPos[g + 1];
-        bool spans = ge > gs && gs / AGG_CHUNK != (ge - 1) / AGG_CHUNK;
-        if (spans) agg[g] = agg[g] / (int32_t)(ge - gs);
+        const long long gs = startPos[g], ge = (g == G - 1) ? n : startPos[g + 1];
+        if (ge > gs) agg[g] = agg[g] / (int32_t)(ge - gs);
     }
 }
 
@@ -1223,10 +1234,9 @@ extern "C" QG_API qg_status qg_aggregate_group_range(qg_ctx *ctx, const void *so
     const long long chunks = (n + AGG_CHUNK - 1) / AGG_CHUNK;
     const int blocks = grid_for(ctx, chunks, AGG_WARPS, 6);
     const bool vec = ((uintptr_t)sorted & 15) == 0;
-    auto kern = op == QG_REDUCE_MAX       ? (vec ? k_agg_chunks<QG_REDUCE_MAX, false, true> : k_agg_chunks<QG_REDUCE_MAX, false, false>)
-                : op == QG_REDUCE_MIN     ? (vec ? k_agg_chunks<QG_REDUCE_MIN, false, true> : k_agg_chunks<QG_REDUCE_MIN, false, false>)
-                : op == QG_REDUCE_AVERAGE ? (vec ? k_agg_chunks<QG_REDUCE_SUM, true, true> : k_agg_chunks<QG_REDUCE_SUM, true, false>)
-                                          : (vec ? k_agg_chunks<QG_REDUCE_SUM, false, true> : k_agg_chunks<QG_REDUCE_SUM, false, false>);
+    auto kern = op == QG_REDUCE_MAX   ? (vec ? k_agg_chunks<QG_REDUCE_MAX, true> : k_agg_chunks<QG_REDUCE_MAX, false>)
+                : op == QG_REDUCE_MIN ? (vec ? k_agg_chunks<QG_REDUCE_MIN, true> : k_agg_chunks<QG_REDUCE_MIN, false>)
+                                      : (vec ? k_agg_chunks<QG_REDUCE_SUM, true> : k_agg_chunks<QG_REDUCE_SUM, false>);
     QG_TRY(qg_launch_chained(ctx, "k_agg_chunks", kern, blocks, 32 * AGG_WARPS, 0, (const uint2 *)sorted, n, startPos,
                              G, g0, g1, agg));
     if (op == QG_REDUCE_AVERAGE) {

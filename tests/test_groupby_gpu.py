@@ -663,3 +663,29 @@ def test_groupby_wide_many_rows(n, cap, groups):
             assert torch.equal(gs, s[cnt > 0]) and torch.equal(gc, cnt[cnt > 0])
     finally:
         c.close()
+
+
+# More chunks than warps: a warp's chunks lie in one group, in several, and begin or
+# end one; wrapping sums, averages of whole groups and of those over many chunks.
+@pytest.mark.parametrize("op", [0, 1, 2, 3])
+@pytest.mark.parametrize("sizes", [[17_000_003], [1, 9_000_000, 5, 7_999_999], [1024] * 9000 + [8_000_000], [7_500_000, 1023] * 2])
+def test_aggregate_chunks_per_warp(ctx, op, sizes):
+    n = sum(sizes)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    sz = torch.tensor(sizes, device="cuda")
+    rank = torch.repeat_interleave(torch.arange(sz.numel(), device="cuda"), sz)
+    x = torch.randint(-(2 ** 31), 2 ** 31, (n,), generator=g, device="cuda")
+    rec = torch.stack([x, rank], 1).to(torch.int32)
+    sp = (sz.cumsum(0) - sz).to(torch.int32)
+    got = ctx.aggregate_groups(rec, sp, op).to(torch.int64)
+    if op in (0, 3):
+        s = torch.zeros(sz.numel(), dtype=torch.int64, device="cuda").index_add_(0, rank, x)
+        exp = (s + 2 ** 31) % 2 ** 32 - 2 ** 31
+        if op == 3:
+            exp = torch.div(exp, sz, rounding_mode="trunc")
+    elif op == 1:
+        exp = torch.zeros(sz.numel(), dtype=torch.int64, device="cuda").scatter_reduce_(0, rank, x, "amax")
+    else:
+        exp = torch.full((sz.numel(),), 1 << 30, device="cuda").scatter_reduce_(0, rank, x, "amin")
+    assert torch.equal(got, exp)
