@@ -74,6 +74,7 @@ struct qg_ctx {
     bool gb_wide_keys;      // last key-ordered group-by's keys spanned too wide a range for the dense order
     uint32_t gb_kbase;      // first key of the next dense-order window (from the last call's keys)
     bool sort_odd_passes;   // the last in-place record sort took an odd number of passes
+    bool sort_no_passes;    // ... or none (all keys equal)
     uint32_t pj_stats[8];   // last qg_join_filter_sort (see qg_join_stats)
     bool pj_sparse;         // the last join's R keys had no dense span: look before launching the counting path
     // Joins that leave out an attempt which was given up at some cost, so that a stream

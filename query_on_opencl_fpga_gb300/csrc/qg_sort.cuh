@@ -83,6 +83,6 @@ size_t qg_radix_dev_work_bytes(long long n_bound);
 // buffer, planned on the device (no synchronisation, nothing read back).
 qg_status qg_sort_rec(qg_ctx *ctx, const unsigned long long *in, unsigned long long *out, unsigned long long *tmp,
                       long long n);
-// After the stream of an in-place qg_sort_rec has been waited for: remember the
-// parity of its passes for the next one.
+// After the stream of an in-place qg_sort_rec has been waited for: remember its
+// passes for the next one.
 void qg_sort_remember(qg_ctx *ctx);

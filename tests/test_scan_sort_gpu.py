@@ -127,3 +127,20 @@ def test_sort_rec_tiles_and_passes(ctx, n, mask):
         heads = np.flatnonzero(np.r_[True, exp[1:, 1] != exp[:-1, 1]])
         assert np.array_equal(start.cpu().numpy(), heads)
         assert np.array_equal(ctx.sort_rec(d).cpu().numpy(), exp)
+
+
+def test_sort_rec_equal_keys_between_others(ctx):
+    # many tiles of equal keys (no pass at all, twice), then keys that need passes, the
+    # same buffer each time
+    n = 10_500_000
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    buf = torch.empty((n, 2), dtype=torch.int32, device="cuda")
+    x = torch.arange(n, dtype=torch.int32, device="cuda")
+    for key in (7, 7, None, 9, -1, None, None):
+        y = torch.full((n,), key, dtype=torch.int32, device="cuda") if key is not None else \
+            torch.randint(-(2 ** 31), 2 ** 31, (n,), generator=g, device="cuda").to(torch.int32)
+        buf[:, 0], buf[:, 1] = x, y
+        ctx.sort_rec(buf)
+        order = torch.sort(y.to(torch.int64) & 0xFFFFFFFF, stable=True).indices
+        assert torch.equal(buf[:, 0], x[order]) and torch.equal(buf[:, 1], y[order])
