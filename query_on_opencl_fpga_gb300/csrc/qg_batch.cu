@@ -241,8 +241,8 @@ QG_API qg_status qg_batch_create(const qg_query *queries, int nq, int autotune, 
         for (int i = 0; i < nq; i++)
             if (b->persistent && b->q[i].op != QG_OP_JOIN) b->order.push_back(i);
     }
-    // Lanes: a group-by query on the default variant (dense window first) is
-    // run once on the dense-window path; when every row fell in the window the
+    // Lanes: a group-by query on the default variant (dense window first; a small one
+    // takes its one launch) is run once on the dense-window path; when every row fell in the window the
     // captured form takes that path too, sync-free (rows outside the window on
     // a later replay are reported, QG_ERR_UNSUPPORTED, not handed over to the
     // two-pass path, which needs a host read).  The others keep the sync-free
@@ -251,7 +251,11 @@ QG_API qg_status qg_batch_create(const qg_query *queries, int nq, int autotune, 
     for (int i = 0; i < nq && st == QG_OK && !b->persistent; i++) {
         const qg_query &q = b->q[i];
         if ((q.op != QG_OP_GROUPBY && q.op != QG_OP_FUSED) || (q.variant >= 0 && q.variant != 0)) continue;
-        bool ok = false;
+        bool ok = q.n > 0 && q.n < QG_GBS_SURE_ROWS;  // one launch whatever the keys: no 70 MB table for it
+        if (ok) {
+            b->gdense[i] = 1;
+            continue;
+        }
         st = qg_groupby_dense_probe(b->own[b->lane[i]], q.in[0], q.in[1], q.op == QG_OP_FUSED ? q.in[2] : nullptr,
                                     q.lo, q.hi, q.n, (int32_t *)q.out[0], (int64_t *)q.out[1], (int64_t *)q.out[2],
                                     q.cap, q.d_count, &ok);

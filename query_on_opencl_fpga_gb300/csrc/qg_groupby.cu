@@ -1540,15 +1540,17 @@ __global__ void k_gbd_outside_error(qg_control *ctl) {
 }
 }  // namespace
 
-// The dense-window path without a host round trip (batches): output in key
-// order, the group count in *d_num; keys outside the sampled window are
+// The dense-window path without a host round trip (batches), or a small input's one
+// launch: output in key order, the group count in *d_num; keys outside the sampled window are
 // reported as QG_ERR_UNSUPPORTED by qg_ctx_check (nothing valid is written).
 qg_status qg_groupby_dense_async(qg_ctx *ctx, const int32_t *key, const int32_t *val, const int32_t *val2,
                                  int32_t lo2, int32_t hi2, int64_t n, int32_t *gkey, int64_t *gsum, int64_t *gcnt,
                                  int64_t cap, int64_t *d_num) {
     if (!ctx || n < 0 || cap < 0 || !d_num || (n > 0 && (!key || !val))) return QG_ERR_INVALID;
     if ((((uintptr_t)key) | ((uintptr_t)val) | ((uintptr_t)val2)) & 15) return QG_ERR_INVALID;
-    if (n < QG_GBS_SURE_ROWS || n >= (1LL << 32))
+    if (n > 0 && n < QG_GBS_SURE_ROWS)  // whatever the process-wide mode is
+        return qg_gbs_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, (long long *)d_num, nullptr);
+    if (n == 0 || n >= (1LL << 32))
         return qg_groupby_cols_async(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, QG_ORDER_NONE, d_num);
     QG_TRY(qg_gbd_launch(ctx, key, val, val2, lo2, hi2, n, gkey, gsum, gcnt, cap, (long long *)d_num, nullptr));
     qg_pre_launch(ctx);

@@ -267,3 +267,30 @@ def test_batch_join_small_capacity(ctx, orc, span, cap):
         _same(qb.OP_JOIN, tuple(t[:skey.size] for t in q["out"]), tuple(torch.from_numpy(x) for x in exp))
     finally:
         b.close()
+
+
+# A small group-by of the default variant runs in its own form whatever the query
+# before it asked for (the group-by mode is process-wide).
+def test_batch_small_group_by_after_another_variant(ctx):
+    rng = np.random.default_rng(35)
+    qs = []
+    for variant in (-1, 1):  # equal row counts: enqueued last first
+        n = 5000
+        key = torch.from_numpy(rng.integers(0, 700, n).astype(np.int32)).cuda()
+        val = torch.from_numpy(rng.integers(0, 1000, n).astype(np.int32)).cuda()
+        qs.append({"op": qb.OP_GROUPBY, "n": n, "n2": 0, "variant": variant, "inp": [key, val, val], "lo": 0, "hi": 0,
+                   "cap": n, "count": torch.zeros(1, dtype=torch.int64, device="cuda"),
+                   "out": [torch.empty(n, dtype=t, device="cuda") for t in (torch.int32, torch.int64, torch.int64)]})
+    plain = qb.run_plain(ctx, qs)
+    assert ctx.lib.qg_batch_set_lanes(1) == 0
+    try:
+        b = qb.Batch(qs, autotune=False)
+    finally:
+        ctx.lib.qg_batch_set_lanes(12)
+    try:
+        b.run()
+        b.check()
+        for g, e in zip(qb.batch_results(qs)[0], plain[0]):
+            assert torch.equal(g, e)
+    finally:
+        b.close()
