@@ -79,7 +79,7 @@ struct qg_ctx {
     bool pj_sparse;         // the last join's R keys had no dense span: look before launching the counting path
     // Joins that leave out an attempt which was given up at some cost, so that a stream
     // of such inputs pays for it once in QG_PJ_LEAVE_OUT + 1 calls.
-    uint8_t pj_no_hash;
+    uint8_t pj_no_hash, pj_no_part;
     char *pj_tmp;           // the join's sort-merge arrays (grow-only)
     size_t pj_tmp_bytes;
     void *pin_join;         // host pinned bucket bounds and group plan of the join (allocated on first use)

@@ -38,9 +38,15 @@ enum { PJ_F_DENSE = 1, PJ_F_DISTINCT = 2, PJ_F_PMIN = 4, PJ_F_PMAX = 5, PJ_F_SEN
 
 // Dense build side, large probe inputs (qg_jpart.cu): four launches, no read
 // back.  r: R's payload table as k_pj_rtab leaves it.  rows: `room` rows of
-// scratch, 16-byte aligned.  Afterwards *result is 1 when the outputs hold the
-// result, *d_count then the match count, else 0; qg_jp_done() is the same word in
-// device memory for kernels that follow.  work: qg_jp_bytes(), 16-byte aligned.
+// scratch, 16-byte aligned.  Afterwards *result is a qg_jp_result, and with QG_JP_DONE
+// the outputs hold the result and *d_count the match count; qg_jp_done() is a word in
+// device memory that is 1 then, for kernels that follow.  work: qg_jp_bytes(), 16-byte
+// aligned.
+enum qg_jp_result : uint32_t {
+    QG_JP_REFUSED = 0,  // no dense build side, or the sample shows uneven rows
+    QG_JP_DONE = 1,
+    QG_JP_OVER = 2,     // a bucket outgrew its room while the rows were partitioned
+};
 struct qg_jp_r {
     const uint32_t *range;  // smallest and largest key
     const uint32_t *flags;  // PJ_F_*

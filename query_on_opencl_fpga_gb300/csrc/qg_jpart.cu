@@ -332,7 +332,7 @@ k_jp_join(JpPlan *__restrict__ P, const unsigned long long *__restrict__ rows, q
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t lt = qg_lanemask_lt();
     if (!P->ok || P->over) {  // the same for all CTAs: only k_jp_part sets it
-        if (blockIdx.x == 0 && tid == 0) *result = 0;
+        if (blockIdx.x == 0 && tid == 0) *result = P->ok ? QG_JP_OVER : QG_JP_REFUSED;
         return;
     }
     const uint32_t nb = P->nb, kmin = P->kmin, sent = r.flags[PJ_F_SENT], by_sent = r.flags[PJ_F_SENT_OK];
@@ -455,7 +455,7 @@ k_jp_join(JpPlan *__restrict__ P, const unsigned long long *__restrict__ rows, q
         if (tid == 0 && b == nb - 1) {
             *d_count = o0 + total;
             P->done = 1;
-            *result = 1;
+            *result = QG_JP_DONE;
         }
     }
     qg_lb_end(lb);

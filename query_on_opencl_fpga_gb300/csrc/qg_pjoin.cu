@@ -2287,7 +2287,12 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     QG_TRY(qg_launch_chained(ctx, "k_pj_distinct", k_pj_distinct, pj_grid(ctx, nR, 256, 8), 256, 0, bitmap, T, L.range,
                              lb2, nR, L.dflags, reinterpret_cast<unsigned long long *>(L.dflags + PJ_F_DISTINCT)));
     // large probe inputs: one partition step, unless the build side is not dense or the rows spread unevenly
-    const bool jp = dflt && nS > PJ_DIRECT_S;
+    const bool large = dflt && nS > PJ_DIRECT_S;
+    bool jp = large;
+    if (jp && ctx->pj_no_part) {
+        ctx->pj_no_part--;
+        jp = false;
+    }
     const bool filter_later = may_hash && !pj_near_size(nS, nR);  // with sparse build keys, if the hash join hands back
     char *jp_work = aux + 2 * rb + 2 * sb + bmb + pj_level_bytes(PJ_MAX_BUCKETS, true);
     if (jp) {
@@ -2301,20 +2306,21 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     QG_TRY(qg_launch_chained(ctx, "k_pj_sfilter", k_pj_sfilter, (unsigned)std::min<long long>(tiles,
                              (long long)ctx->sm_count * 4), SF_THREADS, 0, skey, spay, nS, slo, shi, L.range, S,
                              &L.range->count, ctx->ctl, lb2, L.dh + 512, jp ? qg_jp_done(jp_work) : nullptr,
-                             jp && filter_later ? L.dflags + PJ_F_DENSE : nullptr));
+                             large && filter_later ? L.dflags + PJ_F_DENSE : nullptr));
     // one copy brings R's key range, the S' count, the histograms and the dense flags
     constexpr size_t head = offsetof(PjPin, dflags) + PJ_F_WORDS * 4;
     static_assert(offsetof(PjPin, h) == 256 && offsetof(PjPin, dflags) == 256 + 4096, "as carved");
     QG_TRY_CUDA(ctx, cudaMemcpyAsync(pin, L.range, head, cudaMemcpyDeviceToHost, ctx->stream), "head d2h");
     QG_TRY(qg_collect_error(ctx));
-    if (jp && ctx->hres->aux) {
+    if (jp && ctx->hres->aux == QG_JP_OVER) ctx->pj_no_part = QG_PJ_LEAVE_OUT;
+    if (jp && ctx->hres->aux == QG_JP_DONE) {
         ctx->pj_stats[0] = 4;
         ctx->pj_sparse = false;
         *out_n = ctx->hres->count;
         return *out_n > cap ? QG_ERR_CAPACITY : QG_OK;
     }
     const bool near = (unsigned long long)(pin->range.kmax - pin->range.kmin) + 1ull <= pj_near_span(nS, nR);
-    if (jp && may_hash && !near && pin->dflags[PJ_F_DENSE] == 0u) {  // sparse build keys: the hash join, then what follows it
+    if (large && may_hash && !near && pin->dflags[PJ_F_DENSE] == 0u) {  // sparse build keys: the hash join, then what follows it
         ctx->pj_sparse = true;
         return join_filter_sort_impl(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay, out_spay, cap, out_n);
     }

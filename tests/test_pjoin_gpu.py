@@ -702,3 +702,36 @@ def test_join_hash_without_room_for_a_third_set_of_columns():
             assert c.join_stats()["path"] == "hash_sort"
     finally:
         c.close()
+
+
+def test_join_large_overflow_is_not_repeated():
+    # Probe rows off the sampled ones crowd one bucket's range: the partition step runs
+    # over, the next call leaves it out, and sparse build keys between are hashed.
+    from query_on_opencl_fpga_gb300.api import Context
+
+    nS, nR = 20_000_003, 1_300_000
+    g = torch.Generator(device="cuda")
+    g.manual_seed(13)
+    ints = lambda lo, hi, n: torch.randint(lo, hi, (n,), generator=g, device="cuda")  # noqa: E731
+    r, rpay, soff, spay = torch.randperm(nR, generator=g, device="cuda"), ints(0, 1000, nR), ints(0, nR, nS), ints(0, 1000, nS)
+    row = np.arange(nS // 1024 * 1024)
+    sampled = (row % 1024) // 16 == (_hash32(row // 1024) & np.uint64(63)).astype(np.int64)
+    off = torch.from_numpy(np.flatnonzero(~sampled)).cuda()
+    soff[off] = soff[off] % (nR // 3)
+    sel = spay <= 299
+    table = torch.empty(nR, dtype=torch.int64, device="cuda")
+    table[r] = rpay
+    exp = (soff[sel] * 1000 + spay[sel]).sort().values
+    c = Context()
+    try:
+        for i, stride in enumerate((1, 1, 1000, 1)):
+            args = [t.to(torch.int32) for t in (r * stride, rpay, soff * stride, spay)]
+            got = []
+            names = launched(c, lambda: got.extend(c.join_filter_sort(*args, 0, 299, cap=nS)))
+            k = got[0].to(torch.int64) // stride
+            assert bool((k[1:] >= k[:-1]).all())
+            assert torch.equal((k * 1000 + got[2]).sort().values, exp) and torch.equal(got[1].to(torch.int64), table[k])
+            assert c.join_stats()["path"] == ("hash_sort" if stride > 1 else c.join_stats()["path"])
+            assert ("k_jp_part" in names) == (i == 0), (i, names)
+    finally:
+        c.close()
