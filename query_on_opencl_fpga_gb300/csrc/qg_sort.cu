@@ -195,7 +195,7 @@ __device__ __forceinline__ void rs_copy_tile(const qg_sort_bufs &src, const qg_s
 // One tile of a pass.  ALL: a full tile, with no bounds checks per item.
 template <bool KV3, bool SIDE, int RANK, bool ALL>
 __device__ __forceinline__ void rs_tile(RsSmem<KV3, SIDE> &S, const qg_sort_bufs &src, const qg_sort_bufs &dst,
-                                        int cnt, int shift, uint32_t key_off, const uint32_t *__restrict__ dbase,
+                                        uint32_t n, int cnt, int shift, uint32_t key_off, const uint32_t *__restrict__ dbase,
                                         uint32_t *__restrict__ status, qg_control *ctl, uint32_t spin_limit) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t tile = blockIdx.x;  // started in index order; the status words are cleared before every pass
@@ -335,12 +335,15 @@ __device__ __forceinline__ void rs_tile(RsSmem<KV3, SIDE> &S, const qg_sort_bufs
     __syncthreads();
     // Out, each digit's run with consecutive addresses.  The digit is taken
     // from the key (or id) again: cheaper than a byte array of digits, whose
-    // scattered stores cost shared-memory wavefronts.
+    // scattered stores cost shared-memory wavefronts.  A pass after one whose look-back
+    // gave up (reported as QG_ERR_TIMEOUT) reads items that are not the ones counted, so
+    // a place may lie past the end: those are dropped.
     auto put = [&](int p) {
         const unsigned long long v = S.v[p];
         const uint32_t k = KV3 ? S.k[p] : (uint32_t)(v >> 32);
         const uint32_t d = SIDE ? ((uint32_t)S.bid[p] >> shift) & 255u : rs_digit(k, key_off, shift);
         const uint32_t g = S.goff[d] + (uint32_t)p;
+        if (g >= n) return;
         if (KV3) {
             dst.k[g] = k;
             dst.a[g] = (uint32_t)v;
@@ -421,9 +424,9 @@ k_radix_pass(qg_sort_bufs src, qg_sort_bufs dst, long long n, int shift, uint32_
     for (int i = threadIdx.x; i < RS_WARPS * QG_RADIX; i += RS_THREADS) (&S.whist[0][0])[i] = 0;
     __syncthreads();
     if (left >= RS_TILE)
-        rs_tile<KV3, SIDE, RANK, true>(S, src, dst, RS_TILE, shift, key_off, dbase, status, ctl, spin_limit);
+        rs_tile<KV3, SIDE, RANK, true>(S, src, dst, (uint32_t)n, RS_TILE, shift, key_off, dbase, status, ctl, spin_limit);
     else
-        rs_tile<KV3, SIDE, RANK, false>(S, src, dst, (int)left, shift, key_off, dbase, status, ctl, spin_limit);
+        rs_tile<KV3, SIDE, RANK, false>(S, src, dst, (uint32_t)n, (int)left, shift, key_off, dbase, status, ctl, spin_limit);
 }
 
 }  // namespace

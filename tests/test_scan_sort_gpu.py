@@ -144,3 +144,31 @@ def test_sort_rec_equal_keys_between_others(ctx):
         ctx.sort_rec(buf)
         order = torch.sort(y.to(torch.int64) & 0xFFFFFFFF, stable=True).indices
         assert torch.equal(buf[:, 0], x[order]) and torch.equal(buf[:, 1], y[order])
+
+
+def test_sort_rec_timeout_reports_and_recovers(ctx):
+    # Poll limit 0: look-backs give up, passes after the first read items other than the
+    # counted ones.  The call reports it, writes nothing past the records, and the next
+    # call is exact.
+    from query_on_opencl_fpga_gb300 import QGError
+
+    n = 4_000_001
+    g = torch.Generator(device="cuda")
+    g.manual_seed(6)
+    rec = torch.randint(-(2 ** 31), 2 ** 31, (n + 300_000, 2), generator=g, device="cuda").to(torch.int32)
+    rec[n:] = 77
+    keep = rec[:n].clone()
+    for _ in range(3):
+        ctx.set_spin_limit(0)
+        try:
+            with pytest.raises(QGError) as e:
+                ctx.sort_rec(rec[:n])
+            assert e.value.status == 5
+        finally:
+            ctx.set_spin_limit(1 << 22)
+        assert bool((rec[n:] == 77).all())
+        rec[:n] = keep
+        ctx.sort_rec(rec[:n])
+        order = torch.sort(keep[:, 1].to(torch.int64) & 0xFFFFFFFF, stable=True).indices
+        assert torch.equal(rec[:n], keep[order])
+        rec[:n] = keep
