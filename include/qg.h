@@ -242,6 +242,17 @@ QG_API qg_status qg_groupby_set_single_launch(int enable);
  * out[3] = bucket capacity (the last three 0 on the dense-window path and when
  * partitioned by key range). */
 QG_API qg_status qg_groupby_stats(qg_ctx *ctx, uint32_t *out4);
+/* Which form answered the context's last qg_groupby_cols call. */
+typedef enum {
+    QG_GB_ROUTE_NONE = 0,
+    QG_GB_ROUTE_ONE_CTA = 1,        /* a small input, one launch */
+    QG_GB_ROUTE_EXACT_WINDOW = 2,   /* dense window on the exact key range */
+    QG_GB_ROUTE_SAMPLED_WINDOW = 3, /* dense window on a sample's key range */
+    QG_GB_ROUTE_KEY_RANGES = 4,     /* partitioned by key range */
+    QG_GB_ROUTE_TWO_PASS = 5,
+    QG_GB_ROUTE_GLOBAL_TABLE = 6
+} qg_groupby_route_t;
+QG_API int qg_groupby_route(qg_ctx *ctx);
 
 /* ---- hash join + filter + sort (config 2; kernel/hj_filter_sort/1/hj_filter_sort_op.cl)
  * Inner equi-join of R(rkey, rpay) and S(skey, spay) on uint key equality,
@@ -287,6 +298,17 @@ QG_API qg_status qg_join_set_dense(int enable);
  * out[6] heavy keys among them, out[7] 1 when the automatic choice moved
  * from radix to the learned function. */
 QG_API qg_status qg_join_stats(qg_ctx *ctx, uint32_t *out8);
+/* Which form answered the context's last qg_join_filter_sort call. */
+typedef enum {
+    QG_JOIN_ROUTE_NONE = 0,          /* nothing to join */
+    QG_JOIN_ROUTE_COUNTING = 1,      /* dense build side, counted */
+    QG_JOIN_ROUTE_ONE_STEP = 2,      /* dense build side, one partition step */
+    QG_JOIN_ROUTE_DENSE_BUCKETS = 3, /* dense build side, radix partitioned */
+    QG_JOIN_ROUTE_RADIX = 4,
+    QG_JOIN_ROUTE_LEARNED = 5,
+    QG_JOIN_ROUTE_HASH = 6
+} qg_join_route_t;
+QG_API int qg_join_route(qg_ctx *ctx);
 
 /* ---- whole-column reduce (the check of host/host/Validate.cpp:372-468; the
  * reference ships no kernel) ----  SUM (wrapping modulo 2^32), MAX and MIN

@@ -71,6 +71,7 @@ SIGNATURES: dict[str, tuple] = {
     "qg_groupby_set_knobs": (c_int, [c_int, c_int, c_int, c_uint32]),
     "qg_groupby_set_single_launch": (c_int, [c_int]),
     "qg_groupby_stats": (c_int, [c_void_p, c_void_p]),
+    "qg_groupby_route": (c_int, [c_void_p]),
     "qg_join_filter_sort": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_int64,
                                     c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_int64,
                                     POINTER(c_int64)]),
@@ -89,6 +90,7 @@ SIGNATURES: dict[str, tuple] = {
     "qg_join_set_dense": (c_int, [c_int]),
     "qg_sort_set_rank": (c_int, [c_int]),
     "qg_join_stats": (c_int, [c_void_p, c_void_p]),
+    "qg_join_route": (c_int, [c_void_p]),
     "qg_part_model_bytes": (c_int64, []),
     "qg_reduce_rec": (c_int, [c_void_p, c_void_p, c_int64, c_int, POINTER(c_uint32)]),
     "qg_split_rec": (c_int, [c_void_p, c_void_p, c_int64, c_int32, c_void_p, c_void_p]),

@@ -269,7 +269,9 @@ class Context:
         out = (ctypes.c_uint32 * 4)()
         self.check(self.lib.qg_groupby_stats(self.handle, out), "qg_groupby_stats")
         path = {0: "two_pass", 1: "global_table", 2: "dense"}[out[0]]
-        return {"path": path, "flags": out[1], "fullest_bucket": out[2], "bucket_cap": out[3]}
+        routes = ("none", "one_cta", "exact_window", "sampled_window", "key_ranges", "two_pass", "global_table")
+        return {"path": path, "flags": out[1], "fullest_bucket": out[2], "bucket_cap": out[3],
+                "route": routes[self.lib.qg_groupby_route(self.handle)]}
 
     # ---- join ---------------------------------------------------------------
     def join_filter_sort(self, rkey, rpay, skey, spay, slo: int = INT32_MIN, shi: int = INT32_MAX,
@@ -329,9 +331,10 @@ class Context:
         out = (ctypes.c_uint32 * 8)()
         self.check(self.lib.qg_join_stats(self.handle, out), "qg_join_stats")
         names = {0: "none", 1: "radix", 2: "learned", 3: "hash_sort", 4: "dense"}
+        routes = ("none", "counting", "one_step", "dense_buckets", "radix", "learned", "hash")
         return {"path": names.get(out[0], str(out[0])), "buckets": out[1], "outside_buckets": out[2],
                 "outside_rows": out[3], "merge_buckets": out[4], "knots": out[5], "heavy_keys": out[6],
-                "auto_switched": out[7]}
+                "auto_switched": out[7], "route": routes[self.lib.qg_join_route(self.handle)]}
 
     def part_learn(self, keys: torch.Tensor, nbuckets: int) -> torch.Tensor:
         """Fit the learned partition function on int32/uint32 keys; returns the device model."""

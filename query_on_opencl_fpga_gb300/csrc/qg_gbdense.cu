@@ -83,7 +83,7 @@ constexpr int GBD_THREADS = 1024;
 constexpr int GBM_THREADS = 512;                  // k_gbd_mid
 constexpr int GBM_SLOTS = 4096;
 constexpr int GBM_ROWS = 4096;                    // rows per CTA at least
-constexpr int64_t GBM_MAX_ROWS = 1 << 23;         // largest input of the three-launch form
+constexpr int64_t GBM_MAX_ROWS = QG_GBD_EXACT_ROWS;  // largest input of the three-launch form
 constexpr uint32_t GBD_EMPTY = 0xffffffffu;
 
 // ctl->gbd word indices
@@ -897,6 +897,8 @@ qg_status qg_gbd_range(qg_ctx *ctx, const int32_t *key, int64_t n, uint32_t few_
 }
 
 static int g_gbd_single = 0;  // 1: the four steps in one cooperative launch where it fits
+
+bool qg_gbd_single() { return g_gbd_single != 0; }
 
 extern "C" QG_API qg_status qg_groupby_set_single_launch(int enable) {
     if (enable != 0 && enable != 1) return QG_ERR_INVALID;

@@ -1272,6 +1272,8 @@ static const int g_gb_slog2 = 12;    // fallback kernel: shared-memory table slo
 // out[0] = 0 two-pass / 1 global table / 2 dense window, out[1] = overflow
 // flags (bit 0 spill bucket, bit 1 pass-2 table), out[2] = fullest spill
 // bucket, out[3] = bucket capacity (the last three 0 on the dense path).
+extern "C" QG_API int qg_groupby_route(qg_ctx *ctx) { return ctx ? ctx->gb_route : QG_GB_ROUTE_NONE; }
+
 extern "C" QG_API qg_status qg_groupby_stats(qg_ctx *ctx, uint32_t *out) {
     if (!ctx || !out) return QG_ERR_INVALID;
     for (int i = 0; i < 4; i++) out[i] = ctx->gb_stats[i];
@@ -1625,6 +1627,7 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
                              &ctx->hres->aux));
         QG_TRY(qg_host_count(ctx, &g));
         if (ctx->hres->aux == 0) {
+            ctx->gb_route = QG_GB_ROUTE_ONE_CTA;
             ctx->gb_stats[0] = 2u;
             ctx->gb_stats[1] = ctx->gb_stats[2] = ctx->gb_stats[3] = 0;
             *num_groups = g;
@@ -1649,6 +1652,7 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
         QG_TRY(qg_host_count(ctx, &g));
         *verdict = ctx->hres->aux;
         if (*verdict == QG_GBW_DONE) {
+            ctx->gb_route = QG_GB_ROUTE_KEY_RANGES;
             ctx->gb_stats[0] = 0u;
             ctx->gb_stats[1] = ctx->gb_stats[2] = ctx->gb_stats[3] = 0;
             *num_groups = g;
@@ -1680,6 +1684,7 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
         QG_TRY(qg_host_count(ctx, &g));
         if (ctx->hres->aux == 0) {
             ctx->gb_first = 0;
+            ctx->gb_route = n <= QG_GBD_EXACT_ROWS && !qg_gbd_single() ? QG_GB_ROUTE_EXACT_WINDOW : QG_GB_ROUTE_SAMPLED_WINDOW;
             ctx->gb_stats[0] = 2u;
             ctx->gb_stats[1] = ctx->gb_stats[2] = ctx->gb_stats[3] = 0;
             *num_groups = g;
@@ -1743,6 +1748,7 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
         QG_TRY(gb_launch_global(ctx, key, val, val2, lo2, hi2, n, o, cap, d_num));
         QG_TRY(qg_read_count(ctx, d_num, &g));
     }
+    ctx->gb_route = global ? QG_GB_ROUTE_GLOBAL_TABLE : QG_GB_ROUTE_TWO_PASS;
     *num_groups = g;
     if (g > cap) return QG_ERR_CAPACITY;
     if (done) return QG_OK;

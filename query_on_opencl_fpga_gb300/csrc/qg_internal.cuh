@@ -69,6 +69,7 @@ struct qg_ctx {
     bool unchained;         // launches are not chained: the context shares the device with others (batch lanes)
     bool table_dirty;       // group-by table must be cleared before next use
     uint32_t gb_stats[4];   // last qg_groupby_cols: path, flags, fullest bucket, bucket cap
+    int gb_route, pj_route; // ... and last qg_join_filter_sort: qg_groupby_route_t, qg_join_route_t
     int gb_first;           // what the last default group-by found (qg_groupby.cu): 0 narrow keys, 1 wide ones, 2 uneven, 3 few
                             //   (qg_gbwide.cu), 2 dense window and no attempt at the wide keys' path after it
     bool gb_wide_keys;      // last key-ordered group-by's keys spanned too wide a range for the dense order
@@ -161,6 +162,7 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
                         int32_t lo2, int32_t hi2, int64_t n, int32_t *gkey, int64_t *gsum, int64_t *gcnt,
                         int64_t cap, long long *d_num, volatile uint32_t *outside);
 enum { QG_GBD_OUTSIDE = 6 };
+bool qg_gbd_single();  // the one-launch form is asked for
 // Small column group-by in one launch (qg_gbsmall.cu).
 constexpr int64_t QG_GBS_MAX_ROWS = 16384, QG_GBS_SURE_ROWS = 8192;
 qg_status qg_gbs_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, const int32_t *val2, int32_t lo2,
@@ -177,6 +179,7 @@ qg_status qg_groupby_dense_probe(qg_ctx *ctx, const int32_t *key, const int32_t 
 // context's stream; after the stream is synchronised *result tells whether
 // *d_num and the outputs hold the groups.
 constexpr uint32_t QG_GBD_WINDOW = 1u << 22;  // key values the dense window takes
+constexpr int64_t QG_GBD_EXACT_ROWS = 1 << 23;  // rows up to which it lies on the exact key range
 enum qg_gbw_result : uint32_t {
     QG_GBW_NARROW = 0,  // the keys fit the dense window
     QG_GBW_DONE = 1,

@@ -1977,6 +1977,7 @@ qg_status pj_core(qg_ctx *ctx, const PjLevel &L, PjPin *pin, uint32_t nb, int lb
             kern<<<pk.groups, PB_THREADS, sizeof(PdSmem<PB_SMAX, PB_WARPS>), ctx->stream>>>(da, lb);
             QG_TRY(qg_check_launch(ctx, "k_pj_join_dense"));
             QG_TRY(qg_host_count(ctx, M_out));
+            ctx->pj_route = QG_JOIN_ROUTE_DENSE_BUCKETS;
             ctx->pj_stats[0] = 4;
             ctx->pj_stats[1] = nbu;
             for (int i = 2; i < 8; i++) ctx->pj_stats[i] = 0;
@@ -2097,6 +2098,7 @@ qg_status pj_core(qg_ctx *ctx, const PjLevel &L, PjPin *pin, uint32_t nb, int lb
         const unsigned long long outside = (unsigned long long)ctx->pinned[1] + cross_rows;
         if (outside >= (1ull << 32)) *M_out = (long long)outside;
     }
+    ctx->pj_route = use_learned ? QG_JOIN_ROUTE_LEARNED : QG_JOIN_ROUTE_RADIX;
     ctx->pj_stats[0] = use_learned ? 2 : 1;
     ctx->pj_stats[1] = nbu;
     ctx->pj_stats[2] = no;
@@ -2137,6 +2139,8 @@ extern "C" QG_API qg_status qg_join_stats(qg_ctx *ctx, uint32_t *out8) {
     memcpy(out8, ctx->pj_stats, sizeof(ctx->pj_stats));
     return QG_OK;
 }
+
+extern "C" QG_API int qg_join_route(qg_ctx *ctx) { return ctx ? ctx->pj_route : QG_JOIN_ROUTE_NONE; }
 
 int qg_join_default_variant() { return g_pj_variant; }
 
@@ -2197,6 +2201,7 @@ static qg_status join_direct(qg_ctx *ctx, const int32_t *rkey, const int32_t *rp
     QG_TRY(qg_host_count(ctx, &M));
     ctx->pj_sparse = ctx->hres->aux == QG_JD_SPARSE;
     if (ctx->hres->aux == QG_JD_DONE) {
+        ctx->pj_route = QG_JOIN_ROUTE_COUNTING;
         ctx->pj_stats[0] = 4;
         *out_n = M;
     }
@@ -2214,7 +2219,8 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
         return QG_ERR_INVALID;
     if ((((uintptr_t)skey) | ((uintptr_t)spay)) & 15) return QG_ERR_INVALID;
     if (cap >= (1LL << 30) || nS >= (1LL << 40)) return QG_ERR_UNSUPPORTED;
-    if (variant == 3 || nS >= (1LL << 30) || nR >= (1LL << 30))
+    ctx->pj_route = variant == 3 || nS >= (1LL << 30) || nR >= (1LL << 30) ? QG_JOIN_ROUTE_HASH : QG_JOIN_ROUTE_NONE;
+    if (ctx->pj_route == QG_JOIN_ROUTE_HASH)
         return qg_join_hash_sort(ctx, rkey, rpay, nR, skey, spay, nS, slo, shi, out_key, out_rpay,
                                  out_spay, cap, out_n);
     *out_n = 0;
@@ -2244,6 +2250,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
         if (st == QG_ERR_OOM) end = QG_JH_CROWDED;  // its columns are sized by cap, the arrays below are not
         else if (st != QG_OK && st != QG_ERR_CAPACITY) return st;
         if (end == QG_JH_DONE) {
+            ctx->pj_route = QG_JOIN_ROUTE_HASH;
             ctx->pj_stats[0] = 3;
             return st;
         }
@@ -2314,6 +2321,7 @@ static qg_status join_filter_sort_impl(qg_ctx *ctx, const int32_t *rkey, const i
     QG_TRY(qg_collect_error(ctx));
     if (jp && ctx->hres->aux == QG_JP_OVER) ctx->pj_no_part = QG_PJ_LEAVE_OUT;
     if (jp && ctx->hres->aux == QG_JP_DONE) {
+        ctx->pj_route = QG_JOIN_ROUTE_ONE_STEP;
         ctx->pj_stats[0] = 4;
         ctx->pj_sparse = false;
         *out_n = ctx->hres->count;

@@ -689,3 +689,62 @@ def test_aggregate_chunks_per_warp(ctx, op, sizes):
     else:
         exp = torch.full((sz.numel(),), 1 << 30, device="cuda").scatter_reduce_(0, rank, x, "amin")
     assert torch.equal(got, exp)
+
+
+# The sampled window (above 2^23 rows): a key that no sample run reads and that lies
+# outside the window is seen by the main pass, and another path answers; it moved here
+# when smaller inputs got the exact key range.
+@pytest.mark.parametrize("fused", [False, True])
+def test_groupby_sampled_window_hidden_keys(orc, fused):
+    from query_on_opencl_fpga_gb300.api import Context
+
+    rng = np.random.default_rng(16)
+    n = (1 << 23) + 4099
+    key = rng.integers(100, 100 + 50000, n).astype(np.int32)
+    val = rng.integers(0, 1000, n).astype(np.int32)
+    val2 = rng.integers(0, 1000, n).astype(np.int32) if fused else None
+    runs = 1024
+    starts = np.array([(n - 256) * r // (runs - 1) for r in range(runs)])
+    gap = 5000
+    assert not np.any((starts <= gap + 1) & (gap < starts + 256))
+    c = Context()
+    try:
+        _dense_case(c, orc, key, val, val2, 0, 499, cap=60_000, path="dense")
+        assert c.groupby_stats()["route"] == "sampled_window"
+        key[gap], key[gap + 1] = 2 ** 30, -5
+        if fused:
+            val2[gap: gap + 2] = 7  # (a row outside counts only when it is selected)
+        for _ in range(2):
+            _dense_case(c, orc, key, val, val2, 0, 499, cap=60_000)
+            assert c.groupby_stats()["route"] == "two_pass"
+        _dense_case(c, orc, key[gap + 2:].copy(), val[gap + 2:].copy(), val2[gap + 2:].copy() if fused else None, 0, 499,
+                    cap=60_000, path="dense")
+    finally:
+        c.close()
+
+
+# Which form answers: each new one where it is meant to, and not where it hands over.
+@pytest.mark.parametrize("n,kind,route", [(1, "narrow", "one_cta"), (16_384, "narrow", "one_cta"), (16_384, "own", "exact_window"),
+                                          (16_385, "narrow", "exact_window"), (16_385, "ids", "key_ranges"),
+                                          (1 << 23, "narrow", "exact_window"), ((1 << 23) + 1, "narrow", "sampled_window"),
+                                          (100_000, "ids", "key_ranges"), (4_000_000, "ids", "key_ranges"),
+                                          (100_000, "uneven", "two_pass"), (120_000, "crowded", "two_pass"),
+                                          (8_000_001, "few", "two_pass")])
+def test_groupby_routes(orc, n, kind, route):
+    from query_on_opencl_fpga_gb300.api import Context
+
+    rng = np.random.default_rng(n)
+    ids = rng.integers(-(2 ** 31), 2 ** 31, 1 << 20)
+    key = {"narrow": lambda: rng.integers(5, 3000, n), "own": lambda: rng.permutation(n),
+           "ids": lambda: rng.choice(ids[: max(50, n // 5)], n),
+           "uneven": lambda: rng.choice(np.array([-(2 ** 31), 5, 2 ** 31 - 1]), n),
+           "crowded": lambda: np.where(np.arange(n) < 16_000, np.arange(n), rng.choice(ids[:50], n)),
+           "few": lambda: rng.choice(ids[:60], n)}[kind]().astype(np.int32)
+    val = rng.integers(-5, 1000, n).astype(np.int32)
+    c = Context()
+    try:
+        for _ in range(2):
+            _dense_case(c, orc, key, val, cap=min(n, 1 << 20))  # (key ranges: at most 1.3M groups)
+            assert c.groupby_stats()["route"] == route
+    finally:
+        c.close()

@@ -735,3 +735,46 @@ def test_join_large_overflow_is_not_repeated():
             assert ("k_jp_part" in names) == (i == 0), (i, names)
     finally:
         c.close()
+
+
+# Which form answers: each new one where it is meant to, and not where it hands over.
+@pytest.mark.parametrize("nR,nS,kind,route", [(1000, 20_000, "unique", "counting"), (70_000, 1 << 20, "unique", "counting"),
+                                              (1_000_000, 18_000_000, "unique", "counting"),
+                                              (1_000_000, 18_000_001, "unique", "one_step"),
+                                              (1_300_000, 20_000_003, "hot", "not one_step"),
+                                              (20_000, 300_000, "twice", "radix"), (20_000, 300_000, "sparse", "hash"),
+                                              (8_400_000, 1 << 20, "sparse", "radix"),
+                                              (8_400_000, 1 << 20, "unique", "dense_buckets")])
+def test_join_routes(nR, nS, kind, route):
+    from query_on_opencl_fpga_gb300.api import Context
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nR + nS)
+    ints = lambda lo, hi, n: torch.randint(lo, hi, (n,), generator=g, device="cuda")  # noqa: E731
+    stride = 200 if kind == "sparse" else 1
+    r = torch.randperm(nR, generator=g, device="cuda") * stride
+    rpay, s, spay = ints(0, 1000, nR), ints(-nR, 2 * nR, nS) * stride, ints(0, 1000, nS)
+    if kind == "hot":
+        s[::200] = 12_345
+    if kind == "twice":
+        r[5] = r[6]
+    table = torch.zeros(nR * stride, dtype=torch.int64, device="cuda")
+    table.index_add_(0, r, rpay + (1 << 20))  # rows of the key in the high bits, the sum of their payloads below
+    hit = (spay <= 299) & (s >= 0) & (s < nR * stride)
+    hit[hit.clone()] = table[s[hit]] > 0
+    rows = table[s[hit]]
+    c = Context()
+    try:
+        args = [t.to(torch.int32) for t in (r, rpay, s, spay)]
+        for _ in range(2):
+            k, a, b = c.join_filter_sort(*args, 0, 299, cap=2 * nS)
+            assert k.numel() == int((rows >> 20).sum()) and bool((k[1:] >= k[:-1]).all())
+            assert int(a.sum(dtype=torch.int64)) == int((rows & 0xFFFFF).sum())
+            one = rows >> 20 == 1  # every row once: the pairs themselves
+            if bool(one.all()):
+                assert torch.equal((k.to(torch.int64) * 1000 + b).sort().values, (s[hit] * 1000 + spay[hit]).sort().values)
+                assert torch.equal(a.to(torch.int64), table[k.to(torch.int64)] & 0xFFFFF)
+            got = c.join_stats()["route"]
+            assert got != "one_step" if route == "not one_step" else got == route
+    finally:
+        c.close()
