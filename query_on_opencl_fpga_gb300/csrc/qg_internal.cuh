@@ -80,7 +80,8 @@ struct qg_ctx {
     bool pj_sparse;         // the last join's R keys had no dense span: look before launching the counting path
     // Joins that leave out an attempt which was given up at some cost, so that a stream
     // of such inputs pays for it once in QG_PJ_LEAVE_OUT + 1 calls.
-    uint8_t pj_no_hash, pj_no_part;
+    uint8_t pj_no_hash, pj_no_part, pj_no_count;
+    int64_t pj_hot_rows;    // probe rows of the join that set pj_no_count: much smaller ones count all the same
     char *pj_tmp;           // the join's sort-merge arrays (grow-only)
     size_t pj_tmp_bytes;
     void *pin_join;         // host pinned bucket bounds and group plan of the join (allocated on first use)

@@ -125,7 +125,7 @@ k_jd_table(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, l
         for (int u = 0; u < U; u++)
             if (i0 + u * stride < nR) twice |= jd_put(E + k[u], p[u]);
     }
-    if (twice) jd[JD_OK] = QG_JD_OTHER;
+    if (twice) jd[JD_OK] = QG_JD_TWICE;
 }
 
 // The three steps above in one CTA: with so few rows the launches are what costs.
@@ -176,7 +176,7 @@ k_jd_build(const int32_t *__restrict__ rkey, const int32_t *__restrict__ rpay, u
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < JD_ONE_PER; j++)
-        if (j * JD_ONE_THREADS + tid < nR && jd_put(E + (k[j] - kmin), p[j])) jd[JD_OK] = QG_JD_OTHER;
+        if (j * JD_ONE_THREADS + tid < nR && jd_put(E + (k[j] - kmin), p[j])) jd[JD_OK] = QG_JD_TWICE;
 }
 
 // S rows, 4096 per tile (persistent CTAs): the rows that pass the filter and
@@ -286,7 +286,7 @@ k_jd_count(const int32_t *__restrict__ skey, const int32_t *__restrict__ spay, l
                 heavy |= seen >= JD_KEY_ROWS;
             }
         }
-        if (heavy) jd[JD_OK] = QG_JD_OTHER;
+        if (heavy) jd[JD_OK] = QG_JD_HOT;
         __syncthreads();  // the shared words are rewritten by the next tile
     }
 }

@@ -11,7 +11,8 @@ enum { QG_JD_OK = 4 };
 enum qg_jd_result : uint32_t {
     QG_JD_SPARSE = 0,  // R's keys spread over more than 2 nR values
     QG_JD_DONE = 1,
-    QG_JD_OTHER = 2,   // dense span, but a build key twice or a probe key with too many rows
+    QG_JD_TWICE = 2,   // dense span, but a build key twice
+    QG_JD_HOT = 3,     // ... or a probe key with too many rows
 };
 size_t qg_jd_bytes(int64_t nR, int64_t nS);
 qg_status qg_jd_launch(qg_ctx *ctx, char *work, const int32_t *rkey, const int32_t *rpay, int64_t nR,

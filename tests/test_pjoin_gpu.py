@@ -778,3 +778,37 @@ def test_join_routes(nR, nS, kind, route):
             assert got != "one_step" if route == "not one_step" else got == route
     finally:
         c.close()
+
+
+def test_join_hot_probe_key_is_not_counted_again():
+    # A key with too many rows ends the counting attempt; the next join of that size
+    # leaves it out until one without such a key has been seen, smaller ones do not, and
+    # sparse build keys find the hash join all the same.
+    from query_on_opencl_fpga_gb300.api import Context
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(14)
+    ints = lambda lo, hi, n: torch.randint(lo, hi, (n,), generator=g, device="cuda")  # noqa: E731
+    nR = 20_000
+    r, rpay = torch.randperm(nR, generator=g, device="cuda"), ints(0, 1000, nR)
+    table = torch.empty(nR, dtype=torch.int64, device="cuda")
+    table[r] = rpay
+    c = Context()
+    try:
+        for nS, hot, stride, count, route in [(300_000, True, 1, True, "radix"), (300_000, True, 1, False, "radix"),
+                                              (100_000, False, 1, True, "counting"), (300_000, True, 1, False, "radix"),
+                                              (300_000, False, 1000, False, "hash"), (300_000, False, 1, False, "dense_buckets"),
+                                              (300_000, False, 1, True, "counting")]:
+            s, spay = ints(0, 2 * nR, nS), ints(0, 1000, nS)
+            if hot:
+                s[::20] = 77
+            args = [t.to(torch.int32) for t in (r * stride, rpay, s * stride, spay)]
+            got = []
+            names = launched(c, lambda: got.extend(c.join_filter_sort(*args, 0, 299, cap=nS)))
+            k = got[0].to(torch.int64) // stride
+            hit = (spay <= 299) & (s < nR)
+            assert bool((k[1:] >= k[:-1]).all()) and torch.equal(got[1].to(torch.int64), table[k])
+            assert torch.equal((k * 1000 + got[2]).sort().values, (s[hit] * 1000 + spay[hit]).sort().values)
+            assert ("k_jd_count" in names) == count and c.join_stats()["route"] == route, (nS, hot, stride, names)
+    finally:
+        c.close()
