@@ -757,8 +757,10 @@ qg_status qg_filter_cols_launch(qg_ctx *ctx, const int32_t *key, const int32_t *
     if (variant == 2) {
         // k_filter_two writes rows while other CTAs still read keys
         const bool over = qg_overlap(out, (size_t)std::min(cap, n) * 8, key, (size_t)n * 4);
-        if (over || (n >= F2_TWO_ROWS && f2_two_fits(ctx, n)))
-            return f2_launch_two(ctx, key, pay, n, lo, hi, out, cap, d_count);
+        if (over || (n >= F2_TWO_ROWS && f2_two_fits(ctx, n))) {
+            const qg_status st = f2_launch_two(ctx, key, pay, n, lo, hi, out, cap, d_count);
+            if (st != QG_ERR_OOM || over) return st;  // no room for the bits: nothing was launched
+        }
         return f2_launch<false>(ctx, key, pay, n, lo, hi, out, cap, d_count);
     }
     qg_lookback lb;

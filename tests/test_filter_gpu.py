@@ -256,3 +256,26 @@ def test_filter_rec_over_its_input(ctx, n, shift, sel):
     st = ctx.lib.qg_filter_range_rec(ctx.handle, buf[3000:].data_ptr(), n, -5, hi, out.data_ptr(), n, ctypes.byref(cnt))
     assert st == 0 and cnt.value == exp.shape[0]
     assert torch.equal(out[: cnt.value], exp)
+
+
+def test_filter_cols_without_scratch_takes_one_launch():
+    # No room for the predicate bits: the one-launch form answers.
+    from query_on_opencl_fpga_gb300.api import Context
+
+    n = (1 << 22) + 513
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    key = torch.randint(0, 1000, (n,), generator=g, device="cuda").to(torch.int32)
+    pay = torch.randint(0, 1000, (n,), generator=g, device="cuda").to(torch.int32)
+    at = (key <= 99).nonzero().flatten()
+    exp = torch.stack([at.to(torch.int32), pay[at]], 1)
+    c = Context()
+    try:
+        for limit, kernels in [(200_000, {"k_filter_two"}), (0, {"k_filter_count", "k_filter_write"})]:
+            c.check(c.lib.qg_ctx_set_arena_limit(c.handle, limit), "limit")
+            c.enable_timing(True)
+            got = c.filter_cols(key, pay, 0, 99)
+            assert torch.equal(got, exp) and set(c.timing_report()) == kernels
+            c.enable_timing(False)
+    finally:
+        c.close()
