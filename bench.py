@@ -449,9 +449,9 @@ def operator_lines(ctx, args, peak, stream):
 
     ms, kern, _ = timed(ctx, fstep, steps, 3, 1, stream)
     sel = res["o"].shape[0]
-    # The column filter is one kernel: its roofline is the operator's
-    # algorithmic bytes over its launch time.
-    fk = [k for k in ("k_filter_two", "k_filter_cols") if kern.get(k, (0, 0.0))[0]]
+    # The column filter is one or two kernels, each launched once: its roofline is the
+    # operator's algorithmic bytes over their time.
+    fk = [k for k, v in kern.items() if k.startswith("k_filter") and v[0]]
     f_ms = sum(kern[k][1] / kern[k][0] for k in fk)
     f_alg = n * 8 + sel * 8
     out["filter_config0"] = {"rows_per_s": n / (ms * 1e-3), "ms_per_op": ms, "rows": n, "selected": sel,
@@ -516,7 +516,7 @@ def operator_lines(ctx, args, peak, stream):
 
 def sort_line(ctx, steps, peak, stream):
     """In-place sort of 64M reference Records by unsigned y (radixSortImpl_sm),
-    keys uniform in [0, 2^20): three 8-bit passes.  Every step sorts a fresh
+    keys uniform in [0, 2^20).  Every step sorts a fresh
     copy of the same unsorted records; the copy is outside the timed call."""
     import torch
 
@@ -546,16 +546,18 @@ def sort_line(ctx, steps, peak, stream):
     torch.cuda.synchronize()
     kern = ctx.timing_report()
     ctx.enable_timing(False)
-    # four passes are launched, planned on the device: the one over the keys' high
-    # zero byte ends at once and moves nothing
-    launches = kern.get("k_radix_pass", (0, 0.0))[0] // steps
-    passes = 3
+    # a pass moves the records when the keys differ in its byte; the others are launched
+    # (the plan is made on the device) and end at once
+    digits = base[:, 1].contiguous().view(torch.uint8).view(ns, 4)
+    passes = int((digits.amin(0) != digits.amax(0)).sum())
+    launches, pass_ms = kern.get("k_radix_pass", (0, 0.0))
+    moving = {"k_radix_pass": (passes * steps, pass_ms)}  # the idle launches' time is charged to them
     alg = ns * 16 * passes  # one read and one write of the records per key pass
-    del base, rec
-    return {"rows_per_s": ns / (ms * 1e-3), "ms_per_op": ms, "rows": ns, "passes": passes, "sorted": ok,
-            "op_frac_of_peak": alg / (ms * 1e-3) / 1e9 / peak,
+    del base, rec, digits
+    return {"rows_per_s": ns / (ms * 1e-3), "ms_per_op": ms, "rows": ns, "passes": passes,
+            "pass_launches": launches // steps, "sorted": ok, "op_frac_of_peak": alg / (ms * 1e-3) / 1e9 / peak,
             "kernels_ms": {k: v[1] / steps for k, v in kern.items()},
-            "roofline": roofline(kern, "k_radix_pass", alg / max(launches, 1), peak)}
+            "roofline": roofline(moving, "k_radix_pass", ns * 16, peak)}
 
 
 def skew_line(ctx, stream):
