@@ -134,9 +134,10 @@ QG_API qg_status qg_noalloc_forget(void);
 
 /* Column filter kernel choice (process-wide): 0 = one 4096-row tile per CTA
  * held in registers with a decoupled look-back, 1 = persistent CTAs
- * streaming tiles through a 3-stage bulk-copy (TMA) ring, 2 = two phases of
- * one launch (per-CTA counts from the keys, then the writes) around a single
- * exchange of counts, the default.  Results are identical. */
+ * streaming tiles through a 3-stage bulk-copy (TMA) ring, 2 (the default) = two
+ * phases, the counts from the keys and then the writes, around a single exchange of
+ * counts: in one launch, or from 2^22 rows on in two that keep a bit per row in
+ * scratch.  With variant 2 the output may lie over the keys.  Results are identical. */
 QG_API qg_status qg_filter_set_variant(int variant);
 
 /* ---- scan (ScanLargeArrays/prefixSum/blockAddition, host/host/testScan.cpp:278-340) */
@@ -198,7 +199,9 @@ QG_API qg_status qg_scatter_rec(qg_ctx *ctx, const void *R, int64_t rLen, const 
  * (rows < 2^30, cap up to 1.3M groups), or, where the partitions would be
  * uneven, hold too many groups or few groups meet many rows, the call runs the
  * two-pass hash path; which of these is launched first is what the context's
- * last call found.  On the two-pass path `cap` also sizes the spill partitions (about 1024 groups each), so a
+ * last call found.  Device memory that the context keeps: about 70 MB for the window,
+ * 16 bytes a row when partitioned by key range; when that cannot be had, or outputs
+ * lie over inputs, the call runs the two-pass path.  On the two-pass path `cap` also sizes the spill partitions (about 1024 groups each), so a
  * cap near the true group count is fastest, and for key order the context
  * remembers the key range of its previous call and ranks keys in a bitmap
  * window placed there; results never depend on either, only the path does
@@ -268,8 +271,9 @@ QG_API qg_status qg_join_filter_sort(qg_ctx *ctx, const int32_t *rkey, const int
  * knobs at their defaults, when R's keys are unique over a dense span (at most
  * 2 nR values): a counting join for S up to 18M rows, beyond it one partition
  * step fused with the filter if the rows spread evenly; the hash join (3) when R
- * has up to 2^23 keys of no dense span (over 40M S rows: of a span above half
- * of them); else range partitioning by
+ * has up to 2^23 keys of no dense span that hardly repeat (with many S rows: of a
+ * span well above a dense one); else, and when one of those gives up (a key met
+ * too often, uneven rows, too little memory), range partitioning by
  * radix over the key, switching to the learned CDF partition function when
  * radix leaves more than 2% of the rows in buckets too large for shared memory
  * and the model does better on the same counts; 1 radix
@@ -365,7 +369,9 @@ QG_API qg_status qg_batch_info(const qg_batch *b, int32_t *out4);
 QG_API qg_status qg_batch_destroy(qg_batch *b);
 /* Lanes of the batches created after this call (process-wide, 1..16; default
  * 12): the queries are spread over that many streams, each with a private
- * context, and the graph runs the lanes side by side. */
+ * context, and the graph runs the lanes side by side.  A lane's context keeps the
+ * arenas of its queries: about 70 MB for group-bys of 8192 rows or more, the join's
+ * table and three columns of cap rows. */
 QG_API qg_status qg_batch_set_lanes(int lanes);
 /* Form of the batches created after this call (process-wide): 1
  * persistent -- every filter, group-by and fused query runs inside one

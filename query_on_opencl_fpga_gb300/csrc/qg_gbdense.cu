@@ -13,13 +13,12 @@
 // down).  Larger inputs take four, no host round trip until the caller's one read at
 // the end:
 //  1. k_gbd_sample -- 2^18 keys (1024 runs of 256 consecutive rows spread over
-//                     the column, or every row of a smaller input) are counted
+//                     the column) are counted
 //                     per CTA in shared memory; each CTA adds its distinct
 //                     keys' counts to a two-row count-min sketch in L2 (fire-
 //                     and-forget reductions) and lists the keys.  The
 //                     smallest and largest sampled key are recorded.
-//  2. k_gbd_cands  -- every listed key whose sketch count is at least 2 (at
-//                     least 1 when the whole input was sampled) bids for the
+//  2. k_gbd_cands  -- every listed key whose sketch count is at least 2 bids for the
 //                     heavy-key slot its hash selects with one 64-bit atomicMax
 //                     of (count << 32 | key): each of the 16384 slots ends up
 //                     holding its most frequent candidate.  The key window
@@ -945,6 +944,8 @@ qg_status qg_gbd_launch(qg_ctx *ctx, const int32_t *key, const int32_t *val, con
     auto mainf = pred ? k_gbd_main<true> : k_gbd_main<false>;
     QG_TRY(qg_allow_smem(ctx, site_main[pred], mainf, smem_main));
 
+    // Every row is a sample only in the one cooperative launch: without it inputs that small
+    // take the exact range below.
     const bool every_row = n <= (long long)GBD_SAMPLE_RUNS * GBD_RUN;
     const int runs = every_row ? (int)qg_ceil_div(n, GBD_RUN) : GBD_SAMPLE_RUNS;
     qg_status s = QG_OK;

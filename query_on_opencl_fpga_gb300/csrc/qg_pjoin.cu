@@ -1,8 +1,10 @@
 // qg_pjoin.cu -- range-partitioned join + filter + sort, and the choice among the
 // paths of qg_join_filter_sort: counting (qg_jdirect.cu) for dense build keys and
 // up to 18M probe rows, one partition step (qg_jpart.cu, after steps 1 here) beyond,
-// the hash join (qg_join.cu) for up to 2^23 build keys of no dense span, and the
-// pipeline below for the rest and for what those hand over.
+// the hash join (qg_join.cu) for up to 2^23 build keys of no dense span and not near
+// one (pj_near_size), and the pipeline below for the rest and for what those hand over.
+// An attempt that was given up at some cost is left out of the next calls (pj_no_count,
+// pj_no_hash, pj_no_part in qg_internal.cuh).
 //
 // Reference operators this replaces: buildHashTable / probeHashTable and the
 // filter + bitonic sort of the matches (kernel/hj_filter_sort/1/
