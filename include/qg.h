@@ -200,8 +200,8 @@ QG_API qg_status qg_scatter_rec(qg_ctx *ctx, const void *R, int64_t rLen, const 
  * uneven, hold too many groups or few groups meet many rows, the call runs the
  * two-pass hash path; which of these is launched first is what the context's
  * last call found.  Device memory that the context keeps: about 70 MB for the window,
- * 16 bytes a row when partitioned by key range; when that cannot be had, or outputs
- * lie over inputs, the call runs the two-pass path.  On the two-pass path `cap` also sizes the spill partitions (about 1024 groups each), so a
+ * 16 bytes a row when partitioned by key range (which is left out when that cannot be
+ * had or outputs lie over inputs).  On the two-pass path `cap` also sizes the spill partitions (about 1024 groups each), so a
  * cap near the true group count is fastest, and for key order the context
  * remembers the key range of its previous call and ranks keys in a bitmap
  * window placed there; results never depend on either, only the path does

@@ -684,8 +684,10 @@ k_gbd_emit(unsigned long long *__restrict__ dense, long long *__restrict__ extra
         }
     }
     __syncthreads();
-    gbd_chunk_write(dense, extra, k, s_wsum[0], st[G_KBASE], st[G_EXTRA] != 0u, shift, gkey, gsum, gcnt, cap, s_off,
-                    &s_tot);
+    // With a row outside the window the caller reads its inputs again: nothing is written, as
+    // the outputs may lie over them.
+    gbd_chunk_write(dense, extra, k, s_wsum[0], st[G_KBASE], st[G_EXTRA] != 0u, shift, gkey, gsum, gcnt,
+                    st[G_OUTSIDE] ? 0 : cap, s_off, &s_tot);
     // The last chunk ends after every earlier chunk published (its look-back
     // waited for them), and every CTA took its chunk before that.
     qg_lb_finish_dyn(lb, chunk, C - 1, epoch);
@@ -879,7 +881,8 @@ k_gbd_single(const int32_t *__restrict__ key, const int32_t *__restrict__ val, c
         }
     }
     __syncthreads();
-    gbd_chunk_write(dense, extra, ck, s_base, kbase, xtra, shift, gkey, gsum, gcnt, cap, s_off, &s_tot);
+    gbd_chunk_write(dense, extra, ck, s_base, kbase, xtra, shift, gkey, gsum, gcnt, __ldcg(&st[G_OUTSIDE]) ? 0 : cap,
+                    s_off, &s_tot);
 }
 
 }  // namespace

@@ -723,6 +723,31 @@ def test_groupby_sampled_window_hidden_keys(orc, fused):
         c.close()
 
 
+# The same with the groups' keys over the key column: the path that answers reads it again.
+@pytest.mark.parametrize("single", [0, 1])
+def test_groupby_sampled_window_over_its_keys(orc, single):
+    from query_on_opencl_fpga_gb300.api import Context
+
+    rng = np.random.default_rng(17)
+    n, gap = (1 << 23) + 4099, 5000
+    key = rng.integers(100, 100 + 50000, n).astype(np.int32)
+    val = rng.integers(0, 1000, n).astype(np.int32)
+    key[gap], key[gap + 1] = 2 ** 30, -5
+    exp = orc.groupby_cols(key, val)
+    c = Context()
+    try:
+        c.check(c.lib.qg_groupby_set_single_launch(single), "single")
+        k = dev(key)
+        out = (k[:60_000], torch.empty(60_000, dtype=torch.int64, device="cuda"),
+               torch.empty(60_000, dtype=torch.int64, device="cuda"))
+        got = c.groupby_cols(k, dev(val), cap=60_000, out=out)
+        for g, e in zip(got, exp):
+            assert np.array_equal(g.cpu().numpy(), e)
+    finally:
+        c.lib.qg_groupby_set_single_launch(0)
+        c.close()
+
+
 # Which form answers: each new one where it is meant to, and not where it hands over.
 @pytest.mark.parametrize("n,kind,route", [(1, "narrow", "one_cta"), (16_384, "narrow", "one_cta"), (16_384, "own", "exact_window"),
                                           (16_385, "narrow", "exact_window"), (16_385, "ids", "key_ranges"),
