@@ -1612,8 +1612,22 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
     if (n >= (1LL << 32)) return QG_ERR_UNSUPPORTED;
     long long *d_num = (long long *)&ctx->ctl->counter[1];
     unsigned int *flags = (unsigned int *)&ctx->ctl->counter[2];
+    // Outputs over an input: no path may write them while a path that reads the input may
+    // follow.  The two-pass path then merges into temporaries, as key order does anyway, and
+    // its overflow flags are read before the groups go to the outputs.
+    auto over = [&](const void *out, size_t bytes) {
+        return qg_overlap(out, bytes, key, (size_t)n * 4) || qg_overlap(out, bytes, val, (size_t)n * 4) ||
+               (val2 && qg_overlap(out, bytes, val2, (size_t)n * 4));
+    };
+    const bool in_place = over(gkey, (size_t)cap * 4) || over(gsum, (size_t)cap * 8) || over(gcnt, (size_t)cap * 8);
+    if (in_place) order = QG_ORDER_KEY;
     GbOut o;
-    QG_TRY(gb_outputs(ctx, gkey, gsum, gcnt, cap, order, &o));
+    auto outputs = [&]() -> qg_status {
+        QG_TRY(gb_outputs(ctx, gkey, gsum, gcnt, cap, order, &o));
+        if (in_place) o.k = (int32_t *)(o.c + (cap > 0 ? cap : 1));  // the sort's other buffer, not in use yet
+        return QG_OK;
+    };
+    QG_TRY(outputs());
     long long g = 0;
     const int gm = gb_mode(ctx);
     bool global = gm == 1;
@@ -1661,12 +1675,7 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
     };
     // The partitions' groups are written before it is known whether all of them have a
     // place: not over a column that the path after it would read.
-    auto over = [&](const void *out, size_t bytes) {
-        return qg_overlap(out, bytes, key, (size_t)n * 4) || qg_overlap(out, bytes, val, (size_t)n * 4) ||
-               (val2 && qg_overlap(out, bytes, val2, (size_t)n * 4));
-    };
-    const bool may_wide = gm == 0 && qg_gbw_applies(n, cap) && !over(gkey, (size_t)cap * 4) &&
-                          !over(gsum, (size_t)cap * 8) && !over(gcnt, (size_t)cap * 8);
+    const bool may_wide = gm == 0 && qg_gbw_applies(n, cap) && !in_place;
     bool narrow = true;
     if (may_wide && ctx->gb_first == 1) {
         uint32_t v;
@@ -1699,7 +1708,7 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
             if (v == QG_GBW_DONE) return g > cap ? QG_ERR_CAPACITY : QG_OK;
         }
     }
-    if (wide_tried) QG_TRY(gb_outputs(ctx, gkey, gsum, gcnt, cap, order, &o));  // the arena may have moved
+    if (wide_tried) QG_TRY(outputs());  // the arena may have moved
     const bool dense = o.rec && !ctx->gb_wide_keys;
     const bool dev_order = o.rec && !dense && cap < (1LL << 30);
     uint32_t *mm = (uint32_t *)&ctx->ctl->counter[4];
@@ -1713,8 +1722,15 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
         }
         QG_TRY(gb_launch_twopass(ctx, key, val, val2, lo2, hi2, n, o, cap, d_num, flags,
                                  dev_order ? ctx->ctl->ghist : nullptr, o.rec ? mm : nullptr, bits, kbase));
-        if (dense) QG_TRY(gb_key_order_dense(ctx, o, cap, d_num, mm, bits, kbase, gkey, gsum, gcnt));
-        if (dev_order) QG_TRY(gb_key_order_dev(ctx, o, cap, d_num, gkey, gsum, gcnt));
+        unsigned int over_flags = 0;
+        if (in_place) {
+            QG_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->pinned, flags, 4, cudaMemcpyDeviceToHost, ctx->stream), "flags d2h");
+            QG_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream), "sync");
+            over_flags = *(const unsigned int *)ctx->pinned;
+            if (over_flags && dense) ctx->table_dirty = true;  // the merge's bits are left set
+        }
+        if (dense && !over_flags) QG_TRY(gb_key_order_dense(ctx, o, cap, d_num, mm, bits, kbase, gkey, gsum, gcnt));
+        if (dev_order && !over_flags) QG_TRY(gb_key_order_dev(ctx, o, cap, d_num, gkey, gsum, gcnt));
         // One read of the control block, at the end, brings the error word,
         // the group count (counter[1]) and the overflow flags (counter[2]).
         QG_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->pin_ctl, ctx->ctl, offsetof(qg_control, ghist),
@@ -1764,6 +1780,8 @@ static qg_status groupby_cols_impl(qg_ctx *ctx, const int32_t *key, const int32_
     } else if (order == QG_ORDER_KEY && g == 1) {
         QG_TRY_CUDA(ctx, cudaMemcpyAsync(gsum, o.s, 8, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
         QG_TRY_CUDA(ctx, cudaMemcpyAsync(gcnt, o.c, 8, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
+        if (o.k != gkey)
+            QG_TRY_CUDA(ctx, cudaMemcpyAsync(gkey, o.k, 4, cudaMemcpyDeviceToDevice, ctx->stream), "copy");
         return qg_ctx_check(ctx);
     }
     return QG_OK;

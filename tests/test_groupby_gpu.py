@@ -638,6 +638,36 @@ def test_groupby_outputs_over_inputs(orc, which):
         c.close()
 
 
+# The same where the two-pass path overflows and the global table reads the inputs again:
+# wide keys in a spill bucket that holds one row; one group, both orders.
+@pytest.mark.parametrize("which", [0, 1, 2])
+@pytest.mark.parametrize("groups", [1, 5000])
+def test_groupby_overflow_over_inputs(orc, knobs, which, groups):
+    from query_on_opencl_fpga_gb300.api import QG_ORDER_KEY, QG_ORDER_NONE, Context
+
+    rng = np.random.default_rng(33)
+    n = 200_000
+    key = (rng.integers(0, groups, n) * 429_000 - 2 ** 31).astype(np.int32)
+    val = rng.integers(-1000, 1000, n).astype(np.int32)
+    exp = orc.groupby_cols(key, val)
+    knobs(0, 8, 6, 1)
+    c = Context()
+    try:
+        for order in (QG_ORDER_KEY, QG_ORDER_NONE, QG_ORDER_KEY):
+            k, v = dev(key), dev(val)
+            cap = n // 2
+            out = [torch.empty(cap, dtype=torch.int32, device="cuda"), torch.empty(cap, dtype=torch.int64, device="cuda"),
+                   torch.empty(cap, dtype=torch.int64, device="cuda")]
+            out[which] = k[:cap] if which == 0 else (k if which == 1 else v).view(torch.int64)[:cap]
+            got = [g.cpu().numpy() for g in c.groupby_cols(k, v, cap=cap, order=order, out=tuple(out))]
+            at = np.argsort(got[0].astype(np.uint32), kind="stable")
+            for g, e in zip(got, exp):
+                assert np.array_equal(g[at], e), (order, c.groupby_stats())
+            assert groups == 1 or c.groupby_stats()["route"] == "global_table"
+    finally:
+        c.close()
+
+
 # Rows and capacity around the line above which many groups stay on the two-pass
 # path: the same groups on both sides, and with fewer groups than the capacity allows.
 @pytest.mark.parametrize("n,cap,groups", [(56_000_000, 1 << 20, 900_000), (56_000_001, 1 << 20, 900_000),
